@@ -33,7 +33,7 @@ def build(ref: bool = True) -> None:
     """Compile liboracle.so, and oracle/_ref/ when the reference tree exists
     (the CPU binaries, and the single-GPU binary when nvcc is present)."""
     subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
-    if ref and os.path.isdir(REFERENCE_TREE):
+    if ref and os.path.exists(os.path.join(REFERENCE_TREE, "main.cpp")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF={REFERENCE_TREE}"], check=True)
         if os.path.exists("/usr/local/cuda/bin/nvcc"):
             subprocess.run(["make", "-s", "-C", HERE, "refgpu", f"REF={REFERENCE_TREE}"], check=True)
