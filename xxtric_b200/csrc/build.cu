@@ -64,15 +64,6 @@ __global__ void k_edge_keys(const int32_t *__restrict__ src, const int32_t *__re
   }
 }
 
-__global__ void k_unique_flags(const uint64_t *__restrict__ keys, int64_t n, int b, uint8_t *__restrict__ flags) {
-  const uint64_t mask = (uint64_t(1) << b) - 1;
-  XT_GRID_STRIDE(i, n) {
-    uint64_t k = keys[i];
-    bool first = (i == 0) || (keys[i - 1] != k);
-    flags[i] = (first && ((k >> b) != (k & mask))) ? 1 : 0;
-  }
-}
-
 // every vertex's id (the values of the rank sort, keyed by degree) and the
 // largest degree (how many key bits the sort needs)
 __global__ void k_rank_ids(const int32_t *__restrict__ deg, int64_t nv, int32_t *__restrict__ ids,
@@ -89,16 +80,6 @@ __global__ void k_rank_ids(const int32_t *__restrict__ deg, int64_t nv, int32_t 
 // ids in (degree, id) order -> input->internal map
 __global__ void k_rank_perm(const int32_t *__restrict__ n2o, int64_t nv, int32_t *__restrict__ o2n) {
   XT_GRID_STRIDE(r, nv) o2n[n2o[r]] = int32_t(r);
-}
-
-// (lo,hi) in input ids -> (src<<b|dst) in internal ids, src <= dst
-__global__ void k_relabel_edges(uint64_t *__restrict__ keys, int64_t m, int b, const int32_t *__restrict__ o2n) {
-  const uint64_t mask = (uint64_t(1) << b) - 1;
-  XT_GRID_STRIDE(i, m) {
-    const uint64_t k = keys[i];
-    const uint64_t a = uint64_t(o2n[k >> b]), c = uint64_t(o2n[k & mask]);
-    keys[i] = a < c ? ((a << b) | c) : ((c << b) | a);
-  }
 }
 
 // (lo, hi) in input ids -> (row, col) = (low rank, high rank), in place.
@@ -523,93 +504,181 @@ __global__ void k_rows_emit(const int64_t *__restrict__ rstart, const uint32_t *
   }
 }
 
-// Sorted keys (row << b | col) -> row lengths and columns. The thread at a
-// run's first key adds -start, the one at its last key adds end, so each
-// non-empty row ends with end - start (len must start zeroed). The offsets
-// are then the exclusive scan of the lengths.
-template <class K>
-__global__ void k_csr_runs(const K *__restrict__ keys, int64_t m, int b, int64_t *__restrict__ len,
-                           int32_t *__restrict__ col) {
-  const K mask = (K(1) << b) - 1;
+// Sorted keys (row << b | rest) -> row lengths. The thread at a run's first
+// key adds -start, the one at its last key adds end, so each non-empty row
+// ends with end - start (len must start zeroed). The offsets are then the
+// exclusive scan of the lengths.
+__global__ void k_csr_runs(const uint32_t *__restrict__ keys, int64_t m, int b, int64_t *__restrict__ len) {
   XT_GRID_STRIDE(i, m) {
-    const K k = keys[i];
-    const K row = k >> b;
+    const uint32_t row = keys[i] >> b;
     if (i == 0 || (keys[i - 1] >> b) != row)
       atomicAdd(reinterpret_cast<unsigned long long *>(&len[row]), (unsigned long long)(-i));
     if (i + 1 == m || (keys[i + 1] >> b) != row)
       atomicAdd(reinterpret_cast<unsigned long long *>(&len[row]), (unsigned long long)(i + 1));
-    if (col) col[i] = int32_t(k & mask);
   }
 }
 
-// row index of every CSR entry (warp per row); optional range checks
-__global__ void k_csr_rows(const int64_t *__restrict__ off, int64_t nv, int64_t ne, int32_t *__restrict__ rows,
-                           int *__restrict__ err) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t u = warp; u < nv; u += nwarps) {
-    int64_t e0 = off[u], e1 = off[u + 1];
-    if (e0 < 0 || e1 < e0 || e1 > ne) {
-      if (lane == 0 && err) atomicOr(err, 2);
-      continue;
-    }
-    for (int64_t e = e0 + lane; e < e1; e += 32) rows[e] = int32_t(u);
-  }
-}
+// ---- CSR input ----------------------------------------------------------------
 
-__global__ void k_csr_tails32(const int64_t *__restrict__ tails, int64_t n, int64_t nv, int32_t *__restrict__ out,
-                              int *__restrict__ err) {
-  XT_GRID_STRIDE(i, n) {
-    int64_t t = tails[i];
-    if (t < 0 || t >= nv) {
-      atomicOr(err, 1);
-      t = 0;
-    }
-    out[i] = int32_t(t);
-  }
-}
-
-// Canonical CSR input check, a warp per row, run once the offsets and ids have
-// passed k_csr_rows / k_csr_tails32: every row strictly ascending (no
-// repeats), without its own id, and every entry (u,t) listed back in row t
-// (binary search of row t, whose bounds were checked). The canonical path
-// takes each row's upper part as it stands, so a row out of order would
-// reach the count's member sets unsorted and an edge listed from one end
-// only would lose its triangles; either sets bit 4 of *err.
-__global__ void k_csr_check_canonical(const int64_t *__restrict__ off, const int32_t *__restrict__ t32, int64_t nv,
-                                      int *__restrict__ err) {
-  const int lane = threadIdx.x & 31;
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t u = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; u < nv; u += nwarps) {
+// offsets: not negative, not decreasing, none past ne (bit 2 of *err)
+__global__ void k_csr_offsets(const int64_t *__restrict__ off, int64_t nv, int64_t ne, int *__restrict__ err) {
+  XT_GRID_STRIDE(u, nv) {
     const int64_t e0 = off[u], e1 = off[u + 1];
-    bool bad = false;
-    for (int64_t p = e0 + lane; !bad && p < e1; p += 32) {
-      const int32_t t = t32[p];
-      bad = t == u || (p > e0 && t32[p - 1] >= t);
-      if (!bad) {
-        int64_t lo = off[t], hi = off[t + 1];
-        const int64_t end = hi;
-        while (lo < hi) {
-          const int64_t mid = lo + (hi - lo) / 2;
-          if (t32[mid] < u) lo = mid + 1;
-          else hi = mid;
-        }
-        bad = lo >= end || t32[lo] != u;
-      }
-    }
-    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(err, 4);
+    if (e0 < 0 || e1 < e0 || e1 > ne) atomicOr(err, 2);
   }
 }
 
-// canonical CSR input: each undirected edge once, as the entry (u,t), u < t;
-// the kept entries stay in (row, column) order
-__global__ void k_csr_lower_keys(const int32_t *__restrict__ rows, const int32_t *__restrict__ tails, int64_t n,
-                                 int b, uint64_t *__restrict__ keys, uint8_t *__restrict__ flags) {
-  XT_GRID_STRIDE(i, n) {
-    const int64_t u = rows[i], t = tails[i];
-    flags[i] = u < t ? 1 : 0;
-    keys[i] = (uint64_t(u) << b) | uint64_t(t);
+// What the entries say about the CSR, gathered on the device: word 0 is set
+// when a row is out of order, repeats an id or holds its own id; word 1 is
+// the entries above their row's id less those below it, modulo 2^64; word 2
+// is set when an entry is missing from its other end's row.
+constexpr int kCsrWords = 3;
+
+// row holding entry e, from a row at or before it: a few steps, then a search
+// (a run of empty rows can be long)
+__device__ __forceinline__ int64_t row_from(const int64_t *__restrict__ off, int64_t nv, int64_t r, int64_t e) {
+  for (int i = 0; i < 8; i++) {
+    if (r + 1 >= nv || off[r + 1] > e) return r;
+    r++;
+  }
+  int64_t lo = r, hi = nv;
+  while (hi - lo > 1) {
+    const int64_t mid = lo + (hi - lo) / 2;
+    if (off[mid] <= e) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// Every CSR entry's row and its tail in 32 bits (ids outside [0, nv): bit 1
+// of *err), with the row checks above. A warp takes spans of kCsrSpan
+// consecutive entries whatever their rows, so a hub's row is read by as many
+// warps as its entries fill: a warp per row held a R-MAT 2^20 CSR's first
+// pass at 147 us behind its longest row.
+constexpr int kCsrSpan = 256;
+__global__ void k_csr_entries(const int64_t *__restrict__ off, const int64_t *__restrict__ tails, int64_t nv,
+                              int64_t e_first, int64_t ne, int32_t *__restrict__ rows, int32_t *__restrict__ t32,
+                              int *__restrict__ err, unsigned long long *__restrict__ chk) {
+  if (*err & 2) return;  // the offsets cannot be walked
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  long long tilt = 0;  // entries above their row's id less those below it
+  bool bad = false;
+  for (int64_t w = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; e_first + w * kCsrSpan < ne; w += nw) {
+    const int64_t b0 = e_first + w * kCsrSpan;
+    int64_t r = 0, hi = nv;  // the last row starting at or before b0
+    while (hi - r > 1) {
+      const int64_t mid = r + (hi - r) / 2;
+      if (off[mid] <= b0) r = mid;
+      else hi = mid;
+    }
+    for (int i = 0; i < kCsrSpan; i += 32) {
+      const int64_t e = b0 + i + lane;
+      const bool in = e < ne;
+      const int64_t rr = in ? row_from(off, nv, r, e) : r;
+      int64_t t = in ? tails[e] : 0;
+      if (t < 0 || t >= nv) {
+        atomicOr(err, 1);
+        t = 0;
+      }
+      int64_t prev = __shfl_up_sync(0xffffffffu, t, 1);
+      if (in) {
+        const bool first = e == off[rr];
+        if (lane == 0 && !first) prev = tails[e - 1];
+        bad |= t == rr || (!first && prev >= t);
+        tilt += (t > rr) - (t < rr);
+        rows[e] = int32_t(rr);
+        t32[e] = int32_t(t);
+      }
+      r = __shfl_sync(0xffffffffu, rr, 31);
+    }
+  }
+  using Red = cub::BlockReduce<long long, 256>;
+  __shared__ typename Red::TempStorage ts;
+  const long long tot = Red(ts).Sum(tilt);
+  if (threadIdx.x == 0 && tot) atomicAdd(&chk[1], (unsigned long long)tot);
+  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&chk[0], 1ull);
+}
+
+// Symmetry of sorted rows, a thread per entry: every entry (u, t) above its
+// row's id must be listed back in row t (binary search). With as many entries
+// below as above, and rows without repeats, each entry below is then the one
+// that such a search found, so half the searches decide both directions. (A
+// warp per row searching every entry: 9.7 ms on a R-MAT 2^20 CSR.)
+__global__ void k_csr_back(const int64_t *__restrict__ off, const int32_t *__restrict__ rows,
+                           const int32_t *__restrict__ t32, int64_t e_first, int64_t ne,
+                           const int *__restrict__ err, unsigned long long *__restrict__ chk) {
+  if (*err || chk[0] || chk[1]) return;  // decided already
+  bool bad = false;
+  for (int64_t e = e_first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < ne;
+       e += int64_t(gridDim.x) * blockDim.x) {
+    const int32_t u = rows[e], t = t32[e];
+    if (t <= u) continue;
+    int64_t lo = off[t], hi = off[t + 1];
+    const int64_t end = hi;
+    while (lo < hi) {
+      const int64_t mid = lo + (hi - lo) / 2;
+      if (t32[mid] < u) lo = mid + 1;
+      else hi = mid;
+    }
+    bad |= lo >= end || t32[lo] != u;
+  }
+  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&chk[2], 1ull);
+}
+
+// Canonical CSR input, oriented without sorting the edges: entry (u, t) of
+// the symmetric rows is the oriented edge of rank(u) when rank(t) is the
+// higher, so each row's kept tails are its out-row, in any order (the row
+// tiers sort them). Pass 1 (k_csr_keep) turns each entry into its ranks, in
+// place (-1: not kept), and counts the kept ones per row; pass 2
+// (k_csr_place) writes them at the scanned starts. Entries of one row are
+// consecutive, so a warp adds one count per run of equal rows.
+// run of equal rows around this lane: its first lane, and its lanes
+__device__ __forceinline__ unsigned row_run(int32_t row, int lane, int &first) {
+  const int32_t p = __shfl_up_sync(0xffffffffu, row, 1);
+  const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || p != row);
+  first = 31 - __clz(int(heads & (0xffffffffu >> (31 - lane))));
+  const unsigned above = heads & ~(0xffffffffu >> (31 - lane));
+  const unsigned end = above ? (above & (0u - above)) - 1u : 0xffffffffu;  // lanes below the next run
+  return end & (0xffffffffu << first);
+}
+__global__ void k_csr_keep(int32_t *__restrict__ rows, int32_t *__restrict__ t32, int64_t n,
+                           const int32_t *__restrict__ o2n, int64_t *__restrict__ len) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t b = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) & ~int64_t(31); b < n;
+       b += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t e = b + lane;
+    int32_t u = -1, t = -1;
+    if (e < n) {
+      u = rows[e];
+      t = t32[e];
+      if (o2n) {
+        u = o2n[u];
+        t = o2n[t];
+      }
+      rows[e] = u;
+      t32[e] = t > u ? t : -1;
+    }
+    int first;
+    const unsigned run = row_run(u, lane, first);
+    const int kept = __popc(__ballot_sync(0xffffffffu, t > u) & run);
+    if (lane == first && kept) atomicAdd(reinterpret_cast<unsigned long long *>(&len[u]), (unsigned long long)kept);
+  }
+}
+__global__ void k_csr_place(const int32_t *__restrict__ rows, const int32_t *__restrict__ t32, int64_t n,
+                            unsigned long long *__restrict__ cur, uint32_t *__restrict__ bk) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t b = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) & ~int64_t(31); b < n;
+       b += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t e = b + lane;
+    const int32_t u = e < n ? rows[e] : -1, t = e < n ? t32[e] : -1;
+    int first;
+    const unsigned run = row_run(u, lane, first);
+    const unsigned m = __ballot_sync(0xffffffffu, t >= 0) & run;
+    unsigned long long at = 0;
+    if (lane == first && m) at = atomicAdd(&cur[u], (unsigned long long)__popc(m));
+    at = __shfl_sync(0xffffffffu, at, first);
+    if (t >= 0) bk[at + __popc(m & ((1u << lane) - 1u))] = uint32_t(t);
   }
 }
 
@@ -622,80 +691,7 @@ __global__ void k_pad_len(const int64_t *__restrict__ off, int64_t nv, int64_t *
   XT_GRID_STRIDE(u, nv) plen[u] = (off[u + 1] - off[u] + 7) & ~int64_t(7);
 }
 
-// sorted keys (row << b | col) -> the padded columns: key i, the j-th of its
-// row, goes to colp[poff[row] + j]; the row's last key also fills the rest
-// of the row's padded span with kPadSentinel (a thread per key, so short
-// rows cost no idle lanes)
-__global__ void k_pad_fill(const uint64_t *__restrict__ keys, int64_t m, int b, const int64_t *__restrict__ off,
-                           const int64_t *__restrict__ poff, int32_t *__restrict__ colp) {
-  const uint64_t mask = (uint64_t(1) << b) - 1;
-  XT_GRID_STRIDE(i, m) {
-    const uint64_t k = keys[i];
-    const int64_t row = int64_t(k >> b);
-    const int64_t q = poff[row] + (i - off[row]);
-    colp[q] = int32_t(k & mask);
-    if (i + 1 == off[row + 1])
-      for (int64_t t = q + 1, e = poff[row + 1]; t < e; t++) colp[t] = kPadSentinel;
-  }
-}
-
-// (head << lb | length class) sort key for every out-CSR position, and the
-// position's in-record, both written in position order (rows ascend with
-// positions, so the row reads are near sequential): lb (0..7) bits of the
-// class fit beside the head in 31 bits. The records then travel through the
-// sort as its values, so no gather from random positions follows.
-__global__ void k_in_keys(const uint64_t *__restrict__ keys, int b, const int64_t *__restrict__ off,
-                          const int64_t *__restrict__ poff, int64_t m, int lb, uint32_t *__restrict__ ik,
-                          InRec *__restrict__ recp) {
-  const uint64_t mask = (uint64_t(1) << b) - 1;
-  XT_GRID_STRIDE(p, m) {
-    const uint64_t e = keys[p];  // the out-CSR entry at position p: its row and column
-    const int32_t u = int32_t(e >> b);
-    const int64_t a = off[u], len = off[u + 1] - p - 1;
-    uint32_t k = uint32_t(e & mask) << lb;
-    if (lb > 0) k |= len_class_desc(len) >> (7 - lb);
-    ik[p] = k;
-    recp[p] = make_inrec(poff[u] + (p - a) + 1, len);  // the suffix, in the padded column array
-  }
-}
-
 // ---------------------------------------------------------------------------
-
-static xt_status sort_keys(Ctx *c, const uint64_t *in, uint64_t *out, int64_t n, int end_bit) {
-  size_t bytes = 0;
-  XT_CUDA(c, cub::DeviceRadixSort::SortKeys(nullptr, bytes, in, out, n, 0, end_bit, c->stream));
-  void *tmp = nullptr;
-  XT_TRY(dalloc(c, &tmp, bytes));
-  cudaError_t e = cub::DeviceRadixSort::SortKeys(tmp, bytes, in, out, n, 0, end_bit, c->stream);
-  dfree(c, tmp);
-  XT_CUDA(c, e);
-  return XT_OK;
-}
-
-static xt_status select_flagged(Ctx *c, const uint64_t *in, const uint8_t *flags, uint64_t *out, int64_t n,
-                                int64_t *m_out) {
-  int64_t *d_num = nullptr;
-  XT_TRY(dalloc_n(c, &d_num, 1));
-  size_t bytes = 0;
-  cudaError_t e = cub::DeviceSelect::Flagged(nullptr, bytes, in, flags, out, d_num, n, c->stream);
-  if (e != cudaSuccess) {
-    dfree(c, d_num);
-    return cuda_status(c, e, "DeviceSelect::Flagged");
-  }
-  void *tmp = nullptr;
-  xt_status s = dalloc(c, &tmp, bytes);
-  if (s != XT_OK) {
-    dfree(c, d_num);
-    return s;
-  }
-  e = cub::DeviceSelect::Flagged(tmp, bytes, in, flags, out, d_num, n, c->stream);
-  dfree(c, tmp);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(m_out, d_num, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  dfree(c, d_num);
-  XT_CUDA(c, e);
-  return XT_OK;
-}
 
 // Stable radix sort of (32-bit key, value) pairs on the low end_bit bits,
 // ping-ponging between the caller's two buffers of each (no scratch copies of
@@ -717,14 +713,13 @@ static xt_status sort_pairs_db(Ctx *c, uint32_t *k0, uint32_t *k1, V *v0, V *v1,
   return XT_OK;
 }
 
-// sorted (row << b | col) keys -> off[nv+1] (and col[m] when col != null)
-template <class K>
-static xt_status keys_to_csr(Ctx *c, const K *keys, int64_t m, int64_t nv, int b, int64_t *off, int32_t *col) {
+// sorted (row << b | rest) keys -> off[nv+1]
+static xt_status keys_to_csr(Ctx *c, const uint32_t *keys, int64_t m, int64_t nv, int b, int64_t *off) {
   int64_t *len = nullptr;
   XT_TRY(dalloc_n(c, &len, size_t(nv + 1)));
   cudaError_t e = cudaMemsetAsync(len, 0, sizeof(int64_t) * (nv + 1), c->stream);
   if (e == cudaSuccess && m > 0) {
-    k_csr_runs<K><<<counted(c, grid_for(m, 256, c->sm_count)), 256, 0, c->stream>>>(keys, m, b, len, col);
+    k_csr_runs<<<counted(c, grid_for(m, 256, c->sm_count)), 256, 0, c->stream>>>(keys, m, b, len);
     e = cudaGetLastError();
   }
   size_t bytes = 0;
@@ -756,29 +751,24 @@ static xt_status check_err(Ctx *c, const char *what) {
   XT_CUDA(c, cudaStreamSynchronize(c->stream));
   if (h) {
     XT_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-    const char *why = (h & 1)   ? ": vertex id outside [0,nv)"
-                      : (h & 2) ? ": offsets not monotone in [0,ne]"
-                                : ": a row is out of order, repeats an id or holds its own id, or an edge is "
-                                  "missing from its other end's row (not a canonical CSR)";
+    const char *why = (h & 1) ? ": vertex id outside [0,nv)" : ": offsets not monotone in [0,ne]";
     return set_error(c, XT_ERR_INVALID, std::string(what) + why);
   }
   return XT_OK;
 }
 
 // Degree orientation: ranks the vertices by (deg, id) into g->d_perm
-// (internal -> input id) and relabels n rows in place: packed keys (lo << b
-// | hi, input ids) to (low rank << b | high rank), or, with keys == null,
-// the split ends lo[] / hi[] to (low rank, high rank). The rank is a stable
-// sort of the ids keyed by degree alone (the ids enter in ascending order,
-// so ties keep id order), on as many key bits as the largest degree needs.
-static xt_status rank_and_relabel(Ctx *c, int32_t *deg, int64_t nv, int b, uint64_t *keys, int64_t n, Graph *g,
-                                  uint32_t *lo = nullptr, uint32_t *hi = nullptr) {
+// (internal -> input id) and *o2n (input -> internal, the caller frees it).
+// The rank is a stable sort of the ids keyed by degree alone (the ids enter
+// in ascending order, so ties keep id order), on as many key bits as the
+// largest degree needs; deg is consumed.
+static xt_status rank_vertices(Ctx *c, int32_t *deg, int64_t nv, Graph *g, int32_t **o2n) {
   const int B = 256;
-  int32_t *ids = nullptr, *o2n = nullptr, *dalt = nullptr;
+  int32_t *ids = nullptr, *dalt = nullptr;
   unsigned int *d_dmax = nullptr;
   xt_status s = dalloc_n(c, &ids, size_t(nv));
   if (s == XT_OK) s = dalloc_n(c, &dalt, size_t(nv));
-  if (s == XT_OK) s = dalloc_n(c, &o2n, size_t(nv));
+  if (s == XT_OK) s = dalloc_n(c, o2n, size_t(nv));
   if (s == XT_OK) s = dalloc_n(c, &g->d_perm, size_t(nv));
   if (s == XT_OK) s = dalloc_n(c, &d_dmax, 1);
   unsigned int dmax = 0;
@@ -802,103 +792,23 @@ static xt_status rank_and_relabel(Ctx *c, int32_t *deg, int64_t nv, int b, uint6
     s = cuda_status(c, cudaMemcpyAsync(g->d_perm, perm, sizeof(int32_t) * nv, cudaMemcpyDeviceToDevice, c->stream),
                     "perm");
   if (s == XT_OK) {
-    k_rank_perm<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(g->d_perm, nv, o2n);
-    if (n > 0 && keys) k_relabel_edges<<<counted(c, grid_for(n, B, c->sm_count)), B, 0, c->stream>>>(keys, n, b, o2n);
-    if (n > 0 && !keys) k_relabel_split<<<counted(c, grid_for(n, B, c->sm_count)), B, 0, c->stream>>>(lo, hi, n, o2n);
-    s = cuda_status(c, cudaGetLastError(), "relabel");
+    k_rank_perm<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(g->d_perm, nv, *o2n);
+    s = cuda_status(c, cudaGetLastError(), "rank");
   }
   dfree(c, ids);
   dfree(c, dalt);
-  dfree(c, o2n);
   dfree(c, d_dmax);
   return s;
 }
 
-// In-records grouped by head (d_ioff, d_irec), longest suffix first, from the
-// out-CSR. keys: the out-CSR's m sorted keys (row << b | col), read here and
-// then overwritten; spare: a free buffer of at least m 8-byte entries. The
-// 4-byte sort keys of both sides fit in spare; the records are sorted as
-// values between two record arrays, one of which becomes d_irec.
-static xt_status build_in_records(Ctx *c, uint64_t *keys, uint64_t *spare, int64_t m, int64_t nv, int b, Graph *g) {
-  const int B = 256;
-  const int lb = b + 7 <= 31 ? 7 : 31 - b;  // key = head << lb | class, 31 bits at most
-  uint32_t *kin = reinterpret_cast<uint32_t *>(spare), *kalt = kin + m;
-  InRec *r0 = nullptr, *r1 = nullptr;
-  xt_status s = dalloc_n(c, &r0, size_t(m) + 2);
-  if (s == XT_OK) s = dalloc_n(c, &r1, size_t(m) + 2);
-  if (s == XT_OK) {
-    // the sorted keys still hold each position's row and column
-    k_in_keys<<<counted(c, grid_for(m, B, c->sm_count)), B, 0, c->stream>>>(keys, b, g->d_off, g->d_poff, m, lb,
-                                                                            kin, r0);
-    s = cuda_status(c, cudaGetLastError(), "in-keys");
-  }
-  // stable: records of one (head, class) stay in position order
-  uint32_t *ks = nullptr;
-  InRec *rs = nullptr;
-  if (s == XT_OK) s = sort_pairs_db<InRec>(c, kin, kalt, r0, r1, m, b + lb, &ks, &rs);
-  if (s == XT_OK) s = keys_to_csr<uint32_t>(c, ks, m, nv, lb, g->d_ioff, nullptr);
-  if (s == XT_OK) {
-    g->d_irec = rs;
-    dfree(c, rs == r0 ? r1 : r0);
-  } else {
-    dfree(c, r0);
-    dfree(c, r1);
-  }
-  return s;
-}
-
-// keys: m unique oriented edges (src << b | dst, src < dst, internal ids),
-// sorted; spare: m more 8-byte entries. Emits the out-CSR and the in-records.
-static xt_status finish_csr(Ctx *c, uint64_t *keys, uint64_t *spare, int64_t m, int64_t nv, int b, Graph *g) {
-  g->ne = m;
-  // Columns are read as aligned 32-byte pairs: pad so the last pair of the
-  // last row stays inside the allocation.
-  XT_TRY(dalloc_n(c, &g->d_off, size_t(nv + 1)));
-  XT_TRY(dalloc_n(c, &g->d_col, size_t(m) + kColPad));
-  XT_CUDA(c, cudaMemsetAsync(g->d_col + m, 0xff, sizeof(int32_t) * kColPad, c->stream));
-  XT_TRY(keys_to_csr<uint64_t>(c, keys, m, nv, b, g->d_off, g->d_col));
-  // padded columns: row starts on 8-column boundaries
-  {
-    const int B = 256;
-    int64_t *plen = nullptr;
-    XT_TRY(dalloc_n(c, &g->d_poff, size_t(nv + 1)));
-    XT_TRY(dalloc_n(c, &plen, size_t(nv + 1)));
-    k_pad_len<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(g->d_off, nv, plen);
-    xt_status s = cuda_status(c, cudaMemsetAsync(plen + nv, 0, sizeof(int64_t), c->stream), "memset");
-    if (s == XT_OK) s = exclusive_scan_i64(c, plen, g->d_poff, nv + 1);
-    int64_t total = 0;
-    if (s == XT_OK)
-      s = cuda_status(c, cudaMemcpyAsync(&total, g->d_poff + nv, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream),
-                      "D2H");
-    if (s == XT_OK) s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync");
-    dfree(c, plen);
-    XT_TRY(s);
-    if (total >= kMaxColp) return set_error(c, XT_ERR_OVERFLOW, "2^35 or more padded columns: beyond what the in-records address");
-    XT_TRY(dalloc_n(c, &g->d_colp, size_t(total > 0 ? total : 8)));
-    g->colp_len = total;
-    if (total > 0)
-      k_pad_fill<<<counted(c, grid_for(m, B, c->sm_count)), B, 0, c->stream>>>(keys, m, b, g->d_off, g->d_poff,
-                                                                               g->d_colp);
-    XT_CUDA(c, cudaGetLastError());
-  }
-  XT_TRY(dalloc_n(c, &g->d_ioff, size_t(nv + 1)));
-  if (m == 0) {
-    XT_TRY(dalloc_n(c, &g->d_irec, 2));
-    XT_CUDA(c, cudaMemsetAsync(g->d_ioff, 0, sizeof(int64_t) * (nv + 1), c->stream));
-    return XT_OK;
-  }
-  return build_in_records(c, keys, spare, m, nv, b, g);
-}
-
-// The out-CSR and the in-records from n rows grouped by their low end:
-// rows_s (the low ends, ascending) and cols_s (the high ends, in any order
-// within a row; repeats and self loops allowed). kbuf: n 8-byte entries
-// disjoint from cols_s, which take the in-record sort's keys (both of its
-// buffers).
-static xt_status rows_to_csr(Ctx *c, const uint32_t *rows_s, uint32_t *cols_s, int64_t n, int64_t nv, int b,
+// The out-CSR and the in-records from n rows grouped by their low end: row r
+// holds the high ends cols_s[rstart[r], rstart[r + 1]), in any order (repeats
+// and self loops allowed). kbuf: an 8-byte entry per unique edge, disjoint
+// from cols_s, which take the in-record sort's keys (both of its buffers).
+static xt_status rows_to_csr(Ctx *c, const int64_t *rstart, uint32_t *cols_s, int64_t n, int64_t nv, int b,
                              uint64_t *kbuf, Graph *g) {
   const int B = 256;
-  int64_t *rstart = nullptr, *ulen = nullptr, *spans = nullptr;
+  int64_t *ulen = nullptr, *spans = nullptr;
   int32_t *lists = nullptr;
   unsigned long long *nl = nullptr;
   uint64_t *hk = nullptr;
@@ -906,9 +816,6 @@ static xt_status rows_to_csr(Ctx *c, const uint32_t *rows_s, uint32_t *cols_s, i
   void *tmp = nullptr;
   xt_status s = XT_OK;
   do {
-    // bucket bounds: the runs of the sorted low ends
-    if ((s = dalloc_n(c, &rstart, size_t(nv + 1))) != XT_OK) break;
-    if ((s = keys_to_csr<uint32_t>(c, rows_s, n, nv, 0, rstart, nullptr)) != XT_OK) break;
     if ((s = dalloc_n(c, &ulen, size_t(nv + 1))) != XT_OK) break;
     RowLists rl;
     int64_t ltot = 0;
@@ -1038,12 +945,11 @@ static xt_status rows_to_csr(Ctx *c, const uint32_t *rows_s, uint32_t *cols_s, i
     uint32_t *ks = nullptr;
     InRec *rs = nullptr;
     if ((s = sort_pairs_db<InRec>(c, kin, kalt, r0, r1, m, b + lb, &ks, &rs)) != XT_OK) break;
-    if ((s = keys_to_csr<uint32_t>(c, ks, m, nv, lb, g->d_ioff, nullptr)) != XT_OK) break;
+    if ((s = keys_to_csr(c, ks, m, nv, lb, g->d_ioff)) != XT_OK) break;
     g->d_irec = rs;
     if (rs == r0) r0 = nullptr;
     else r1 = nullptr;
   } while (0);
-  dfree(c, rstart);
   dfree(c, ulen);
   dfree(c, spans);
   dfree(c, lists);
@@ -1108,7 +1014,8 @@ xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src,
   // k0 = the rows' low ends then, from the next 16-byte boundary, their
   // high ends (4 bytes each); k1 = the same for the sort's other buffers
   uint64_t *k0 = nullptr, *k1 = nullptr;
-  int32_t *deg = nullptr;
+  int32_t *deg = nullptr, *o2n = nullptr;
+  int64_t *rstart = nullptr;
   xt_status s = XT_OK;
   const size_t n1 = size_t(ne > 0 ? ne : 1);
   const int64_t ne4 = (ne + 3) & ~int64_t(3);
@@ -1135,20 +1042,80 @@ xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src,
     }
     // rank, then relabel every row in place
     if (orient == XT_ORIENT_DEGREE) {
-      if ((s = rank_and_relabel(c, deg, nv, b, nullptr, ne, g, lo, hi)) != XT_OK) break;
+      if ((s = rank_vertices(c, deg, nv, g, &o2n)) != XT_OK) break;
+      if (ne > 0)
+        k_relabel_split<<<counted(c, grid_for(ne, B, c->sm_count)), B, 0, c->stream>>>(lo, hi, ne, o2n);
+      if ((s = cuda_status(c, cudaGetLastError(), "relabel")) != XT_OK) break;
       dfree(c, deg);
-      deg = nullptr;
+      dfree(c, o2n);
+      deg = o2n = nullptr;
     }
     // rows grouped by their low end: a radix sort on the low end's b bits
     uint32_t *rows_s = lo, *cols_s = hi;
     if (ne > 0 && (s = sort_pairs_db<uint32_t>(c, lo, lo2, hi, hi2, ne, b, &rows_s, &cols_s)) != XT_OK) break;
     const bool in_k0 = cols_s == hi;  // the sorted rows are in k0
-    s = rows_to_csr(c, rows_s, cols_s, ne, nv, b, in_k0 ? k1 : k0, g);
+    // bucket bounds: the runs of the sorted low ends
+    if ((s = dalloc_n(c, &rstart, size_t(nv + 1))) != XT_OK) break;
+    if ((s = keys_to_csr(c, rows_s, ne, nv, 0, rstart)) != XT_OK) break;
+    s = rows_to_csr(c, rstart, cols_s, ne, nv, b, in_k0 ? k1 : k0, g);
   } while (0);
   dfree(c, k0);
   dfree(c, k1);
   dfree(c, deg);
+  dfree(c, o2n);
+  dfree(c, rstart);
   if (s != XT_OK) free_graph_device(g);
+  return s;
+}
+
+// Canonical CSR entries (rows and tails in 32 bits, n of them, m = n / 2
+// undirected edges; both arrays are overwritten) -> the graph: ranks from the
+// offsets' degrees, then the oriented rows placed by counting, no edge sort.
+static xt_status build_canonical(Ctx *c, int64_t nv, const int64_t *d_off, int32_t *rows, int32_t *t32, int64_t n,
+                                 int orient, Graph *g) {
+  const int B = 256, b = bits_for(nv);
+  const int64_t m = n / 2;
+  int32_t *deg = nullptr, *o2n = nullptr;
+  int64_t *len = nullptr, *rstart = nullptr;
+  uint32_t *bk = nullptr;
+  uint64_t *kbuf = nullptr;
+  xt_status s = XT_OK;
+  do {
+    if (orient == XT_ORIENT_DEGREE) {
+      if ((s = dalloc_n(c, &deg, size_t(nv))) != XT_OK) break;
+      k_degree_from_off<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(d_off, nv, deg);
+      if ((s = rank_vertices(c, deg, nv, g, &o2n)) != XT_OK) break;
+      dfree(c, deg);
+      deg = nullptr;
+    }
+    if ((s = dalloc_n(c, &len, size_t(nv + 1))) != XT_OK) break;
+    if ((s = dalloc_n(c, &rstart, size_t(nv + 1))) != XT_OK) break;
+    if ((s = dalloc_n(c, &bk, size_t(m > 0 ? m : 1))) != XT_OK) break;
+    if ((s = cuda_status(c, cudaMemsetAsync(len, 0, sizeof(int64_t) * (nv + 1), c->stream), "memset")) != XT_OK) break;
+    if (n > 0)
+      k_csr_keep<<<counted(c, grid_for(n, B, c->sm_count)), B, 0, c->stream>>>(rows, t32, n, o2n, len);
+    if ((s = exclusive_scan_i64(c, len, rstart, nv + 1)) != XT_OK) break;
+    int64_t *cur = len;  // the rows' next free slots
+    if ((s = cuda_status(c, cudaMemcpyAsync(cur, rstart, sizeof(int64_t) * nv, cudaMemcpyDeviceToDevice, c->stream),
+                         "D2D")) != XT_OK)
+      break;
+    if (n > 0)
+      k_csr_place<<<counted(c, grid_for(n, B, c->sm_count)), B, 0, c->stream>>>(
+          rows, t32, n, reinterpret_cast<unsigned long long *>(cur), bk);
+    if ((s = cuda_status(c, cudaGetLastError(), "k_csr_place")) != XT_OK) break;
+    dfree(c, len);
+    dfree(c, o2n);
+    len = nullptr;
+    o2n = nullptr;
+    if ((s = dalloc_n(c, &kbuf, size_t(m > 0 ? m : 1))) != XT_OK) break;
+    s = rows_to_csr(c, rstart, bk, m, nv, b, kbuf, g);
+  } while (0);
+  dfree(c, deg);
+  dfree(c, o2n);
+  dfree(c, len);
+  dfree(c, rstart);
+  dfree(c, bk);
+  dfree(c, kbuf);
   return s;
 }
 
@@ -1157,31 +1124,46 @@ xt_status build_from_csr(Ctx *c, int64_t nv, const int64_t *d_off, const int64_t
   if (nv < 1) return set_error(c, XT_ERR_INVALID, "nv must be >= 1");
   if (nv > (int64_t(1) << 31) - 1) return set_error(c, XT_ERR_OVERFLOW, "nv must be below 2^31");
   if (orient != XT_ORIENT_ID && orient != XT_ORIENT_DEGREE) return set_error(c, XT_ERR_INVALID, "bad orientation");
-  int64_t ne_in = 0;
-  XT_CUDA(c, cudaMemcpyAsync(&ne_in, d_off + nv, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+  int64_t ends[2] = {0, 0};
+  XT_CUDA(c, cudaMemcpyAsync(&ends[0], d_off, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+  XT_CUDA(c, cudaMemcpyAsync(&ends[1], d_off + nv, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
   XT_CUDA(c, cudaStreamSynchronize(c->stream));
+  const int64_t e_first = ends[0], ne_in = ends[1];
   if (ne_in < 0) return set_error(c, XT_ERR_INVALID, "offsets[nv] is negative");
+  if (e_first < 0 || e_first > ne_in) return set_error(c, XT_ERR_INVALID, "csr: offsets not monotone in [0,ne]");
   const int B = 256;
+  const int64_t n = ne_in - e_first;  // entries of the rows
   int32_t *rows = nullptr, *t32 = nullptr;
+  unsigned long long *chk = nullptr;
+  unsigned long long h[kCsrWords] = {0, 0, 0};
   xt_status s = XT_OK;
   const size_t n1 = size_t(ne_in > 0 ? ne_in : 1);
   do {
     if ((s = dalloc_n(c, &rows, n1)) != XT_OK) break;
     if ((s = dalloc_n(c, &t32, n1)) != XT_OK) break;
-    k_csr_rows<<<counted(c, grid_for(nv * 32, B, c->sm_count)), B, 0, c->stream>>>(d_off, nv, ne_in, rows,
-                                                                                   c->d_err);
-    k_csr_tails32<<<counted(c, grid_for(ne_in, B, c->sm_count)), B, 0, c->stream>>>(d_tails, ne_in, nv, t32,
-                                                                                    c->d_err);
-    if ((s = cuda_status(c, cudaGetLastError(), "k_csr_rows")) != XT_OK) break;
-    if ((s = check_err(c, "csr")) != XT_OK) break;
-    if (canonical) {  // the rows are used as they stand: check the promise first
-      k_csr_check_canonical<<<counted(c, grid_for(nv * 32, B, c->sm_count)), B, 0, c->stream>>>(d_off, t32, nv,
-                                                                                                c->d_err);
-      if ((s = cuda_status(c, cudaGetLastError(), "k_csr_check_canonical")) != XT_OK) break;
-      if ((s = check_err(c, "canonical csr")) != XT_OK) break;
+    if ((s = dalloc_n(c, &chk, kCsrWords)) != XT_OK) break;
+    if ((s = cuda_status(c, cudaMemsetAsync(chk, 0, kCsrWords * sizeof(*chk), c->stream), "memset")) != XT_OK) break;
+    k_csr_offsets<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(d_off, nv, ne_in, c->d_err);
+    if (n > 0) {
+      const int64_t warps = (n + kCsrSpan - 1) / kCsrSpan;
+      k_csr_entries<<<counted(c, grid_for(warps * 32, B, c->sm_count)), B, 0, c->stream>>>(
+          d_off, d_tails, nv, e_first, ne_in, rows, t32, c->d_err, chk);
+      k_csr_back<<<counted(c, grid_for(n, B, c->sm_count)), B, 0, c->stream>>>(d_off, rows, t32, e_first, ne_in,
+                                                                               c->d_err, chk);
     }
-    if (!canonical) {
-      s = build_from_edges(c, nv, ne_in, rows, t32, orient, g);
+    if ((s = cuda_status(c, cudaGetLastError(), "csr check")) != XT_OK) break;
+    if ((s = cuda_status(c, cudaMemcpyAsync(h, chk, sizeof(h), cudaMemcpyDeviceToHost, c->stream), "D2H")) != XT_OK)
+      break;
+    if ((s = check_err(c, "csr")) != XT_OK) break;
+    // rows that are canonical, promised or not, need no edge sort
+    const bool sorted = h[0] == 0 && h[1] == 0 && h[2] == 0;
+    if (canonical && !sorted) {
+      s = set_error(c, XT_ERR_INVALID, "canonical csr: a row is out of order, repeats an id or holds its own id, or "
+                                       "an edge is missing from its other end's row (not a canonical CSR)");
+      break;
+    }
+    if (!sorted) {
+      s = build_from_edges(c, nv, n, rows + e_first, t32 + e_first, orient, g);
       if (s == XT_OK) g->n_input = ne_in;
       break;
     }
@@ -1189,44 +1171,12 @@ xt_status build_from_csr(Ctx *c, int64_t nv, const int64_t *d_off, const int64_t
     g->nv = nv;
     g->n_input = ne_in;
     g->orient = orient;
-    const int b = bits_for(nv);
-    uint64_t *keys = nullptr, *sel = nullptr;
-    uint8_t *flags = nullptr;
-    int32_t *deg = nullptr;
-    int64_t m = 0;
-    do {
-      if ((s = dalloc_n(c, &keys, n1)) != XT_OK) break;
-      if ((s = dalloc_n(c, &sel, n1)) != XT_OK) break;
-      if ((s = dalloc_n(c, &flags, n1)) != XT_OK) break;
-      if (ne_in > 0) {
-        // the u < t entries of sorted symmetric rows: the sorted undirected set
-        k_csr_lower_keys<<<counted(c, grid_for(ne_in, B, c->sm_count)), B, 0, c->stream>>>(rows, t32, ne_in, b,
-                                                                                           keys, flags);
-        if ((s = cuda_status(c, cudaGetLastError(), "k_csr_lower_keys")) != XT_OK) break;
-        if ((s = select_flagged(c, keys, flags, sel, ne_in, &m)) != XT_OK) break;
-      }
-      dfree(c, flags);
-      flags = nullptr;
-      if (orient == XT_ORIENT_DEGREE) {
-        if ((s = dalloc_n(c, &deg, size_t(nv))) != XT_OK) break;
-        k_degree_from_off<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(d_off, nv, deg);
-        if ((s = rank_and_relabel(c, deg, nv, b, sel, m, g)) != XT_OK) break;
-        dfree(c, deg);
-        deg = nullptr;
-        if (m > 0 && (s = sort_keys(c, sel, keys, m, 2 * b)) != XT_OK) break;
-        s = finish_csr(c, keys, sel, m, nv, b, g);
-      } else {
-        s = finish_csr(c, sel, keys, m, nv, b, g);
-      }
-    } while (0);
-    dfree(c, keys);
-    dfree(c, sel);
-    dfree(c, flags);
-    dfree(c, deg);
+    s = build_canonical(c, nv, d_off, rows + e_first, t32 + e_first, n, orient, g);
     if (s != XT_OK) free_graph_device(g);
   } while (0);
   dfree(c, rows);
   dfree(c, t32);
+  dfree(c, chk);
   return s;
 }
 
