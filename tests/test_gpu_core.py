@@ -1,0 +1,80 @@
+"""The dense core (blocks of the top ranks counted on the tensor cores) against
+the oracle, at the edges of its row blocks (128), column steps (256) and
+widths, and beside rows that are streamed."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import xxtric_b200 as xt
+    with xt.Context(0) as c:
+        yield c
+
+
+def dense(n, p, rng):
+    a, b = np.triu_indices(n, 1)
+    keep = rng.random(len(a)) < p
+    return a[keep], b[keep]
+
+
+def graph(kind):
+    rng = np.random.default_rng(11)
+    if isinstance(kind, int):  # a dense graph of that many vertices
+        return kind, *dense(kind, 0.8, rng)
+    if kind == "complete":
+        return 1700, *np.triu_indices(1700, 1)
+    if kind == "core and tail":  # a dense core, a band of rows half in it, and a sparse tail
+        n, k = 60000, 1500
+        a, b = dense(k, 0.6, rng)
+        m = rng.integers(k, 6000, 250000)
+        t = rng.integers(0, n, (2, 200000))
+        s = np.concatenate([a, m, t[0]])
+        d = np.concatenate([b, rng.integers(0, k, len(m)), t[1]])
+        p = rng.permutation(n)
+        return n, p[s], p[d]
+    raise ValueError(kind)
+
+
+CASES = [1151, 1152, 1153, 1279, 1280, 1281, 1535, 1537, "complete", "core and tail"]
+
+
+@pytest.mark.parametrize("kind", CASES)
+def test_core_counts_match_the_oracle(ctx, kind):
+    nv, src, dst = graph(kind)
+    off, tails = oracle.canon_csr(nv, src.astype(np.int64), dst.astype(np.int64))
+    want, pv = oracle.count_merge(off, tails, per_vertex=True)
+    for orient in (1, 0):
+        g = ctx.graph_from_edges(nv, src.astype(np.int32), dst.astype(np.int32), orient)
+        before = ctx.launches
+        assert g.count() == want
+        if orient == 1 or kind != "core and tail":  # under the id order the permuted core is not at the top
+            assert ctx.launches == before + 2, "the core's kernel beside the streaming one"
+        total, each = g.count(per_vertex=True)
+        assert total == want
+        np.testing.assert_array_equal(each, pv)
+        total, sup = g.count_edges()
+        assert total == want and int(sup.sum()) == 3 * want
+        g.set_tiers(0, 0)
+        assert g.count() == want
+        g.free()
+
+
+@pytest.mark.parametrize("nshards", [2, 7])
+def test_core_shards_sum_to_the_count(ctx, nshards):
+    import torch
+    nv, src, dst = graph("core and tail")
+    g = ctx.graph_from_edges(nv, src.astype(np.int32), dst.astype(np.int32))
+    want = g.count()
+    part = torch.zeros(1, dtype=torch.int64, device="cuda")
+    got = 0
+    for i in range(nshards):
+        g.count_shard_async(i, nshards, part)
+        ctx.synchronize()
+        got += int(part)
+    assert got == want
+    g.free()

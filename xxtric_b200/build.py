@@ -24,7 +24,7 @@ BUILD = os.path.join(ROOT, "_build")
 LIB = os.path.join(PKG, "libxtb200.so")
 CLI = os.path.join(PKG, "xtric")
 
-CUDA_SOURCES = ["csrc/capi.cu", "csrc/build.cu", "csrc/count.cu", "csrc/gen.cu", "csrc/rgg.cu",
+CUDA_SOURCES = ["csrc/capi.cu", "csrc/build.cu", "csrc/count.cu", "csrc/core.cu", "csrc/gen.cu", "csrc/rgg.cu",
                 "csrc/vite.cu", "csrc/count_static.cu", "csrc/batch.cu", "csrc/serve.cu"]
 HOST_SOURCES = ["host/host_io.cpp"]
 CLI_SOURCES = ["host/xtric_main.cpp"]

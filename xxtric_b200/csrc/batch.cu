@@ -121,6 +121,7 @@ xt_status build_batch(Ctx *c, int64_t ng, const int64_t *h_voff, const int64_t *
       s = set_error(c, XT_ERR_INVALID, "batch: a vertex id is outside its graph");
       break;
     }
+    g->no_core = true;
     if ((s = build_from_edges(c, nv, ne, gs, gd, orient, g)) != XT_OK) break;
     dfree(c, gs);
     dfree(c, gd);
@@ -525,7 +526,7 @@ static std::string tune_key(const Graph *g) {
   };
   char buf[512];
   // the schedule revision keeps timings of an older kernel from being reused
-  snprintf(buf, sizeof buf, "sched10|%s|sm%d|orient%d|nv2^%d|ne2^%d|work2^%d|groups%lld", p.name, p.multiProcessorCount,
+  snprintf(buf, sizeof buf, "sched11|%s|sm%d|orient%d|nv2^%d|ne2^%d|work2^%d|groups%lld", p.name, p.multiProcessorCount,
            g->orient, lg(g->nv), lg(g->ne), lg(g->stream_work), (long long)g->n_groups);
   for (char *q = buf; *q; q++)
     if (*q == ' ') *q = '_';

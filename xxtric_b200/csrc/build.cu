@@ -465,9 +465,17 @@ __device__ __forceinline__ uint32_t len_class_desc(int64_t len) {
 // ulen[u] (kPadSentinel after it); its out-CSR position p = off[u] + t also
 // gets the in-record of edge u->v (the suffix after t: colp[poff[u] + t + 1,
 // poff[u] + ulen[u])) and its sort key, v << lb | the suffix length's class
-// (lb of its 7 bits, as many as fit beside v in 31 bits).
+// (lb of its 7 bits, as many as fit beside v in 31 bits). With a core (cut !=
+// null) the top of the lb bits marks the records of row block b of the core's
+// nb whose head is cut[b] or above: they sort last among their head's, still
+// longest first.
+__device__ __forceinline__ uint32_t rec_class(int64_t len, bool flagged, bool core, int lb) {
+  const int cb = flagged ? lb - 1 : lb;  // bits of the length class
+  const uint32_t c = cb > 0 ? len_class_desc(len) >> (7 - cb) : 0u;
+  return core ? c | (1u << cb) : c;
+}
 __global__ void k_rows_emit(const int64_t *__restrict__ rstart, const uint32_t *__restrict__ bk, int64_t nv, int lb,
-                            const int64_t *__restrict__ off, const int64_t *__restrict__ poff,
+                            const int32_t *__restrict__ cut, int nb, const int64_t *__restrict__ off, const int64_t *__restrict__ poff,
                             int32_t *__restrict__ col, int32_t *__restrict__ colp, uint32_t *__restrict__ ik,
                             InRec *__restrict__ rec) {
   const int lane = threadIdx.x & 31;
@@ -477,6 +485,8 @@ __global__ void k_rows_emit(const int64_t *__restrict__ rstart, const uint32_t *
     const int64_t r = base + lane, rc = r < nv ? r : nv;  // lanes past nv: empty rows at the end
     const int64_t o = off[rc], len = off[r < nv ? r + 1 : nv] - o, p = poff[rc];
     const int64_t a = r < nv ? rstart[r] : 0;
+    const int64_t blk = (nv - 1 - r) >> 7;
+    const int32_t cu = cut && r < nv && blk < nb ? cut[blk] : 0x7fffffff;
     const int64_t p0 = __shfl_sync(0xffffffffu, p, 0);
     const int64_t pend = poff[base + 32 < nv ? base + 32 : nv];
     for (int64_t q0 = p0; q0 < pend; q0 += 32) {
@@ -487,6 +497,7 @@ __global__ void k_rows_emit(const int64_t *__restrict__ rstart, const uint32_t *
         if (__shfl_sync(0xffffffffu, p, j + step) <= q) j += step;
       const int64_t pj = __shfl_sync(0xffffffffu, p, j), lj = __shfl_sync(0xffffffffu, len, j);
       const int64_t oj = __shfl_sync(0xffffffffu, o, j), aj = __shfl_sync(0xffffffffu, a, j);
+      const int32_t cj = __shfl_sync(0xffffffffu, cu, j);
       if (q < pend) {
         const int64_t t = q - pj;
         if (t < lj) {
@@ -494,7 +505,7 @@ __global__ void k_rows_emit(const int64_t *__restrict__ rstart, const uint32_t *
           const int64_t sl = lj - t - 1;
           col[oj + t] = int32_t(x);
           colp[q] = int32_t(x);
-          ik[oj + t] = (x << lb) | (lb > 0 ? len_class_desc(sl) >> (7 - lb) : 0u);
+          ik[oj + t] = (x << lb) | rec_class(sl, cut != nullptr, int32_t(x) >= cj, lb);
           rec[oj + t] = make_inrec(q + 1, sl);
         } else {
           colp[q] = kPadSentinel;
@@ -504,18 +515,40 @@ __global__ void k_rows_emit(const int64_t *__restrict__ rstart, const uint32_t *
   }
 }
 
-// Sorted keys (row << b | rest) -> row lengths. The thread at a run's first
+// Sorted rows -> row lengths. The thread at a run's first
 // key adds -start, the one at its last key adds end, so each non-empty row
 // ends with end - start (len must start zeroed). The offsets are then the
 // exclusive scan of the lengths.
-__global__ void k_csr_runs(const uint32_t *__restrict__ keys, int64_t m, int b, int64_t *__restrict__ len) {
+__global__ void k_csr_runs(const uint32_t *__restrict__ rows, int64_t m, int64_t *__restrict__ len) {
   XT_GRID_STRIDE(i, m) {
-    const uint32_t row = keys[i] >> b;
-    if (i == 0 || (keys[i - 1] >> b) != row)
+    const uint32_t row = rows[i];
+    if (i == 0 || rows[i - 1] != row)
       atomicAdd(reinterpret_cast<unsigned long long *>(&len[row]), (unsigned long long)(-i));
-    if (i + 1 == m || (keys[i + 1] >> b) != row)
+    if (i + 1 == m || rows[i + 1] != row)
       atomicAdd(reinterpret_cast<unsigned long long *>(&len[row]), (unsigned long long)(i + 1));
   }
+}
+
+// The in-records' sorted keys (head << lb | class) -> records per head (as
+// k_csr_runs) and, beside them, those whose class is below `dead`: the ones
+// that have candidates and are not the core's come first among a head's.
+__global__ void k_rec_runs(const uint32_t *__restrict__ keys, int64_t m, int lb, uint32_t dead,
+                           unsigned long long *__restrict__ len, unsigned long long *__restrict__ live) {
+  const uint32_t mask = (1u << lb) - 1u;
+  XT_GRID_STRIDE(i, m) {
+    const uint32_t k = keys[i], head = k >> lb;
+    const uint32_t p = i > 0 ? keys[i - 1] : 0u, q = i + 1 < m ? keys[i + 1] : 0u;
+    const bool first = i == 0 || (p >> lb) != head, last = i + 1 == m || (q >> lb) != head;
+    const bool on = (k & mask) < dead;
+    if (first) atomicAdd(&len[head], (unsigned long long)(-i));
+    if (last) atomicAdd(&len[head], (unsigned long long)(i + 1));
+    if (on && first) atomicAdd(&live[head], (unsigned long long)(-i));
+    if (on && (last || (q & mask) >= dead)) atomicAdd(&live[head], (unsigned long long)(i + 1));
+  }
+}
+// live records per head -> the end of the head's live records, in place
+__global__ void k_rec_ends(const int64_t *__restrict__ ioff, int64_t nv, int64_t *__restrict__ live) {
+  XT_GRID_STRIDE(v, nv) live[v] += ioff[v];
 }
 
 // ---- CSR input ----------------------------------------------------------------
@@ -713,27 +746,6 @@ static xt_status sort_pairs_db(Ctx *c, uint32_t *k0, uint32_t *k1, V *v0, V *v1,
   return XT_OK;
 }
 
-// sorted (row << b | rest) keys -> off[nv+1]
-static xt_status keys_to_csr(Ctx *c, const uint32_t *keys, int64_t m, int64_t nv, int b, int64_t *off) {
-  int64_t *len = nullptr;
-  XT_TRY(dalloc_n(c, &len, size_t(nv + 1)));
-  cudaError_t e = cudaMemsetAsync(len, 0, sizeof(int64_t) * (nv + 1), c->stream);
-  if (e == cudaSuccess && m > 0) {
-    k_csr_runs<<<counted(c, grid_for(m, 256, c->sm_count)), 256, 0, c->stream>>>(keys, m, b, len);
-    e = cudaGetLastError();
-  }
-  size_t bytes = 0;
-  void *tmp = nullptr;
-  if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, bytes, len, off, nv + 1, c->stream);
-  xt_status s = cuda_status(c, e, "csr offsets");
-  if (s == XT_OK) s = dalloc(c, &tmp, bytes);
-  if (s == XT_OK)
-    s = cuda_status(c, cub::DeviceScan::ExclusiveSum(tmp, bytes, len, off, nv + 1, c->stream), "csr offsets");
-  dfree(c, tmp);
-  dfree(c, len);
-  return s;
-}
-
 static xt_status exclusive_scan_i64(Ctx *c, const int64_t *in, int64_t *out, int64_t n) {
   size_t bytes = 0;
   XT_CUDA(c, cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, n, c->stream));
@@ -743,6 +755,48 @@ static xt_status exclusive_scan_i64(Ctx *c, const int64_t *in, int64_t *out, int
   dfree(c, tmp);
   XT_CUDA(c, e);
   return XT_OK;
+}
+
+// sorted rows -> off[nv+1]
+static xt_status rows_to_offsets(Ctx *c, const uint32_t *rows, int64_t m, int64_t nv, int64_t *off) {
+  int64_t *len = nullptr;
+  XT_TRY(dalloc_n(c, &len, size_t(nv + 1)));
+  cudaError_t e = cudaMemsetAsync(len, 0, sizeof(int64_t) * (nv + 1), c->stream);
+  if (e == cudaSuccess && m > 0) {
+    k_csr_runs<<<counted(c, grid_for(m, 256, c->sm_count)), 256, 0, c->stream>>>(rows, m, len);
+    e = cudaGetLastError();
+  }
+  xt_status s = cuda_status(c, e, "csr offsets");
+  if (s == XT_OK) s = exclusive_scan_i64(c, len, off, nv + 1);
+  dfree(c, len);
+  return s;
+}
+
+// sorted record keys -> g->d_ioff and g->d_iend
+static xt_status records_to_csr(Ctx *c, const uint32_t *keys, int64_t m, int lb, Graph *g) {
+  const int64_t nv = g->nv;
+  int64_t *len = nullptr;
+  XT_TRY(dalloc_n(c, &g->d_iend, size_t(nv)));
+  XT_TRY(dalloc_n(c, &len, size_t(nv + 1)));
+  cudaError_t e = cudaMemsetAsync(len, 0, sizeof(int64_t) * (nv + 1), c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(g->d_iend, 0, sizeof(int64_t) * nv, c->stream);
+  // class bits: 7 hold a zero length apart (127); fewer do not, so nothing but the core's mark then
+  const bool core = g->core.n_items > 0;
+  const uint32_t dead = lb - (core ? 1 : 0) == 7 ? 127u : core ? 1u << (lb - 1) : 1u << lb;
+  xt_status s = cuda_status(c, e, "records");
+  if (s == XT_OK) {
+    k_rec_runs<<<counted(c, grid_for(m, 256, c->sm_count)), 256, 0, c->stream>>>(
+        keys, m, lb, dead, reinterpret_cast<unsigned long long *>(len),
+        reinterpret_cast<unsigned long long *>(g->d_iend));
+    s = cuda_status(c, cudaGetLastError(), "k_rec_runs");
+  }
+  if (s == XT_OK) s = exclusive_scan_i64(c, len, g->d_ioff, nv + 1);
+  if (s == XT_OK) {
+    k_rec_ends<<<counted(c, grid_for(nv, 256, c->sm_count)), 256, 0, c->stream>>>(g->d_ioff, nv, g->d_iend);
+    s = cuda_status(c, cudaGetLastError(), "k_rec_ends");
+  }
+  dfree(c, len);
+  return s;
 }
 
 static xt_status check_err(Ctx *c, const char *what) {
@@ -812,6 +866,7 @@ static xt_status rows_to_csr(Ctx *c, const int64_t *rstart, uint32_t *cols_s, in
   int32_t *lists = nullptr;
   unsigned long long *nl = nullptr;
   uint64_t *hk = nullptr;
+  int64_t *d_sums = nullptr;
   InRec *r0 = nullptr, *r1 = nullptr;
   void *tmp = nullptr;
   xt_status s = XT_OK;
@@ -904,6 +959,8 @@ static xt_status rows_to_csr(Ctx *c, const int64_t *rstart, uint32_t *cols_s, in
       break;
     if ((s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync")) != XT_OK) break;
     g->ne = m;
+    // the dense core's widths
+    if ((s = core_plan(c, g, rstart, cols_s, m, &d_sums)) != XT_OK) break;
     // Columns are read as aligned 32-byte pairs: pad so the last pair of the
     // last row stays inside the allocation.
     if ((s = dalloc_n(c, &g->d_col, size_t(m) + kColPad)) != XT_OK) break;
@@ -915,9 +972,12 @@ static xt_status rows_to_csr(Ctx *c, const int64_t *rstart, uint32_t *cols_s, in
     k_pad_len<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(g->d_off, nv, plen);
     if ((s = cuda_status(c, cudaMemsetAsync(plen + nv, 0, sizeof(int64_t), c->stream), "memset")) != XT_OK) break;
     if ((s = exclusive_scan_i64(c, plen, g->d_poff, nv + 1)) != XT_OK) break;
-    int64_t total = 0;
+    int64_t total = 0, sums[kCoreSums] = {};
     if ((s = cuda_status(c, cudaMemcpyAsync(&total, g->d_poff + nv, sizeof(int64_t), cudaMemcpyDeviceToHost,
                                             c->stream), "D2H")) != XT_OK)
+      break;
+    if (d_sums && (s = cuda_status(c, cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, c->stream),
+                                   "D2H")) != XT_OK)
       break;
     if ((s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync")) != XT_OK) break;
     if (total >= kMaxColp) {
@@ -929,23 +989,28 @@ static xt_status rows_to_csr(Ctx *c, const int64_t *rstart, uint32_t *cols_s, in
     if ((s = dalloc_n(c, &g->d_ioff, size_t(nv + 1))) != XT_OK) break;
     if (m == 0) {
       if ((s = dalloc_n(c, &g->d_irec, 2)) != XT_OK) break;
+      if ((s = dalloc_n(c, &g->d_iend, size_t(nv))) != XT_OK) break;
+      if ((s = cuda_status(c, cudaMemsetAsync(g->d_iend, 0, sizeof(int64_t) * nv, c->stream), "memset")) != XT_OK)
+        break;
       s = cuda_status(c, cudaMemsetAsync(g->d_ioff, 0, sizeof(int64_t) * (nv + 1), c->stream), "memset");
       break;
     }
     // the out-CSR, with the in-records in position order and their sort keys
     // (head << lb | class, in kbuf), sorted by head and then class (stable:
     // records of one (head, class) stay in position order)
-    const int lb = b + 7 <= 31 ? 7 : 31 - b;
+    if ((s = core_decide(c, g, sums)) != XT_OK) break;
+    const int lb = g->core.n_items > 0 ? std::min(8, 32 - b) : (b + 7 <= 31 ? 7 : 31 - b);
     uint32_t *kin = reinterpret_cast<uint32_t *>(kbuf), *kalt = kin + m;
     if ((s = dalloc_n(c, &r0, size_t(m) + 2)) != XT_OK) break;
     if ((s = dalloc_n(c, &r1, size_t(m) + 2)) != XT_OK) break;
-    k_rows_emit<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(rstart, cols_s, nv, lb, g->d_off,
-                                                                               g->d_poff, g->d_col, g->d_colp, kin, r0);
+    k_rows_emit<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(
+        rstart, cols_s, nv, lb, g->core.d_cut, g->core.nb, g->d_off, g->d_poff, g->d_col, g->d_colp, kin, r0);
     if ((s = cuda_status(c, cudaGetLastError(), "row emit")) != XT_OK) break;
     uint32_t *ks = nullptr;
     InRec *rs = nullptr;
     if ((s = sort_pairs_db<InRec>(c, kin, kalt, r0, r1, m, b + lb, &ks, &rs)) != XT_OK) break;
-    if ((s = keys_to_csr(c, ks, m, nv, lb, g->d_ioff)) != XT_OK) break;
+    if ((s = records_to_csr(c, ks, m, lb, g)) != XT_OK) break;
+    if ((s = core_finish(c, g)) != XT_OK) break;
     g->d_irec = rs;
     if (rs == r0) r0 = nullptr;
     else r1 = nullptr;
@@ -955,6 +1020,7 @@ static xt_status rows_to_csr(Ctx *c, const int64_t *rstart, uint32_t *cols_s, in
   dfree(c, lists);
   dfree(c, nl);
   dfree(c, hk);
+  dfree(c, d_sums);
   dfree(c, tmp);
   dfree(c, r0);
   dfree(c, r1);
@@ -1056,7 +1122,7 @@ xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src,
     const bool in_k0 = cols_s == hi;  // the sorted rows are in k0
     // bucket bounds: the runs of the sorted low ends
     if ((s = dalloc_n(c, &rstart, size_t(nv + 1))) != XT_OK) break;
-    if ((s = keys_to_csr(c, rows_s, ne, nv, 0, rstart)) != XT_OK) break;
+    if ((s = rows_to_offsets(c, rows_s, ne, nv, rstart)) != XT_OK) break;
     s = rows_to_csr(c, rstart, cols_s, ne, nv, b, in_k0 ? k1 : k0, g);
   } while (0);
   dfree(c, k0);
@@ -1187,9 +1253,11 @@ void free_graph_device(Graph *g) {
   dfree(g->ctx, g->d_res);
   g->d_res = nullptr;
   free_plan(g);
+  core_free(g);
   dfree(g->ctx, g->d_off);
   dfree(g->ctx, g->d_col);
   dfree(g->ctx, g->d_ioff);
+  dfree(g->ctx, g->d_iend);
   dfree(g->ctx, g->d_irec);
   dfree(g->ctx, g->d_irec_u);
   g->d_irec_u = nullptr;
@@ -1200,6 +1268,7 @@ void free_graph_device(Graph *g) {
   g->d_off = nullptr;
   g->d_col = nullptr;
   g->d_ioff = nullptr;
+  g->d_iend = nullptr;
   g->d_irec = nullptr;
   g->d_colp = nullptr;
   g->d_poff = nullptr;

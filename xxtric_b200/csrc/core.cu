@@ -1,0 +1,555 @@
+// The dense core of the oriented graph, counted on the tensor cores.
+//
+// In (degree, id) rank order the columns of a power-law graph crowd the top
+// ranks: on R-MAT 2^22, 44% of the candidates the count streams lie in blocks
+// of the adjacency matrix that hold an edge in every 10th to 50th place. There
+// a contraction does 8,192 multiply-adds per SM and cycle where the streaming
+// kernel (count.cu) spends about 15 instructions on a candidate, so those
+// blocks leave its schedule and are counted here.
+//
+// Notation: rank position i of a vertex counts from the top, i = nv - 1 - id,
+// so N+(u) are positions below u's. Rows are taken in blocks of 128 positions,
+// columns in chunks of 128. Row block b has a width T_b (a multiple of 256,
+// at most kCoreWidth; 0: none): the triangles u < v < w (ids) with u in block b
+// and v among the top T_b positions (w, above v, is then too) are
+//     sum over v of X[u][v] * (sum over w of X[u][w] * X[v][w]),
+// X the 0/1 adjacency matrix, the inner sum a product of the rows of block b
+// with the rows of the top T_b vertices. Every one of them has its streamed
+// candidates in the in-records u->v, which the builder puts last among v's
+// records (Graph::d_iend[v] is the first of them) and the schedule leaves out.
+// The reference has no counterpart: its kernels intersect sorted lists
+// (counting.cu:95-131).
+//
+// Operands: one byte per element in 16 KB tiles of 128 rows x 128 columns, laid
+// out in memory as a 128-byte-swizzled K-major operand sits in shared memory
+// (16-byte piece p of row r at p ^ (r & 7)), so a tile is one bulk copy.
+#include <cub/cub.cuh>
+
+#include <algorithm>
+
+#include "xt_internal.cuh"
+
+namespace xt {
+
+constexpr int kCoreRows = 128;          // rows of a block, columns of a chunk
+constexpr int kCoreTile = kCoreRows * 128;
+constexpr int kCoreStep = 256;          // widths are multiples of this: the columns of one work item
+constexpr int kCoreMaxJ = 64;           // widths up to 64 * 256
+constexpr int kCoreWidth = kCoreMaxJ * kCoreStep;
+constexpr int kCoreMinBlk = kCoreWidth / kCoreRows;  // the core's own rows
+constexpr int kCoreMaxBlk = 8192;       // row blocks looked at: the top 2^20 vertices
+constexpr int kCoreMinRow = 16;         // shorter rows gain less than their share of a step
+
+// The rule of T_b weighs, per block, the streamed candidates it takes away
+// against the chunk steps (128 x 256 x 128 multiply-adds) it adds, each at the
+// rate the whole GPU runs it: a candidate of these long suffixes 0.4 ps, a
+// chunk step 2.2 ns (3.8e15 operations a second), both measured on R-MAT 2^24
+// and 2^22 and Chung-Lu 2^22. The optimum is flat: steps taken at 1 or 4 ns
+// move those counts by 2%.
+constexpr int64_t kCandFs = 400;
+constexpr int64_t kStepFs = 2200000;
+// below this gain in all (20 us) the second launch is not worth it
+constexpr int64_t kCoreMinFs = int64_t(20) * 1000 * 1000 * 1000;
+
+// the kCoreSums words: tiles, items, widest J, gain in fs
+
+// J = T_b / 256 of row block blockIdx.x: four rows a warp, each lane holding
+// the benefit of two widths. A row has C(c, 2) candidates whose v lies in the
+// top T positions, c its columns there: its entries from the end on, 128 at a
+// time, go into a histogram of 256 positions a bin, whose prefix sum is c.
+// (Sixteen rows a warp, or binary searches for every width, took 190 us on
+// R-MAT 2^21: chains of misses in the widest rows' blocks.)
+__global__ void __launch_bounds__(1024) k_core_pick(int64_t nv, const int64_t *__restrict__ rstart,
+                                                    const int64_t *__restrict__ off, const uint32_t *__restrict__ cols,
+                                                    int32_t *__restrict__ jw, int32_t *__restrict__ cut,
+                                                    unsigned long long *__restrict__ gain) {
+  __shared__ unsigned long long s_ben[kCoreMaxJ];
+  __shared__ int s_hist[32][kCoreMaxJ];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int b = blockIdx.x;
+  if (threadIdx.x < kCoreMaxJ) s_ben[threadIdx.x] = 0;
+  __syncthreads();
+  unsigned long long ben0 = 0, ben1 = 0;
+  // lane l < 4 holds the warp's row l: its end and length
+  int64_t end = 0;
+  int32_t len = 0;
+  {
+    const int64_t u = nv - 1 - (int64_t(b) * kCoreRows + warp * 4 + lane);
+    if (lane < 4 && u >= 0) {
+      len = int32_t(off[u + 1] - off[u]);
+      end = rstart[u] + len;
+    }
+    if (len < kCoreMinRow) len = 0;
+  }
+  const uint32_t top = uint32_t(nv - 1);
+  for (int q = 0; q < 4; q++) {
+    const int32_t n = __shfl_sync(0xffffffffu, len, q);
+    if (n == 0) continue;
+    const uint32_t *last = cols + __shfl_sync(0xffffffffu, end, q) - 1 - lane;
+    s_hist[warp][lane] = 0;
+    s_hist[warp][lane + 32] = 0;
+    __syncwarp();
+    for (int32_t at = 0; at < n; at += 128) {
+      uint32_t x[4];
+#pragma unroll
+      for (int h = 0; h < 4; h++) x[h] = at + 32 * h + lane < n ? top - last[-(at + 32 * h)] : 0xffffffffu;
+#pragma unroll
+      for (int h = 0; h < 4; h++)
+        if (x[h] < uint32_t(kCoreWidth)) atomicAdd(&s_hist[warp][x[h] / kCoreStep], 1);
+      if (!__any_sync(0xffffffffu, x[3] < uint32_t(kCoreWidth))) break;
+    }
+    __syncwarp();
+    int c0 = s_hist[warp][lane], c1 = s_hist[warp][lane + 32];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a0 = __shfl_up_sync(0xffffffffu, c0, o), a1 = __shfl_up_sync(0xffffffffu, c1, o);
+      if (lane >= o) {
+        c0 += a0;
+        c1 += a1;
+      }
+    }
+    c1 += __shfl_sync(0xffffffffu, c0, 31);
+    ben0 += (unsigned long long)c0 * (unsigned long long)(c0 - (c0 > 0)) / 2;
+    ben1 += (unsigned long long)c1 * (unsigned long long)(c1 - (c1 > 0)) / 2;
+    __syncwarp();
+  }
+  if (ben0) atomicAdd(&s_ben[lane], ben0);
+  if (ben1) atomicAdd(&s_ben[lane + 32], ben1);
+  __syncthreads();
+  if (warp != 0) return;
+  const int jmax = b / 2 + 1;  // the rows' own positions bound their columns
+  long long best = 0;
+  int bj = 0;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int j = lane + 32 * h + 1;
+    const unsigned long long ben = s_ben[j - 1];
+    // item i of the block runs 2 i + 2 chunk steps; reading its accumulator
+    // and building its operand cost about two more
+    const long long net = (long long)(ben * kCandFs) - (long long)(int64_t(j) * (j + 3) * kStepFs);
+    if (j <= jmax && net > best) {
+      best = net;
+      bj = j;
+    }
+  }
+  for (int o = 16; o; o >>= 1) {
+    const long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oj = __shfl_xor_sync(0xffffffffu, bj, o);
+    if (ob > best || (ob == best && oj < bj)) {
+      best = ob;
+      bj = oj;
+    }
+  }
+  if (lane == 0) {
+    jw[b] = bj;
+    const int64_t c = nv - int64_t(bj) * kCoreStep;
+    cut[b] = bj ? int32_t(c > 0 ? c : 0) : 0x7fffffff;
+    if (best > 0) atomicAdd(gain, (unsigned long long)best);
+  }
+}
+
+// chunks stored for row block b: a core row's own columns (an even number of
+// chunks, so that an item reads whole pairs), any other's width
+__device__ __forceinline__ int core_chunks(int b, int j, int jtop) { return b < 2 * jtop ? (b | 1) + 1 : 2 * j; }
+
+// Tile and item offsets of the nb row blocks (one CTA, at most 8 blocks a
+// thread; tiles and items scanned as the halves of one 64-bit sum).
+__global__ void __launch_bounds__(1024) k_core_layout(int nb, const int32_t *__restrict__ jw,
+                                                      int64_t *__restrict__ tile0, int32_t *__restrict__ item0,
+                                                      int64_t *__restrict__ sums) {
+  using Scan = cub::BlockScan<unsigned long long, 1024>;
+  __shared__ typename Scan::TempStorage ts;
+  __shared__ int s_top;
+  constexpr int kPer = kCoreMaxBlk / 1024;
+  if (threadIdx.x == 0) s_top = 0;
+  __syncthreads();
+  int j[kPer], top = 0;
+#pragma unroll
+  for (int i = 0; i < kPer; i++) {
+    const int b = threadIdx.x * kPer + i;
+    j[i] = b < nb ? jw[b] : 0;
+    top = max(top, j[i]);
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0 && top) atomicMax(&s_top, top);
+  __syncthreads();
+  top = s_top;
+  unsigned long long own = 0, at, tot;
+#pragma unroll
+  for (int i = 0; i < kPer; i++) {
+    const int b = threadIdx.x * kPer + i;
+    if (b < nb) own += (unsigned long long)core_chunks(b, j[i], top) << 32 | (unsigned long long)j[i];
+  }
+  Scan(ts).ExclusiveSum(own, at, tot);
+#pragma unroll
+  for (int i = 0; i < kPer; i++) {
+    const int b = threadIdx.x * kPer + i;
+    if (b >= nb) break;
+    tile0[b] = int64_t(at >> 32);
+    item0[b] = int32_t(at & 0xffffffffu);
+    at += (unsigned long long)core_chunks(b, j[i], top) << 32 | (unsigned long long)j[i];
+  }
+  if (threadIdx.x == 0) {
+    tile0[nb] = int64_t(tot >> 32);
+    sums[0] = int64_t(tot >> 32);
+    sums[1] = int64_t(tot & 0xffffffffu);
+    sums[2] = top;
+  }
+}
+
+// Work items (row block, column step): groups of 32 row blocks, within one the
+// longest items first, so the CTAs that run together share the operand of
+// their columns and the last ones are short.
+__global__ void k_core_items(int nb, const int32_t *__restrict__ jw, const int32_t *__restrict__ item0,
+                             int2 *__restrict__ items) {
+  const int lane = threadIdx.x & 31;
+  const int b = (blockIdx.x * blockDim.x + threadIdx.x);
+  if ((b & ~31) >= nb) return;
+  const int j = b < nb ? jw[b] : 0;
+  int at = __shfl_sync(0xffffffffu, b < nb ? item0[b] : 0, 0);
+  for (int t = kCoreMaxJ - 1; t >= 0; t--) {
+    const unsigned m = __ballot_sync(0xffffffffu, j > t);
+    if (j > t) items[at + __popc(m & ((1u << lane) - 1u))] = make_int2(b, t);
+    at += __popc(m);
+  }
+}
+
+// The operand tiles, two chunks (32 KB) per CTA, set in shared memory and
+// written out whole: two threads a row set the row's bytes from the first of
+// its positions in these chunks (the positions ascend from the row's end).
+__global__ void __launch_bounds__(256) k_core_tiles(int64_t nv, int nb, const int64_t *__restrict__ off,
+                                                    const int32_t *__restrict__ col,
+                                                    const int64_t *__restrict__ tile0, uint8_t *__restrict__ tiles) {
+  __shared__ __align__(16) uint8_t s_t[2 * kCoreTile];
+  const int lane = threadIdx.x & 31, r = threadIdx.x >> 1;
+  const int64_t t = 2 * int64_t(blockIdx.x);
+  for (int i = threadIdx.x; i < 2 * kCoreTile / 16; i += 256)
+    reinterpret_cast<int4 *>(s_t)[i] = make_int4(0, 0, 0, 0);
+  int b = 0, end = nb;  // the row block holding tile t, by 32-way steps
+  while (end - b > 1) {
+    const int w = (end - b + 31) / 32, x = b + lane * w;
+    const unsigned m = __ballot_sync(0xffffffffu, x < end && tile0[x] <= t);
+    b += (31 - __clz(int(m))) * w;
+    end = min(end, b + w);
+  }
+  const int64_t c0 = (t - tile0[b]) * kCoreRows;  // first position of these columns
+  const int64_t u = nv - 1 - (int64_t(b) * kCoreRows + r);
+  __syncthreads();
+  if (u >= 0) {
+    const int64_t e0 = off[u], e1 = off[u + 1];
+    int64_t lo = e0, hi = e1;  // entries [e0, lo) lie at positions >= c0
+    while (lo < hi) {
+      const int64_t mid = (lo + hi) >> 1;
+      if (nv - 1 - int64_t(col[mid]) >= c0) lo = mid + 1;
+      else hi = mid;
+    }
+    for (int64_t p = lo - 1 - (threadIdx.x & 1); p >= e0; p -= 2) {
+      const int64_t c = nv - 1 - int64_t(col[p]) - c0;
+      if (c >= kCoreStep) break;
+      const int x = int(c) & 127;
+      s_t[(int(c) >> 7) * kCoreTile + r * 128 + (((x >> 4) ^ (r & 7)) << 4) + (x & 15)] = 1;
+    }
+  }
+  __syncthreads();
+  int4 *out = reinterpret_cast<int4 *>(tiles + t * kCoreTile);
+  for (int i = threadIdx.x; i < 2 * kCoreTile / 16; i += 256) out[i] = reinterpret_cast<int4 *>(s_t)[i];
+}
+
+// ---- the product --------------------------------------------------------------
+
+constexpr int kCoreStages = 4;
+constexpr int kCoreStageBytes = 3 * kCoreTile;  // 128 rows of X, 256 rows of the core
+constexpr int kCoreThreads = 192;
+constexpr size_t kCoreSmem = size_t(kCoreStages) * kCoreStageBytes + 1024;
+constexpr uint32_t kCoreWaitLimit = 1u << 22;
+
+struct CoreArgs {
+  const uint8_t *tiles;
+  const int64_t *tile0;
+  const int2 *items;
+  int64_t n;       // items of this launch: items[0], items[stride], ...
+  int64_t stride;
+  unsigned long long *global;
+  int *err;
+};
+
+__device__ __forceinline__ uint32_t core_smem(const void *p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void core_bar_init(uint64_t *bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(core_smem(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void core_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(core_smem(bar)) : "memory");
+}
+__device__ __forceinline__ void core_expect(uint64_t *bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(core_smem(bar)), "r"(bytes)
+               : "memory");
+}
+// waits for the barrier's phase, at most kCoreWaitLimit tries; gives up early
+// once another warp of the CTA has
+__device__ __forceinline__ bool core_wait(uint64_t *bar, uint32_t parity, volatile int *fail) {
+  for (uint32_t it = 0; it < kCoreWaitLimit; it++) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(core_smem(bar)), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if ((it & 255u) == 255u && *fail) return false;
+  }
+  *fail = 1;
+  return false;
+}
+__device__ __forceinline__ void core_copy(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   core_smem(dst)),
+               "l"(src), "r"(bytes), "r"(core_smem(bar))
+               : "memory");
+}
+// 128-byte-swizzled K-major operand at a 1,024-byte aligned shared address:
+// 8-row groups 1,024 bytes apart
+__device__ __forceinline__ uint64_t core_desc(uint32_t saddr) {
+  return uint64_t((saddr & 0x3ffffu) >> 4) | (uint64_t(1) << 16) | (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) |
+         (uint64_t(2) << 61);
+}
+__device__ __forceinline__ void core_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(uint32_t(acc))
+      : "memory");
+}
+__device__ __forceinline__ void core_commit(uint64_t *bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(core_smem(bar))
+               : "memory");
+}
+// 32 columns of this warp's 32 accumulator rows
+__device__ __forceinline__ void core_ld32(uint32_t taddr, int32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(taddr));
+}
+
+// One persistent CTA per SM. Warp 0 brings in the tiles of each chunk step,
+// warp 1 issues the products of unsigned bytes into one of two 256-column
+// accumulators (32-bit integers: exact), warps 2 to 5 read the other, multiply
+// it by X[u][v] (the item's last two chunks of X) and sum. Bound by the tile
+// reads from L2: 48 KB a step against 512 cycles of tensor work.
+__global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *st = smem_raw + ((1024 - (core_smem(smem_raw) & 1023)) & 1023);
+  __shared__ __align__(8) uint64_t s_full[kCoreStages], s_empty[kCoreStages], s_tfull[2], s_tempty[2], s_drain;
+  __shared__ uint32_t s_tmem;
+  __shared__ int s_fail;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kCoreStages; i++) {
+      core_bar_init(&s_full[i], 1);
+      core_bar_init(&s_empty[i], 1);
+    }
+    for (int i = 0; i < 2; i++) {
+      core_bar_init(&s_tfull[i], 1);
+      core_bar_init(&s_tempty[i], 4);
+    }
+    core_bar_init(&s_drain, 1);
+    s_fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(core_smem(&s_tmem)),
+                 "r"(512u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = s_tmem;
+  volatile int *fail = &s_fail;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      uint32_t k = 0;  // loads issued
+      for (int64_t i = blockIdx.x; i < a.n && !*fail; i += gridDim.x) {
+        const int2 it = a.items[i * a.stride];
+        const uint8_t *x = a.tiles + a.tile0[it.x] * kCoreTile;
+        const uint8_t *y0 = a.tiles + a.tile0[2 * it.y] * kCoreTile, *y1 = a.tiles + a.tile0[2 * it.y + 1] * kCoreTile;
+        const int steps = 2 * it.y + 2;
+        for (int c = 0; c < steps; c++, k++) {
+          const uint32_t sg = k % kCoreStages, ph = (k / kCoreStages) & 1u;
+          if (!core_wait(&s_empty[sg], ph ^ 1u, fail)) break;
+          uint8_t *d = st + sg * kCoreStageBytes;
+          core_expect(&s_full[sg], kCoreStageBytes);
+          core_copy(d, x + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
+          core_copy(d + kCoreTile, y0 + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
+          core_copy(d + 2 * kCoreTile, y1 + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
+        }
+      }
+      if (*fail)  // the copies in flight land before the CTA leaves
+        for (uint32_t q = k > kCoreStages ? k - kCoreStages : 0; q < k; q++) {
+          int quiet = 0;
+          core_wait(&s_full[q % kCoreStages], (q / kCoreStages) & 1u, &quiet);
+        }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = (2u << 4) | (uint32_t(kCoreStep / 8) << 17) | (uint32_t(kCoreRows / 16) << 24);
+      uint32_t k = 0, t = 0;
+      for (int64_t i = blockIdx.x; i < a.n && !*fail; i += gridDim.x, t++) {
+        const int steps = 2 * a.items[i * a.stride].y + 2;
+        if (!core_wait(&s_tempty[t & 1], ((t >> 1) & 1u) ^ 1u, fail)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t d = tmem + (t & 1) * kCoreStep;
+        bool ok = true;
+        for (int c = 0; c < steps; c++, k++) {
+          const uint32_t sg = k % kCoreStages;
+          if (!core_wait(&s_full[sg], (k / kCoreStages) & 1u, fail)) {
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t sa = core_smem(st + sg * kCoreStageBytes);
+          const uint64_t da = core_desc(sa), db = core_desc(sa + kCoreTile);
+#pragma unroll
+          for (int q = 0; q < 4; q++)  // 32 of the chunk's 128 columns each
+            core_mma(d, da + 2 * q, db + 2 * q, idesc, c > 0 || q > 0);
+          core_commit(&s_empty[sg]);
+        }
+        if (!ok) break;
+        core_commit(&s_tfull[t & 1]);
+      }
+      core_commit(&s_drain);  // every product issued is done before the accumulators are given back
+      int quiet = 0;
+      core_wait(&s_drain, 0, &quiet);
+    }
+    __syncwarp();
+  } else {
+    const int quad = warp & 3, r = quad * 32 + lane;  // this warp's accumulator rows
+    int64_t acc = 0;
+    uint32_t t = 0;
+    for (int64_t i = blockIdx.x; i < a.n; i += gridDim.x, t++) {
+      const int2 it = a.items[i * a.stride];
+      const uint8_t *x = a.tiles + (a.tile0[it.x] + 2 * it.y) * kCoreTile + r * 128;
+      uint4 m[16];  // X[u][v] of the item's 256 columns
+#pragma unroll
+      for (int q = 0; q < 16; q++)
+        m[q] = __ldg(reinterpret_cast<const uint4 *>(x + (q >> 3) * kCoreTile + (((q & 7) ^ (r & 7)) << 4)));
+      if (!__all_sync(0xffffffffu, core_wait(&s_tfull[t & 1], (t >> 1) & 1u, fail))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      int32_t sum = 0;
+#pragma unroll
+      for (int g = 0; g < kCoreStep / 32; g++) {
+        int32_t v[32];
+        core_ld32(tmem + (t & 1) * kCoreStep + g * 32 + (uint32_t(quad * 32) << 16), v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int h = 0; h < 8; h++) {
+          const uint4 &q = m[2 * g + (h >> 2)];
+          const uint32_t w = (h & 3) == 0 ? q.x : (h & 3) == 1 ? q.y : (h & 3) == 2 ? q.z : q.w;
+          sum += int32_t(w & 0xffu) * v[4 * h] + int32_t((w >> 8) & 0xffu) * v[4 * h + 1] +
+                 int32_t((w >> 16) & 0xffu) * v[4 * h + 2] + int32_t(w >> 24) * v[4 * h + 3];
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) core_arrive(&s_tempty[t & 1]);
+      acc += sum;
+    }
+    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0 && acc) atomicAdd(a.global, (unsigned long long)acc);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+  if (threadIdx.x == 0 && s_fail && a.err) atomicOr(a.err, kErrCoreTimeout);
+}
+
+// ---- host side ------------------------------------------------------------------
+
+// Widths of the row blocks from the unique rows (row u: cols[rstart[u]] on, as
+// many as off says), and their layout; *d_sums has kCoreSums words once the
+// stream gets there. Leaves g->core empty (and *d_sums null) for graphs that
+// cannot gain.
+xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *cols, int64_t m, int64_t **d_sums) {
+  *d_sums = nullptr;
+  Core &k = g->core;
+  // m edges have at most (2m)^1.5 / 6 candidates: below 2^17 edges, less than the least gain
+  if (g->no_core || m < (int64_t(1) << 17)) return XT_OK;
+  const int64_t blocks = (g->nv + kCoreRows - 1) / kCoreRows;
+  k.nb = int(std::max<int64_t>(kCoreMinBlk, std::min<int64_t>(blocks, kCoreMaxBlk)));
+  // one allocation for the row blocks' tables: tile0, then jw, cut, item0
+  XT_TRY(dalloc_n(c, &k.d_tile0, size_t(k.nb + 1) + size_t(3 * k.nb + 1) / 2));
+  k.d_jw = reinterpret_cast<int32_t *>(k.d_tile0 + k.nb + 1);
+  k.d_cut = k.d_jw + k.nb;
+  k.d_item0 = k.d_cut + k.nb;
+  XT_TRY(dalloc_n(c, d_sums, kCoreSums));
+  XT_CUDA(c, cudaMemsetAsync(*d_sums, 0, kCoreSums * sizeof(int64_t), c->stream));
+  k_core_pick<<<counted(c, dim3(k.nb)), 1024, 0, c->stream>>>(g->nv, rstart, g->d_off, cols, k.d_jw, k.d_cut,
+                                                             reinterpret_cast<unsigned long long *>(*d_sums) + 3);
+  k_core_layout<<<counted(c, dim3(1)), 1024, 0, c->stream>>>(k.nb, k.d_jw, k.d_tile0, k.d_item0, *d_sums);
+  XT_CUDA(c, cudaGetLastError());
+  return XT_OK;
+}
+
+// sums read back: keeps the core (its memory allocated) or drops it
+xt_status core_decide(Ctx *c, Graph *g, const int64_t *sums) {
+  Core &k = g->core;
+  if (k.nb == 0) return XT_OK;
+  if (sums[3] < kCoreMinFs || sums[1] == 0) {
+    core_free(g);
+    return XT_OK;
+  }
+  k.n_tiles = sums[0];
+  k.n_items = sums[1];
+  XT_TRY(dalloc_n(c, &k.d_tiles, size_t(sums[0]) * kCoreTile));
+  return dalloc_n(c, &k.d_items, size_t(sums[1]));
+}
+
+// operands and work items from the finished out-CSR
+xt_status core_finish(Ctx *c, Graph *g) {
+  Core &k = g->core;
+  if (k.n_items == 0) return XT_OK;
+  k_core_tiles<<<counted(c, dim3(unsigned(k.n_tiles / 2))), 256, 0, c->stream>>>(g->nv, k.nb, g->d_off, g->d_col,
+                                                                                 k.d_tile0, k.d_tiles);
+  k_core_items<<<counted(c, dim3(unsigned((k.nb + 255) / 256))), 256, 0, c->stream>>>(k.nb, k.d_jw, k.d_item0,
+                                                                                     k.d_items);
+  XT_CUDA(c, cudaGetLastError());
+  XT_CUDA(c, cudaFuncSetAttribute(k_core_count, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCoreSmem)));
+  return XT_OK;
+}
+
+// adds the core's triangles of every nshards-th item from `shard` to *d_global
+xt_status core_count(Graph *g, int64_t *d_global, int shard, int nshards) {
+  Ctx *c = g->ctx;
+  const Core &k = g->core;
+  if (k.n_items <= shard) return XT_OK;
+  CoreArgs a;
+  a.tiles = k.d_tiles;
+  a.tile0 = k.d_tile0;
+  a.items = k.d_items + shard;
+  a.n = (k.n_items - shard + nshards - 1) / nshards;
+  a.stride = nshards;
+  a.global = reinterpret_cast<unsigned long long *>(d_global);
+  a.err = c->d_err;
+  const unsigned grid = unsigned(std::min<int64_t>(a.n, c->sm_count));
+  k_core_count<<<counted(c, dim3(grid)), kCoreThreads, kCoreSmem, c->stream>>>(a);
+  XT_CUDA(c, cudaGetLastError());
+  return XT_OK;
+}
+
+void core_free(Graph *g) {
+  Core &k = g->core;
+  for (void *p : {(void *)k.d_tile0, (void *)k.d_tiles, (void *)k.d_items}) dfree(g->ctx, p);
+  g->core = Core{};
+}
+
+}  // namespace xt

@@ -186,37 +186,45 @@ struct RecLen {
 // Graph statistics in one pass over the vertices: st[0] the largest degree
 // (out + in), st[1] the largest out-degree, st[2] the largest in-degree,
 // st[3] the tail-grouped work sum over edges u->v of d+(v) = sum over v of
-// d-(v) d+(v)
-__global__ void k_vertex_stats(const int64_t *__restrict__ off, const int64_t *__restrict__ ioff, int64_t nv,
+// d-(v) d+(v); st[4] the candidates of the records up to iend[v] (P: the
+// records' prefix sum)
+__global__ void __launch_bounds__(256) k_vertex_stats(const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
+                               const int64_t *__restrict__ iend, const int64_t *__restrict__ P, int64_t nv,
                                unsigned long long *__restrict__ st) {
-  unsigned long long md = 0, mo = 0, mi = 0, wsum = 0;
+  unsigned long long md = 0, mo = 0, mi = 0, wsum = 0, live = 0;
   XT_GRID_STRIDE(i, nv) {
     const unsigned long long dout = off[i + 1] - off[i], din = ioff[i + 1] - ioff[i];
     md = max(md, dout + din);
     mo = max(mo, dout);
     mi = max(mi, din);
     wsum += dout * din;
+    live += (unsigned long long)(P[iend[i]] - P[ioff[i]]);
   }
-  for (int o = 16; o; o >>= 1) {
-    md = max(md, __shfl_xor_sync(0xffffffffu, md, o));
-    mo = max(mo, __shfl_xor_sync(0xffffffffu, mo, o));
-    mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, o));
-    wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
+  // one atomic a CTA and word: with one a warp, 38,000 warps queued at these
+  // five words (88 us on a graph of 2^20 vertices)
+  using Red = cub::BlockReduce<unsigned long long, 256>;
+  __shared__ typename Red::TempStorage ts[5];
+  const auto larger = [](unsigned long long a, unsigned long long b) { return a > b ? a : b; };
+  md = Red(ts[0]).Reduce(md, larger);
+  mo = Red(ts[1]).Reduce(mo, larger);
+  mi = Red(ts[2]).Reduce(mi, larger);
+  wsum = Red(ts[3]).Sum(wsum);
+  live = Red(ts[4]).Sum(live);
+  if (threadIdx.x == 0) {
     atomicMax(&st[0], md);
     atomicMax(&st[1], mo);
     atomicMax(&st[2], mi);
     atomicAdd(&st[3], wsum);
+    atomicAdd(&st[4], live);
   }
 }
 
 // tasks of head v: nb CTA tasks (parts x chunks), nw warp tasks, nt lane tasks (0 or 1 each)
 __device__ __forceinline__ void classify(int64_t v, const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
-                                         const int64_t *__restrict__ P, const PlanParams pp, int64_t &nb,
+                                         const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp, int64_t &nb,
                                          int64_t &nw, int64_t &nt, int64_t &parts, int64_t &chunks, int64_t &work) {
   const int64_t dp = off[v + 1] - off[v];
-  const int64_t k0 = ioff[v], k1 = ioff[v + 1];
+  const int64_t k0 = ioff[v], k1 = iend[v];
   nb = nw = nt = parts = chunks = 0;
   work = P[k1] - P[k0];
   if (dp == 0 || work == 0) return;
@@ -234,11 +242,11 @@ __device__ __forceinline__ void classify(int64_t v, const int64_t *__restrict__ 
 }
 
 __global__ void k_plan_count(int64_t nv, const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
-                             const int64_t *__restrict__ P, const PlanParams pp, int64_t *__restrict__ nb_out,
+                             const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp, int64_t *__restrict__ nb_out,
                              int64_t *__restrict__ nw_out, int64_t *__restrict__ nt_out) {
   XT_GRID_STRIDE(v, nv) {
     int64_t nb, nw, nt, parts, chunks, work;
-    classify(v, off, ioff, P, pp, nb, nw, nt, parts, chunks, work);
+    classify(v, off, ioff, iend, P, pp, nb, nw, nt, parts, chunks, work);
     nb_out[v] = nb;
     nw_out[v] = nw;
     nt_out[v] = nt;
@@ -281,26 +289,30 @@ __device__ __forceinline__ Task make_task(int64_t v, int64_t k0, int64_t k1, int
 }
 
 __global__ void k_plan_fill(int64_t nv, const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
-                            const int64_t *__restrict__ P, const PlanParams pp, const int64_t *__restrict__ nb_pos,
+                            const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp, const int64_t *__restrict__ nb_pos,
                             const int64_t *__restrict__ nw_pos, const int64_t *__restrict__ nt_pos,
                             Task *__restrict__ bt, Task *__restrict__ wt, int32_t *__restrict__ tt) {
   XT_GRID_STRIDE(v, nv) {
     int64_t nb, nw, nt, parts, chunks, work;
-    classify(v, off, ioff, P, pp, nb, nw, nt, parts, chunks, work);
-    const int64_t k0 = ioff[v], k1 = ioff[v + 1];
+    classify(v, off, ioff, iend, P, pp, nb, nw, nt, parts, chunks, work);
+    const int64_t k0 = ioff[v], k1 = iend[v];
     if (nt) tt[nt_pos[v]] = int32_t(v);
     if (nw) {
       // The lanes per record that take the warp the fewest steps. Records
       // are stored longest first, so a batch of 32 / S records runs as many
       // steps as its first record needs on S lanes (its pairs: the suffix
       // length plus an average offset into its first pair, over 8); each
-      // batch also costs about one step of set-up.
+      // batch also costs about one step of set-up. Heads of many records are
+      // sampled, at most 64 batches for each choice (one thread walking all
+      // of a head's 4,000 short records held the R-MAT 2^18 plan for 440 us).
       int32_t lg_s = 0;
       int64_t best = INT64_MAX;
       for (int32_t ls = 0; ls <= 5; ls++) {
         const int64_t B = int64_t(32) >> ls, S = int64_t(1) << ls;
+        const int64_t every = ((k1 - k0) / B + 63) / 64, skip = B * (every > 1 ? every : 1);
         int64_t steps = 0;
-        for (int64_t i = k0; i < k1; i += B) steps += 1 + ((P[i + 1] - P[i] + 11) / 8 + S - 1) / S;
+        for (int64_t i = k0; i < k1; i += skip) steps += 1 + ((P[i + 1] - P[i] + 11) / 8 + S - 1) / S;
+        steps *= skip / B;
         if (steps < best) {
           best = steps;
           lg_s = ls;
@@ -351,11 +363,11 @@ __global__ void k_task_gather(const Task *__restrict__ bt, const int32_t *__rest
 // members): parts of kClusterDmax members x chunks of kCluster * block_work
 // items. Returns how many (0 for every other head).
 __device__ __forceinline__ int64_t cluster_tasks(int64_t v, const int64_t *__restrict__ off,
-                                                 const int64_t *__restrict__ ioff, const int64_t *__restrict__ P,
-                                                 const PlanParams pp, int64_t &parts, int64_t &chunks,
+                                                 const int64_t *__restrict__ ioff, const int64_t *__restrict__ iend,
+                                                 const int64_t *__restrict__ P, const PlanParams pp, int64_t &parts, int64_t &chunks,
                                                  int64_t &work) {
   int64_t nb, nw, nt, bparts, bchunks;
-  classify(v, off, ioff, P, pp, nb, nw, nt, bparts, bchunks, work);
+  classify(v, off, ioff, iend, P, pp, nb, nw, nt, bparts, bchunks, work);
   parts = chunks = 0;
   if (nb == 0 || bparts <= 1) return 0;
   parts = (off[v + 1] - off[v] + kClusterDmax - 1) / kClusterDmax;
@@ -365,21 +377,21 @@ __device__ __forceinline__ int64_t cluster_tasks(int64_t v, const int64_t *__res
 }
 
 __global__ void k_plan_ccount(int64_t nv, const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
-                              const int64_t *__restrict__ P, const PlanParams pp, int64_t *__restrict__ nc_out) {
+                              const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp, int64_t *__restrict__ nc_out) {
   XT_GRID_STRIDE(v, nv) {
     int64_t parts, chunks, work;
-    nc_out[v] = cluster_tasks(v, off, ioff, P, pp, parts, chunks, work);
+    nc_out[v] = cluster_tasks(v, off, ioff, iend, P, pp, parts, chunks, work);
   }
 }
 
 __global__ void k_plan_cfill(int64_t nv, const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
-                             const int64_t *__restrict__ P, const PlanParams pp, const int64_t *__restrict__ nc_pos,
+                             const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp, const int64_t *__restrict__ nc_pos,
                              Task *__restrict__ ct) {
   XT_GRID_STRIDE(v, nv) {
     int64_t parts, chunks, work;
-    const int64_t n = cluster_tasks(v, off, ioff, P, pp, parts, chunks, work);
+    const int64_t n = cluster_tasks(v, off, ioff, iend, P, pp, parts, chunks, work);
     if (!n) continue;
-    const int64_t k0 = ioff[v], k1 = ioff[v + 1], base = P[k0];
+    const int64_t k0 = ioff[v], k1 = iend[v], base = P[k0];
     int64_t t = nc_pos[v], prev = k0;
     for (int64_t c = 0; c < chunks; c++) {
       const int64_t kend = (c + 1 == chunks) ? k1 : lower_bound_i64(P, prev, k1, base + (work * (c + 1)) / chunks);
@@ -910,6 +922,7 @@ struct CountArgs {
   const int32_t *colp;  // padded columns (suffixes are streamed from here)
   const int64_t *poff;  // padded row starts
   const int64_t *ioff;
+  const int64_t *iend;  // the end of each head's streamed records
   const InRec *rec;
   const int32_t *rec_u;  // the records' tails (per-vertex and per-edge modes)
   const Task *bt;  // CTA tasks
@@ -1347,7 +1360,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
       for (int j = 0; j < kLaneRegs; j++) mm[j] = (regs && j < r1 - r0) ? col[r0 + j] : -1;
       int64_t hv = 0;
       const int32_t *__restrict__ colp = a.colp;
-      for (int64_t k = ioff[v]; k < ioff[v + 1]; k++) {
+      for (int64_t k = ioff[v]; k < a.iend[v]; k++) {
         const InRec r = rec[k];
         const int64_t rs = rec_s(r), re = rs + rec_len(r);
         const int32_t ru = MODE == 1 ? a.rec_u[k] : 0;
@@ -1546,17 +1559,21 @@ static xt_status exclusive_scan(Ctx *c, const int64_t *in, int64_t *out, int64_t
   return XT_OK;
 }
 
+static void free_one_plan(Ctx *c, Plan *pl) {
+  if (!pl) return;
+  dfree(c, pl->d_bt);
+  dfree(c, pl->d_ct);
+  dfree(c, pl->d_bt0);
+  dfree(c, pl->d_wt);
+  dfree(c, pl->d_tt);
+  dfree(c, pl->d_cursor);
+  delete pl;
+}
+
 void free_plan(Graph *g) {
-  if (!g->plan) return;
-  Ctx *c = g->ctx;
-  dfree(c, g->plan->d_bt);
-  dfree(c, g->plan->d_ct);
-  dfree(c, g->plan->d_bt0);
-  dfree(c, g->plan->d_wt);
-  dfree(c, g->plan->d_tt);
-  dfree(c, g->plan->d_cursor);
-  delete g->plan;
-  g->plan = nullptr;
+  free_one_plan(g->ctx, g->plan);
+  free_one_plan(g->ctx, g->plan_all);
+  g->plan = g->plan_all = nullptr;
 }
 
 static xt_status d2h(Ctx *c, void *h, const void *d, size_t bytes) {
@@ -1565,7 +1582,8 @@ static xt_status d2h(Ctx *c, void *h, const void *d, size_t bytes) {
 
 // The cluster tasks (d_ct) and the CTA tasks of the other heads (d_bt0,
 // chunk-major order kept), and the cluster kernel's persistent grid.
-static xt_status plan_cluster(Ctx *c, Graph *g, Plan *pl, const int64_t *P, const PlanParams &pp) {
+static xt_status plan_cluster(Ctx *c, Graph *g, Plan *pl, const int64_t *iend, const int64_t *P,
+                              const PlanParams &pp) {
   const int64_t nv = g->nv;
   const int B = 256;
   int64_t *nc = nullptr, *ncp = nullptr, *d_num = nullptr;
@@ -1574,7 +1592,8 @@ static xt_status plan_cluster(Ctx *c, Graph *g, Plan *pl, const int64_t *P, cons
   do {
     if ((s = dalloc_n(c, &nc, size_t(nv + 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &ncp, size_t(nv + 1))) != XT_OK) break;
-    k_plan_ccount<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(nv, g->d_off, g->d_ioff, P, pp, nc);
+    k_plan_ccount<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(nv, g->d_off, g->d_ioff, iend, P, pp,
+                                                                                 nc);
     if ((s = cuda_status(c, cudaMemsetAsync(nc + nv, 0, sizeof(int64_t), c->stream), "memset")) != XT_OK) break;
     if ((s = exclusive_scan(c, nc, ncp, nv + 1)) != XT_OK) break;
     int64_t n = 0;
@@ -1582,7 +1601,7 @@ static xt_status plan_cluster(Ctx *c, Graph *g, Plan *pl, const int64_t *P, cons
     if ((s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync")) != XT_OK) break;
     if (n == 0) break;
     if ((s = dalloc_n(c, &pl->d_ct, size_t(n))) != XT_OK) break;
-    k_plan_cfill<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(nv, g->d_off, g->d_ioff, P, pp, ncp,
+    k_plan_cfill<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(nv, g->d_off, g->d_ioff, iend, P, pp, ncp,
                                                                                 pl->d_ct);
     if ((s = cuda_status(c, cudaGetLastError(), "k_plan_cfill")) != XT_OK) break;
     if ((s = dalloc_n(c, &pl->d_bt0, size_t(pl->n_btask))) != XT_OK) break;
@@ -1623,11 +1642,11 @@ static xt_status plan_cluster(Ctx *c, Graph *g, Plan *pl, const int64_t *P, cons
   return s;
 }
 
-xt_status make_plan(Graph *g) {
+// the schedule of the records up to iend[v] of every head
+static xt_status plan_records(Graph *g, const int64_t *iend, Plan **out) {
   Ctx *c = g->ctx;
-  free_plan(g);
   Plan *pl = new Plan();
-  g->plan = pl;
+  *out = pl;
   const int64_t nv = g->nv, ne = g->ne;
   const int B = 256;
   int64_t *P = nullptr, *nb = nullptr, *nw = nullptr, *nt = nullptr, *nbp = nullptr, *nwp = nullptr,
@@ -1636,12 +1655,11 @@ xt_status make_plan(Graph *g) {
   xt_status s = XT_OK;
   do {
     if ((s = dalloc_n(c, &pl->d_cursor, 4)) != XT_OK) break;
-    if ((s = dalloc_n(c, &stats, 4)) != XT_OK) break;
+    if ((s = dalloc_n(c, &stats, 5)) != XT_OK) break;
     if ((s = dalloc_n(c, &P, size_t(ne + 1))) != XT_OK) break;
-    if ((s = cuda_status(c, cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), c->stream), "memset")) !=
+    if ((s = cuda_status(c, cudaMemsetAsync(stats, 0, 5 * sizeof(unsigned long long), c->stream), "memset")) !=
         XT_OK)
       break;
-    k_vertex_stats<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(g->d_off, g->d_ioff, nv, stats);
     // suffix lengths, prefix-summed in head order
     {
       const auto lens = thrust::make_transform_iterator(thrust::counting_iterator<int64_t>(0), RecLen{g->d_irec, ne});
@@ -1655,6 +1673,8 @@ xt_status make_plan(Graph *g) {
       dfree(c, tmp);
       if (s != XT_OK) break;
     }
+    k_vertex_stats<<<counted(c, std::min(grid_for(nv, B, c->sm_count), unsigned(c->sm_count) * 8)), B, 0, c->stream>>>(
+        g->d_off, g->d_ioff, iend, P, nv, stats);
     // persistent grids: every CTA that fits on the device at once
     int occ[3] = {0, 0, 0};
     for (int mode = 0; mode < 3 && s == XT_OK; mode++) {
@@ -1674,7 +1694,7 @@ xt_status make_plan(Graph *g) {
     // CTA task size: large tasks amortise the member-set build and the task
     // barrier, but every CTA should still get about 16 of them
     int64_t total_work = 0;
-    if ((s = d2h(c, &total_work, P + ne, sizeof(int64_t))) != XT_OK) break;
+    if ((s = d2h(c, &total_work, stats + 4, sizeof(int64_t))) != XT_OK) break;
     if ((s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync")) != XT_OK) break;
     PlanParams pp;
     pp.warp_dmax = kWarpDmax;
@@ -1704,7 +1724,7 @@ xt_status make_plan(Graph *g) {
     if ((s = dalloc_n(c, &nwp, size_t(nv + 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &nt, size_t(nv + 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &ntp, size_t(nv + 1))) != XT_OK) break;
-    k_plan_count<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(nv, g->d_off, g->d_ioff, P, pp, nb,
+    k_plan_count<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(nv, g->d_off, g->d_ioff, iend, P, pp, nb,
                                                                                 nw, nt);
     if ((s = cuda_status(c, cudaMemsetAsync(nb + nv, 0, sizeof(int64_t), c->stream), "memset")) != XT_OK) break;
     if ((s = cuda_status(c, cudaMemsetAsync(nw + nv, 0, sizeof(int64_t), c->stream), "memset")) != XT_OK) break;
@@ -1713,7 +1733,7 @@ xt_status make_plan(Graph *g) {
     if ((s = exclusive_scan(c, nw, nwp, nv + 1)) != XT_OK) break;
     if ((s = exclusive_scan(c, nt, ntp, nv + 1)) != XT_OK) break;
     int64_t h[4] = {0, 0, 0, 0};
-    unsigned long long hs[4] = {0, 0, 0, 0};
+    unsigned long long hs[5] = {0, 0, 0, 0, 0};
     if ((s = d2h(c, &h[0], nbp + nv, sizeof(int64_t))) != XT_OK) break;
     if ((s = d2h(c, &h[1], nwp + nv, sizeof(int64_t))) != XT_OK) break;
     if ((s = d2h(c, &h[2], P + ne, sizeof(int64_t))) != XT_OK) break;
@@ -1736,7 +1756,7 @@ xt_status make_plan(Graph *g) {
     if ((s = dalloc_n(c, &pl->d_wt, size_t(pl->n_wtask > 0 ? pl->n_wtask : 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &pl->d_tt, size_t(pl->n_ttask > 0 ? pl->n_ttask : 1))) != XT_OK) break;
     k_plan_fill<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(
-        nv, g->d_off, g->d_ioff, P, pp, nbp, nwp, ntp, pl->d_bt, pl->d_wt, pl->d_tt);
+        nv, g->d_off, g->d_ioff, iend, P, pp, nbp, nwp, ntp, pl->d_bt, pl->d_wt, pl->d_tt);
     if ((s = cuda_status(c, cudaGetLastError(), "k_plan_fill")) != XT_OK) break;
     if (pl->n_btask > 1) {  // chunk-major order
       uint64_t *k1 = nullptr, *k2 = nullptr;
@@ -1775,7 +1795,7 @@ xt_status make_plan(Graph *g) {
     // global count: heads whose members overflow a CTA's set go to the
     // cluster tier instead of CTA tasks over parts of their members
     if (g->cluster_tier != 0 && g->max_out_degree > kBlockDmax && pl->n_btask > 0)
-      s = plan_cluster(c, g, pl, P, pp);
+      s = plan_cluster(c, g, pl, iend, P, pp);
   } while (0);
   dfree(c, P);
   dfree(c, nb);
@@ -1785,8 +1805,16 @@ xt_status make_plan(Graph *g) {
   dfree(c, nt);
   dfree(c, ntp);
   dfree(c, stats);
-  if (s != XT_OK) free_plan(g);
+  if (s != XT_OK) {
+    free_one_plan(c, pl);
+    *out = nullptr;
+  }
   return s;
+}
+
+xt_status make_plan(Graph *g) {
+  free_plan(g);
+  return plan_records(g, g->d_iend, &g->plan);
 }
 
 int64_t cluster_task_count(const Graph *g) { return g->plan ? g->plan->n_ctask : 0; }
@@ -1799,9 +1827,9 @@ xt_status count_status(Ctx *c) {
   int h = 0;
   XT_CUDA(c, cudaMemcpyAsync(&h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   XT_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (h & kErrStageTimeout) {
+  if (h & (kErrStageTimeout | kErrCoreTimeout)) {
     XT_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-    return set_error(c, XT_ERR_TIMEOUT, "count: a CTA's wait for its staged member list timed out");
+    return set_error(c, XT_ERR_TIMEOUT, "count: a CTA's wait for its staged data timed out");
   }
   return XT_OK;
 }
@@ -1852,7 +1880,10 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   if (nshards < 1 || shard < 0 || shard >= nshards)
     return set_error(c, XT_ERR_INVALID, "shard must lie in [0, nshards) and nshards be at least 1");
   if (!g->plan) XT_TRY(make_plan(g));
-  Plan *pl = g->plan;
+  // with a core, the per-vertex and per-edge counts stream every record
+  const bool core = g->core.n_items > 0 && !d_pv && !d_support, all = g->core.n_items > 0 && !core;
+  if (all && !g->plan_all) XT_TRY(plan_records(g, g->d_ioff + 1, &g->plan_all));
+  Plan *pl = all ? g->plan_all : g->plan;
   // pairs of columns are read with 32-byte vector loads
   if (reinterpret_cast<uintptr_t>(g->d_colp) % 32 != 0)
     return set_error(c, XT_ERR_CUDA, "padded column array is not 32-byte aligned");
@@ -1890,6 +1921,7 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   a.colp = g->d_colp;
   a.poff = g->d_poff;
   a.ioff = g->d_ioff;
+  a.iend = all ? g->d_ioff + 1 : g->d_iend;
   a.rec = g->d_irec;
   a.rec_u = g->d_irec_u;
   a.bt = shard_first(pl->d_bt, pl->n_btask, shard);
@@ -1919,6 +1951,7 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
       k_count<1, false><<<counted(c, pl->grid_pv), kThreads, count_smem_bytes(true), c->stream>>>(a);
     else {
       // cluster heads leave the CTA task list to the cluster tier
+      if (core) XT_TRY(core_count(g, d_global, shard, nshards));
       CountArgs a0 = a;
       if (pl->n_ctask > 0) {
         a0.bt = shard_first(pl->d_bt0, pl->n_btask0, shard);

@@ -99,6 +99,20 @@ __host__ __device__ inline InRec make_inrec(int64_t s, int64_t len) {
 __host__ __device__ inline int64_t rec_s(InRec r) { return (int64_t(r.pair) << 3) | int64_t(r.lw >> kRecLenBits); }
 __host__ __device__ inline int32_t rec_len(InRec r) { return int32_t(r.lw & uint32_t(kMaxRecLen - 1)); }
 
+// The graph's dense core (core.cu): operand tiles and work items of the part
+// of the count that runs on the tensor cores. Empty (n_items 0) for graphs
+// that gain nothing by it.
+struct Core {
+  int nb = 0;                 // row blocks of 128, from the highest id down
+  int64_t *d_tile0 = nullptr;  // per row block: its first operand tile (nb + 1; one allocation with the next three)
+  int32_t *d_jw = nullptr;     // ... its width / 256 (0: none)
+  int32_t *d_cut = nullptr;    // ... the first head id whose record from the block is counted here
+  int32_t *d_item0 = nullptr;  // ... its items' place in the list
+  uint8_t *d_tiles = nullptr;
+  int2 *d_items = nullptr;    // (row block, column step)
+  int64_t n_tiles = 0, n_items = 0;
+};
+
 struct Graph {
   Ctx *ctx = nullptr;
   int64_t nv = 0;
@@ -114,6 +128,11 @@ struct Graph {
   int64_t *d_ioff = nullptr;  // in-record offsets per head v, nv+1
   InRec *d_irec = nullptr;    // one record per edge u->v, grouped by v (ne + 2: the last 16 bytes are slack
                               //   for 16-byte aligned bulk prefetches)
+  // the first in-record of each head that the global count does not stream
+  // (no candidates, or the core's): nv
+  int64_t *d_iend = nullptr;
+  Core core;
+  bool no_core = false;         // the batch form counts per graph: no core
   int32_t *d_irec_u = nullptr;  // the tail u of each record, built on first use (per-vertex, per-edge)
   // The columns again, each row starting on an 8-column (32-byte) boundary
   // and padded with kPadSentinel: the count streams suffixes from here in
@@ -145,7 +164,8 @@ struct Graph {
   int64_t wedge_work = 0;   // sum over oriented (u,v) of d+(v)
   int64_t stream_work = 0;  // sum over u of C(d+(u), 2): the suffix columns the count streams
   int64_t colp_len = 0;     // entries of the padded column array
-  Plan *plan = nullptr;
+  Plan *plan = nullptr;      // the global count's schedule
+  Plan *plan_all = nullptr;  // every record's schedule (per-vertex and per-edge counts of a graph with a core)
 };
 
 // Optional: the rows still in host memory. build_from_edges then copies
@@ -173,6 +193,17 @@ xt_status build_from_vite(Ctx *c, const char *path, int elem_bytes, bool canonic
 // rows with graph-local ids) as one graph with a per-vertex group map.
 xt_status build_batch(Ctx *c, int64_t ng, const int64_t *h_voff, const int64_t *h_eoff, const int32_t *d_src,
                       const int32_t *d_dst, int orient, Graph *g);
+
+// The dense core (core.cu), in the builder's order: widths chosen from the
+// unique rows, kept or dropped once their sums are read back, then operands
+// and items from the finished graph; its part of a count.
+constexpr int kCoreSums = 4;
+constexpr int kErrCoreTimeout = 16;  // bit of the context's error word: a bounded wait of the core's kernel gave up
+xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *cols, int64_t m, int64_t **d_sums);
+xt_status core_decide(Ctx *c, Graph *g, const int64_t *sums);
+xt_status core_finish(Ctx *c, Graph *g);
+xt_status core_count(Graph *g, int64_t *d_global, int shard, int nshards);
+void core_free(Graph *g);
 
 // Builds (or rebuilds) the per-graph schedule and graph statistics.
 xt_status make_plan(Graph *g);
