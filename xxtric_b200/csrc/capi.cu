@@ -91,8 +91,12 @@ const char *xt_strerror(xt_status s) {
 
 const char *xt_last_error(const xt_ctx *ctx) { return ctx ? ctx->c.last_error.c_str() : "null context"; }
 
-xt_status xt_open(int device, xt_ctx **out) {
-  if (!out) return XT_ERR_INVALID;
+// A context on `device` (made current): on the given stream, or on one of its
+// own. Only the attributes it needs are read (cudaGetDeviceProperties takes 5
+// to 190 ms on these hosts, more than a small graph's whole build and count),
+// and its result block comes from the stream-ordered pool, so opening a context
+// waits for no other stream's work.
+static xt_status open_ctx(int device, bool own_stream, cudaStream_t stream, xt_ctx **out) {
   *out = nullptr;
   int n = 0;
   if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0) {
@@ -100,34 +104,49 @@ xt_status xt_open(int device, xt_ctx **out) {
     return XT_ERR_NO_DEVICE;
   }
   if (device < 0 || device >= n) return XT_ERR_INVALID;
-  cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return XT_ERR_CUDA;
-  if (prop.major < 10) return XT_ERR_NO_DEVICE;  // built for sm_100a only
+  int major = 0, sms = 0;
+  if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+    cudaGetLastError();
+    return XT_ERR_CUDA;
+  }
+  if (major < 10) return XT_ERR_NO_DEVICE;  // built for sm_100a only
   if (cudaSetDevice(device) != cudaSuccess) return XT_ERR_CUDA;
   xt_ctx *ctx = new (std::nothrow) xt_ctx();
   if (!ctx) return XT_ERR_OOM;
   Ctx *c = &ctx->c;
   c->device = device;
-  c->sm_count = prop.multiProcessorCount;
-  c->smem_optin = prop.sharedMemPerBlockOptin;
-  if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
+  c->sm_count = sms;
+  c->stream = stream;
+  if (own_stream && cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete ctx;
     return XT_ERR_CUDA;
   }
-  c->own_stream = true;
+  c->own_stream = own_stream;
   // keep freed pool memory cached: graphs are rebuilt and counted repeatedly
   cudaMemPool_t pool;
   if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
     uint64_t thr = UINT64_MAX;
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
   }
-  if (cudaMalloc(&c->d_err, sizeof(int)) != cudaSuccess || cudaMemset(c->d_err, 0, sizeof(int)) != cudaSuccess) {
-    cudaStreamDestroy(c->stream);
+  void *blk = nullptr;
+  if (cudaMallocAsync(&blk, sizeof(CountOut), c->stream) != cudaSuccess ||
+      cudaMemsetAsync(blk, 0, sizeof(CountOut), c->stream) != cudaSuccess) {
+    cudaGetLastError();
+    if (blk) cudaFreeAsync(blk, c->stream);
+    if (own_stream) cudaStreamDestroy(c->stream);
     delete ctx;
     return XT_ERR_CUDA;
   }
+  c->d_out = static_cast<CountOut *>(blk);
+  c->d_err = &c->d_out->err;
   *out = ctx;
   return XT_OK;
+}
+
+xt_status xt_open(int device, xt_ctx **out) {
+  if (!out) return XT_ERR_INVALID;
+  return open_ctx(device, true, nullptr, out);
 }
 
 xt_status xt_close(xt_ctx *ctx) {
@@ -135,7 +154,10 @@ xt_status xt_close(xt_ctx *ctx) {
   Ctx *c = &ctx->c;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  cudaFree(c->d_err);
+  if (cudaFreeAsync(c->d_out, c->stream) != cudaSuccess) {  // e.g. a caller's stream that is gone
+    cudaGetLastError();
+    cudaFree(c->d_out);
+  }
   if (c->copy_stream) {
     cudaStreamSynchronize(c->copy_stream);
     cudaStreamDestroy(c->copy_stream);
@@ -344,16 +366,13 @@ xt_status xt_count(xt_graph *gr, int64_t *global, int64_t *per_vertex) {
   Ctx *c = g.ctx;
   cudaSetDevice(c->device);
   int64_t *d = nullptr;
-  XT_TRY(dalloc_n(c, &d, size_t(1 + (per_vertex ? g.nv : 0))));
-  xt_status s = count_graph(&g, d, per_vertex ? d + 1 : nullptr);
-  if (s == XT_OK)
-    s = cuda_status(c, cudaMemcpyAsync(global, d, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream), "D2H");
+  if (per_vertex) XT_TRY(dalloc_n(c, &d, size_t(g.nv)));
+  xt_status s = count_graph(&g, &c->d_out->total, d);
   if (s == XT_OK && per_vertex)
-    s = cuda_status(c, cudaMemcpyAsync(per_vertex, d + 1, sizeof(int64_t) * g.nv, cudaMemcpyDeviceToHost, c->stream),
+    s = cuda_status(c, cudaMemcpyAsync(per_vertex, d, sizeof(int64_t) * g.nv, cudaMemcpyDeviceToHost, c->stream),
                     "D2H");
   dfree(c, d);
-  if (s == XT_OK) s = cuda_status(c, cudaStreamSynchronize(c->stream), "count");
-  if (s == XT_OK) s = count_status(c);
+  if (s == XT_OK) s = count_status(c, global);
   return s;
 }
 
@@ -363,16 +382,13 @@ xt_status xt_count_edges(xt_graph *gr, int64_t *global, int64_t *support) {
   Ctx *c = g.ctx;
   cudaSetDevice(c->device);
   int64_t *d = nullptr;
-  XT_TRY(dalloc_n(c, &d, size_t(1 + g.ne)));
-  xt_status s = count_graph(&g, d, nullptr, nullptr, d + 1);
-  if (s == XT_OK)
-    s = cuda_status(c, cudaMemcpyAsync(global, d, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream), "D2H");
+  XT_TRY(dalloc_n(c, &d, size_t(g.ne > 0 ? g.ne : 1)));
+  xt_status s = count_graph(&g, &c->d_out->total, nullptr, nullptr, d);
   if (s == XT_OK && g.ne > 0)
-    s = cuda_status(c, cudaMemcpyAsync(support, d + 1, sizeof(int64_t) * g.ne, cudaMemcpyDeviceToHost, c->stream),
+    s = cuda_status(c, cudaMemcpyAsync(support, d, sizeof(int64_t) * g.ne, cudaMemcpyDeviceToHost, c->stream),
                     "D2H");
   dfree(c, d);
-  if (s == XT_OK) s = cuda_status(c, cudaStreamSynchronize(c->stream), "count");
-  if (s == XT_OK) s = count_status(c);
+  if (s == XT_OK) s = count_status(c, global);
   return s;
 }
 
@@ -401,11 +417,8 @@ xt_status xt_count_device(int64_t nv, const int64_t *d_indices, const int64_t *d
   if (cudaGetDevice(&dev) != cudaSuccess) return XT_ERR_NO_DEVICE;
   // a transient context on the caller's device and stream
   xt_ctx *ctx = nullptr;
-  XT_TRY(xt_open(dev, &ctx));
+  XT_TRY(open_ctx(dev, false, static_cast<cudaStream_t>(stream), &ctx));
   Ctx *c = &ctx->c;
-  cudaStreamDestroy(c->stream);
-  c->stream = static_cast<cudaStream_t>(stream);
-  c->own_stream = false;
   Graph g;
   xt_status s = build_from_csr(c, nv, d_indices, d_edge_list, true, XT_ORIENT_DEGREE, &g);
   int64_t *tmp = nullptr;
@@ -426,9 +439,8 @@ xt_status xt_count_device(int64_t nv, const int64_t *d_indices, const int64_t *d
   }
   dfree(c, tmp);
   free_graph_device(&g);
+  cudaFreeAsync(c->d_out, c->stream);
   cudaStreamSynchronize(c->stream);
-  c->stream = nullptr;
-  cudaFree(c->d_err);
   delete ctx;
   return s;
 }

@@ -1823,10 +1823,12 @@ int64_t lane_task_count(const Graph *g) { return g->plan ? g->plan->n_ttask : 0;
 // After a count has finished on the context stream: XT_ERR_TIMEOUT if a
 // CTA's bounded wait for its staged members gave up (the count is then
 // incomplete), which clears the flag; XT_OK otherwise.
-xt_status count_status(Ctx *c) {
-  int h = 0;
-  XT_CUDA(c, cudaMemcpyAsync(&h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+xt_status count_status(Ctx *c, int64_t *total) {
+  CountOut o = {};
+  XT_CUDA(c, cudaMemcpyAsync(&o, c->d_out, sizeof(o), cudaMemcpyDeviceToHost, c->stream));
   XT_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (total) *total = o.total;
+  const int h = o.err;
   if (h & (kErrStageTimeout | kErrCoreTimeout)) {
     XT_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
     return set_error(c, XT_ERR_TIMEOUT, "count: a CTA's wait for its staged data timed out");

@@ -17,17 +17,24 @@ constexpr int kWarp = 32;
 constexpr size_t kColPad = 8;
 
 // ---- context ---------------------------------------------------------------
+// device block read back by the synchronous counts in one copy: the error word
+// that kernels set when their input or a bounded wait fails, and a total
+struct CountOut {
+  int err;
+  int reserved;
+  int64_t total;
+};
+
 struct Ctx {
   int device = 0;
   int sm_count = 148;
-  size_t smem_optin = 0;  // max dynamic shared memory per block (opt-in)
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   cudaStream_t copy_stream = nullptr;  // host-to-device copies that overlap the build (created on first use)
   std::string last_error;
   int64_t fail_alloc_countdown = 0;  // test hook: >0 counts down to a failing allocation
-  // device-side error word reused by kernels that check their own inputs
-  int *d_err = nullptr;
+  CountOut *d_out = nullptr;
+  int *d_err = nullptr;  // &d_out->err: reused by kernels that check their own inputs
   int64_t launches = 0;  // kernels of this library launched on this context
   // device bytes this context holds (its own allocations) and their high-water mark
   std::unordered_map<void *, size_t> live;
@@ -221,7 +228,8 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
                       int64_t *d_support = nullptr, int shard = 0, int nshards = 1);
 // Synchronises the context stream and reports a count whose bounded device
 // wait gave up (XT_ERR_TIMEOUT); the synchronous count calls end with it.
-xt_status count_status(Ctx *c);
+// total (nullable) receives the context block's total.
+xt_status count_status(Ctx *c, int64_t *total = nullptr);
 // tasks of the global count's thread-block cluster tier in the graph's plan (0 without a plan)
 int64_t cluster_task_count(const Graph *g);
 // lane tasks in the graph's plan (0 without a plan)
