@@ -17,7 +17,7 @@ xt_status gen_chunglu(Ctx *c, int64_t n, const uint64_t *cdf, int64_t ne, uint64
                       int32_t *d_src, int32_t *d_dst);
 xt_status gen_er(Ctx *c, int64_t n, int64_t ne, uint64_t seed, int32_t *d_src, int32_t *d_dst);
 xt_status gen_rgg(Ctx *c, int64_t nv, int nprocs, double radius, int64_t cap, int64_t *n_pairs, int32_t *d_src,
-                  int32_t *d_dst);
+                  int32_t *d_dst, int32_t **own = nullptr);
 
 xt_status set_error(Ctx *c, xt_status s, const std::string &msg) {
   if (c) c->last_error = msg;
@@ -478,23 +478,20 @@ xt_status xt_graph_from_rgg(xt_ctx *ctx, int64_t nv, int nprocs, double radius, 
   Ctx *c = &ctx->c;
   cudaSetDevice(c->device);
   int64_t m = 0;
-  XT_TRY(gen_rgg(c, nv, nprocs, radius, 0, &m, nullptr, nullptr));
-  int32_t *ds = nullptr, *dd = nullptr;
-  XT_TRY(dalloc_n(c, &ds, size_t(m > 0 ? m : 1)));
-  xt_status s = dalloc_n(c, &dd, size_t(m > 0 ? m : 1));
-  if (s == XT_OK && m > 0) s = gen_rgg(c, nv, nprocs, radius, m, &m, ds, dd);
+  int32_t *rows[2] = {nullptr, nullptr};
+  xt_status s = gen_rgg(c, nv, nprocs, radius, 0, &m, nullptr, nullptr, rows);
   xt_graph *gr = nullptr;
   if (s == XT_OK) {
     gr = new (std::nothrow) xt_graph();
     if (!gr) s = XT_ERR_OOM;
   }
   if (s == XT_OK) {
-    s = build_from_edges(c, nv, m, ds, dd, orient, &gr->g);
+    s = build_from_edges(c, nv, m, rows[0], rows[1], orient, &gr->g);
     if (s == XT_OK) gr->g.n_input = 2 * m;  // the reference's directed entries
     s = finish_build(ctx, gr, s, out);
   }
-  dfree(c, ds);
-  dfree(c, dd);
+  dfree(c, rows[0]);
+  dfree(c, rows[1]);
   cudaStreamSynchronize(c->stream);
   return s;
 }

@@ -291,10 +291,12 @@ xt_status xt_rgg_setup(int64_t nv, int nprocs, double radius, double *rn_out, in
       }
     std::memcpy(c, t, sizeof(t));
   };
-  const int64_t M[4] = {16807, 0, 0, 1};
-  int64_t Mk[4];
-  std::memcpy(Mk, M, sizeof(M));
-  for (int64_t p = 0; p < nl - 1; p++) mat2(Mk, Mk, M);
+  // M^nl by squaring: the wrapped products are those of nl - 1 steps
+  int64_t M[4] = {16807, 0, 0, 1}, Mk[4] = {1, 0, 0, 1};
+  for (int64_t e = nl; e > 0; e >>= 1) {
+    if (e & 1) mat2(Mk, Mk, M);
+    mat2(M, M, M);
+  }
   std::vector<std::array<int64_t, 4>> G(P), R(P), Pf(P);
   for (int r = 0; r < P; r++) {
     std::memcpy(G[r].data(), Mk, sizeof(Mk));
