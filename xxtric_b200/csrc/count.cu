@@ -20,11 +20,14 @@
 //              binary-searched in the row itself
 //   warp tier: d+(v) <= kWarpDmax and work(v) <= warp_work -> one warp per
 //              head, member set in the warp's slice of shared memory
+//   pack     : 2 to 32 consecutive heads of few members and little work
+//              between them -> one warp, their members in one set keyed by
+//              (member, head)
 //   CTA tier : otherwise -> CTA tasks over chunks of v's in-records of about
 //              block_work items; N+(v) beyond kBlockDmax members is split
 //              into parts, one task per (part, chunk)
 // One persistent kernel drains the CTA tasks first (the large ones), then the
-// warp tasks, then the lane tasks, each from its own global atomic cursor.
+// warp tasks, the packs and the lane tasks, each from its own global atomic cursor.
 // Inside a task, lanes walk whole suffixes in aligned 32-byte pairs of the
 // padded column array, with no masking (see stream_kind).
 #include <cooperative_groups.h>
@@ -70,6 +73,7 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kMinBlocks = XT_MIN_BLOCKS;
 constexpr int kBlockWords = 8192;  // CTA region: 8192-slot hash or 2^18-bit bitmap
 // warp tasks run after the CTA tasks and split the CTA region among the warps
+constexpr int kWarpLg = 10;
 constexpr int kWarpWords = kBlockWords / kWarps;  // 1024: a 1024-slot hash or a 32K-bit bitmap
 constexpr int kWarpDmax = kWarpWords / 4;         // hash load factor <= 1/4
 constexpr int64_t kWarpWork = XT_WARP_WORK;
@@ -79,6 +83,7 @@ constexpr int64_t kWarpWork = XT_WARP_WORK;
 constexpr int kBlockDmax = XT_BLOCK_DMAX;
 // the warps' member counters share the CTA's
 static_assert(kWarps * kWarpDmax <= kBlockDmax, "warp member counters exceed the CTA's");
+static_assert(kWarpWords == 1 << kWarpLg, "a warp's slice is a power of two");
 // Cluster tier (global count): a head whose members overflow a CTA's set
 // (more than kBlockDmax, as the id orientation gives hubs) is counted by a
 // cluster of kCluster CTAs holding up to kClusterDmax members per part
@@ -92,6 +97,7 @@ struct PlanParams {
   int64_t tiny_work;   // a head with at most this much work is a lane task
   int64_t warp_work;   // ... else one with d+(v) <= warp_dmax and at most this much work is a warp task
   int64_t block_work;  // items per CTA task
+  int64_t pack_work;   // candidates of a pack, at most (0: no packs)
   int32_t warp_dmax;
   int32_t batches_per_warp;  // CTA task: record batches per warp, at least
   int32_t lane_pairs;        // CTA task: pairs per lane on an average record, at least
@@ -135,7 +141,8 @@ constexpr int kErrStageTimeout = 8;
 constexpr int32_t kEmpty = -1;
 
 // A warp or CTA task: the in-records [k0, k0 + nrec) of head v streamed
-// through the members col[r0, r0 + nmem), 2^lg_s lanes per record.
+// through the members col[r0, r0 + nmem), 2^lg_s lanes per record. A pack: the
+// same of the heads v .. v + g - 1 together, lg_s | g << 8.
 struct __align__(16) Task {
   int64_t k0;
   int64_t r0;
@@ -145,14 +152,18 @@ struct __align__(16) Task {
   int32_t lg_s;
 };
 
+constexpr int kCursors = 5;
+
 struct Plan {
   int64_t n_btask = 0;         // CTA tasks
   Task *d_bt = nullptr;
   int64_t n_wtask = 0;         // warp tasks
   Task *d_wt = nullptr;
+  int64_t n_ptask = 0;         // packs
+  Task *d_pt = nullptr;
   int64_t n_ttask = 0;         // lane tasks: one head per lane
   int32_t *d_tt = nullptr;
-  unsigned long long *d_cursor = nullptr;  // [0] CTA, [1] warp, [2] lane, [3] cluster task cursors
+  unsigned long long *d_cursor = nullptr;  // [0] CTA, [1] warp, [2] lane, [3] cluster task, [4] pack cursors
   int64_t n_ctask = 0;         // cluster tasks (global count)
   Task *d_ct = nullptr;
   int64_t n_btask0 = 0;        // the CTA tasks of the other heads, which the global count
@@ -241,15 +252,54 @@ __device__ __forceinline__ void classify(int64_t v, const int64_t *__restrict__ 
   nb = parts * chunks;
 }
 
+// Tasks of every head: CTA tasks in nb, warp tasks and packs in the halves of
+// nwp (packs high), lane tasks in nt (null: none). Packs are aligned blocks of g = 2
+// to 32 heads, the largest g whose heads have at most warp_dmax members and
+// pack_work candidates between them: a warp that takes such heads one by one
+// spends its time waiting (claim, members, first pair: 3 to 5 us a head).
+// pk[v]: log2 g for a pack's first head, kPackRest for its others, 0 elsewhere.
+constexpr uint8_t kPackRest = 0xff;
+constexpr int64_t kPackRecs = 4096;
+// Candidates of a pack, at most: one pack for each warp of the GPU, within
+// these bounds. Swept at 64 to 2,048 (counts in us, 0: no packs): geometric
+// graph of 2^16 vertices 52 without, 31 at 512, 44 at 2,048; of 2^20 656, 238 at
+// 512, 220 at 1,024; Chung-Lu 2^22 6,133, 5,686, 5,630; R-MAT 2^22 3,538, 3,507,
+// 3,507 (3,533 at 2,048); a batch of 256 graphs 1,860, 1,409, 1,359.
+constexpr int64_t kPackWorkMin = 256, kPackWorkMax = 1024;
 __global__ void k_plan_count(int64_t nv, const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
-                             const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp, int64_t *__restrict__ nb_out,
-                             int64_t *__restrict__ nw_out, int64_t *__restrict__ nt_out) {
-  XT_GRID_STRIDE(v, nv) {
-    int64_t nb, nw, nt, parts, chunks, work;
-    classify(v, off, ioff, iend, P, pp, nb, nw, nt, parts, chunks, work);
+                             const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp,
+                             int64_t *__restrict__ nb_out, int64_t *__restrict__ nwp_out,
+                             int64_t *__restrict__ nt_out, uint8_t *__restrict__ pk) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t base = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) & ~int64_t(31); base < nv;
+       base += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t v = base + lane;
+    int64_t nb = 0, nw = 0, nt = 0, parts, chunks, work = 0, mem = 0, rec = 0;
+    if (v < nv) {
+      classify(v, off, ioff, iend, P, pp, nb, nw, nt, parts, chunks, work);
+      mem = off[v + 1] - off[v];
+      rec = ioff[v + 1] - ioff[v];
+    }
+    uint8_t code = 0;
+    if (pp.pack_work > 0) {
+      int busy = nb + nw + nt > 0;
+#pragma unroll
+      for (int lg = 1; lg <= 5; lg++) {
+        const int o = 1 << (lg - 1);
+        mem += __shfl_xor_sync(0xffffffffu, mem, o);
+        work += __shfl_xor_sync(0xffffffffu, work, o);
+        rec += __shfl_xor_sync(0xffffffffu, rec, o);
+        busy += __shfl_xor_sync(0xffffffffu, busy, o);
+        if (busy > 1 && mem <= pp.warp_dmax && work <= pp.pack_work && rec <= kPackRecs)
+          code = (lane & (2 * o - 1)) == 0 ? uint8_t(lg) : kPackRest;
+      }
+    }
+    if (v >= nv) continue;
+    if (code) nb = nw = nt = 0;
     nb_out[v] = nb;
-    nw_out[v] = nw;
-    nt_out[v] = nt;
+    nwp_out[v] = nw | (code && code != kPackRest ? int64_t(1) << 32 : 0);
+    if (nt_out) nt_out[v] = nt;
+    pk[v] = code;
   }
 }
 
@@ -290,9 +340,22 @@ __device__ __forceinline__ Task make_task(int64_t v, int64_t k0, int64_t k1, int
 
 __global__ void k_plan_fill(int64_t nv, const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
                             const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp, const int64_t *__restrict__ nb_pos,
-                            const int64_t *__restrict__ nw_pos, const int64_t *__restrict__ nt_pos,
-                            Task *__restrict__ bt, Task *__restrict__ wt, int32_t *__restrict__ tt) {
+                            const int64_t *__restrict__ nwp_pos, const int64_t *__restrict__ nt_pos,
+                            const uint8_t *__restrict__ pk, Task *__restrict__ bt, Task *__restrict__ wt,
+                            Task *__restrict__ pt, int32_t *__restrict__ tt) {
   XT_GRID_STRIDE(v, nv) {
+    if (pk[v]) {
+      if (pk[v] == kPackRest) continue;
+      const int g = 1 << pk[v];
+      const int64_t h1 = v + g < nv ? v + g : nv, k0 = ioff[v], k1 = ioff[h1];
+      // lanes per record: as many as the pack's records leave idle, while a
+      // record of average length has a pair for each
+      const int64_t pairs = (P[k1] - P[k0]) / (8 * (k1 - k0)) + 1;
+      int32_t lg_s = 0;
+      while (lg_s < 5 && (pairs >> (lg_s + 1)) > 0 && ((k1 - k0) << (lg_s + 1)) <= 32) lg_s++;
+      pt[nwp_pos[v] >> 32] = make_task(v, k0, k1, off[v], off[h1], lg_s | int32_t(h1 - v) << 8);
+      continue;
+    }
     int64_t nb, nw, nt, parts, chunks, work;
     classify(v, off, ioff, iend, P, pp, nb, nw, nt, parts, chunks, work);
     const int64_t k0 = ioff[v], k1 = iend[v];
@@ -318,7 +381,7 @@ __global__ void k_plan_fill(int64_t nv, const int64_t *__restrict__ off, const i
           lg_s = ls;
         }
       }
-      wt[nw_pos[v]] = make_task(v, k0, k1, off[v], off[v + 1], lg_s);
+      wt[nwp_pos[v] & 0xffffffff] = make_task(v, k0, k1, off[v], off[v + 1], lg_s);
     }
     if (!nb) continue;
     const int64_t base = P[k0];
@@ -929,6 +992,8 @@ struct CountArgs {
   int64_t n_bt;
   const Task *wt;  // warp tasks
   int64_t n_wt;
+  const Task *pt;  // packs
+  int64_t n_pt;
   const int32_t *tt;  // lane tasks (heads)
   int64_t n_tt;
   const Task *ct;  // cluster tasks
@@ -936,7 +1001,7 @@ struct CountArgs {
   int lane_merge;  // lane tasks: members found by a two-pointer merge (1) or binary search (0)
   int64_t stride;  // task lists hold every stride-th task of the schedule (a shard of it), else 1
   int claim;       // warp tasks (and groups of 32 lane tasks) taken from their cursor per atomic
-  unsigned long long *cursor;     // [0] CTA, [1] warp, [2] lane task cursors
+  unsigned long long *cursor;     // [0] CTA, [1] warp, [2] lane, [4] pack cursors
   unsigned long long *global;     // the total
   int64_t *pv;                    // per-vertex counts (per-vertex mode)
   unsigned int *es;               // per-edge counts, out-CSR order (per-edge mode)
@@ -1031,8 +1096,18 @@ __device__ __forceinline__ Task claim_task(unsigned long long *cursor, const Tas
 // that atomic is the limit; elsewhere a block lengthens the tail (R-MAT s22
 // 4.69 -> 4.79 ms with 4; s24 and Chung-Lu unchanged), so a plain graph
 // claims one at a time and a batch four (xt_graph_set_claim, the autotuner).
+// Where no CTA tasks come first, every warp starts on the block of its own
+// index, without an atomic (first != 0: the blocks given out that way).
 struct ClaimBlock {
   unsigned long long next = 0, end = 0;  // lane 0: the unclaimed rest of its block
+  unsigned long long first = 0;
+  __device__ __forceinline__ ClaimBlock(bool own, int claim) {
+    if (!own) return;
+    const unsigned long long w = (unsigned long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    next = w * claim;
+    end = next + claim;
+    first = (unsigned long long)gridDim.x * kWarps * claim;
+  }
 };
 __device__ __forceinline__ Task claim_task_block(ClaimBlock &cb, unsigned long long *cursor,
                                                  const Task *__restrict__ tasks, int64_t n, int64_t stride, int claim,
@@ -1040,7 +1115,7 @@ __device__ __forceinline__ Task claim_task_block(ClaimBlock &cb, unsigned long l
   unsigned long long i = 0;
   if (lane == 0) {
     if (cb.next == cb.end) {
-      cb.next = atomicAdd(cursor, (unsigned long long)claim);
+      cb.next = cb.first + atomicAdd(cursor, (unsigned long long)claim);
       cb.end = cb.next + claim;
     }
     i = cb.next++;
@@ -1103,6 +1178,114 @@ __device__ __forceinline__ int stage_task_bulk(int32_t *stage, uint64_t *bar, co
   return int(t.r0 & 3);
 }
 
+// ---- packs ----------------------------------------------------------------------
+//
+// A pack's members are keyed with their head: (x << 5 | head) + 1 in a cuckoo
+// table (0 empty), (x << 5 | head) in a linear-probing one (kEmpty empty), so
+// ids must lie below 2^26 (kPackMaxNv).
+constexpr int64_t kPackMaxNv = (int64_t(1) << 26) - 2;
+
+// the pack's heads, one a lane: first record, end of the live records (both
+// from the pack's first) and first member
+struct PackHeads {
+  int32_t rec, live, mem;
+};
+__device__ __forceinline__ PackHeads pack_heads(const CountArgs &a, const Task &t, int lane) {
+  PackHeads h;
+  h.rec = h.live = h.mem = 0x7fffffff;
+  if (t.nrec >= 0 && lane < (t.lg_s >> 8)) {
+    h.rec = int32_t(a.ioff[t.v + lane] - t.k0);
+    h.live = int32_t(a.iend[t.v + lane] - t.k0);
+    h.mem = int32_t(a.off[t.v + lane] - t.r0);
+  }
+  return h;
+}
+// the last lane whose value is at most x (lane 0's always is)
+__device__ __forceinline__ int pack_find(int32_t start, int32_t x) {
+  int h = 0;
+#pragma unroll
+  for (int step = 16; step; step >>= 1)
+    if (__shfl_sync(0xffffffffu, start, h + step) <= x) h += step;
+  return h;
+}
+
+// the candidate w of a record of head `hl` at padded column pos
+template <int MODE, bool CUCKOO>
+__device__ __forceinline__ int pack_probe(const Members &m, int32_t w, uint32_t hl, unsigned int *__restrict__ es,
+                                          int64_t pos) {
+  if (CUCKOO) {
+    const uint32_t key = uint32_t(w) * 32u + hl + 1u;
+    const uint32_t x = uint32_t(m.words[cuckoo_h1(key, m.shift)]);
+    const uint32_t y = uint32_t(m.words[cuckoo_h2(key, m.shift)]);
+    return int(uint32_t(x == key) | uint32_t(y == key));
+  }
+  if (uint32_t(w - m.lo) > uint32_t(m.hi - m.lo)) return 0;  // sentinels too
+  const int slot = hash_find(m.words, m.mask, m.shift, int32_t(uint32_t(w) * 32u + hl));
+  if (slot < 0) return 0;
+  if (MODE != 0) atomicAdd(&m.mcnt[m.idx[slot]], 1);
+  if (MODE == 2) atomicAdd(&es[pos], 1u);
+  return 1;
+}
+
+// Streams a pack's records through its set (as stream_kind: records two
+// batches ahead, the next pair in flight); hits of each head go to hcnt when
+// HEADS. Returns this lane's hits.
+template <int MODE, bool CUCKOO, bool HEADS>
+__device__ __forceinline__ int64_t stream_pack(const CountArgs &a, const Task &t, const PackHeads &ph,
+                                               const Members &m, int *hcnt, int lane) {
+  const int lg_s = t.lg_s & 0xff, S = 1 << lg_s, bsz = 32 >> lg_s;
+  const int j = lane >> lg_s, k = lane & (S - 1);
+  const int4 sent = make_int4(kSentinel, kSentinel, kSentinel, kSentinel);
+  const InRec *rec = a.rec + t.k0;
+  auto fetch = [&](int32_t base) -> uint2 {
+    return base + j < t.nrec ? __ldg(reinterpret_cast<const uint2 *>(rec) + base + j) : make_uint2(0u, 0u);
+  };
+  uint2 r4 = fetch(0), n4 = fetch(bsz);
+  int64_t hits = 0;
+  for (int32_t b = 0; b < t.nrec; b += bsz) {
+    const uint2 nn4 = fetch(b + 2 * bsz);
+    const int32_t r = b + j;
+    const int hl = pack_find(ph.rec, r);
+    const bool live = r < __shfl_sync(0xffffffffu, ph.live, hl);
+    const int32_t len = live ? int32_t(r4.y & uint32_t(kMaxRecLen - 1)) : 0, lead = int32_t(r4.y >> kRecLenBits);
+    const int32_t np = len > 0 ? (lead + len + 7) >> 3 : 0;
+    const int32_t cnt = np > k ? ((np - k + S - 1) >> lg_s) : 0;
+    const int32_t steps = int32_t(__reduce_max_sync(0xffffffffu, uint32_t(cnt)));
+    PairIdx P = PairIdx(r4.x) + PairIdx(k);
+    int4 xa = sent, xb = sent;
+    if (cnt > 0) load_pair(a.colp, P, xa, xb);
+    int h = 0;
+    for (int32_t it = 0; it < steps; it++) {
+      const int4 ca = xa, cb = xb;
+      const int64_t pos = 8 * int64_t(P);
+      P += S;
+      if (it + 1 < cnt) {
+        load_pair(a.colp, P, xa, xb);
+      } else {
+        xa = sent;
+        xb = sent;
+      }
+      h += pack_probe<MODE, CUCKOO>(m, ca.x, hl, a.es, pos) + pack_probe<MODE, CUCKOO>(m, ca.y, hl, a.es, pos + 1) +
+           pack_probe<MODE, CUCKOO>(m, ca.z, hl, a.es, pos + 2) + pack_probe<MODE, CUCKOO>(m, ca.w, hl, a.es, pos + 3) +
+           pack_probe<MODE, CUCKOO>(m, cb.x, hl, a.es, pos + 4) + pack_probe<MODE, CUCKOO>(m, cb.y, hl, a.es, pos + 5) +
+           pack_probe<MODE, CUCKOO>(m, cb.z, hl, a.es, pos + 6) + pack_probe<MODE, CUCKOO>(m, cb.w, hl, a.es, pos + 7);
+    }
+    hits += h;
+    if (HEADS) {
+      for (int o = S >> 1; o; o >>= 1) h += __shfl_down_sync(0xffffffffu, h, o, S);
+      if (k == 0 && h) {
+        atomicAdd(&hcnt[hl], h);
+        if (MODE == 1)
+          atomicAdd(reinterpret_cast<unsigned long long *>(&a.pv[a.rec_u[t.k0 + r]]), (unsigned long long)h);
+        if (MODE == 2) atomicAdd(&a.es[8 * int64_t(r4.x) + lead - 1], unsigned(h));  // the edge u->v
+      }
+    }
+    r4 = n4;
+    n4 = nn4;
+  }
+  return hits;
+}
+
 // clears the first nclear words of the member set (thread t of nt)
 template <bool PV>
 __device__ __forceinline__ void clear_members(const Members &m, int nclear, int t, int nt) {
@@ -1143,7 +1326,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
   if (tid == 0) mbar_init(&s_stage_bar, 1);
   __syncthreads();
   uint32_t stage_parity = 0;
-  if (warp == 0) {
+  if (a.n_bt > 0 && warp == 0) {
     const Task t0 = claim_task(&cursor[0], a.bt, a.n_bt, a.stride, lane);
     const int so = stage_task_bulk(s_stage, &s_stage_bar, col, rec, t0, lane);
     if (lane == 0) {
@@ -1151,7 +1334,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
       s_soff[0] = so;
     }
   }
-  for (int cur = 0;; cur ^= 1) {
+  for (int cur = 0; a.n_bt > 0; cur ^= 1) {
     // every thread waits for the staged members (bounded: on a timeout the
     // CTA leaves its task loop and reports it through the error word)
     const bool landed = mbar_wait_bounded(&s_stage_bar, stage_parity);
@@ -1226,8 +1409,9 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
   }
 
   // ---- warp tasks: the CTA region split among the warps ----
-  ClaimBlock wclaim;
-  if (MODE == 0 && kWarpCuckoo) {
+  ClaimBlock wclaim(a.n_bt == 0, a.claim);
+  if (a.n_wt == 0) {
+  } else if (MODE == 0 && kWarpCuckoo) {
     // The slice holds the CTA tasks' last set: zero it once. A task then
     // builds its bitmap or cuckoo table into the zeroed slice and, when done,
     // clears only the words or slots its members took, instead of clearing
@@ -1314,6 +1498,103 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
       __syncwarp();
       so = stage_task(wstage, col, rec, tn, lane);
       t = tn;
+    }
+  }
+
+  // ---- packs: several small heads per warp, in the warp's slice ----
+  if (a.n_pt > 0) {
+    __shared__ int s_hcnt[kWarps][32];
+    int32_t *wstage = s_stage + warp * kStageWarp;
+    int32_t *words = bwords + warp * kWarpWords;
+    int *hcnt = s_hcnt[warp];
+    const bool heads = PV || a.group;
+    ClaimBlock pclaim(a.n_bt == 0 && a.n_wt == 0, a.claim);
+    Task t = claim_task_block(pclaim, &cursor[4], a.pt, a.n_pt, a.stride, a.claim, lane);
+    int so = stage_task(wstage, col, rec, t, lane);
+    PackHeads ph = pack_heads(a, t, lane);
+    if (t.nrec >= 0 && MODE == 0) zero_words(words, kWarpWords, lane, 32);
+    while (true) {
+      cp_async_wait_all();
+      __syncwarp();
+      if (t.nrec < 0) break;
+      const int32_t *mem = wstage + so;
+      Members m;
+      m.words = words;
+      m.idx = bidx + warp * kWarpWords;
+      m.mcnt = bmcnt + warp * kWarpDmax;
+      m.mask = kWarpWords - 1;
+      m.shift = 32 - kWarpLg;
+      bool ok = MODE == 0;  // the global count's set is a cuckoo table, in a slice that is all zero
+      if (heads) hcnt[lane] = 0;
+      if (MODE == 0) {
+        for (int i0 = 0; i0 < t.nmem; i0 += 32) {
+          const int i = i0 + lane, hl = pack_find(ph.mem, i);
+          if (i < t.nmem)
+            ok &= cuckoo_insert(words, m.shift, uint32_t(mem[i]) * 32u + uint32_t(hl) + 1u, a.cuckoo_iters);
+        }
+        ok = __all_sync(0xffffffffu, ok);
+      }
+      if (!ok) {  // linear probing (with member counters), or a cuckoo chain ran too long
+        int32_t lo = 0x7fffffff, hi = -1;
+        for (int i = lane; i < kWarpWords; i += 32) words[i] = kEmpty;
+        __syncwarp();
+        for (int i0 = 0; i0 < t.nmem; i0 += 32) {
+          const int i = i0 + lane, hl = pack_find(ph.mem, i);
+          if (i < t.nmem) {
+            lo = min(lo, mem[i]);
+            hi = max(hi, mem[i]);
+            const uint32_t slot = hash_insert(words, m.mask, m.shift, int32_t(uint32_t(mem[i]) * 32u + uint32_t(hl)));
+            if (PV) {
+              m.idx[slot] = uint16_t(i);
+              m.mcnt[i] = 0;
+            }
+          }
+        }
+        m.lo = __reduce_min_sync(0xffffffffu, lo);
+        m.hi = __reduce_max_sync(0xffffffffu, hi);
+      }
+      __syncwarp();
+      const Task tn = claim_task_block(pclaim, &cursor[4], a.pt, a.n_pt, a.stride, a.claim, lane);
+      const PackHeads phn = pack_heads(a, tn, lane);
+      if (PV) acc += stream_pack<MODE, false, true>(a, t, ph, m, hcnt, lane);
+      else if (!ok) acc += stream_pack<0, false, true>(a, t, ph, m, hcnt, lane);
+      else if (a.group) acc += stream_pack<0, true, true>(a, t, ph, m, hcnt, lane);
+      else acc += stream_pack<0, true, false>(a, t, ph, m, hcnt, lane);
+      __syncwarp();
+      if (MODE == 0 && ok) {
+        for (int i0 = 0; i0 < t.nmem; i0 += 32) {
+          const int i = i0 + lane, hl = pack_find(ph.mem, i);
+          if (i < t.nmem) {
+            const uint32_t key = uint32_t(mem[i]) * 32u + uint32_t(hl) + 1u, x = cuckoo_h1(key, m.shift);
+            if (uint32_t(words[x]) == key) words[x] = 0;
+            else words[cuckoo_h2(key, m.shift)] = 0;
+          }
+        }
+      } else if (MODE == 0) {
+        zero_words(words, kWarpWords, lane, 32);
+      }
+      const int32_t v = t.v + lane;  // this lane's head
+      if (heads && lane < (t.lg_s >> 8) && hcnt[lane]) {
+        if (MODE == 1)
+          atomicAdd(reinterpret_cast<unsigned long long *>(&pv[v]), (unsigned long long)hcnt[lane]);
+        if (a.group) atomicAdd(&a.group_out[a.group[v]], (unsigned long long)hcnt[lane]);
+      }
+      if (MODE == 1) {
+        for (int i = lane; i < t.nmem; i += 32)
+          if (m.mcnt[i])
+            atomicAdd(reinterpret_cast<unsigned long long *>(&pv[mem[i]]), (unsigned long long)m.mcnt[i]);
+      }
+      if (MODE == 2) {
+        for (int i0 = 0; i0 < t.nmem; i0 += 32) {
+          const int i = i0 + lane, hl = pack_find(ph.mem, i);
+          const int32_t r0 = __shfl_sync(0xffffffffu, ph.mem, hl);
+          if (i < t.nmem && m.mcnt[i]) atomicAdd(&es[a.poff[t.v + hl] + (i - r0)], unsigned(m.mcnt[i]));
+        }
+      }
+      __syncwarp();
+      so = stage_task(wstage, col, rec, tn, lane);
+      t = tn;
+      ph = phn;
     }
   }
 
@@ -1411,7 +1692,8 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
       }
     }
   };
-  if (a.lane_merge) lane_tasks(std::true_type{});
+  if (a.n_tt == 0) {
+  } else if (a.lane_merge) lane_tasks(std::true_type{});
   else lane_tasks(std::false_type{});
 
   // ---- reduce ----
@@ -1565,6 +1847,7 @@ static void free_one_plan(Ctx *c, Plan *pl) {
   dfree(c, pl->d_ct);
   dfree(c, pl->d_bt0);
   dfree(c, pl->d_wt);
+  dfree(c, pl->d_pt);
   dfree(c, pl->d_tt);
   dfree(c, pl->d_cursor);
   delete pl;
@@ -1651,10 +1934,11 @@ static xt_status plan_records(Graph *g, const int64_t *iend, Plan **out) {
   const int B = 256;
   int64_t *P = nullptr, *nb = nullptr, *nw = nullptr, *nt = nullptr, *nbp = nullptr, *nwp = nullptr,
           *ntp = nullptr;
+  uint8_t *pk = nullptr;
   unsigned long long *stats = nullptr;
   xt_status s = XT_OK;
   do {
-    if ((s = dalloc_n(c, &pl->d_cursor, 4)) != XT_OK) break;
+    if ((s = dalloc_n(c, &pl->d_cursor, kCursors)) != XT_OK) break;
     if ((s = dalloc_n(c, &stats, 5)) != XT_OK) break;
     if ((s = dalloc_n(c, &P, size_t(ne + 1))) != XT_OK) break;
     if ((s = cuda_status(c, cudaMemsetAsync(stats, 0, 5 * sizeof(unsigned long long), c->stream), "memset")) !=
@@ -1709,6 +1993,12 @@ static xt_status plan_records(Graph *g, const int64_t *iend, Plan **out) {
     pp.lane_pairs = XT_LANE_PAIRS;
     pp.warp_work = g->tune_warp_work > 0 ? g->tune_warp_work : (large ? XT_WARP_WORK_LARGE : kWarpWork);
     if (g->tier_warp_work >= 0) pp.warp_work = g->tier_warp_work;
+    // packs fill every warp once before they grow (tiers set by hand: none)
+    pp.pack_work = 0;
+    if (nv <= kPackMaxNv && g->tier_lane_work < 0 && g->tier_warp_work < 0) {
+      const int64_t warps = int64_t(pl->grid_global) * kWarps;
+      pp.pack_work = std::min(kPackWorkMax, std::max(kPackWorkMin, total_work / warps));
+    }
     if (g->tune_block_work > 0) {
       pp.block_work = g->tune_block_work;
     } else {
@@ -1722,26 +2012,30 @@ static xt_status plan_records(Graph *g, const int64_t *iend, Plan **out) {
     if ((s = dalloc_n(c, &nw, size_t(nv + 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &nbp, size_t(nv + 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &nwp, size_t(nv + 1))) != XT_OK) break;
-    if ((s = dalloc_n(c, &nt, size_t(nv + 1))) != XT_OK) break;
-    if ((s = dalloc_n(c, &ntp, size_t(nv + 1))) != XT_OK) break;
+    if ((s = dalloc_n(c, &pk, size_t(nv))) != XT_OK) break;
+    const bool lanes = pp.tiny_work > 0;  // without lane tasks there is nothing to scan
+    if (lanes && (s = dalloc_n(c, &nt, size_t(nv + 1))) != XT_OK) break;
+    if (lanes && (s = dalloc_n(c, &ntp, size_t(nv + 1))) != XT_OK) break;
     k_plan_count<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(nv, g->d_off, g->d_ioff, iend, P, pp, nb,
-                                                                                nw, nt);
+                                                                                nw, nt, pk);
     if ((s = cuda_status(c, cudaMemsetAsync(nb + nv, 0, sizeof(int64_t), c->stream), "memset")) != XT_OK) break;
     if ((s = cuda_status(c, cudaMemsetAsync(nw + nv, 0, sizeof(int64_t), c->stream), "memset")) != XT_OK) break;
-    if ((s = cuda_status(c, cudaMemsetAsync(nt + nv, 0, sizeof(int64_t), c->stream), "memset")) != XT_OK) break;
+    if (lanes && (s = cuda_status(c, cudaMemsetAsync(nt + nv, 0, sizeof(int64_t), c->stream), "memset")) != XT_OK)
+      break;
     if ((s = exclusive_scan(c, nb, nbp, nv + 1)) != XT_OK) break;
     if ((s = exclusive_scan(c, nw, nwp, nv + 1)) != XT_OK) break;
-    if ((s = exclusive_scan(c, nt, ntp, nv + 1)) != XT_OK) break;
+    if (lanes && (s = exclusive_scan(c, nt, ntp, nv + 1)) != XT_OK) break;
     int64_t h[4] = {0, 0, 0, 0};
     unsigned long long hs[5] = {0, 0, 0, 0, 0};
     if ((s = d2h(c, &h[0], nbp + nv, sizeof(int64_t))) != XT_OK) break;
     if ((s = d2h(c, &h[1], nwp + nv, sizeof(int64_t))) != XT_OK) break;
     if ((s = d2h(c, &h[2], P + ne, sizeof(int64_t))) != XT_OK) break;
-    if ((s = d2h(c, &h[3], ntp + nv, sizeof(int64_t))) != XT_OK) break;
+    if (lanes && (s = d2h(c, &h[3], ntp + nv, sizeof(int64_t))) != XT_OK) break;
     if ((s = d2h(c, hs, stats, sizeof(hs))) != XT_OK) break;
     if ((s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync")) != XT_OK) break;
     pl->n_btask = h[0];
-    pl->n_wtask = h[1];
+    pl->n_wtask = h[1] & 0xffffffff;
+    pl->n_ptask = h[1] >> 32;
     pl->n_ttask = h[3];
     g->max_degree = int64_t(hs[0]);
     g->max_out_degree = int64_t(hs[1]);
@@ -1754,9 +2048,10 @@ static xt_status plan_records(Graph *g, const int64_t *iend, Plan **out) {
     }
     if ((s = dalloc_n(c, &pl->d_bt, size_t(pl->n_btask > 0 ? pl->n_btask : 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &pl->d_wt, size_t(pl->n_wtask > 0 ? pl->n_wtask : 1))) != XT_OK) break;
+    if ((s = dalloc_n(c, &pl->d_pt, size_t(pl->n_ptask > 0 ? pl->n_ptask : 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &pl->d_tt, size_t(pl->n_ttask > 0 ? pl->n_ttask : 1))) != XT_OK) break;
     k_plan_fill<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(
-        nv, g->d_off, g->d_ioff, iend, P, pp, nbp, nwp, ntp, pl->d_bt, pl->d_wt, pl->d_tt);
+        nv, g->d_off, g->d_ioff, iend, P, pp, nbp, nwp, ntp, pk, pl->d_bt, pl->d_wt, pl->d_pt, pl->d_tt);
     if ((s = cuda_status(c, cudaGetLastError(), "k_plan_fill")) != XT_OK) break;
     if (pl->n_btask > 1) {  // chunk-major order
       uint64_t *k1 = nullptr, *k2 = nullptr;
@@ -1804,6 +2099,7 @@ static xt_status plan_records(Graph *g, const int64_t *iend, Plan **out) {
   dfree(c, nwp);
   dfree(c, nt);
   dfree(c, ntp);
+  dfree(c, pk);
   dfree(c, stats);
   if (s != XT_OK) {
     free_one_plan(c, pl);
@@ -1865,6 +2161,12 @@ __global__ void k_es_unpad(const unsigned int *__restrict__ esp, const int64_t *
   }
 }
 
+// the task cursors and the total start at zero (one launch for two memsets)
+__global__ void k_count_begin(unsigned long long *__restrict__ cursor, int64_t *__restrict__ total) {
+  if (threadIdx.x < kCursors) cursor[threadIdx.x] = 0;
+  if (threadIdx.x == kCursors) *total = 0;
+}
+
 // tasks of a list of n that fall to shard `shard` of nshards (every
 // nshards-th, from index shard on)
 static int64_t shard_len(int64_t n, int shard, int nshards) {
@@ -1889,8 +2191,8 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   // pairs of columns are read with 32-byte vector loads
   if (reinterpret_cast<uintptr_t>(g->d_colp) % 32 != 0)
     return set_error(c, XT_ERR_CUDA, "padded column array is not 32-byte aligned");
-  XT_CUDA(c, cudaMemsetAsync(pl->d_cursor, 0, 4 * sizeof(unsigned long long), c->stream));
-  XT_CUDA(c, cudaMemsetAsync(d_global, 0, sizeof(int64_t), c->stream));
+  k_count_begin<<<counted(c, dim3(1)), 32, 0, c->stream>>>(pl->d_cursor, d_global);
+  XT_CUDA(c, cudaGetLastError());
   if (d_groups) {
     if (!g->d_group) return set_error(c, XT_ERR_INVALID, "per-group counts need a graph built as a batch");
     XT_CUDA(c, cudaMemsetAsync(d_groups, 0, sizeof(int64_t) * g->n_groups, c->stream));
@@ -1930,6 +2232,8 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   a.n_bt = shard_len(pl->n_btask, shard, nshards);
   a.wt = shard_first(pl->d_wt, pl->n_wtask, shard);
   a.n_wt = shard_len(pl->n_wtask, shard, nshards);
+  a.pt = shard_first(pl->d_pt, pl->n_ptask, shard);
+  a.n_pt = shard_len(pl->n_ptask, shard, nshards);
   a.tt = shard_first(pl->d_tt, pl->n_ttask, shard);
   a.n_tt = shard_len(pl->n_ttask, shard, nshards);
   a.ct = shard_first(pl->d_ct, pl->n_ctask, shard);
