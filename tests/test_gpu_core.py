@@ -48,6 +48,10 @@ def test_core_counts_match_the_oracle(ctx, kind):
     nv, src, dst = graph(kind)
     off, tails = oracle.canon_csr(nv, src.astype(np.int64), dst.astype(np.int64))
     want, pv = oracle.count_merge(off, tails, per_vertex=True)
+    want_sup = oracle.edge_support(off, tails)
+    u = np.repeat(np.arange(nv), np.diff(off))
+    up = u < tails
+    want_sup = want_sup[up]
     g = ctx.graph_from_edges(3, np.array([0, 0, 1], np.int32), np.array([1, 2, 2], np.int32))
     before = ctx.launches
     assert g.count() == 1
@@ -62,8 +66,9 @@ def test_core_counts_match_the_oracle(ctx, kind):
         total, each = g.count(per_vertex=True)
         assert total == want
         np.testing.assert_array_equal(each, pv)
-        total, sup = g.count_edges()
-        assert total == want and int(sup.sum()) == 3 * want
+        a, b, sup = g.edge_support()
+        order = np.lexsort((b, a))
+        np.testing.assert_array_equal(sup[order], want_sup[np.lexsort((tails[up], u[up]))])
         g.set_tiers(0, 0)
         assert g.count() == want
         g.free()
@@ -74,12 +79,28 @@ def test_core_shards_sum_to_the_count(ctx, nshards):
     import torch
     nv, src, dst = graph("core and tail")
     g = ctx.graph_from_edges(nv, src.astype(np.int32), dst.astype(np.int32))
-    want = g.count()
+    want, pv = g.count(per_vertex=True)
+    total, sup = g.count_edges()
+    assert g.count() == total == want
     part = torch.zeros(1, dtype=torch.int64, device="cuda")
-    got = 0
+    each = torch.zeros(nv, dtype=torch.int64, device="cuda")
+    edge = torch.zeros(len(sup), dtype=torch.int64, device="cuda")
+    got = np.zeros(3, np.int64)
+    pvs, sups = np.zeros_like(pv), np.zeros_like(sup)
+    torch.cuda.synchronize()
     for i in range(nshards):
         g.count_shard_async(i, nshards, part)
         ctx.synchronize()
-        got += int(part)
-    assert got == want
+        got[0] += int(part)
+        g.count_shard_async(i, nshards, part, each)
+        ctx.synchronize()
+        got[1] += int(part)
+        pvs += each.cpu().numpy()
+        g.count_edges_shard_async(i, nshards, part, edge)
+        ctx.synchronize()
+        got[2] += int(part)
+        sups += edge.cpu().numpy()
+    assert (got == want).all()
+    np.testing.assert_array_equal(pvs, pv)
+    np.testing.assert_array_equal(sups, sup)
     g.free()

@@ -20,6 +20,14 @@
 // The reference has no counterpart: its kernels intersect sorted lists
 // (counting.cu:95-131).
 //
+// Per vertex and per edge the same blocks give every triangle's other corners
+// and edges. With S the symmetric adjacency matrix of the core, D = X S under the
+// mask X holds for each edge u->c of the row block its core triangles whose lowest
+// corner is u: D's row sums are twice u's, its column sums are those of c as a
+// middle or highest corner, and its entries the supports. The third edge v->w
+// needs the sum over u of X[u][v] X[u][w], a product along the row blocks (their
+// tiles transposed), cut into segments of row blocks.
+//
 // Operands: one byte per element in 16 KB tiles of 128 rows x 128 columns, laid
 // out in memory as a 128-byte-swizzled K-major operand sits in shared memory
 // (16-byte piece p of row r at p ^ (r & 7)), so a tile is one bulk copy.
@@ -217,9 +225,11 @@ __global__ void k_core_items(int nb, const int32_t *__restrict__ jw, const int32
 // The operand tiles, two chunks (32 KB) per CTA, set in shared memory and
 // written out whole: two threads a row set the row's bytes from the first of
 // its positions in these chunks (the positions ascend from the row's end).
+// before: per tile pair and row, the row's entries at positions before them.
 __global__ void __launch_bounds__(256) k_core_tiles(int64_t nv, int nb, const int64_t *__restrict__ off,
                                                     const int32_t *__restrict__ col,
-                                                    const int64_t *__restrict__ tile0, uint8_t *__restrict__ tiles) {
+                                                    const int64_t *__restrict__ tile0, uint8_t *__restrict__ tiles,
+                                                    uint16_t *__restrict__ before) {
   __shared__ __align__(16) uint8_t s_t[2 * kCoreTile];
   const int lane = threadIdx.x & 31, r = threadIdx.x >> 1;
   const int64_t t = 2 * int64_t(blockIdx.x);
@@ -243,6 +253,7 @@ __global__ void __launch_bounds__(256) k_core_tiles(int64_t nv, int nb, const in
       if (nv - 1 - int64_t(col[mid]) >= c0) lo = mid + 1;
       else hi = mid;
     }
+    if ((threadIdx.x & 1) == 0) before[t / 2 * kCoreRows + r] = uint16_t(e1 - lo);
     for (int64_t p = lo - 1 - (threadIdx.x & 1); p >= e0; p -= 2) {
       const int64_t c = nv - 1 - int64_t(col[p]) - c0;
       if (c >= kCoreStep) break;
@@ -263,6 +274,11 @@ constexpr int kCoreThreads = 192;
 constexpr size_t kCoreSmem = size_t(kCoreStages) * kCoreStageBytes + 1024;
 constexpr uint32_t kCoreWaitLimit = 1u << 22;
 
+// what a product gives: the total; every vertex's count; every edge's, for the
+// edges from the row blocks, and for the edges inside the core
+enum CoreKind { kCoreTotal = 0, kCoreVertices = 1, kCoreEdges = 2, kCoreInner = 3 };
+constexpr int kCoreSeg = 64;  // kCoreInner: row blocks of one item, at most
+
 struct CoreArgs {
   const uint8_t *tiles;
   const int64_t *tile0;
@@ -271,6 +287,22 @@ struct CoreArgs {
   int64_t stride;
   unsigned long long *global;
   int *err;
+  // per vertex and per edge
+  const uint8_t *sym;      // S: tile (row block, chunk) at row block * 2 jtop + chunk
+  const int32_t *jw;
+  int jtop;
+  int shard, nshards;      // of the row blocks (kCoreInner: of the items)
+  int64_t nv;
+  const int64_t *off, *poff;
+  const uint16_t *before;
+  unsigned long long *rows2;  // twice the count of each row as the lowest corner
+  unsigned long long *pv;
+  unsigned int *es;
+  // kCoreInner
+  const uint8_t *xt;       // the transposed tiles
+  const int32_t *list;     // level t: first tiles of the row blocks wider than t steps, nb entries each
+  const int32_t *count;    // ... how many
+  int nb;
 };
 
 __device__ __forceinline__ uint32_t core_smem(const void *p) {
@@ -337,17 +369,53 @@ __device__ __forceinline__ void core_ld32(uint32_t taddr, int32_t (&v)[32]) {
       : "r"(taddr));
 }
 
+// An item of one kind: its accumulator's rows are row block b, its columns the
+// positions 256 j on; `steps` chunk steps.
+struct CoreItem {
+  int b, j, steps;
+  int level, first;  // kCoreInner: the list, and the first of its entries
+};
+// item i of the launch; false when it is another shard's
+template <int KIND>
+__device__ __forceinline__ bool core_item(const CoreArgs &a, const int32_t *pfx, int64_t i, CoreItem &it) {
+  it.level = it.first = 0;
+  if (KIND == kCoreInner) {
+    if (a.nshards > 1 && i % a.nshards != a.shard) return false;
+    int t = 0;  // the level holding item i
+    while (int64_t(pfx[t + 1]) <= i) t++;
+    const int segs = (a.count[t] + kCoreSeg - 1) / kCoreSeg, k = int(i - pfx[t]);
+    const int cell = k / segs;  // (row block 2t or 2t + 1, column step 0 .. t)
+    it.b = 2 * t + (cell > t);
+    it.j = cell > t ? cell - t - 1 : cell;
+    it.level = t;
+    it.first = (k - cell * segs) * kCoreSeg;
+    it.steps = min(kCoreSeg, a.count[t] - it.first);
+    return true;
+  }
+  const int2 x = a.items[i * a.stride];
+  it.b = x.x;
+  it.j = x.y;
+  if (KIND == kCoreTotal) {
+    it.steps = 2 * x.y + 2;
+    return true;
+  }
+  it.steps = 2 * a.jw[x.x];
+  return a.nshards <= 1 || x.x % a.nshards == a.shard;
+}
+
 // One persistent CTA per SM. Warp 0 brings in the tiles of each chunk step,
 // warp 1 issues the products of unsigned bytes into one of two 256-column
-// accumulators (32-bit integers: exact), warps 2 to 5 read the other, multiply
-// it by X[u][v] (the item's last two chunks of X) and sum. Bound by the tile
-// reads from L2: 48 KB a step against 512 cycles of tensor work.
+// accumulators (32-bit integers: exact), warps 2 to 5 read the other and add it
+// up under its mask (the item's two chunks of X): 3.8e15 operations/s on R-MAT
+// 2^24, near the tensor rate; 48 KB are read from L2 a step.
+template <int KIND>
 __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *st = smem_raw + ((1024 - (core_smem(smem_raw) & 1023)) & 1023);
   __shared__ __align__(8) uint64_t s_full[kCoreStages], s_empty[kCoreStages], s_tfull[2], s_tempty[2], s_drain;
   __shared__ uint32_t s_tmem;
   __shared__ int s_fail;
+  __shared__ int32_t s_pfx[kCoreMaxJ + 2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kCoreStages; i++) {
@@ -360,6 +428,14 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
     }
     core_bar_init(&s_drain, 1);
     s_fail = 0;
+    if (KIND == kCoreInner) {  // items before each level
+      int32_t at = 0;
+      for (int t = 0; t < a.jtop; t++) {
+        s_pfx[t] = at;
+        at += 2 * (t + 1) * ((a.count[t] + kCoreSeg - 1) / kCoreSeg);
+      }
+      s_pfx[a.jtop] = at;
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -373,42 +449,69 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = s_tmem;
   volatile int *fail = &s_fail;
+  const int64_t n = KIND == kCoreInner ? int64_t(s_pfx[a.jtop]) : a.n;
+  CoreItem it;
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t k = 0;  // loads issued
-      for (int64_t i = blockIdx.x; i < a.n && !*fail; i += gridDim.x) {
-        const int2 it = a.items[i * a.stride];
-        const uint8_t *x = a.tiles + a.tile0[it.x] * kCoreTile;
-        const uint8_t *y0 = a.tiles + a.tile0[2 * it.y] * kCoreTile, *y1 = a.tiles + a.tile0[2 * it.y + 1] * kCoreTile;
-        const int steps = 2 * it.y + 2;
-        for (int c = 0; c < steps; c++, k++) {
-          const uint32_t sg = k % kCoreStages, ph = (k / kCoreStages) & 1u;
-          if (!core_wait(&s_empty[sg], ph ^ 1u, fail)) break;
-          uint8_t *d = st + sg * kCoreStageBytes;
-          core_expect(&s_full[sg], kCoreStageBytes);
-          core_copy(d, x + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
-          core_copy(d + kCoreTile, y0 + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
-          core_copy(d + 2 * kCoreTile, y1 + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
-        }
+    uint32_t k = 0;  // loads issued
+    for (int64_t i = blockIdx.x; i < n; i += gridDim.x) {
+      if (!core_item<KIND>(a, s_pfx, i, it)) continue;
+      const uint8_t *x = nullptr, *y0 = nullptr, *y1 = nullptr;
+      if (KIND != kCoreInner) x = a.tiles + a.tile0[it.b] * kCoreTile;
+      if (KIND == kCoreTotal) {
+        y0 = a.tiles + a.tile0[2 * it.j] * kCoreTile;
+        y1 = a.tiles + a.tile0[2 * it.j + 1] * kCoreTile;
+      } else if (KIND != kCoreInner) {
+        y0 = a.sym + int64_t(2 * it.j) * (2 * a.jtop) * kCoreTile;
+        y1 = y0 + int64_t(2 * a.jtop) * kCoreTile;
       }
-      if (*fail)  // the copies in flight land before the CTA leaves
-        for (uint32_t q = k > kCoreStages ? k - kCoreStages : 0; q < k; q++) {
-          int quiet = 0;
-          core_wait(&s_full[q % kCoreStages], (q / kCoreStages) & 1u, &quiet);
+      bool ok = true;
+      int32_t ahead = 0;  // kCoreInner: the first tiles of 32 row blocks, one a lane
+      for (int c = 0; c < it.steps && ok; c++, k++) {
+        int64_t t = 0;
+        if (KIND == kCoreInner) {
+          if ((c & 31) == 0 && c + lane < it.steps) ahead = a.list[int64_t(it.level) * a.nb + it.first + c + lane];
+          t = __shfl_sync(0xffffffffu, ahead, c & 31);
         }
+        if (lane == 0) {
+          const uint32_t sg = k % kCoreStages, ph = (k / kCoreStages) & 1u;
+          ok = core_wait(&s_empty[sg], ph ^ 1u, fail);
+          if (ok) {
+            uint8_t *d = st + sg * kCoreStageBytes;
+            core_expect(&s_full[sg], kCoreStageBytes);
+            if (KIND == kCoreInner) {
+              core_copy(d, a.xt + (t + it.b) * kCoreTile, kCoreTile, &s_full[sg]);
+              core_copy(d + kCoreTile, a.xt + (t + 2 * it.j) * kCoreTile, 2 * kCoreTile, &s_full[sg]);
+            } else {
+              core_copy(d, x + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
+              core_copy(d + kCoreTile, y0 + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
+              core_copy(d + 2 * kCoreTile, y1 + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
+            }
+          }
+        }
+        ok = __shfl_sync(0xffffffffu, int(ok), 0);
+      }
+      if (!ok) {
+        k--;  // the last step issued none
+        break;
+      }
     }
+    if (lane == 0 && *fail)  // the copies in flight land before the CTA leaves
+      for (uint32_t q = k > kCoreStages ? k - kCoreStages : 0; q < k; q++) {
+        int quiet = 0;
+        core_wait(&s_full[q % kCoreStages], (q / kCoreStages) & 1u, &quiet);
+      }
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc = (2u << 4) | (uint32_t(kCoreStep / 8) << 17) | (uint32_t(kCoreRows / 16) << 24);
       uint32_t k = 0, t = 0;
-      for (int64_t i = blockIdx.x; i < a.n && !*fail; i += gridDim.x, t++) {
-        const int steps = 2 * a.items[i * a.stride].y + 2;
+      for (int64_t i = blockIdx.x; i < n && !*fail; i += gridDim.x) {
+        if (!core_item<KIND>(a, s_pfx, i, it)) continue;
         if (!core_wait(&s_tempty[t & 1], ((t >> 1) & 1u) ^ 1u, fail)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d = tmem + (t & 1) * kCoreStep;
         bool ok = true;
-        for (int c = 0; c < steps; c++, k++) {
+        for (int c = 0; c < it.steps; c++, k++) {
           const uint32_t sg = k % kCoreStages;
           if (!core_wait(&s_full[sg], (k / kCoreStages) & 1u, fail)) {
             ok = false;
@@ -424,6 +527,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
         }
         if (!ok) break;
         core_commit(&s_tfull[t & 1]);
+        t++;
       }
       core_commit(&s_drain);  // every product issued is done before the accumulators are given back
       int quiet = 0;
@@ -434,13 +538,18 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
     const int quad = warp & 3, r = quad * 32 + lane;  // this warp's accumulator rows
     int64_t acc = 0;
     uint32_t t = 0;
-    for (int64_t i = blockIdx.x; i < a.n; i += gridDim.x, t++) {
-      const int2 it = a.items[i * a.stride];
-      const uint8_t *x = a.tiles + (a.tile0[it.x] + 2 * it.y) * kCoreTile + r * 128;
-      uint4 m[16];  // X[u][v] of the item's 256 columns
+    for (int64_t i = blockIdx.x; i < n; i += gridDim.x) {
+      if (!core_item<KIND>(a, s_pfx, i, it)) continue;
+      const int64_t mt = a.tile0[it.b] + 2 * it.j;  // the mask's first tile
+      const uint8_t *x = a.tiles + mt * kCoreTile + r * 128;
+      uint4 m[16];  // X of the item's 256 columns
 #pragma unroll
       for (int q = 0; q < 16; q++)
         m[q] = __ldg(reinterpret_cast<const uint4 *>(x + (q >> 3) * kCoreTile + (((q & 7) ^ (r & 7)) << 4)));
+      const int64_t row = int64_t(it.b) * kCoreRows + r, u = a.nv - 1 - row;
+      unsigned int *es = nullptr;  // per edge: the row's entry at the next position
+      if ((KIND == kCoreEdges || KIND == kCoreInner) && u >= 0)
+        es = a.es + a.poff[u] + (a.off[u + 1] - a.off[u]) - 1 - a.before[mt / 2 * kCoreRows + r];
       if (!__all_sync(0xffffffffu, core_wait(&s_tfull[t & 1], (t >> 1) & 1u, fail))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       int32_t sum = 0;
@@ -449,21 +558,44 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
         int32_t v[32];
         core_ld32(tmem + (t & 1) * kCoreStep + g * 32 + (uint32_t(quad * 32) << 16), v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        int32_t cs = 0;  // per vertex: column sum of column 32 g + lane over this warp's rows
 #pragma unroll
         for (int h = 0; h < 8; h++) {
           const uint4 &q = m[2 * g + (h >> 2)];
           const uint32_t w = (h & 3) == 0 ? q.x : (h & 3) == 1 ? q.y : (h & 3) == 2 ? q.z : q.w;
-          sum += int32_t(w & 0xffu) * v[4 * h] + int32_t((w >> 8) & 0xffu) * v[4 * h + 1] +
-                 int32_t((w >> 16) & 0xffu) * v[4 * h + 2] + int32_t(w >> 24) * v[4 * h + 3];
+          if (KIND == kCoreTotal) {
+            sum += int32_t(w & 0xffu) * v[4 * h] + int32_t((w >> 8) & 0xffu) * v[4 * h + 1] +
+                   int32_t((w >> 16) & 0xffu) * v[4 * h + 2] + int32_t(w >> 24) * v[4 * h + 3];
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              const bool in = (w >> (8 * e)) & 1u;
+              const int32_t d = in ? v[4 * h + e] : 0;
+              if (KIND != kCoreInner) sum += d;
+              if (KIND == kCoreVertices) {
+                const int32_t c = __reduce_add_sync(0xffffffffu, d);
+                if (lane == 4 * h + e) cs = c;
+              } else {
+                if (d) atomicAdd(es, unsigned(d));
+                es -= in ? 1 : 0;
+              }
+            }
+          }
         }
+        if (KIND == kCoreVertices && cs)
+          atomicAdd(&a.pv[a.nv - 1 - (int64_t(it.j) * kCoreStep + g * 32 + lane)], (unsigned long long)cs);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) core_arrive(&s_tempty[t & 1]);
-      acc += sum;
+      t++;
+      if (KIND == kCoreTotal) acc += sum;
+      else if (KIND != kCoreInner && sum) atomicAdd(&a.rows2[row], (unsigned long long)sum);
     }
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0 && acc) atomicAdd(a.global, (unsigned long long)acc);
+    if (KIND == kCoreTotal) {
+      for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0 && acc) atomicAdd(a.global, (unsigned long long)acc);
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -471,6 +603,91 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
   if (threadIdx.x == 0 && s_fail && a.err) atomicOr(a.err, kErrCoreTimeout);
+}
+
+// ---- operands of the per-vertex and per-edge products ------------------------------
+
+// byte (row, column) of a tile
+__device__ __forceinline__ int core_at(int row, int col) {
+  return row * 128 + (((col >> 4) ^ (row & 7)) << 4) + (col & 15);
+}
+// 16 columns (piece p) of row r of the transpose of a tile in shared memory
+__device__ __forceinline__ uint4 core_transposed(const uint8_t *s, int r, int p) {
+  uint32_t w[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    w[q] = 0;
+#pragma unroll
+    for (int e = 0; e < 4; e++) w[q] |= uint32_t(s[core_at(16 * p + 4 * q + e, r)]) << (8 * e);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// S, tile by tile: the core's own tiles below the diagonal, their transposes
+// above it, both on it
+__global__ void __launch_bounds__(256) k_core_sym(int width, const int64_t *__restrict__ tile0,
+                                                  const uint8_t *__restrict__ tiles, uint8_t *__restrict__ sym) {
+  __shared__ __align__(16) uint8_t s_t[kCoreTile];
+  const int i = blockIdx.x / width, k = blockIdx.x % width;
+  const uint8_t *src = tiles + (i >= k ? tile0[i] + k : tile0[k] + i) * kCoreTile;
+  uint4 *out = reinterpret_cast<uint4 *>(sym + int64_t(blockIdx.x) * kCoreTile);
+  for (int q = threadIdx.x; q < kCoreTile / 16; q += 256)
+    reinterpret_cast<uint4 *>(s_t)[q] = reinterpret_cast<const uint4 *>(src)[q];
+  __syncthreads();
+  for (int q = threadIdx.x; q < kCoreTile / 16; q += 256) {
+    const int r = q >> 3, p = (q & 7) ^ (r & 7);
+    uint4 x = i >= k ? reinterpret_cast<uint4 *>(s_t)[q] : make_uint4(0, 0, 0, 0);
+    if (i <= k) {
+      const uint4 y = core_transposed(s_t, r, p);
+      x = make_uint4(x.x | y.x, x.y | y.y, x.z | y.z, x.w | y.w);
+    }
+    out[q] = x;
+  }
+}
+// every tile's transpose, in its place of a second array
+__global__ void __launch_bounds__(256) k_core_turn(const uint8_t *__restrict__ tiles, uint8_t *__restrict__ xt) {
+  __shared__ __align__(16) uint8_t s_t[kCoreTile];
+  const uint4 *src = reinterpret_cast<const uint4 *>(tiles + int64_t(blockIdx.x) * kCoreTile);
+  uint4 *out = reinterpret_cast<uint4 *>(xt + int64_t(blockIdx.x) * kCoreTile);
+  for (int q = threadIdx.x; q < kCoreTile / 16; q += 256) reinterpret_cast<uint4 *>(s_t)[q] = src[q];
+  __syncthreads();
+  for (int q = threadIdx.x; q < kCoreTile / 16; q += 256) {
+    const int r = q >> 3;
+    out[q] = core_transposed(s_t, r, (q & 7) ^ (r & 7));
+  }
+}
+// level blockIdx.x: the row blocks wider than that many steps, by their first tiles
+__global__ void __launch_bounds__(1024) k_core_levels(int nb, const int32_t *__restrict__ jw,
+                                                      const int64_t *__restrict__ tile0, int32_t *__restrict__ list,
+                                                      int32_t *__restrict__ count) {
+  using Scan = cub::BlockScan<int, 1024>;
+  __shared__ typename Scan::TempStorage ts;
+  int at = 0;
+  for (int b0 = 0; b0 < nb; b0 += 1024) {
+    const int b = b0 + threadIdx.x, in = b < nb && jw[b] > int(blockIdx.x);
+    int pos, tot;
+    Scan(ts).ExclusiveSum(in, pos, tot);
+    if (in) list[int64_t(blockIdx.x) * nb + at + pos] = int32_t(tile0[b]);
+    at += tot;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) count[blockIdx.x] = at;
+}
+// half of each row's doubled count: to its vertex, and all of them to the total
+__global__ void __launch_bounds__(256) k_core_halves(const unsigned long long *__restrict__ rows2, int64_t rows,
+                                                     int64_t nv, unsigned long long *__restrict__ total,
+                                                     unsigned long long *__restrict__ pv) {
+  unsigned long long sum = 0;
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < rows; i += int64_t(gridDim.x) * blockDim.x) {
+    const unsigned long long h = rows2[i] / 2;
+    if (!h) continue;
+    sum += h;
+    if (pv) atomicAdd(&pv[nv - 1 - i], h);
+  }
+  using Red = cub::BlockReduce<unsigned long long, 256>;
+  __shared__ typename Red::TempStorage ts;
+  sum = Red(ts).Sum(sum);
+  if (threadIdx.x == 0 && sum) atomicAdd(total, sum);
 }
 
 // ---- host side ------------------------------------------------------------------
@@ -510,7 +727,9 @@ xt_status core_decide(Ctx *c, Graph *g, const int64_t *sums) {
   }
   k.n_tiles = sums[0];
   k.n_items = sums[1];
+  k.jtop = int(sums[2]);
   XT_TRY(dalloc_n(c, &k.d_tiles, size_t(sums[0]) * kCoreTile));
+  XT_TRY(dalloc_n(c, &k.d_before, size_t(sums[0] / 2) * kCoreRows));
   return dalloc_n(c, &k.d_items, size_t(sums[1]));
 }
 
@@ -519,36 +738,107 @@ xt_status core_finish(Ctx *c, Graph *g) {
   Core &k = g->core;
   if (k.n_items == 0) return XT_OK;
   k_core_tiles<<<counted(c, dim3(unsigned(k.n_tiles / 2))), 256, 0, c->stream>>>(g->nv, k.nb, g->d_off, g->d_col,
-                                                                                 k.d_tile0, k.d_tiles);
+                                                                                 k.d_tile0, k.d_tiles, k.d_before);
   k_core_items<<<counted(c, dim3(unsigned((k.nb + 255) / 256))), 256, 0, c->stream>>>(k.nb, k.d_jw, k.d_item0,
                                                                                      k.d_items);
   XT_CUDA(c, cudaGetLastError());
-  XT_CUDA(c, cudaFuncSetAttribute(k_core_count, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCoreSmem)));
+  for (auto fn : {k_core_count<kCoreTotal>, k_core_count<kCoreVertices>, k_core_count<kCoreEdges>,
+                  k_core_count<kCoreInner>})
+    XT_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCoreSmem)));
   return XT_OK;
 }
 
-// adds the core's triangles of every nshards-th item from `shard` to *d_global
-xt_status core_count(Graph *g, int64_t *d_global, int shard, int nshards) {
+// adds the core's triangles to *d_global: of every nshards-th item from
+// `shard`, or, with d_pv (internal numbering) or d_es (padded column positions),
+// of every nshards-th row block, with each triangle credited to its vertices
+// or edges. The operands of the latter are built by their first count and kept;
+// a count recorded into a CUDA graph before that builds its own each time.
+xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d_es, int shard, int nshards) {
   Ctx *c = g->ctx;
-  const Core &k = g->core;
-  if (k.n_items <= shard) return XT_OK;
-  CoreArgs a;
+  Core &k = g->core;
+  CoreArgs a = {};
   a.tiles = k.d_tiles;
   a.tile0 = k.d_tile0;
-  a.items = k.d_items + shard;
-  a.n = (k.n_items - shard + nshards - 1) / nshards;
-  a.stride = nshards;
+  a.items = k.d_items;
+  a.n = k.n_items;
+  a.stride = 1;
   a.global = reinterpret_cast<unsigned long long *>(d_global);
   a.err = c->d_err;
-  const unsigned grid = unsigned(std::min<int64_t>(a.n, c->sm_count));
-  k_core_count<<<counted(c, dim3(grid)), kCoreThreads, kCoreSmem, c->stream>>>(a);
+  a.nv = g->nv;
+  if (!d_pv && !d_es) {
+    if (k.n_items <= shard) return XT_OK;
+    a.items = k.d_items + shard;
+    a.n = (k.n_items - shard + nshards - 1) / nshards;
+    a.stride = nshards;
+    const unsigned grid = unsigned(std::min<int64_t>(a.n, c->sm_count));
+    k_core_count<kCoreTotal><<<counted(c, dim3(grid)), kCoreThreads, kCoreSmem, c->stream>>>(a);
+    XT_CUDA(c, cudaGetLastError());
+    return XT_OK;
+  }
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) cudaGetLastError();
+  const bool keep = cap == cudaStreamCaptureStatusNone;
+  const int width = 2 * k.jtop;
+  uint8_t *sym = k.d_sym, *xt = k.d_xt;
+  int32_t *list = k.d_list;
+  if (!sym) {
+    XT_TRY(dalloc_n(c, &sym, size_t(width) * width * kCoreTile));
+    if (keep) k.d_sym = sym;
+    k_core_sym<<<counted(c, dim3(unsigned(width * width))), 256, 0, c->stream>>>(width, k.d_tile0, k.d_tiles, sym);
+  }
+  if (d_es && !xt) {
+    if (!list) XT_TRY(dalloc_n(c, &list, size_t(k.jtop) * k.nb + k.jtop));
+    if (keep) k.d_list = list;
+    XT_TRY(dalloc_n(c, &xt, size_t(k.n_tiles) * kCoreTile));
+    if (keep) k.d_xt = xt;
+    k_core_turn<<<counted(c, dim3(unsigned(k.n_tiles))), 256, 0, c->stream>>>(k.d_tiles, xt);
+    k_core_levels<<<counted(c, dim3(unsigned(k.jtop))), 1024, 0, c->stream>>>(k.nb, k.d_jw, k.d_tile0, list,
+                                                                             list + int64_t(k.jtop) * k.nb);
+  }
   XT_CUDA(c, cudaGetLastError());
+  const int64_t rows = int64_t(k.nb) * kCoreRows;
+  unsigned long long *rows2 = nullptr;
+  XT_TRY(dalloc_n(c, &rows2, size_t(rows)));
+  cudaError_t e = cudaMemsetAsync(rows2, 0, sizeof(*rows2) * rows, c->stream);
+  a.sym = sym;
+  a.jw = k.d_jw;
+  a.jtop = k.jtop;
+  a.shard = shard;
+  a.nshards = nshards;
+  a.off = g->d_off;
+  a.poff = g->d_poff;
+  a.before = k.d_before;
+  a.rows2 = rows2;
+  a.pv = reinterpret_cast<unsigned long long *>(d_pv);
+  a.es = d_es;
+  a.xt = xt;
+  a.list = list;
+  a.count = list + int64_t(k.jtop) * k.nb;
+  a.nb = k.nb;
+  const unsigned grid = unsigned(c->sm_count);
+  if (e == cudaSuccess) {
+    if (d_es) {
+      k_core_count<kCoreEdges><<<counted(c, dim3(grid)), kCoreThreads, kCoreSmem, c->stream>>>(a);
+      k_core_count<kCoreInner><<<counted(c, dim3(grid)), kCoreThreads, kCoreSmem, c->stream>>>(a);
+    } else {
+      k_core_count<kCoreVertices><<<counted(c, dim3(grid)), kCoreThreads, kCoreSmem, c->stream>>>(a);
+    }
+    k_core_halves<<<counted(c, dim3(unsigned(std::min<int64_t>(rows / 256 + 1, c->sm_count * 4)))), 256, 0,
+                    c->stream>>>(rows2, std::min(rows, g->nv), g->nv, a.global, a.pv);
+    e = cudaGetLastError();
+  }
+  dfree(c, rows2);
+  if (sym != k.d_sym) dfree(c, sym);
+  if (xt != k.d_xt) dfree(c, xt);
+  if (list != k.d_list) dfree(c, list);
+  XT_CUDA(c, e);
   return XT_OK;
 }
 
 void core_free(Graph *g) {
   Core &k = g->core;
-  for (void *p : {(void *)k.d_tile0, (void *)k.d_tiles, (void *)k.d_items}) dfree(g->ctx, p);
+  for (void *p : {(void *)k.d_tile0, (void *)k.d_tiles, (void *)k.d_before, (void *)k.d_items, (void *)k.d_sym, (void *)k.d_xt,
+                  (void *)k.d_list}) dfree(g->ctx, p);
   g->core = Core{};
 }
 

@@ -1841,8 +1841,10 @@ static xt_status exclusive_scan(Ctx *c, const int64_t *in, int64_t *out, int64_t
   return XT_OK;
 }
 
-static void free_one_plan(Ctx *c, Plan *pl) {
+void free_plan(Graph *g) {
+  Plan *pl = g->plan;
   if (!pl) return;
+  Ctx *c = g->ctx;
   dfree(c, pl->d_bt);
   dfree(c, pl->d_ct);
   dfree(c, pl->d_bt0);
@@ -1851,12 +1853,7 @@ static void free_one_plan(Ctx *c, Plan *pl) {
   dfree(c, pl->d_tt);
   dfree(c, pl->d_cursor);
   delete pl;
-}
-
-void free_plan(Graph *g) {
-  free_one_plan(g->ctx, g->plan);
-  free_one_plan(g->ctx, g->plan_all);
-  g->plan = g->plan_all = nullptr;
+  g->plan = nullptr;
 }
 
 static xt_status d2h(Ctx *c, void *h, const void *d, size_t bytes) {
@@ -1925,11 +1922,12 @@ static xt_status plan_cluster(Ctx *c, Graph *g, Plan *pl, const int64_t *iend, c
   return s;
 }
 
-// the schedule of the records up to iend[v] of every head
-static xt_status plan_records(Graph *g, const int64_t *iend, Plan **out) {
+xt_status make_plan(Graph *g) {
   Ctx *c = g->ctx;
+  free_plan(g);
   Plan *pl = new Plan();
-  *out = pl;
+  g->plan = pl;
+  const int64_t *iend = g->d_iend;
   const int64_t nv = g->nv, ne = g->ne;
   const int B = 256;
   int64_t *P = nullptr, *nb = nullptr, *nw = nullptr, *nt = nullptr, *nbp = nullptr, *nwp = nullptr,
@@ -2101,16 +2099,8 @@ static xt_status plan_records(Graph *g, const int64_t *iend, Plan **out) {
   dfree(c, ntp);
   dfree(c, pk);
   dfree(c, stats);
-  if (s != XT_OK) {
-    free_one_plan(c, pl);
-    *out = nullptr;
-  }
+  if (s != XT_OK) free_plan(g);
   return s;
-}
-
-xt_status make_plan(Graph *g) {
-  free_plan(g);
-  return plan_records(g, g->d_iend, &g->plan);
 }
 
 int64_t cluster_task_count(const Graph *g) { return g->plan ? g->plan->n_ctask : 0; }
@@ -2184,10 +2174,7 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   if (nshards < 1 || shard < 0 || shard >= nshards)
     return set_error(c, XT_ERR_INVALID, "shard must lie in [0, nshards) and nshards be at least 1");
   if (!g->plan) XT_TRY(make_plan(g));
-  // with a core, the per-vertex and per-edge counts stream every record
-  const bool core = g->core.n_items > 0 && !d_pv && !d_support, all = g->core.n_items > 0 && !core;
-  if (all && !g->plan_all) XT_TRY(plan_records(g, g->d_ioff + 1, &g->plan_all));
-  Plan *pl = all ? g->plan_all : g->plan;
+  Plan *pl = g->plan;
   // pairs of columns are read with 32-byte vector loads
   if (reinterpret_cast<uintptr_t>(g->d_colp) % 32 != 0)
     return set_error(c, XT_ERR_CUDA, "padded column array is not 32-byte aligned");
@@ -2225,7 +2212,7 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   a.colp = g->d_colp;
   a.poff = g->d_poff;
   a.ioff = g->d_ioff;
-  a.iend = all ? g->d_ioff + 1 : g->d_iend;
+  a.iend = g->d_iend;
   a.rec = g->d_irec;
   a.rec_u = g->d_irec_u;
   a.bt = shard_first(pl->d_bt, pl->n_btask, shard);
@@ -2250,14 +2237,15 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   a.bitmap_bits = pl->bitmap_bits;
   a.cuckoo_iters = g->cuckoo_iters >= 0 ? g->cuckoo_iters : kCuckooIters;
   a.err = c->d_err;
-  if (g->ne > 0) {
+  xt_status s = XT_OK;
+  if (g->core.n_items > 0) s = core_count(g, d_global, pv_int, es, shard, nshards);
+  if (g->ne > 0 && s == XT_OK) {
     if (d_support)
       k_count<2, false><<<counted(c, pl->grid_es), kThreads, count_smem_bytes(true), c->stream>>>(a);
     else if (d_pv)
       k_count<1, false><<<counted(c, pl->grid_pv), kThreads, count_smem_bytes(true), c->stream>>>(a);
     else {
       // cluster heads leave the CTA task list to the cluster tier
-      if (core) XT_TRY(core_count(g, d_global, shard, nshards));
       CountArgs a0 = a;
       if (pl->n_ctask > 0) {
         a0.bt = shard_first(pl->d_bt0, pl->n_btask0, shard);
@@ -2271,14 +2259,15 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
         k_count_cluster<<<counted(c, dim3(pl->grid_cluster)), kThreads, sizeof(int32_t) * kBlockWords, c->stream>>>(a);
     }
   }
-  if (d_support && g->ne > 0)
+  if (d_support && g->ne > 0 && s == XT_OK)
     k_es_unpad<<<counted(c, grid_for(g->nv * 32, 256, c->sm_count)), 256, 0, c->stream>>>(es, g->d_off, g->d_poff,
                                                                                           g->nv, d_support);
-  if (d_pv && g->d_perm)
+  if (d_pv && g->d_perm && s == XT_OK)
     k_unpermute<<<counted(c, grid_for(g->nv, 256, c->sm_count)), 256, 0, c->stream>>>(pv_int, g->d_perm, g->nv, d_pv);
   cudaError_t e = cudaGetLastError();
   if (pv_int && pv_int != d_pv) dfree(c, pv_int);
   dfree(c, es);
+  XT_TRY(s);
   XT_CUDA(c, e);
   return XT_OK;
 }

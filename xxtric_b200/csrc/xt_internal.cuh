@@ -116,7 +116,13 @@ struct Core {
   int32_t *d_cut = nullptr;    // ... the first head id whose record from the block is counted here
   int32_t *d_item0 = nullptr;  // ... its items' place in the list
   uint8_t *d_tiles = nullptr;
+  uint16_t *d_before = nullptr;  // per tile pair and row: the row's entries at positions before them
   int2 *d_items = nullptr;    // (row block, column step)
+  int jtop = 0;               // the widest row block's d_jw
+  // per-vertex and per-edge counts, built by their first: the symmetric core, the
+  // transposed tiles, the row blocks wider than each step
+  uint8_t *d_sym = nullptr, *d_xt = nullptr;
+  int32_t *d_list = nullptr;
   int64_t n_tiles = 0, n_items = 0;
 };
 
@@ -135,8 +141,8 @@ struct Graph {
   int64_t *d_ioff = nullptr;  // in-record offsets per head v, nv+1
   InRec *d_irec = nullptr;    // one record per edge u->v, grouped by v (ne + 2: the last 16 bytes are slack
                               //   for 16-byte aligned bulk prefetches)
-  // the first in-record of each head that the global count does not stream
-  // (no candidates, or the core's): nv
+  // the first in-record of each head that the count does not stream (no
+  // candidates, or the core's): nv
   int64_t *d_iend = nullptr;
   Core core;
   bool no_core = false;         // the batch form counts per graph: no core
@@ -171,8 +177,7 @@ struct Graph {
   int64_t wedge_work = 0;   // sum over oriented (u,v) of d+(v)
   int64_t stream_work = 0;  // sum over u of C(d+(u), 2): the suffix columns the count streams
   int64_t colp_len = 0;     // entries of the padded column array
-  Plan *plan = nullptr;      // the global count's schedule
-  Plan *plan_all = nullptr;  // every record's schedule (per-vertex and per-edge counts of a graph with a core)
+  Plan *plan = nullptr;
 };
 
 // Optional: the rows still in host memory. build_from_edges then copies
@@ -209,7 +214,7 @@ constexpr int kErrCoreTimeout = 16;  // bit of the context's error word: a bound
 xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *cols, int64_t m, int64_t **d_sums);
 xt_status core_decide(Ctx *c, Graph *g, const int64_t *sums);
 xt_status core_finish(Ctx *c, Graph *g);
-xt_status core_count(Graph *g, int64_t *d_global, int shard, int nshards);
+xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d_es, int shard, int nshards);
 void core_free(Graph *g);
 
 // Builds (or rebuilds) the per-graph schedule and graph statistics.
