@@ -454,46 +454,60 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
 
   if (warp == 0) {
     uint32_t k = 0;  // loads issued
-    for (int64_t i = blockIdx.x; i < n; i += gridDim.x) {
-      if (!core_item<KIND>(a, s_pfx, i, it)) continue;
-      const uint8_t *x = nullptr, *y0 = nullptr, *y1 = nullptr;
-      if (KIND != kCoreInner) x = a.tiles + a.tile0[it.b] * kCoreTile;
-      if (KIND == kCoreTotal) {
-        y0 = a.tiles + a.tile0[2 * it.j] * kCoreTile;
-        y1 = a.tiles + a.tile0[2 * it.j + 1] * kCoreTile;
-      } else if (KIND != kCoreInner) {
-        y0 = a.sym + int64_t(2 * it.j) * (2 * a.jtop) * kCoreTile;
-        y1 = y0 + int64_t(2 * a.jtop) * kCoreTile;
-      }
+    // stage k's buffer once it is free, its barrier expecting the step's bytes
+    auto stage = [&]() -> uint8_t * {
+      const uint32_t sg = k % kCoreStages;
+      if (!core_wait(&s_empty[sg], ((k / kCoreStages) & 1u) ^ 1u, fail)) return nullptr;
+      core_expect(&s_full[sg], kCoreStageBytes);
+      return st + sg * kCoreStageBytes;
+    };
+    if (KIND != kCoreInner && lane == 0) {
       bool ok = true;
-      int32_t ahead = 0;  // kCoreInner: the first tiles of 32 row blocks, one a lane
-      for (int c = 0; c < it.steps && ok; c++, k++) {
-        int64_t t = 0;
-        if (KIND == kCoreInner) {
-          if ((c & 31) == 0 && c + lane < it.steps) ahead = a.list[int64_t(it.level) * a.nb + it.first + c + lane];
-          t = __shfl_sync(0xffffffffu, ahead, c & 31);
+      for (int64_t i = blockIdx.x; i < n && ok; i += gridDim.x) {
+        if (!core_item<KIND>(a, s_pfx, i, it)) continue;
+        const uint8_t *x = a.tiles + a.tile0[it.b] * kCoreTile, *y0, *y1;
+        if (KIND == kCoreTotal) {
+          y0 = a.tiles + a.tile0[2 * it.j] * kCoreTile;
+          y1 = a.tiles + a.tile0[2 * it.j + 1] * kCoreTile;
+        } else {
+          y0 = a.sym + int64_t(2 * it.j) * (2 * a.jtop) * kCoreTile;
+          y1 = y0 + int64_t(2 * a.jtop) * kCoreTile;
         }
-        if (lane == 0) {
-          const uint32_t sg = k % kCoreStages, ph = (k / kCoreStages) & 1u;
-          ok = core_wait(&s_empty[sg], ph ^ 1u, fail);
-          if (ok) {
-            uint8_t *d = st + sg * kCoreStageBytes;
-            core_expect(&s_full[sg], kCoreStageBytes);
-            if (KIND == kCoreInner) {
-              core_copy(d, a.xt + (t + it.b) * kCoreTile, kCoreTile, &s_full[sg]);
-              core_copy(d + kCoreTile, a.xt + (t + 2 * it.j) * kCoreTile, 2 * kCoreTile, &s_full[sg]);
-            } else {
-              core_copy(d, x + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
-              core_copy(d + kCoreTile, y0 + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
-              core_copy(d + 2 * kCoreTile, y1 + int64_t(c) * kCoreTile, kCoreTile, &s_full[sg]);
+        for (int c = 0; c < it.steps; c++, k++) {
+          uint8_t *d = stage();
+          if (!d) {
+            ok = false;
+            break;
+          }
+          uint64_t *bar = &s_full[k % kCoreStages];
+          core_copy(d, x + int64_t(c) * kCoreTile, kCoreTile, bar);
+          core_copy(d + kCoreTile, y0 + int64_t(c) * kCoreTile, kCoreTile, bar);
+          core_copy(d + 2 * kCoreTile, y1 + int64_t(c) * kCoreTile, kCoreTile, bar);
+        }
+      }
+    }
+    if (KIND == kCoreInner) {  // the whole warp: each lane reads one of 32 row blocks' first tiles
+      bool ok = true;
+      for (int64_t i = blockIdx.x; i < n && ok; i += gridDim.x) {
+        if (!core_item<KIND>(a, s_pfx, i, it)) continue;
+        for (int c0 = 0; c0 < it.steps && ok; c0 += 32) {
+          const int m = min(32, it.steps - c0);
+          const int32_t own = lane < m ? a.list[int64_t(it.level) * a.nb + it.first + c0 + lane] : 0;
+          for (int c = 0; c < m && ok; c++) {
+            const int64_t t = __shfl_sync(0xffffffffu, own, c);
+            if (lane == 0) {
+              uint8_t *d = stage();
+              ok = d != nullptr;
+              if (ok) {
+                uint64_t *bar = &s_full[k % kCoreStages];
+                core_copy(d, a.xt + (t + it.b) * kCoreTile, kCoreTile, bar);
+                core_copy(d + kCoreTile, a.xt + (t + 2 * it.j) * kCoreTile, 2 * kCoreTile, bar);
+                k++;
+              }
             }
+            ok = __shfl_sync(0xffffffffu, int(ok), 0);
           }
         }
-        ok = __shfl_sync(0xffffffffu, int(ok), 0);
-      }
-      if (!ok) {
-        k--;  // the last step issued none
-        break;
       }
     }
     if (lane == 0 && *fail)  // the copies in flight land before the CTA leaves
