@@ -456,15 +456,41 @@ __device__ __forceinline__ uint32_t len_class_desc(int64_t len) {
   return 127u - (c < 127u ? c : 127u);
 }
 
-// Unique rows -> the out-CSR and the unsorted in-records. A warp takes 32
-// consecutive rows, whose padded spans are contiguous in colp (and their
-// columns in col): it walks those spans 32 entries at a time, each lane
-// finding its entry's row among the 32 by a binary search over the rows'
-// padded starts, held one per lane, so the writes coalesce however short the
-// rows are. Entry t of row u is column v = bk[rstart[u] + t] while t <
-// ulen[u] (kPadSentinel after it); its out-CSR position p = off[u] + t also
-// gets the in-record of edge u->v (the suffix after t: colp[poff[u] + t + 1,
-// poff[u] + ulen[u])) and its sort key, v << lb | the suffix length's class
+// row holding position e, from a row at or before it: a few steps, then a search
+// (a run of empty rows can be long)
+__device__ __forceinline__ int64_t row_from(const int64_t *__restrict__ off, int64_t nv, int64_t r, int64_t e) {
+  for (int i = 0; i < 8; i++) {
+    if (r + 1 >= nv || off[r + 1] > e) return r;
+    r++;
+  }
+  int64_t lo = r, hi = nv;
+  while (hi - lo > 1) {
+    const int64_t mid = lo + (hi - lo) / 2;
+    if (off[mid] <= e) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+// the last row of nv starting at or before e, searched by the whole warp (33 ways a step)
+__device__ __forceinline__ int64_t row_of(const int64_t *__restrict__ off, int64_t nv, int64_t e, int lane) {
+  int64_t lo = 0, hi = nv;
+  while (hi - lo > 1) {
+    const int64_t w = (hi - lo + 31) / 32, x = lo + lane * w;
+    const unsigned m = __ballot_sync(0xffffffffu, x < hi && off[x] <= e);
+    if (m) lo += (31 - __clz(int(m))) * w;  // lane 0 fails only where e lies before every row
+    hi = lo + w < hi ? lo + w : hi;
+  }
+  return lo;
+}
+
+// Unique rows -> the out-CSR and the unsorted in-records. A warp takes spans of
+// kEmitSpan consecutive padded positions whatever their rows, 32 at a time, so
+// loads and writes coalesce and long rows are shared out (a warp per 32 rows
+// held a R-MAT 2^21 build for 0.7 ms behind its 32 longest). Entry t of row u is
+// column v = bk[rstart[u] + t] while t < ulen[u] (kPadSentinel after it); its
+// out-CSR position p = off[u] + t also gets the in-record of edge u->v (the
+// suffix after t: colp[poff[u] + t + 1, poff[u] + ulen[u])) and its sort key,
+// v << lb | the suffix length's class
 // (lb of its 7 bits, as many as fit beside v in 31 bits). With a core (cut !=
 // null) the top of the lb bits marks the records of row block b of the core's
 // nb whose head is cut[b] or above: they sort last among their head's, still
@@ -474,31 +500,39 @@ __device__ __forceinline__ uint32_t rec_class(int64_t len, bool flagged, bool co
   const uint32_t c = cb > 0 ? len_class_desc(len) >> (7 - cb) : 0u;
   return core ? c | (1u << cb) : c;
 }
-__global__ void k_rows_emit(const int64_t *__restrict__ rstart, const uint32_t *__restrict__ bk, int64_t nv, int lb,
-                            const int32_t *__restrict__ cut, int nb, const int64_t *__restrict__ off, const int64_t *__restrict__ poff,
-                            int32_t *__restrict__ col, int32_t *__restrict__ colp, uint32_t *__restrict__ ik,
-                            InRec *__restrict__ rec) {
+constexpr int kEmitSpan = 512;
+__global__ void __launch_bounds__(256) k_rows_emit(const int64_t *__restrict__ rstart,
+                                                   const uint32_t *__restrict__ bk, int64_t nv, int lb,
+                                                   const int32_t *__restrict__ cut, int nb,
+                                                   const int64_t *__restrict__ off, const int64_t *__restrict__ poff,
+                                                   int64_t total, int32_t *__restrict__ col,
+                                                   int32_t *__restrict__ colp, uint32_t *__restrict__ ik,
+                                                   InRec *__restrict__ rec) {
   const int lane = threadIdx.x & 31;
-  const int64_t w0 = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
   const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t base = w0 * 32; base < nv; base += nw * 32) {
-    const int64_t r = base + lane, rc = r < nv ? r : nv;  // lanes past nv: empty rows at the end
-    const int64_t o = off[rc], len = off[r < nv ? r + 1 : nv] - o, p = poff[rc];
-    const int64_t a = r < nv ? rstart[r] : 0;
-    const int64_t blk = (nv - 1 - r) >> 7;
-    const int32_t cu = cut && r < nv && blk < nb ? cut[blk] : 0x7fffffff;
-    const int64_t p0 = __shfl_sync(0xffffffffu, p, 0);
-    const int64_t pend = poff[base + 32 < nv ? base + 32 : nv];
-    for (int64_t q0 = p0; q0 < pend; q0 += 32) {
-      const int64_t q = q0 + lane;
-      int j = 0;  // the last row starting at or before q
+  for (int64_t w = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; w * kEmitSpan < total; w += nw) {
+    int64_t q0 = w * kEmitSpan;
+    const int64_t qend = q0 + kEmitSpan < total ? q0 + kEmitSpan : total;
+    int64_t base = row_of(poff, nv, q0, lane);
+    while (q0 < qend) {
+      // 32 rows, one a lane: padded start, out-CSR start, length, bucket, core cut
+      const int64_t r = base + lane, rc = r < nv ? r : nv;
+      const int64_t p = poff[rc], o = off[rc], a = r < nv ? rstart[r] : 0;
+      const int32_t len = int32_t(off[r < nv ? r + 1 : nv] - o);
+      const int64_t blk = (nv - 1 - r) >> 7;
+      const int32_t cu = cut && r < nv && blk < nb ? cut[blk] : 0x7fffffff;
+      const int64_t pnext = poff[base + 32 < nv ? base + 32 : nv], end = pnext < qend ? pnext : qend;
+      const bool any = end > q0;
+      for (; q0 < end; q0 += 32) {
+        const int64_t q = q0 + lane;
+        int j = 0;  // the last row starting at or before q
 #pragma unroll
-      for (int step = 16; step; step >>= 1)
-        if (__shfl_sync(0xffffffffu, p, j + step) <= q) j += step;
-      const int64_t pj = __shfl_sync(0xffffffffu, p, j), lj = __shfl_sync(0xffffffffu, len, j);
-      const int64_t oj = __shfl_sync(0xffffffffu, o, j), aj = __shfl_sync(0xffffffffu, a, j);
-      const int32_t cj = __shfl_sync(0xffffffffu, cu, j);
-      if (q < pend) {
+        for (int step = 16; step; step >>= 1)
+          if (__shfl_sync(0xffffffffu, p, j + step) <= q) j += step;
+        const int64_t pj = __shfl_sync(0xffffffffu, p, j), oj = __shfl_sync(0xffffffffu, o, j);
+        const int64_t aj = __shfl_sync(0xffffffffu, a, j);
+        const int32_t lj = __shfl_sync(0xffffffffu, len, j), cj = __shfl_sync(0xffffffffu, cu, j);
+        if (q >= end) continue;
         const int64_t t = q - pj;
         if (t < lj) {
           const uint32_t x = bk[aj + t];
@@ -511,6 +545,8 @@ __global__ void k_rows_emit(const int64_t *__restrict__ rstart, const uint32_t *
           colp[q] = kPadSentinel;
         }
       }
+      if (any) q0 = end;
+      base = any ? base + 32 : row_of(poff, nv, q0, lane);  // past a run of empty rows at once
     }
   }
 }
@@ -567,22 +603,6 @@ __global__ void k_csr_offsets(const int64_t *__restrict__ off, int64_t nv, int64
 // is set when an entry is missing from its other end's row.
 constexpr int kCsrWords = 3;
 
-// row holding entry e, from a row at or before it: a few steps, then a search
-// (a run of empty rows can be long)
-__device__ __forceinline__ int64_t row_from(const int64_t *__restrict__ off, int64_t nv, int64_t r, int64_t e) {
-  for (int i = 0; i < 8; i++) {
-    if (r + 1 >= nv || off[r + 1] > e) return r;
-    r++;
-  }
-  int64_t lo = r, hi = nv;
-  while (hi - lo > 1) {
-    const int64_t mid = lo + (hi - lo) / 2;
-    if (off[mid] <= e) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
 // Every CSR entry's row and its tail in 32 bits (ids outside [0, nv): bit 1
 // of *err), with the row checks above. A warp takes spans of kCsrSpan
 // consecutive entries whatever their rows, so a hub's row is read by as many
@@ -599,12 +619,7 @@ __global__ void k_csr_entries(const int64_t *__restrict__ off, const int64_t *__
   bool bad = false;
   for (int64_t w = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; e_first + w * kCsrSpan < ne; w += nw) {
     const int64_t b0 = e_first + w * kCsrSpan;
-    int64_t r = 0, hi = nv;  // the last row starting at or before b0
-    while (hi - r > 1) {
-      const int64_t mid = r + (hi - r) / 2;
-      if (off[mid] <= b0) r = mid;
-      else hi = mid;
-    }
+    int64_t r = row_of(off, nv, b0, lane);
     for (int i = 0; i < kCsrSpan; i += 32) {
       const int64_t e = b0 + i + lane;
       const bool in = e < ne;
@@ -1003,8 +1018,8 @@ static xt_status rows_to_csr(Ctx *c, const int64_t *rstart, uint32_t *cols_s, in
     uint32_t *kin = reinterpret_cast<uint32_t *>(kbuf), *kalt = kin + m;
     if ((s = dalloc_n(c, &r0, size_t(m) + 2)) != XT_OK) break;
     if ((s = dalloc_n(c, &r1, size_t(m) + 2)) != XT_OK) break;
-    k_rows_emit<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(
-        rstart, cols_s, nv, lb, g->core.d_cut, g->core.nb, g->d_off, g->d_poff, g->d_col, g->d_colp, kin, r0);
+    k_rows_emit<<<counted(c, grid_for((total + kEmitSpan - 1) / kEmitSpan * 32, B, c->sm_count)), B, 0, c->stream>>>(
+        rstart, cols_s, nv, lb, g->core.d_cut, g->core.nb, g->d_off, g->d_poff, total, g->d_col, g->d_colp, kin, r0);
     if ((s = cuda_status(c, cudaGetLastError(), "row emit")) != XT_OK) break;
     uint32_t *ks = nullptr;
     InRec *rs = nullptr;
