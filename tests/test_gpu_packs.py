@@ -1,5 +1,5 @@
-"""Packs (several small heads per warp) against the oracle: groups cut by large
-heads, empty heads, ragged ends, the linear-probing fallback, the id limit, and
+"""Packs (several small heads per warp; graphs with a batch of 32 edges for each
+of the GPU's 4,736 warps) against the oracle: groups cut by large heads, empty heads, ragged ends, the linear-probing fallback, the id limit, and
 their credits per vertex, per edge, per graph and per shard."""
 import numpy as np
 import pytest
@@ -19,21 +19,21 @@ def ctx():
 def graph(kind):
     rng = np.random.default_rng(5)
     if kind == "ring":  # two triangles a vertex, every head alike
-        n = 1009
+        n = 100003
         i = np.arange(n)
         return n, np.concatenate([i, i]), np.concatenate([(i + 1) % n, (i + 2) % n])
     if kind == "gaps":  # triangles between runs of vertices without edges
-        n = 5003
-        v = np.sort(rng.choice(n // 3, 300, replace=False)) * 3
+        n = 500003
+        v = np.sort(rng.choice(n // 3, 60000, replace=False)) * 3
         return n, np.concatenate([v, v, v + 1]), np.concatenate([v + 1, v + 2, v + 2])
     if kind == "er":
-        n, m = 4097, 30011
+        n, m = 30017, 200011
         return n, rng.integers(0, n, m), rng.integers(0, n, m)
     if kind == "mixed":  # small heads beside some with hundreds of members
-        n = 3001
+        n = 40001
         a, b = np.triu_indices(700, 1)
         keep = rng.random(len(a)) < 0.5
-        m = rng.integers(0, n, (2, 9000))
+        m = rng.integers(0, n, (2, 200000))
         p = rng.permutation(n)
         return n, p[np.concatenate([a[keep], m[0]])], p[np.concatenate([b[keep], m[1]])]
     raise ValueError(kind)
@@ -87,7 +87,7 @@ def test_packs_credit_graphs_and_shards(ctx):
 @pytest.mark.parametrize("nv", [(1 << 26) - 2, (1 << 26) - 1, (1 << 26) + 5])
 def test_ids_at_the_pack_limit(ctx, nv):
     # triangles at both ends of the ids; past the limit the heads run one by one
-    v = np.concatenate([np.arange(0, 300, 3), np.arange(nv - 300, nv - 2, 3)])
+    v = np.concatenate([np.arange(0, 90000, 3), np.arange(nv - 90000, nv - 2, 3)])
     src = np.concatenate([v, v, v + 1]).astype(np.int32)
     dst = np.concatenate([v + 1, v + 2, v + 2]).astype(np.int32)
     for orient in (0, 1):

@@ -98,6 +98,7 @@ struct PlanParams {
   int64_t warp_work;   // ... else one with d+(v) <= warp_dmax and at most this much work is a warp task
   int64_t block_work;  // items per CTA task
   int64_t pack_work;   // candidates of a pack, at most (0: no packs)
+  int64_t pack_cost;   // ... and candidates + kPackRecCost a record
   int32_t warp_dmax;
   int32_t batches_per_warp;  // CTA task: record batches per warp, at least
   int32_t lane_pairs;        // CTA task: pairs per lane on an average record, at least
@@ -259,13 +260,17 @@ __device__ __forceinline__ void classify(int64_t v, const int64_t *__restrict__ 
 // spends its time waiting (claim, members, first pair: 3 to 5 us a head).
 // pk[v]: log2 g for a pack's first head, kPackRest for its others, 0 elsewhere.
 constexpr uint8_t kPackRest = 0xff;
-constexpr int64_t kPackRecs = 4096;
-// Candidates of a pack, at most: one pack for each warp of the GPU, within
-// these bounds. Swept at 64 to 2,048 (counts in us, 0: no packs): geometric
-// graph of 2^16 vertices 52 without, 31 at 512, 44 at 2,048; of 2^20 656, 238 at
-// 512, 220 at 1,024; Chung-Lu 2^22 6,133, 5,686, 5,630; R-MAT 2^22 3,538, 3,507,
-// 3,507 (3,533 at 2,048); a batch of 256 graphs 1,860, 1,409, 1,359.
-constexpr int64_t kPackWorkMin = 256, kPackWorkMax = 1024;
+constexpr int64_t kPackRecs = 4096, kPackRecCost = 8;
+// Candidates of a pack, at most. Swept at 64 to 2,048 (counts in us, 0: no
+// packs): geometric graph of 2^20 vertices 656 without, 238 at 512, 220 at 1,024;
+// Chung-Lu 2^22 6,133, 5,686, 5,630; R-MAT 2^22 3,538, 3,507, 3,507 (3,533 at
+// 2,048); a batch of 256 graphs 1,860, 1,409, 1,359. Small graphs are cut finer, so
+// that there is a pack for every warp of the GPU: a batch of 32 records takes a warp 1
+// to 2 us, so a record counts as kPackRecCost candidates there (a geometric graph of
+// 2^16 vertices 52 us without packs, 31 with 6,600, 44 with 3,200), and graphs
+// without a batch for every warp have none (a uniform one of 9,645 vertices: 11 us
+// without, 13 with).
+constexpr int64_t kPackWorkMax = 1024;
 __global__ void k_plan_count(int64_t nv, const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
                              const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp,
                              int64_t *__restrict__ nb_out, int64_t *__restrict__ nwp_out,
@@ -290,7 +295,8 @@ __global__ void k_plan_count(int64_t nv, const int64_t *__restrict__ off, const 
         work += __shfl_xor_sync(0xffffffffu, work, o);
         rec += __shfl_xor_sync(0xffffffffu, rec, o);
         busy += __shfl_xor_sync(0xffffffffu, busy, o);
-        if (busy > 1 && mem <= pp.warp_dmax && work <= pp.pack_work && rec <= kPackRecs)
+        if (busy > 1 && mem <= pp.warp_dmax && work <= pp.pack_work && rec <= kPackRecs &&
+            work + kPackRecCost * rec <= pp.pack_cost)
           code = (lane & (2 * o - 1)) == 0 ? uint8_t(lg) : kPackRest;
       }
     }
@@ -404,14 +410,14 @@ __global__ void k_plan_fill(int64_t nv, const int64_t *__restrict__ off, const i
 }
 
 // CTA tasks run chunk-major: every head's first chunk, then every head's
-// second, ... (key: chunk index within its head, then head). Tasks that run
-// together then belong to many heads and read the same rows' suffixes while
-// they are in L2 (R-MAT s24: 40.2 -> 38.6 ms against head-major order).
+// second, ... (a stable sort by chunk within the head; the tasks are filled in
+// by head). Tasks that run together then belong to many heads and read the
+// same rows' suffixes while they are in L2 (R-MAT s24: 40.2 -> 38.6 ms against
+// head-major order).
 __global__ void k_task_keys(const Task *__restrict__ bt, int64_t n, const int64_t *__restrict__ nb_pos,
-                            uint64_t *__restrict__ key, int32_t *__restrict__ idx) {
+                            uint32_t *__restrict__ key, int32_t *__restrict__ idx) {
   XT_GRID_STRIDE(i, n) {
-    const int64_t v = bt[i].v;
-    key[i] = (uint64_t(i - nb_pos[v]) << 32) | uint64_t(v);
+    key[i] = uint32_t(i - nb_pos[bt[i].v]);
     idx[i] = int32_t(i);
   }
 }
@@ -1991,11 +1997,13 @@ xt_status make_plan(Graph *g) {
     pp.lane_pairs = XT_LANE_PAIRS;
     pp.warp_work = g->tune_warp_work > 0 ? g->tune_warp_work : (large ? XT_WARP_WORK_LARGE : kWarpWork);
     if (g->tier_warp_work >= 0) pp.warp_work = g->tier_warp_work;
-    // packs fill every warp once before they grow (tiers set by hand: none)
-    pp.pack_work = 0;
-    if (nv <= kPackMaxNv && g->tier_lane_work < 0 && g->tier_warp_work < 0) {
-      const int64_t warps = int64_t(pl->grid_global) * kWarps;
-      pp.pack_work = std::min(kPackWorkMax, std::max(kPackWorkMin, total_work / warps));
+    // packs, where every warp has a batch of records to itself; they fill every
+    // warp once before they grow (tiers set by hand: none)
+    const int64_t warps = int64_t(pl->grid_global) * kWarps;
+    pp.pack_work = pp.pack_cost = 0;
+    if (nv <= kPackMaxNv && ne >= 32 * warps && g->tier_lane_work < 0 && g->tier_warp_work < 0) {
+      pp.pack_work = kPackWorkMax;
+      pp.pack_cost = (total_work + kPackRecCost * ne) / warps;
     }
     if (g->tune_block_work > 0) {
       pp.block_work = g->tune_block_work;
@@ -2052,11 +2060,13 @@ xt_status make_plan(Graph *g) {
         nv, g->d_off, g->d_ioff, iend, P, pp, nbp, nwp, ntp, pk, pl->d_bt, pl->d_wt, pl->d_pt, pl->d_tt);
     if ((s = cuda_status(c, cudaGetLastError(), "k_plan_fill")) != XT_OK) break;
     if (pl->n_btask > 1) {  // chunk-major order
-      uint64_t *k1 = nullptr, *k2 = nullptr;
+      uint32_t *k1 = nullptr, *k2 = nullptr;
       int32_t *i1 = nullptr, *i2 = nullptr;
       Task *tmp = nullptr;
       void *tb = nullptr;
       const int64_t nt = pl->n_btask;
+      int bits = 1;  // of the largest task index of a head
+      while (bits < 32 && (int64_t(1) << bits) < nt) bits++;
       size_t bytes = 0;
       s = dalloc_n(c, &k1, size_t(nt));
       if (s == XT_OK) s = dalloc_n(c, &k2, size_t(nt));
@@ -2065,17 +2075,17 @@ xt_status make_plan(Graph *g) {
       if (s == XT_OK) s = dalloc_n(c, &tmp, size_t(nt));
       if (s == XT_OK) {
         k_task_keys<<<counted(c, grid_for(nt, B, c->sm_count)), B, 0, c->stream>>>(pl->d_bt, nt, nbp, k1, i1);
-        s = cuda_status(c, cub::DeviceRadixSort::SortPairs(nullptr, bytes, k1, k2, i1, i2, nt, 0, 64, c->stream),
+        s = cuda_status(c, cub::DeviceRadixSort::SortPairs(nullptr, bytes, k1, k2, i1, i2, nt, 0, bits, c->stream),
                         "task order");
       }
       if (s == XT_OK) s = dalloc(c, &tb, bytes);
       if (s == XT_OK)
-        s = cuda_status(c, cub::DeviceRadixSort::SortPairs(tb, bytes, k1, k2, i1, i2, nt, 0, 64, c->stream),
+        s = cuda_status(c, cub::DeviceRadixSort::SortPairs(tb, bytes, k1, k2, i1, i2, nt, 0, bits, c->stream),
                         "task order");
       if (s == XT_OK) {
         k_task_gather<<<counted(c, grid_for(nt, B, c->sm_count)), B, 0, c->stream>>>(pl->d_bt, i2, nt, tmp);
-        s = cuda_status(c, cudaMemcpyAsync(pl->d_bt, tmp, sizeof(Task) * nt, cudaMemcpyDeviceToDevice, c->stream),
-                        "task order");
+        s = cuda_status(c, cudaGetLastError(), "task order");
+        std::swap(pl->d_bt, tmp);
       }
       dfree(c, tb);
       dfree(c, k1);
