@@ -58,23 +58,6 @@ __device__ __forceinline__ int64_t find_seg(const int64_t *__restrict__ off, int
 
 // ---- union build ----------------------------------------------------------
 
-__global__ void k_globalize(const int32_t *__restrict__ src, const int32_t *__restrict__ dst, int64_t ne,
-                            const int64_t *__restrict__ eoff, const int64_t *__restrict__ voff, int64_t ng,
-                            int32_t *__restrict__ gsrc, int32_t *__restrict__ gdst, int *__restrict__ err) {
-  XT_GRID_STRIDE(e, ne) {
-    const int64_t g = find_seg(eoff, ng, e);
-    const int64_t n = voff[g + 1] - voff[g];
-    int64_t s = src[e], d = dst[e];
-    if (s < 0 || d < 0 || s >= n || d >= n) {
-      atomicOr(err, 1);
-      s = 0;
-      d = 0;
-    }
-    gsrc[e] = int32_t(voff[g] + s);
-    gdst[e] = int32_t(voff[g] + d);
-  }
-}
-
 // internal id -> graph
 __global__ void k_group_of(const int32_t *__restrict__ perm, int64_t nv, const int64_t *__restrict__ voff, int64_t ng,
                            int32_t *__restrict__ group) {
@@ -85,7 +68,7 @@ __global__ void k_group_of(const int32_t *__restrict__ perm, int64_t nv, const i
 }
 
 xt_status build_batch(Ctx *c, int64_t ng, const int64_t *h_voff, const int64_t *h_eoff, const int32_t *d_src,
-                      const int32_t *d_dst, int orient, Graph *g) {
+                      const int32_t *d_dst, int orient, Graph *g, const HostRows *upload) {
   if (ng < 1 || !h_voff || !h_eoff) return set_error(c, XT_ERR_INVALID, "batch: bad graph tables");
   if (h_voff[0] != 0 || h_eoff[0] != 0) return set_error(c, XT_ERR_INVALID, "batch: offsets must start at 0");
   for (int64_t i = 0; i < ng; i++)
@@ -95,37 +78,22 @@ xt_status build_batch(Ctx *c, int64_t ng, const int64_t *h_voff, const int64_t *
   if (nv < 1) return set_error(c, XT_ERR_INVALID, "batch: no vertices");
   if (nv > (int64_t(1) << 31) - 1) return set_error(c, XT_ERR_OVERFLOW, "batch: 2^31 or more vertices in all");
   int64_t *d_voff = nullptr, *d_eoff = nullptr;
-  int32_t *gs = nullptr, *gd = nullptr;
   xt_status s = XT_OK;
   do {
     if ((s = dalloc_n(c, &d_voff, size_t(ng + 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &d_eoff, size_t(ng + 1))) != XT_OK) break;
-    if ((s = dalloc_n(c, &gs, size_t(ne > 0 ? ne : 1))) != XT_OK) break;
-    if ((s = dalloc_n(c, &gd, size_t(ne > 0 ? ne : 1))) != XT_OK) break;
     if ((s = cuda_status(c, cudaMemcpyAsync(d_voff, h_voff, sizeof(int64_t) * (ng + 1), cudaMemcpyHostToDevice,
                                             c->stream), "H2D")) != XT_OK)
       break;
     if ((s = cuda_status(c, cudaMemcpyAsync(d_eoff, h_eoff, sizeof(int64_t) * (ng + 1), cudaMemcpyHostToDevice,
                                             c->stream), "H2D")) != XT_OK)
       break;
-    if (ne > 0)
-      k_globalize<<<counted(c, grid_for(ne, 256, c->sm_count)), 256, 0, c->stream>>>(d_src, d_dst, ne, d_eoff, d_voff,
-                                                                                     ng, gs, gd, c->d_err);
-    int h = 0;
-    if ((s = cuda_status(c, cudaMemcpyAsync(&h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "D2H")) !=
-        XT_OK)
-      break;
-    if ((s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync")) != XT_OK) break;
-    if (h) {
-      cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
-      s = set_error(c, XT_ERR_INVALID, "batch: a vertex id is outside its graph");
-      break;
-    }
     g->no_core = true;
-    if ((s = build_from_edges(c, nv, ne, gs, gd, orient, g)) != XT_OK) break;
-    dfree(c, gs);
-    dfree(c, gd);
-    gs = gd = nullptr;
+    BatchTables bt;
+    bt.eoff = d_eoff;
+    bt.voff = d_voff;
+    bt.ng = ng;
+    if ((s = build_from_edges(c, nv, ne, d_src, d_dst, orient, g, upload, bt)) != XT_OK) break;
     if ((s = dalloc_n(c, &g->d_group, size_t(nv))) != XT_OK) break;
     k_group_of<<<counted(c, grid_for(nv, 256, c->sm_count)), 256, 0, c->stream>>>(g->d_perm, nv, d_voff, ng,
                                                                                    g->d_group);
@@ -134,8 +102,6 @@ xt_status build_batch(Ctx *c, int64_t ng, const int64_t *h_voff, const int64_t *
   } while (0);
   dfree(c, d_voff);
   dfree(c, d_eoff);
-  dfree(c, gs);
-  dfree(c, gd);
   return s;
 }
 
@@ -698,16 +664,13 @@ xt_status xt_device_free(xt_ctx *ctx, void *p) {
   return XT_OK;
 }
 
-xt_status xt_graph_from_device_batch(xt_ctx *ctx, int64_t n_graphs, const int64_t *vertex_offsets,
-                                     const int64_t *edge_offsets, const int32_t *d_src, const int32_t *d_dst,
-                                     int orient, xt_graph **out) {
-  if (!ctx || !out || !vertex_offsets || !edge_offsets) return XT_ERR_INVALID;
-  *out = nullptr;
+static xt_status batch_graph(xt_ctx *ctx, int64_t n_graphs, const int64_t *vertex_offsets, const int64_t *edge_offsets,
+                             const int32_t *d_src, const int32_t *d_dst, int orient, const HostRows *upload,
+                             xt_graph **out) {
   Ctx *c = &ctx->c;
-  cudaSetDevice(c->device);
   xt_graph *gr = new (std::nothrow) xt_graph();
   if (!gr) return XT_ERR_OOM;
-  xt_status s = build_batch(c, n_graphs, vertex_offsets, edge_offsets, d_src, d_dst, orient, &gr->g);
+  xt_status s = build_batch(c, n_graphs, vertex_offsets, edge_offsets, d_src, d_dst, orient, &gr->g, upload);
   if (s == XT_OK) s = make_plan(&gr->g);
   if (s == XT_OK) s = cuda_status(c, cudaStreamSynchronize(c->stream), "build");
   if (s != XT_OK) {
@@ -720,10 +683,20 @@ xt_status xt_graph_from_device_batch(xt_ctx *ctx, int64_t n_graphs, const int64_
   return XT_OK;
 }
 
+xt_status xt_graph_from_device_batch(xt_ctx *ctx, int64_t n_graphs, const int64_t *vertex_offsets,
+                                     const int64_t *edge_offsets, const int32_t *d_src, const int32_t *d_dst,
+                                     int orient, xt_graph **out) {
+  if (!ctx || !out || !vertex_offsets || !edge_offsets) return XT_ERR_INVALID;
+  *out = nullptr;
+  cudaSetDevice(ctx->c.device);
+  return batch_graph(ctx, n_graphs, vertex_offsets, edge_offsets, d_src, d_dst, orient, nullptr, out);
+}
+
 xt_status xt_graph_from_batch(xt_ctx *ctx, int64_t n_graphs, const int64_t *vertex_offsets,
                               const int64_t *edge_offsets, const int32_t *src, const int32_t *dst, int orient,
                               xt_graph **out) {
   if (!ctx || !out || !vertex_offsets || !edge_offsets || n_graphs < 1) return XT_ERR_INVALID;
+  *out = nullptr;
   Ctx *c = &ctx->c;
   cudaSetDevice(c->device);
   const int64_t ne = edge_offsets[n_graphs];
@@ -731,12 +704,11 @@ xt_status xt_graph_from_batch(xt_ctx *ctx, int64_t n_graphs, const int64_t *vert
   int32_t *ds = nullptr, *dd = nullptr;
   XT_TRY(dalloc_n(c, &ds, size_t(ne > 0 ? ne : 1)));
   xt_status s = dalloc_n(c, &dd, size_t(ne > 0 ? ne : 1));
-  if (s == XT_OK && ne > 0) {
-    s = cuda_status(c, cudaMemcpyAsync(ds, src, sizeof(int32_t) * ne, cudaMemcpyHostToDevice, c->stream), "H2D");
-    if (s == XT_OK)
-      s = cuda_status(c, cudaMemcpyAsync(dd, dst, sizeof(int32_t) * ne, cudaMemcpyHostToDevice, c->stream), "H2D");
+  if (s == XT_OK) {
+    // the copy-in runs in chunks beside the first build step
+    const HostRows up{src, dst};
+    s = batch_graph(ctx, n_graphs, vertex_offsets, edge_offsets, ds, dd, orient, &up, out);
   }
-  if (s == XT_OK) s = xt_graph_from_device_batch(ctx, n_graphs, vertex_offsets, edge_offsets, ds, dd, orient, out);
   dfree(c, ds);
   dfree(c, dd);
   return s;

@@ -41,22 +41,59 @@ static unsigned grid_for(int64_t n, int block, int sm_count) {
 #define XT_GRID_STRIDE(i, n) \
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < (n); i += int64_t(gridDim.x) * blockDim.x)
 
+// row holding position e, from a row at or before it: a few steps, then a search
+// (a run of empty rows can be long)
+__device__ __forceinline__ int64_t row_from(const int64_t *__restrict__ off, int64_t nv, int64_t r, int64_t e) {
+  for (int i = 0; i < 8; i++) {
+    if (r + 1 >= nv || off[r + 1] > e) return r;
+    r++;
+  }
+  int64_t lo = r, hi = nv;
+  while (hi - lo > 1) {
+    const int64_t mid = lo + (hi - lo) / 2;
+    if (off[mid] <= e) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+// the last row of nv starting at or before e, searched by the whole warp (33 ways a step)
+__device__ __forceinline__ int64_t row_of(const int64_t *__restrict__ off, int64_t nv, int64_t e, int lane) {
+  int64_t lo = 0, hi = nv;
+  while (hi - lo > 1) {
+    const int64_t w = (hi - lo + 31) / 32, x = lo + lane * w;
+    const unsigned m = __ballot_sync(0xffffffffu, x < hi && off[x] <= e);
+    if (m) lo += (31 - __clz(int(m))) * w;  // lane 0 fails only where e lies before every row
+    hi = lo + w < hi ? lo + w : hi;
+  }
+  return lo;
+}
+
 // (lo[i], hi[i]) = (min, max) of row i's ends; self loops keep lo == hi and
 // are dropped later. With deg != null, every non-loop row also counts one
 // for each end: the degree with repeated rows counted again, which orders
 // the vertices as well as the true degree does (any total order gives the
-// same triangle count).
+// same triangle count). BATCH: row e0 + i's ids are local to its graph of the
+// tables (a warp looks its first row's graph up, the others step from it).
+template <bool BATCH>
 __global__ void k_edge_keys(const int32_t *__restrict__ src, const int32_t *__restrict__ dst, int64_t ne,
                             int64_t nv, uint32_t *__restrict__ lo, uint32_t *__restrict__ hi,
-                            int32_t *__restrict__ deg, int *__restrict__ err) {
-  XT_GRID_STRIDE(i, ne) {
-    int64_t s = src[i], d = dst[i];
-    if (s < 0 || d < 0 || s >= nv || d >= nv) {
-      atomicOr(err, 1);
-      s = 0;
-      d = 0;
+                            int32_t *__restrict__ deg, int *__restrict__ err, int64_t e0, const BatchTables bt) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t b = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) & ~int64_t(31); b < ne;
+       b += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t i = b + lane, g0 = BATCH ? row_of(bt.eoff, bt.ng, e0 + b, lane) : 0;
+    if (i >= ne) continue;
+    int64_t s = src[i], d = dst[i], v0 = 0, n = nv;
+    if (BATCH) {
+      const int64_t g = row_from(bt.eoff, bt.ng, g0, e0 + i);
+      v0 = bt.voff[g];
+      n = bt.voff[g + 1] - v0;
     }
-    const uint32_t l = uint32_t(s < d ? s : d), h = uint32_t(s < d ? d : s);
+    if (s < 0 || d < 0 || s >= n || d >= n) {
+      atomicOr(err, 1);
+      s = d = v0 = 0;
+    }
+    const uint32_t l = uint32_t(v0 + (s < d ? s : d)), h = uint32_t(v0 + (s < d ? d : s));
     lo[i] = l;
     hi[i] = h;
     if (deg && l != h) {
@@ -456,33 +493,6 @@ __device__ __forceinline__ uint32_t len_class_desc(int64_t len) {
     c = 32u + 4u * uint32_t(lg - 5) + uint32_t((len >> (lg - 2)) & 3);
   }
   return 127u - (c < 127u ? c : 127u);
-}
-
-// row holding position e, from a row at or before it: a few steps, then a search
-// (a run of empty rows can be long)
-__device__ __forceinline__ int64_t row_from(const int64_t *__restrict__ off, int64_t nv, int64_t r, int64_t e) {
-  for (int i = 0; i < 8; i++) {
-    if (r + 1 >= nv || off[r + 1] > e) return r;
-    r++;
-  }
-  int64_t lo = r, hi = nv;
-  while (hi - lo > 1) {
-    const int64_t mid = lo + (hi - lo) / 2;
-    if (off[mid] <= e) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-// the last row of nv starting at or before e, searched by the whole warp (33 ways a step)
-__device__ __forceinline__ int64_t row_of(const int64_t *__restrict__ off, int64_t nv, int64_t e, int lane) {
-  int64_t lo = 0, hi = nv;
-  while (hi - lo > 1) {
-    const int64_t w = (hi - lo + 31) / 32, x = lo + lane * w;
-    const unsigned m = __ballot_sync(0xffffffffu, x < hi && off[x] <= e);
-    if (m) lo += (31 - __clz(int(m))) * w;  // lane 0 fails only where e lies before every row
-    hi = lo + w < hi ? lo + w : hi;
-  }
-  return lo;
 }
 
 // Unique rows -> the out-CSR and the unsorted in-records. A warp takes spans of
@@ -1039,7 +1049,7 @@ static xt_status rows_to_csr(Ctx *c, const int64_t *rstart, uint32_t *cols_s, in
 // context stream turns each chunk into keys (and degree counts) once it has
 // landed.
 static xt_status upload_and_key(Ctx *c, const HostRows &up, int64_t nv, int64_t ne, int32_t *d_src, int32_t *d_dst,
-                                uint32_t *lo, uint32_t *hi, int32_t *deg) {
+                                uint32_t *lo, uint32_t *hi, int32_t *deg, const BatchTables &bt) {
   constexpr int kChunks = 8;
   const int B = 256;
   if (!c->copy_stream) XT_CUDA(c, cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
@@ -1062,8 +1072,9 @@ static xt_status upload_and_key(Ctx *c, const HostRows &up, int64_t nv, int64_t 
     if (s == XT_OK) s = cuda_status(c, cudaEventRecord(ev[i], c->copy_stream), "event");
     if (s == XT_OK) s = cuda_status(c, cudaStreamWaitEvent(c->stream, ev[i], 0), "event");
     if (s == XT_OK) {
-      k_edge_keys<<<counted(c, grid_for(n, B, c->sm_count)), B, 0, c->stream>>>(d_src + a, d_dst + a, n, nv,
-                                                                               lo + a, hi + a, deg, c->d_err);
+      const auto keys = bt.ng > 0 ? k_edge_keys<true> : k_edge_keys<false>;
+      keys<<<counted(c, grid_for(n, B, c->sm_count)), B, 0, c->stream>>>(d_src + a, d_dst + a, n, nv, lo + a, hi + a,
+                                                                        deg, c->d_err, a, bt);
       s = cuda_status(c, cudaGetLastError(), "k_edge_keys");
     }
   }
@@ -1075,7 +1086,7 @@ static xt_status upload_and_key(Ctx *c, const HostRows &up, int64_t nv, int64_t 
 }
 
 xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src, const int32_t *d_dst, int orient,
-                           Graph *g, const HostRows *upload) {
+                           Graph *g, const HostRows *upload, const BatchTables &bt) {
   if (nv < 1 || ne < 0) return set_error(c, XT_ERR_INVALID, "nv must be >= 1 and ne >= 0");
   if (nv > (int64_t(1) << 31) - 1) return set_error(c, XT_ERR_OVERFLOW, "nv must be below 2^31");
   if (orient != XT_ORIENT_ID && orient != XT_ORIENT_DEGREE) return set_error(c, XT_ERR_INVALID, "bad orientation");
@@ -1105,14 +1116,15 @@ xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src,
     if (ne > 0) {
       if (upload) {
         s = upload_and_key(c, *upload, nv, ne, const_cast<int32_t *>(d_src), const_cast<int32_t *>(d_dst), lo, hi,
-                           deg);
+                           deg, bt);
         if (s != XT_OK) break;
       } else {
-        k_edge_keys<<<counted(c, grid_for(ne, B, c->sm_count)), B, 0, c->stream>>>(d_src, d_dst, ne, nv, lo, hi,
-                                                                                   deg, c->d_err);
+        const auto keys = bt.ng > 0 ? k_edge_keys<true> : k_edge_keys<false>;
+        keys<<<counted(c, grid_for(ne, B, c->sm_count)), B, 0, c->stream>>>(d_src, d_dst, ne, nv, lo, hi, deg, c->d_err,
+                                                                           0, bt);
         if ((s = cuda_status(c, cudaGetLastError(), "k_edge_keys")) != XT_OK) break;
       }
-      if ((s = check_err(c, "edge list")) != XT_OK) break;
+      if ((s = check_err(c, bt.ng > 0 ? "batch" : "edge list")) != XT_OK) break;
     }
     // rank, then relabel every row in place
     if (orient == XT_ORIENT_DEGREE) {

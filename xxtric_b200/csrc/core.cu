@@ -58,6 +58,7 @@ constexpr int64_t kCandFs = 400;
 constexpr int64_t kStepFs = 2200000;
 // below this gain in all (20 us) the second launch is not worth it
 constexpr int64_t kCoreMinFs = int64_t(20) * 1000 * 1000 * 1000;
+constexpr int64_t kCoreMaxBytes = 16;  // operand bytes per edge, at most
 
 // the kCoreSums words: tiles, items, widest J, gain in fs
 
@@ -735,7 +736,9 @@ xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *col
 xt_status core_decide(Ctx *c, Graph *g, const int64_t *sums) {
   Core &k = g->core;
   if (k.nb == 0) return XT_OK;
-  if (sums[3] < kCoreMinFs || sums[1] == 0) {
+  // dropped also where the operands would outgrow the edges' own memory (a few
+  // dense rows that reach far into a sparse core)
+  if (sums[3] < kCoreMinFs || sums[1] == 0 || sums[0] * kCoreTile > kCoreMaxBytes * g->ne) {
     core_free(g);
     return XT_OK;
   }

@@ -188,10 +188,17 @@ struct HostRows {
   const int32_t *src, *dst;
 };
 
+// The graphs of a batch (device tables; ng 0: one graph): graph g's rows are
+// [eoff[g], eoff[g+1]), its ids, local in those rows, [voff[g], voff[g+1]).
+struct BatchTables {
+  const int64_t *eoff = nullptr, *voff = nullptr;
+  int64_t ng = 0;
+};
+
 // Builds the oriented CSR from a device edge list (int32 ids) of ne rows.
 // Rows may repeat, be one-directional or self loops.
 xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src, const int32_t *d_dst,
-                           int orient, Graph *g, const HostRows *upload = nullptr);
+                           int orient, Graph *g, const HostRows *upload = nullptr, const BatchTables &bt = {});
 // Builds from a device CSR (int64 offsets and tails). canonical: rows already
 // sorted, deduped, symmetric and loop-free, so no sort is needed.
 xt_status build_from_csr(Ctx *c, int64_t nv, const int64_t *d_off, const int64_t *d_tails, bool canonical,
@@ -204,7 +211,7 @@ xt_status build_from_vite(Ctx *c, const char *path, int elem_bytes, bool canonic
 // Builds the disjoint union of ng graphs (host offset tables, device edge
 // rows with graph-local ids) as one graph with a per-vertex group map.
 xt_status build_batch(Ctx *c, int64_t ng, const int64_t *h_voff, const int64_t *h_eoff, const int32_t *d_src,
-                      const int32_t *d_dst, int orient, Graph *g);
+                      const int32_t *d_dst, int orient, Graph *g, const HostRows *upload = nullptr);
 
 // The dense core (core.cu), in the builder's order: widths chosen from the
 // unique rows, kept or dropped once their sums are read back, then operands
