@@ -41,33 +41,6 @@ static unsigned grid_for(int64_t n, int block, int sm_count) {
 #define XT_GRID_STRIDE(i, n) \
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < (n); i += int64_t(gridDim.x) * blockDim.x)
 
-// row holding position e, from a row at or before it: a few steps, then a search
-// (a run of empty rows can be long)
-__device__ __forceinline__ int64_t row_from(const int64_t *__restrict__ off, int64_t nv, int64_t r, int64_t e) {
-  for (int i = 0; i < 8; i++) {
-    if (r + 1 >= nv || off[r + 1] > e) return r;
-    r++;
-  }
-  int64_t lo = r, hi = nv;
-  while (hi - lo > 1) {
-    const int64_t mid = lo + (hi - lo) / 2;
-    if (off[mid] <= e) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-// the last row of nv starting at or before e, searched by the whole warp (33 ways a step)
-__device__ __forceinline__ int64_t row_of(const int64_t *__restrict__ off, int64_t nv, int64_t e, int lane) {
-  int64_t lo = 0, hi = nv;
-  while (hi - lo > 1) {
-    const int64_t w = (hi - lo + 31) / 32, x = lo + lane * w;
-    const unsigned m = __ballot_sync(0xffffffffu, x < hi && off[x] <= e);
-    if (m) lo += (31 - __clz(int(m))) * w;  // lane 0 fails only where e lies before every row
-    hi = lo + w < hi ? lo + w : hi;
-  }
-  return lo;
-}
-
 // (lo[i], hi[i]) = (min, max) of row i's ends; self loops keep lo == hi and
 // are dropped later. With deg != null, every non-loop row also counts one
 // for each end: the degree with repeated rows counted again, which orders
@@ -678,21 +651,50 @@ __global__ void k_csr_entries(const int64_t *__restrict__ off, const int64_t *__
 }
 
 // Symmetry of sorted rows, a thread per entry: every entry (u, t) above its
-// row's id must be listed back in row t (binary search). With as many entries
+// row's id must be listed back in row t (a search from where even spacing would
+// put it). With as many entries
 // below as above, and rows without repeats, each entry below is then the one
 // that such a search found, so half the searches decide both directions. (A
 // warp per row searching every entry: 9.7 ms on a R-MAT 2^20 CSR.)
-__global__ void k_csr_back(const int64_t *__restrict__ off, const int32_t *__restrict__ rows,
+__global__ void k_csr_back(const int64_t *__restrict__ off, int64_t nv, const int32_t *__restrict__ rows,
                            const int32_t *__restrict__ t32, int64_t e_first, int64_t ne,
                            const int *__restrict__ err, unsigned long long *__restrict__ chk) {
   if (*err || chk[0] || chk[1]) return;  // decided already
   bool bad = false;
+  const double per = 1.0 / double(nv);
   for (int64_t e = e_first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < ne;
        e += int64_t(gridDim.x) * blockDim.x) {
     const int32_t u = rows[e], t = t32[e];
     if (t <= u) continue;
     int64_t lo = off[t], hi = off[t + 1];
     const int64_t end = hi;
+    // where u would stand were the row's ids spread evenly, and from there out
+    // until the two sides enclose it
+    if (hi - lo > 16) {
+      int64_t g = lo + int64_t(double(u) * per * double(hi - lo));
+      g = g < hi ? g : hi - 1;
+      int64_t w = 1;
+      while (w * w < hi - lo) w <<= 1;  // about the spread of such a guess
+      if (t32[g] < u) {
+        lo = g + 1;
+        for (; lo + w < hi; w <<= 1) {
+          if (t32[lo + w] >= u) {
+            hi = lo + w;
+            break;
+          }
+          lo += w + 1;
+        }
+      } else {
+        hi = g;
+        for (; hi - w > lo; w <<= 1) {
+          if (t32[hi - w] < u) {
+            lo = hi - w + 1;
+            break;
+          }
+          hi -= w;
+        }
+      }
+    }
     while (lo < hi) {
       const int64_t mid = lo + (hi - lo) / 2;
       if (t32[mid] < u) lo = mid + 1;
@@ -1234,7 +1236,7 @@ xt_status build_from_csr(Ctx *c, int64_t nv, const int64_t *d_off, const int64_t
       const int64_t warps = (n + kCsrSpan - 1) / kCsrSpan;
       k_csr_entries<<<counted(c, grid_for(warps * 32, B, c->sm_count)), B, 0, c->stream>>>(
           d_off, d_tails, nv, e_first, ne_in, rows, t32, c->d_err, chk);
-      k_csr_back<<<counted(c, grid_for(n, B, c->sm_count)), B, 0, c->stream>>>(d_off, rows, t32, e_first, ne_in,
+      k_csr_back<<<counted(c, grid_for(n, B, c->sm_count)), B, 0, c->stream>>>(d_off, nv, rows, t32, e_first, ne_in,
                                                                                c->d_err, chk);
     }
     if ((s = cuda_status(c, cudaGetLastError(), "csr check")) != XT_OK) break;

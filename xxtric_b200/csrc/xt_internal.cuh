@@ -247,6 +247,34 @@ int64_t cluster_task_count(const Graph *g);
 // lane tasks in the graph's plan (0 without a plan)
 int64_t lane_task_count(const Graph *g);
 
+// ---- device helpers ----------------------------------------------------------
+// row holding position e, from a row at or before it: a few steps, then a search
+// (a run of empty rows can be long)
+__device__ __forceinline__ int64_t row_from(const int64_t *__restrict__ off, int64_t nv, int64_t r, int64_t e) {
+  for (int i = 0; i < 8; i++) {
+    if (r + 1 >= nv || off[r + 1] > e) return r;
+    r++;
+  }
+  int64_t lo = r, hi = nv;
+  while (hi - lo > 1) {
+    const int64_t mid = lo + (hi - lo) / 2;
+    if (off[mid] <= e) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+// the last row of nv starting at or before e, searched by the whole warp (33 ways a step)
+__device__ __forceinline__ int64_t row_of(const int64_t *__restrict__ off, int64_t nv, int64_t e, int lane) {
+  int64_t lo = 0, hi = nv;
+  while (hi - lo > 1) {
+    const int64_t w = (hi - lo + 31) / 32, x = lo + lane * w;
+    const unsigned m = __ballot_sync(0xffffffffu, x < hi && off[x] <= e);
+    if (m) lo += (31 - __clz(int(m))) * w;  // lane 0 fails only where e lies before every row
+    hi = lo + w < hi ? lo + w : hi;
+  }
+  return lo;
+}
+
 }  // namespace xt
 
 // The host set-up of the reference's random geometric graph (host_io.cpp):
