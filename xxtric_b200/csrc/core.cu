@@ -418,6 +418,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
   __shared__ int s_fail;
   __shared__ int32_t s_pfx[kCoreMaxJ + 2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_launch_dependents();  // the streaming kernel's CTAs start as this one's leave
   if (threadIdx.x == 0) {
     for (int i = 0; i < kCoreStages; i++) {
       core_bar_init(&s_full[i], 1);

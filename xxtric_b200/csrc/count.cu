@@ -1006,6 +1006,7 @@ struct CountArgs {
   int64_t n_ct;
   int lane_merge;  // lane tasks: members found by a two-pointer merge (1) or binary search (0)
   int64_t stride;  // task lists hold every stride-th task of the schedule (a shard of it), else 1
+  int beside;      // launched as the core's kernel drains: waits for it at the end
   int claim;       // warp tasks (and groups of 32 lane tasks) taken from their cursor per atomic
   unsigned long long *cursor;     // [0] CTA, [1] warp, [2] lane, [4] pack cursors
   unsigned long long *global;     // the total
@@ -1711,6 +1712,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
     unsigned long long tot = 0;
     for (int w = 0; w < kWarps; w++) tot += s_red[w];
     atomicAdd(a.global, tot);
+    if (a.beside) pdl_wait();  // this kernel is not complete before the core's is
   }
 }
 
@@ -2186,6 +2188,24 @@ static const T *shard_first(const T *p, int64_t n, int shard) {
   return p && n > shard ? p + shard : nullptr;
 }
 
+// The streaming kernel; `beside`: it may start while the core's kernel ahead of
+// it in the stream drains, whose CTAs hold an SM each and leave one by one (R-MAT
+// 2^18 167 -> 157 us; started early behind the zeroing launch instead, the count
+// of a 65,536-vertex geometric graph went 43 -> 46 us).
+static xt_status launch_count(Ctx *c, void (*fn)(const CountArgs), int grid, size_t smem, const CountArgs &a) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = counted(c, dim3(unsigned(grid)));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = a.beside ? 1 : 0;
+  return cuda_status(c, cudaLaunchKernelEx(&cfg, fn, a), "k_count");
+}
+
 xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_groups, int64_t *d_support, int shard,
                       int nshards) {
   Ctx *c = g->ctx;
@@ -2244,6 +2264,7 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   a.ct = shard_first(pl->d_ct, pl->n_ctask, shard);
   a.n_ct = shard_len(pl->n_ctask, shard, nshards);
   a.stride = nshards;
+  a.beside = 0;
   a.claim = g->claim_block > 0 ? g->claim_block : (g->n_groups > 0 ? 4 : 1);
   a.lane_merge = g->lane_merge;
   a.cursor = pl->d_cursor;
@@ -2256,6 +2277,8 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   a.cuckoo_iters = g->cuckoo_iters >= 0 ? g->cuckoo_iters : kCuckooIters;
   a.err = c->d_err;
   xt_status s = XT_OK;
+  // the core's total is one launch, straight ahead of the streaming kernel
+  const bool core = g->core.n_items > shard && !d_pv && !d_support;
   if (g->core.n_items > 0) s = core_count(g, d_global, pv_int, es, shard, nshards);
   if (g->ne > 0 && s == XT_OK) {
     if (d_support)
@@ -2269,10 +2292,9 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
         a0.bt = shard_first(pl->d_bt0, pl->n_btask0, shard);
         a0.n_bt = shard_len(pl->n_btask0, shard, nshards);
       }
-      if (g->prefetch_suffix > 0)
-        k_count<0, true><<<counted(c, pl->grid_global), kThreads, count_smem_bytes(false), c->stream>>>(a0);
-      else
-        k_count<0, false><<<counted(c, pl->grid_global), kThreads, count_smem_bytes(false), c->stream>>>(a0);
+      a0.beside = core ? 1 : 0;
+      s = launch_count(c, g->prefetch_suffix > 0 ? k_count<0, true> : k_count<0, false>, pl->grid_global,
+                       count_smem_bytes(false), a0);
       if (pl->n_ctask > 0)
         k_count_cluster<<<counted(c, dim3(pl->grid_cluster)), kThreads, sizeof(int32_t) * kBlockWords, c->stream>>>(a);
     }

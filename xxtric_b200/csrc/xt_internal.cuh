@@ -248,6 +248,14 @@ int64_t cluster_task_count(const Graph *g);
 int64_t lane_task_count(const Graph *g);
 
 // ---- device helpers ----------------------------------------------------------
+// Programmatic dependent launch: the next kernel of the stream, if it was
+// launched so, may start now; and that kernel's wait until this one is complete
+// and its writes are visible (at once in a kernel launched the plain way).
+__device__ __forceinline__ void pdl_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // row holding position e, from a row at or before it: a few steps, then a search
 // (a run of empty rows can be long)
 __device__ __forceinline__ int64_t row_from(const int64_t *__restrict__ off, int64_t nv, int64_t r, int64_t e) {
