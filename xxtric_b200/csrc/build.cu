@@ -817,40 +817,48 @@ static xt_status exclusive_scan_i64(Ctx *c, In in, int64_t *out, int64_t n) {
   return XT_OK;
 }
 
+// the error word of the context's block, as read from the device
+static xt_status check_err_word(Ctx *c, int h, const char *what) {
+  if (!h) return XT_OK;
+  XT_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
+  const char *why = (h & 1) ? ": vertex id outside [0,nv)" : ": offsets not monotone in [0,ne]";
+  return set_error(c, XT_ERR_INVALID, std::string(what) + why);
+}
 static xt_status check_err(Ctx *c, const char *what) {
-  int h = 0;
-  XT_CUDA(c, cudaMemcpyAsync(&h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  XT_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (h) {
-    XT_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-    const char *why = (h & 1) ? ": vertex id outside [0,nv)" : ": offsets not monotone in [0,ne]";
-    return set_error(c, XT_ERR_INVALID, std::string(what) + why);
-  }
-  return XT_OK;
+  int64_t h = 0;
+  const void *at = c->d_out;
+  XT_TRY(read_words(c, 1, &at, &h));
+  return check_err_word(c, int(h & 0xffffffff), what);
 }
 
 // Degree orientation: ranks the vertices by (deg, id) into g->d_perm
 // (internal -> input id) and *o2n (input -> internal, the caller frees it).
 // The rank is a stable sort of the ids keyed by degree alone (the ids enter
 // in ascending order, so ties keep id order), on as many key bits as the
-// largest degree needs; deg is consumed.
-static xt_status rank_vertices(Ctx *c, int32_t *deg, int64_t nv, Graph *g, int32_t **o2n) {
+// largest degree needs; deg is consumed. The error word is read with that
+// degree: `what` names the input its checks belong to.
+static xt_status rank_vertices(Ctx *c, int32_t *deg, int64_t nv, Graph *g, int32_t **o2n, const char *what) {
   const int B = 256;
   int32_t *ids = nullptr, *dalt = nullptr;
-  unsigned int *d_dmax = nullptr;
+  unsigned int *d_dmax = nullptr;  // two words, to be read as one of 64 bits
   xt_status s = dalloc_n(c, &ids, size_t(nv));
   if (s == XT_OK) s = dalloc_n(c, &dalt, size_t(nv));
   if (s == XT_OK) s = dalloc_n(c, o2n, size_t(nv));
   if (s == XT_OK) s = dalloc_n(c, &g->d_perm, size_t(nv));
-  if (s == XT_OK) s = dalloc_n(c, &d_dmax, 1);
+  if (s == XT_OK) s = dalloc_n(c, &d_dmax, 2);
   unsigned int dmax = 0;
-  if (s == XT_OK) s = cuda_status(c, cudaMemsetAsync(d_dmax, 0, sizeof(unsigned int), c->stream), "memset");
+  if (s == XT_OK) s = cuda_status(c, cudaMemsetAsync(d_dmax, 0, 2 * sizeof(unsigned int), c->stream), "memset");
   if (s == XT_OK) {
     k_rank_ids<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(deg, nv, ids, d_dmax);
-    s = cuda_status(c, cudaMemcpyAsync(&dmax, d_dmax, sizeof(unsigned int), cudaMemcpyDeviceToHost, c->stream),
-                    "D2H");
+    s = cuda_status(c, cudaGetLastError(), "k_rank_ids");
   }
-  if (s == XT_OK) s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync");
+  if (s == XT_OK) {
+    const void *from[2] = {d_dmax, c->d_out};
+    int64_t h[2] = {0, 0};
+    s = read_words(c, 2, from, h);
+    dmax = (unsigned int)h[0];
+    if (s == XT_OK) s = check_err_word(c, int(h[1] & 0xffffffff), what);
+  }
   uint32_t *dk = nullptr;
   int32_t *perm = nullptr;
   if (s == XT_OK) {
@@ -971,31 +979,25 @@ static xt_status rows_to_csr(Ctx *c, const int64_t *rstart, uint32_t *cols_s, in
     // offsets of the unique rows, then the padded offsets
     if ((s = dalloc_n(c, &g->d_off, size_t(nv + 1))) != XT_OK) break;
     if ((s = exclusive_scan_i64(c, ulen, g->d_off, nv + 1)) != XT_OK) break;
-    int64_t m = 0;
-    if ((s = cuda_status(c, cudaMemcpyAsync(&m, g->d_off + nv, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream),
-                         "D2H")) != XT_OK)
-      break;
-    if ((s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync")) != XT_OK) break;
-    g->ne = m;
+    const auto plen = thrust::make_transform_iterator(thrust::counting_iterator<int64_t>(0), PadLen{g->d_off, nv});
+    if ((s = dalloc_n(c, &g->d_poff, size_t(nv + 1))) != XT_OK) break;
+    if ((s = exclusive_scan_i64(c, plen, g->d_poff, nv + 1)) != XT_OK) break;
     // the dense core's widths
-    if ((s = core_plan(c, g, rstart, cols_s, m, &d_sums)) != XT_OK) break;
+    if ((s = core_plan(c, g, rstart, cols_s, n, &d_sums)) != XT_OK) break;
+    int64_t size[2 + kCoreSums] = {};
+    {
+      const void *from[2 + kCoreSums] = {g->d_off + nv, g->d_poff + nv};
+      for (int i = 0; i < kCoreSums; i++) from[2 + i] = d_sums + i;
+      if ((s = read_words(c, d_sums ? 2 + kCoreSums : 2, from, size)) != XT_OK) break;
+    }
+    const int64_t m = size[0], total = size[1], *sums = size + 2;
+    g->ne = m;
     // Columns are read as aligned 32-byte pairs: pad so the last pair of the
     // last row stays inside the allocation.
     if ((s = dalloc_n(c, &g->d_col, size_t(m) + kColPad)) != XT_OK) break;
     if ((s = cuda_status(c, cudaMemsetAsync(g->d_col + m, 0xff, sizeof(int32_t) * kColPad, c->stream), "memset")) !=
         XT_OK)
       break;
-    if ((s = dalloc_n(c, &g->d_poff, size_t(nv + 1))) != XT_OK) break;
-    const auto plen = thrust::make_transform_iterator(thrust::counting_iterator<int64_t>(0), PadLen{g->d_off, nv});
-    if ((s = exclusive_scan_i64(c, plen, g->d_poff, nv + 1)) != XT_OK) break;
-    int64_t total = 0, sums[kCoreSums] = {};
-    if ((s = cuda_status(c, cudaMemcpyAsync(&total, g->d_poff + nv, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                                            c->stream), "D2H")) != XT_OK)
-      break;
-    if (d_sums && (s = cuda_status(c, cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, c->stream),
-                                   "D2H")) != XT_OK)
-      break;
-    if ((s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync")) != XT_OK) break;
     if (total >= kMaxColp) {
       s = set_error(c, XT_ERR_OVERFLOW, "2^35 or more padded columns: beyond what the in-records address");
       break;
@@ -1106,6 +1108,7 @@ xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src,
   xt_status s = XT_OK;
   const size_t n1 = size_t(ne > 0 ? ne : 1);
   const int64_t ne4 = (ne + 3) & ~int64_t(3);
+  const char *what = bt.ng > 0 ? "batch" : "edge list";
   do {
     if ((s = dalloc_n(c, &k0, n1 + 2)) != XT_OK) break;
     if ((s = dalloc_n(c, &k1, n1 + 2)) != XT_OK) break;
@@ -1126,11 +1129,11 @@ xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src,
                                                                            0, bt);
         if ((s = cuda_status(c, cudaGetLastError(), "k_edge_keys")) != XT_OK) break;
       }
-      if ((s = check_err(c, bt.ng > 0 ? "batch" : "edge list")) != XT_OK) break;
+      if (orient != XT_ORIENT_DEGREE && (s = check_err(c, what)) != XT_OK) break;  // else with the largest degree
     }
     // rank, then relabel every row in place
     if (orient == XT_ORIENT_DEGREE) {
-      if ((s = rank_vertices(c, deg, nv, g, &o2n)) != XT_OK) break;
+      if ((s = rank_vertices(c, deg, nv, g, &o2n, what)) != XT_OK) break;
       if (ne > 0)
         k_relabel_split<<<counted(c, grid_for(ne, B, c->sm_count)), B, 0, c->stream>>>(lo, hi, ne, o2n);
       if ((s = cuda_status(c, cudaGetLastError(), "relabel")) != XT_OK) break;
@@ -1172,7 +1175,7 @@ static xt_status build_canonical(Ctx *c, int64_t nv, const int64_t *d_off, int32
     if (orient == XT_ORIENT_DEGREE) {
       if ((s = dalloc_n(c, &deg, size_t(nv))) != XT_OK) break;
       k_degree_from_off<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(d_off, nv, deg);
-      if ((s = rank_vertices(c, deg, nv, g, &o2n)) != XT_OK) break;
+      if ((s = rank_vertices(c, deg, nv, g, &o2n, "csr")) != XT_OK) break;
       dfree(c, deg);
       deg = nullptr;
     }
@@ -1208,14 +1211,15 @@ static xt_status build_canonical(Ctx *c, int64_t nv, const int64_t *d_off, int32
 }
 
 xt_status build_from_csr(Ctx *c, int64_t nv, const int64_t *d_off, const int64_t *d_tails, bool canonical,
-                         int orient, Graph *g) {
+                         int orient, Graph *g, int64_t ne_known) {
   if (nv < 1) return set_error(c, XT_ERR_INVALID, "nv must be >= 1");
   if (nv > (int64_t(1) << 31) - 1) return set_error(c, XT_ERR_OVERFLOW, "nv must be below 2^31");
   if (orient != XT_ORIENT_ID && orient != XT_ORIENT_DEGREE) return set_error(c, XT_ERR_INVALID, "bad orientation");
-  int64_t ends[2] = {0, 0};
-  XT_CUDA(c, cudaMemcpyAsync(&ends[0], d_off, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
-  XT_CUDA(c, cudaMemcpyAsync(&ends[1], d_off + nv, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
-  XT_CUDA(c, cudaStreamSynchronize(c->stream));
+  int64_t ends[2] = {0, ne_known};
+  if (ne_known < 0) {
+    const void *from[2] = {d_off, d_off + nv};
+    XT_TRY(read_words(c, 2, from, ends));
+  }
   const int64_t e_first = ends[0], ne_in = ends[1];
   if (ne_in < 0) return set_error(c, XT_ERR_INVALID, "offsets[nv] is negative");
   if (e_first < 0 || e_first > ne_in) return set_error(c, XT_ERR_INVALID, "csr: offsets not monotone in [0,ne]");
@@ -1223,7 +1227,7 @@ xt_status build_from_csr(Ctx *c, int64_t nv, const int64_t *d_off, const int64_t
   const int64_t n = ne_in - e_first;  // entries of the rows
   int32_t *rows = nullptr, *t32 = nullptr;
   unsigned long long *chk = nullptr;
-  unsigned long long h[kCsrWords] = {0, 0, 0};
+  int64_t h[kCsrWords + 1] = {};
   xt_status s = XT_OK;
   const size_t n1 = size_t(ne_in > 0 ? ne_in : 1);
   do {
@@ -1240,9 +1244,11 @@ xt_status build_from_csr(Ctx *c, int64_t nv, const int64_t *d_off, const int64_t
                                                                                c->d_err, chk);
     }
     if ((s = cuda_status(c, cudaGetLastError(), "csr check")) != XT_OK) break;
-    if ((s = cuda_status(c, cudaMemcpyAsync(h, chk, sizeof(h), cudaMemcpyDeviceToHost, c->stream), "D2H")) != XT_OK)
-      break;
-    if ((s = check_err(c, "csr")) != XT_OK) break;
+    {
+      const void *from[kCsrWords + 1] = {chk, chk + 1, chk + 2, c->d_out};
+      if ((s = read_words(c, kCsrWords + 1, from, h)) != XT_OK) break;
+    }
+    if ((s = check_err_word(c, int(h[kCsrWords] & 0xffffffff), "csr")) != XT_OK) break;
     // rows that are canonical, promised or not, need no edge sort
     const bool sorted = h[0] == 0 && h[1] == 0 && h[2] == 0;
     if (canonical && !sorted) {

@@ -66,6 +66,26 @@ void dfree(Ctx *c, void *p) {
   cudaFreeAsync(p, c->stream);
 }
 
+struct WordList {
+  const int64_t *p[12];
+};
+__global__ void k_read_words(const WordList from, int n, int64_t *__restrict__ to) {
+  if (threadIdx.x < n) to[threadIdx.x] = *from.p[threadIdx.x];
+}
+xt_status read_words(Ctx *c, int n, const void *const *from, int64_t *to) {
+  const void *at = from[0];
+  if (n > 1) {
+    WordList w;
+    for (int i = 0; i < 12; i++) w.p[i] = static_cast<const int64_t *>(from[i < n ? i : 0]);
+    k_read_words<<<counted(c, dim3(1)), 32, 0, c->stream>>>(w, n, c->d_out->words);
+    XT_CUDA(c, cudaGetLastError());
+    at = c->d_out->words;
+  }
+  XT_CUDA(c, cudaMemcpyAsync(to, at, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, c->stream));
+  XT_CUDA(c, cudaStreamSynchronize(c->stream));
+  return XT_OK;
+}
+
 }  // namespace xt
 
 using namespace xt;
@@ -270,7 +290,7 @@ xt_status xt_graph_from_csr(xt_ctx *ctx, int64_t nv, const int64_t *offsets, con
     if (!gr) s = XT_ERR_OOM;
   }
   if (s == XT_OK) {
-    s = build_from_csr(c, nv, doff, dt, (flags & XT_CSR_CANONICAL) != 0, orient, &gr->g);
+    s = build_from_csr(c, nv, doff, dt, (flags & XT_CSR_CANONICAL) != 0, orient, &gr->g, ne);
     s = finish_build(ctx, gr, s, out);
   }
   dfree(c, doff);

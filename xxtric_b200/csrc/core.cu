@@ -712,11 +712,11 @@ __global__ void __launch_bounds__(256) k_core_halves(const unsigned long long *_
 // many as off says), and their layout; *d_sums has kCoreSums words once the
 // stream gets there. Leaves g->core empty (and *d_sums null) for graphs that
 // cannot gain.
-xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *cols, int64_t m, int64_t **d_sums) {
+xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *cols, int64_t n, int64_t **d_sums) {
   *d_sums = nullptr;
   Core &k = g->core;
-  // m edges have at most (2m)^1.5 / 6 candidates: below 2^17 edges, less than the least gain
-  if (g->no_core || m < (int64_t(1) << 17)) return XT_OK;
+  // m edges have at most (2m)^1.5 / 6 candidates: below 2^17 edges (of at most n rows), less than the least gain
+  if (g->no_core || n < (int64_t(1) << 17)) return XT_OK;
   const int64_t blocks = (g->nv + kCoreRows - 1) / kCoreRows;
   k.nb = int(std::max<int64_t>(kCoreMinBlk, std::min<int64_t>(blocks, kCoreMaxBlk)));
   // one allocation for the row blocks' tables: tile0, then jw, cut, item0

@@ -1984,8 +1984,12 @@ xt_status make_plan(Graph *g) {
     // CTA task size: large tasks amortise the member-set build and the task
     // barrier, but every CTA should still get about 16 of them
     int64_t total_work = 0;
-    if ((s = d2h(c, &total_work, stats + 4, sizeof(int64_t))) != XT_OK) break;
-    if ((s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync")) != XT_OK) break;
+    // below 2^17 edges there are at most 2^24.5 candidates and no packs: nothing
+    // here depends on how many
+    if (ne >= (int64_t(1) << 17)) {
+      const void *from = stats + 4;
+      if ((s = read_words(c, 1, &from, &total_work)) != XT_OK) break;
+    }
     PlanParams pp;
     pp.warp_dmax = kWarpDmax;
     // graphs of 2^34 or more candidates (R-MAT s24 has 2^35.3) take larger
@@ -2033,14 +2037,14 @@ xt_status make_plan(Graph *g) {
     if ((s = exclusive_scan(c, nb, nbp, nv + 1)) != XT_OK) break;
     if ((s = exclusive_scan(c, nw, nwp, nv + 1)) != XT_OK) break;
     if (lanes && (s = exclusive_scan(c, nt, ntp, nv + 1)) != XT_OK) break;
-    int64_t h[4] = {0, 0, 0, 0};
-    unsigned long long hs[5] = {0, 0, 0, 0, 0};
-    if ((s = d2h(c, &h[0], nbp + nv, sizeof(int64_t))) != XT_OK) break;
-    if ((s = d2h(c, &h[1], nwp + nv, sizeof(int64_t))) != XT_OK) break;
-    if ((s = d2h(c, &h[2], P + ne, sizeof(int64_t))) != XT_OK) break;
-    if (lanes && (s = d2h(c, &h[3], ntp + nv, sizeof(int64_t))) != XT_OK) break;
-    if ((s = d2h(c, hs, stats, sizeof(hs))) != XT_OK) break;
-    if ((s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync")) != XT_OK) break;
+    int64_t h[8] = {};
+    {
+      const void *from[8] = {nbp + nv, nwp + nv, P + ne, lanes ? ntp + nv : nullptr, stats, stats + 1, stats + 2, stats + 3};
+      if (!lanes) from[3] = nbp + nv;
+      if ((s = read_words(c, 8, from, h)) != XT_OK) break;
+      if (!lanes) h[3] = 0;
+    }
+    const int64_t *hs = h + 4;
     pl->n_btask = h[0];
     pl->n_wtask = h[1] & 0xffffffff;
     pl->n_ptask = h[1] >> 32;

@@ -23,6 +23,7 @@ struct CountOut {
   int err;
   int reserved;
   int64_t total;
+  int64_t words[12];  // read_words
 };
 
 struct Ctx {
@@ -58,6 +59,10 @@ template <class T>
 xt_status dalloc_n(Ctx *c, T **p, size_t n) {
   return dalloc(c, reinterpret_cast<void **>(p), n * sizeof(T));
 }
+
+// Waits for the context's stream and brings n words from device addresses to the
+// host in one copy (each copy into pageable memory holds the host for 7 us).
+xt_status read_words(Ctx *c, int n, const void *const *from, int64_t *to);
 
 // Records a CUDA error (if any) and converts it to a status.
 xt_status cuda_status(Ctx *c, cudaError_t e, const char *what);
@@ -200,9 +205,10 @@ struct BatchTables {
 xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src, const int32_t *d_dst,
                            int orient, Graph *g, const HostRows *upload = nullptr, const BatchTables &bt = {});
 // Builds from a device CSR (int64 offsets and tails). canonical: rows already
-// sorted, deduped, symmetric and loop-free, so no sort is needed.
+// sorted, deduped, symmetric and loop-free, so no sort is needed. ne_known: the
+// entries, where the caller has seen that the offsets start at 0 and end there.
 xt_status build_from_csr(Ctx *c, int64_t nv, const int64_t *d_off, const int64_t *d_tails, bool canonical,
-                         int orient, Graph *g);
+                         int orient, Graph *g, int64_t ne_known = -1);
 void free_graph_device(Graph *g);
 // Reads a vite binary file (8- or 4-byte fields) through pinned staging
 // buffers into a device CSR and builds from it (vite.cu).
