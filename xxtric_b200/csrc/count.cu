@@ -596,7 +596,7 @@ __device__ __forceinline__ void members_insert_at(const Members &m, const int32_
   const int32_t x = mem[i];
   if (m.bitmap) {
     const uint32_t wd = uint32_t(x >> 5) - m.base;
-    atomicOr(reinterpret_cast<unsigned int *>(&m.words[wd]), 1u << (x & 31));
+    atomicOr(reinterpret_cast<unsigned int *>(&m.words[wd]), PV ? 1u << (x & 31) : 0x80000000u >> (x & 31));
     if (PV && (i == 0 || uint32_t(mem[i - 1] >> 5) - m.base != wd)) m.idx[wd] = uint16_t(i);
   } else {
     const uint32_t slot = hash_insert(m.words, m.mask, m.shift, x);
@@ -607,7 +607,7 @@ __device__ __forceinline__ void members_insert_at(const Members &m, const int32_
 
 __device__ __forceinline__ void members_insert(const Members &m, int32_t x) {
   if (m.bitmap) {
-    atomicOr(reinterpret_cast<unsigned int *>(&m.words[uint32_t(x >> 5) - m.base]), 1u << (x & 31));
+    atomicOr(reinterpret_cast<unsigned int *>(&m.words[uint32_t(x >> 5) - m.base]), 0x80000000u >> (x & 31));
   } else {
     hash_insert(m.words, m.mask, m.shift, x);
   }
@@ -710,13 +710,18 @@ __device__ __forceinline__ void prefetch_line_l2(const void *p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
-// bitmap membership: bit (w & 31) of word (w >> 5) - base; every w outside
-// the bitmap's words lands on the zero guard word
-__device__ __forceinline__ uint32_t bitmap_test(const Members &m, int32_t w) {
+// Bitmap membership in the global count: bit 31 - (w & 31) of word (w >> 5) -
+// base, added to h; every w outside the bitmap's words lands on the zero guard
+// word. The bits stand reversed in their words, so that one shift by w brings a
+// candidate's to the top, from where it is added: R-MAT 2^22 3.50 -> 3.46 ms, 2^24
+// 20.57 -> 20.48, Chung-Lu 2^22 5.64 -> 5.615 against a shift down and a mask.
+// (The shifts by constants as multiply-adds, to spare the integer ALU: 3.63 to
+// 3.96 ms; the bits shifted into a word and counted there: 3.50.)
+__device__ __forceinline__ uint32_t bitmap_count(const Members &m, int32_t w, uint32_t h) {
   uint32_t i = uint32_t(w >> 5) - m.base;
   i = i < m.nwords ? i : m.nwords;
-  const uint32_t x = uint32_t(m.words[i]);
-  return __funnelshift_r(x, x, uint32_t(w)) & 1u;
+  const uint32_t x = __funnelshift_l(0u, uint32_t(m.words[i]), uint32_t(w));
+  return h + (x >> 31);
 }
 
 template <bool PV>
@@ -776,8 +781,9 @@ __device__ __forceinline__ int probe_pair(const int4 a, const int4 b, const Memb
                (cluster_test(m, b.x) + cluster_test(m, b.y)) + (cluster_test(m, b.z) + cluster_test(m, b.w)));
   }
   if (KIND == kKindBitmap) {
-    return int((bitmap_test(m, a.x) + bitmap_test(m, a.y)) + (bitmap_test(m, a.z) + bitmap_test(m, a.w)) +
-               (bitmap_test(m, b.x) + bitmap_test(m, b.y)) + (bitmap_test(m, b.z) + bitmap_test(m, b.w)));
+    const uint32_t p = bitmap_count(m, a.w, bitmap_count(m, a.z, bitmap_count(m, a.y, bitmap_count(m, a.x, 0u))));
+    const uint32_t q = bitmap_count(m, b.w, bitmap_count(m, b.z, bitmap_count(m, b.y, bitmap_count(m, b.x, 0u))));
+    return int(p + q);
   }
   if (KIND == kKindCuckoo) {
     return int((cuckoo_test(m, a.x) + cuckoo_test(m, a.y)) + (cuckoo_test(m, a.z) + cuckoo_test(m, a.w)) +
