@@ -74,9 +74,11 @@ __global__ void __launch_bounds__(1024) k_core_pick(int64_t nv, const int64_t *_
                                                     unsigned long long *__restrict__ gain) {
   __shared__ unsigned long long s_ben[kCoreMaxJ];
   __shared__ int s_hist[32][kCoreMaxJ];
+  __shared__ unsigned s_all;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int b = blockIdx.x;
   if (threadIdx.x < kCoreMaxJ) s_ben[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_all = 0;
   __syncthreads();
   unsigned long long ben0 = 0, ben1 = 0;
   // lane l < 4 holds the warp's row l: its end and length
@@ -89,6 +91,18 @@ __global__ void __launch_bounds__(1024) k_core_pick(int64_t nv, const int64_t *_
       end = rstart[u] + len;
     }
     if (len < kCoreMinRow) len = 0;
+    const unsigned all = __reduce_add_sync(0xffffffffu, unsigned(min(int64_t(len) * (len - 1) / 2, int64_t(1) << 20)));
+    if (lane == 0 && all) atomicAdd(&s_all, all);
+  }
+  __syncthreads();
+  // all candidates of its rows cannot pay for the narrowest width: no columns read
+  // (R-MAT 2^21 107 -> 94 us, a geometric graph of 2^20 vertices 48 -> 31)
+  if ((unsigned long long)s_all * kCandFs <= (unsigned long long)(4 * kStepFs)) {
+    if (threadIdx.x == 0) {
+      jw[b] = 0;
+      cut[b] = 0x7fffffff;
+    }
+    return;
   }
   const uint32_t top = uint32_t(nv - 1);
   for (int q = 0; q < 4; q++) {
