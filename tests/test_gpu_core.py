@@ -104,3 +104,52 @@ def test_core_shards_sum_to_the_count(ctx, nshards):
     np.testing.assert_array_equal(pvs, pv)
     np.testing.assert_array_equal(sups, sup)
     g.free()
+
+
+@pytest.mark.parametrize("first", ["recorded", "run"])
+def test_core_counts_recorded_and_replayed(ctx, first):
+    """Counts recorded into a CUDA graph and replayed twice, before and after
+    the operands of the per-edge product exist."""
+    import torch
+    import xxtric_b200 as xt
+    nv, src, dst = graph("core and tail")
+    off, tails = oracle.canon_csr(nv, src.astype(np.int64), dst.astype(np.int64))
+    want, pv = oracle.count_merge(off, tails, per_vertex=True)
+    stream = torch.cuda.Stream()
+    with xt.Context(0) as c:
+        c.set_stream(stream.cuda_stream)
+        g = c.graph_from_edges(nv, src.astype(np.int32), dst.astype(np.int32))
+        m = g.info()["n_edges"]
+        each = torch.zeros(nv, dtype=torch.int64, device="cuda")
+        edge = torch.zeros(m, dtype=torch.int64, device="cuda")
+        total = torch.zeros(3, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+
+        def counts():
+            g.count_async(total[0:1])
+            g.count_edges_async(total[1:2], edge)
+            if first == "run":  # the records' tails, which any graph's per-vertex count keeps, exist by then
+                g.count_async(total[2:3], each)
+
+        if first == "run":
+            counts()
+            c.synchronize()
+        rec = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(rec, stream=stream):
+            counts()
+        for _ in range(2):
+            total.zero_(), each.zero_(), edge.zero_()
+            torch.cuda.synchronize()
+            rec.replay()
+            torch.cuda.synchronize()
+            assert total.tolist()[:2] == [want] * 2
+            if first == "run":
+                assert int(total[2]) == want
+                np.testing.assert_array_equal(each.cpu().numpy(), pv)
+            assert int(edge.sum()) == 3 * want
+        del rec
+        torch.cuda.synchronize()
+        assert g.count() == want  # and uncaptured again
+        g.capture()
+        assert g.count() == g.count_groups()[0] == want
+        g.free()
