@@ -609,7 +609,8 @@ constexpr int kCsrWords = 3;
 // of *err), with the row checks above. A warp takes spans of kCsrSpan
 // consecutive entries whatever their rows, so a hub's row is read by as many
 // warps as its entries fill: a warp per row held a R-MAT 2^20 CSR's first
-// pass at 147 us behind its longest row.
+// pass at 147 us behind its longest row. (Rows found by a chain of loads in each lane
+// took 265 us there, by row_near 225.)
 constexpr int kCsrSpan = 256;
 __global__ void k_csr_entries(const int64_t *__restrict__ off, const int64_t *__restrict__ tails, int64_t nv,
                               int64_t e_first, int64_t ne, int32_t *__restrict__ rows, int32_t *__restrict__ t32,
@@ -625,7 +626,7 @@ __global__ void k_csr_entries(const int64_t *__restrict__ off, const int64_t *__
     for (int i = 0; i < kCsrSpan; i += 32) {
       const int64_t e = b0 + i + lane;
       const bool in = e < ne;
-      const int64_t rr = in ? row_from(off, nv, r, e) : r;
+      const int64_t rr = row_near(off, nv, r, in ? e : ne - 1, lane);
       int64_t t = in ? tails[e] : 0;
       if (t < 0 || t >= nv) {
         atomicOr(err, 1);

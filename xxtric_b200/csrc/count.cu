@@ -2164,17 +2164,33 @@ __global__ void k_rec_tails(const InRec *__restrict__ rec, int64_t ne, const int
 // per-edge counts from padded positions (row u at poff[u]) to the out-CSR's
 // (row u at off[u]), widened to 64 bits: warps take spans of out-CSR positions
 // whatever their rows (a warp per row spent 0.12 ms on R-MAT 2^20's mostly short
-// rows, spans 0.08)
+// rows, spans 0.08). A span is 256 positions, or less where the graph has too few
+// to keep every SM's warps busy: a warp walks its span 32 at a time, each step
+// a chain of loads (uniform graph of 1,639 vertices 25 us, 35 with 256 always).
+// Graphs of at most two rows a warp, or of rows that fill one on average, none
+// longer than a span, take a warp per row (span 0): no search (uniform graph of 8,739 vertices and out-degree 30 40 us
+// with spans, 38 without; R-MAT in id order, 8,192 vertices, 134 us without, 118 with).
 constexpr int kUnpadSpan = 256;
+static int unpad_span(const Graph *g, int sms) {
+  if (g->max_out_degree <= kUnpadSpan && (g->nv <= int64_t(sms) * 128 || g->ne >= 16 * g->nv)) return 0;
+  int span = kUnpadSpan;
+  while (span > 32 && g->ne < int64_t(span) * sms * 64) span /= 2;
+  return span;
+}
 __global__ void k_es_unpad(const unsigned int *__restrict__ esp, const int64_t *__restrict__ off,
-                           const int64_t *__restrict__ poff, int64_t nv, int64_t ne, int64_t *__restrict__ out) {
+                           const int64_t *__restrict__ poff, int64_t nv, int64_t ne, int span,
+                           int64_t *__restrict__ out) {
   const int lane = threadIdx.x & 31;
-  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t w = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w * kUnpadSpan < ne; w += nw) {
-    const int64_t p0 = w * kUnpadSpan;
+  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5, w0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  for (int64_t u = w0; span == 0 && u < nv; u += nw) {
+    const int64_t r0 = off[u], r1 = off[u + 1], shift = poff[u] - r0;
+    for (int64_t p = r0 + lane; p < r1; p += 32) out[p] = int64_t(esp[p + shift]);
+  }
+  for (int64_t w = w0; span != 0 && w * span < ne; w += nw) {
+    const int64_t p0 = w * span;
     int64_t r = row_of(off, nv, p0, lane);
-    for (int i = 0; i < kUnpadSpan; i += 32) {
-      const int64_t p = p0 + i + lane, u = p < ne ? row_from(off, nv, r, p) : r;
+    for (int i = 0; i < span; i += 32) {
+      const int64_t p = p0 + i + lane, u = row_near(off, nv, r, min(p, ne - 1), lane);
       if (p < ne) out[p] = int64_t(esp[poff[u] + (p - off[u])]);
       r = __shfl_sync(0xffffffffu, u, 31);
     }
@@ -2309,9 +2325,12 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
         k_count_cluster<<<counted(c, dim3(pl->grid_cluster)), kThreads, sizeof(int32_t) * kBlockWords, c->stream>>>(a);
     }
   }
-  if (d_support && g->ne > 0 && s == XT_OK)
-    k_es_unpad<<<counted(c, grid_for((g->ne + kUnpadSpan - 1) / kUnpadSpan * 32, 256, c->sm_count)), 256, 0,
-                 c->stream>>>(es, g->d_off, g->d_poff, g->nv, g->ne, d_support);
+  if (d_support && g->ne > 0 && s == XT_OK) {
+    const int span = unpad_span(g, c->sm_count);
+    const int64_t warps = span ? (g->ne + span - 1) / span : g->nv;
+    k_es_unpad<<<counted(c, grid_for(warps * 32, 256, c->sm_count)), 256, 0, c->stream>>>(
+        es, g->d_off, g->d_poff, g->nv, g->ne, span, d_support);
+  }
   if (d_pv && g->d_perm && s == XT_OK)
     k_unpermute<<<counted(c, grid_for(g->nv, 256, c->sm_count)), 256, 0, c->stream>>>(pv_int, g->d_perm, g->nv, d_pv);
   cudaError_t e = cudaGetLastError();

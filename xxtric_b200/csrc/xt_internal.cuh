@@ -277,6 +277,17 @@ __device__ __forceinline__ int64_t row_from(const int64_t *__restrict__ off, int
   }
   return lo;
 }
+// The same for a whole warp with ascending e and one r: the next 32 starts are
+// read at once and searched by shuffles, so the lanes wait for one load
+__device__ __forceinline__ int64_t row_near(const int64_t *__restrict__ off, int64_t nv, int64_t r, int64_t e, int lane) {
+  const int64_t next = r + 1 + lane < nv ? off[r + 1 + lane] : INT64_MAX;
+  int j = 0;
+#pragma unroll
+  for (int s = 16; s; s >>= 1)
+    if (__shfl_sync(0xffffffffu, next, j + s - 1) <= e) j += s;
+  if (__shfl_sync(0xffffffffu, next, j) <= e) j++;
+  return j < 32 ? r + j : row_from(off, nv, r + 32, e);
+}
 // the last row of nv starting at or before e, searched by the whole warp (33 ways a step)
 __device__ __forceinline__ int64_t row_of(const int64_t *__restrict__ off, int64_t nv, int64_t e, int lane) {
   int64_t lo = 0, hi = nv;
