@@ -1,4 +1,4 @@
-"""Packs (several small heads per warp; graphs with a batch of 32 edges for each
+"""Packs (several small heads per warp; graphs with 8 vertices and 16 edges for each
 of the GPU's 4,736 warps) against the oracle: groups cut by large heads, empty heads, ragged ends, the linear-probing fallback, the id limit, and
 their credits per vertex, per edge, per graph and per shard."""
 import numpy as np
@@ -27,7 +27,7 @@ def graph(kind):
         v = np.sort(rng.choice(n // 3, 60000, replace=False)) * 3
         return n, np.concatenate([v, v, v + 1]), np.concatenate([v + 1, v + 2, v + 2])
     if kind == "er":
-        n, m = 30017, 200011
+        n, m = 40017, 200011
         return n, rng.integers(0, n, m), rng.integers(0, n, m)
     if kind == "mixed":  # small heads beside some with hundreds of members
         n = 40001
@@ -94,3 +94,36 @@ def test_ids_at_the_pack_limit(ctx, nv):
         g = ctx.graph_from_edges(nv, src, dst, orient)
         assert g.count() == len(v)
         g.free()
+
+
+@pytest.mark.parametrize("orient", [0, 1])
+@pytest.mark.parametrize("span", [0, 40000])
+def test_long_warp_tasks_match_the_oracle(ctx, span, orient):
+    """Heads of 250 members and up to 32,000 candidates, their members' ids
+    within a warp's bitmap or (span) beyond it, some with many short records."""
+    rng = np.random.default_rng(3)
+    n, k = 70000, 500
+    hub = rng.permutation(k) * (1 + span // k)  # the ids of a dense part
+    a, b = np.triu_indices(k, 1)
+    keep = rng.random(len(a)) < 0.9
+    m = rng.integers(0, n, (2, 300000))
+    f = rng.integers(0, n, 60000)  # vertices with two neighbours in the dense part
+    h = rng.integers(0, k, (2, 60000))
+    src = np.concatenate([hub[a[keep]], m[0], f, f])
+    dst = np.concatenate([hub[b[keep]], m[1], hub[h[0]], hub[h[1]]])
+    off, tails = oracle.canon_csr(n, src.astype(np.int64), dst.astype(np.int64))
+    want, pv = oracle.count_merge(off, tails, per_vertex=True)
+    sup = oracle.edge_support(off, tails)
+    g = ctx.graph_from_edges(n, src.astype(np.int32), dst.astype(np.int32), orient)
+    for work in (0, 1 << 20, 1):  # automatic; every head of 256 members on a warp; on CTAs
+        g.set_tuning(0, work, 0)
+        assert g.count() == want
+        total, each = g.count(per_vertex=True)
+        assert total == want
+        np.testing.assert_array_equal(each, pv)
+    g.set_tuning(0, 0, 0)
+    u = np.repeat(np.arange(n), np.diff(off))
+    up = u < tails
+    a, b, s = g.edge_support()
+    np.testing.assert_array_equal(s[np.lexsort((b, a))], sup[up][np.lexsort((tails[up], u[up]))])
+    g.free()

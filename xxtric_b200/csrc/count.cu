@@ -18,8 +18,9 @@
 // Schedule (make_plan): per head v, work(v) = total suffix length.
 //   lane tier: work(v) <= tiny_work -> one lane per head, members
 //              binary-searched in the row itself
-//   warp tier: d+(v) <= kWarpDmax and work(v) <= warp_work -> one warp per
-//              head, member set in the warp's slice of shared memory
+//   warp tier: d+(v) <= kWarpDmax and work(v) and v's records within what a
+//              warp does in time (kWarpCost) -> one warp per head, member
+//              set in the warp's slice of shared memory
 //   pack     : 2 to 32 consecutive heads of few members and little work
 //              between them -> one warp, their members in one set keyed by
 //              (member, head)
@@ -44,21 +45,28 @@ namespace xt {
 #ifndef XT_THREADS
 #define XT_THREADS 256
 #endif
-// CTA tasks of up to 2^17 candidates, warp tasks of up to 4,096 (8,192 on
-// graphs of 2^34 or more candidates): swept with the cuckoo member sets
-// (R-MAT s24 / s22 / Chung-Lu 27.32 / 4.70 / 7.99 ms at 2^17 and 8,192
-// against 28.09 / 4.99 / 8.39 at 2^16 and 4,096; at 2^17, 4,096 gave 27.69 /
-// 4.72 / 7.97; 2^18 28.52 ms at s24; 32,768 9.49 ms on Chung-Lu). On small
-// graphs the larger warp limit moves heads onto warp tasks, which run last
-// and leave a tail: R-MAT s18 0.195 -> 0.35 ms with 8,192.
+// CTA tasks of up to 2^17 candidates: swept with the cuckoo member sets
+// (R-MAT s24 / s22 / Chung-Lu 27.32 / 4.70 / 7.99 ms at 2^17, 28.09 / 4.99 /
+// 8.39 at 2^16 with smaller warp tasks, 28.52 at s24 with 2^18) and again with
+// the core and packs (s24 20.5 ms, 21.1 at 2^16, 22.0 at 2^18).
+// Warp tasks: a head costs its warp its candidates and kWarpRecCost for each
+// record (a batch of 32 records is a step's wait however short they are), at
+// most kWarpCost between them and one warp's share of the graph's (half of that
+// share in candidates); where a warp's slice serves a head by a hashed set (two slots
+// read and two products a candidate, where a CTA's bitmap of 2^18 ids often still
+// reads one word) and not by a bitmap, at most kWarpWork candidates. With 4,096 candidates (8,192 on graphs of
+// 2^34 or more) and no look at records or ids, against this: R-MAT 2^18 159.5 ->
+// 134.7 us, 2^20 609 -> 572 (per edge 1,818 -> 1,608), 2^21 per vertex 3,164 ->
+// 3,095, 2^22 3,460 -> 3,449, Chung-Lu 2^19 546 -> 509, 2^22 5,602 -> 5,538. Around it: 16,384
+// candidates where hashed 3,524 on R-MAT 2^22; kWarpCost 16,384 1,709 us and 131,072
+// 1,634 on the per-edge 2^20; a record as 4 or 8 candidates 145 us on 2^18; a quarter
+// of a warp's share 130 us against 124 on 2^17; all of it in candidates 159 us against
+// 137 per vertex on 65,536 vertices of R-MAT in id order.
 #ifndef XT_BLOCK_WORK_LOG2
 #define XT_BLOCK_WORK_LOG2 17
 #endif
 #ifndef XT_WARP_WORK
-#define XT_WARP_WORK 4096
-#endif
-#ifndef XT_WARP_WORK_LARGE
-#define XT_WARP_WORK_LARGE 8192
+#define XT_WARP_WORK 8192
 #endif
 constexpr int kThreads = XT_THREADS;
 constexpr int kWarps = kThreads / 32;
@@ -77,6 +85,11 @@ constexpr int kWarpLg = 10;
 constexpr int kWarpWords = kBlockWords / kWarps;  // 1024: a 1024-slot hash or a 32K-bit bitmap
 constexpr int kWarpDmax = kWarpWords / 4;         // hash load factor <= 1/4
 constexpr int64_t kWarpWork = XT_WARP_WORK;
+constexpr int64_t kWarpCost = 32768, kWarpRecCost = 16;
+// ... and on graphs with less for every warp at least this, kWarpMostMin of it
+// candidates (kWarpCostMin 12,288 / 8,192 / 4,096: Chung-Lu 2^14 50 / 53 / 60 us,
+// R-MAT 2^12 49 / 39 / 37)
+constexpr int64_t kWarpCostMin = 8192, kWarpMostMin = 4096;
 #ifndef XT_BLOCK_DMAX
 #define XT_BLOCK_DMAX 2048
 #endif
@@ -95,13 +108,18 @@ constexpr int64_t kBlockWorkMax = int64_t(1) << XT_BLOCK_WORK_LOG2;
 // Run-time schedule thresholds (the binning of make_plan).
 struct PlanParams {
   int64_t tiny_work;   // a head with at most this much work is a lane task
-  int64_t warp_work;   // ... else one with d+(v) <= warp_dmax and at most this much work is a warp task
+  int64_t warp_work;   // ... else one with d+(v) <= warp_dmax and at most this much work is a warp task,
+  int64_t warp_bits;   // with a member id range of at most this (a warp's bitmap) whatever its work,
+  int64_t warp_cost;   // while work + kWarpRecCost a record stays within this
+  int64_t warp_most;   // and work alone within this
   int64_t block_work;  // items per CTA task
   int64_t pack_work;   // candidates of a pack, at most (0: no packs)
   int64_t pack_cost;   // ... and candidates + kPackRecCost a record
   int32_t warp_dmax;
   int32_t batches_per_warp;  // CTA task: record batches per warp, at least
   int32_t lane_pairs;        // CTA task: pairs per lane on an average record, at least
+  const int32_t *col;
+  bool high_first;           // warp tasks from the last head to the first
 };
 #ifndef XT_BATCHES_PER_WARP
 #define XT_BATCHES_PER_WARP 4
@@ -231,6 +249,12 @@ __global__ void __launch_bounds__(256) k_vertex_stats(const int64_t *__restrict_
   }
 }
 
+// whether n ascending members' ids fit a bitmap of `bits` ids in a warp's slice (as members_layout decides)
+__device__ __forceinline__ bool warp_bitmap(const int32_t *__restrict__ mem, int n, int64_t bits) {
+  const int32_t lo = mem[0], hi = mem[n - 1];
+  return (hi >> 5) - (lo >> 5) + 2 <= kWarpWords && int64_t(hi) - int64_t(lo) + 1 <= bits;
+}
+
 // tasks of head v: nb CTA tasks (parts x chunks), nw warp tasks, nt lane tasks (0 or 1 each)
 __device__ __forceinline__ void classify(int64_t v, const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
                                          const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp, int64_t &nb,
@@ -244,7 +268,8 @@ __device__ __forceinline__ void classify(int64_t v, const int64_t *__restrict__ 
     nt = 1;
     return;
   }
-  if (dp <= pp.warp_dmax && work <= pp.warp_work) {
+  if (dp <= pp.warp_dmax && work <= pp.warp_most && work + kWarpRecCost * (k1 - k0) <= pp.warp_cost &&
+      (work <= pp.warp_work || warp_bitmap(pp.col + off[v], int(dp), pp.warp_bits))) {
     nw = 1;
     return;
   }
@@ -260,16 +285,23 @@ __device__ __forceinline__ void classify(int64_t v, const int64_t *__restrict__ 
 // spends its time waiting (claim, members, first pair: 3 to 5 us a head).
 // pk[v]: log2 g for a pack's first head, kPackRest for its others, 0 elsewhere.
 constexpr uint8_t kPackRest = 0xff;
-constexpr int64_t kPackRecs = 4096, kPackRecCost = 8;
+// What a pack saves is a head's wait for its few records, so its heads have on
+// average at most kPackRecs of them (beyond that a head fills its own batches:
+// uniform graph of 139,811 vertices and mean out-degree 30 221 us with such heads
+// packed, 172 without packs; a limit of 24 costs a batch of 256 graphs 70 us), none
+// of more than kPackLen candidates (one lane walks a record: Chung-Lu in id order, 65,536
+// vertices, 99 us without the limit, 74 with 128; Chung-Lu 2^22 5,590 with 32, 5,534
+// with 128), and the graph has kPackHeads vertices
+// and kPackGraphRecs records for every warp (a uniform one of 17,477 vertices 57 us with
+// packs, 45 without; a geometric one of 104,857 vertices, mean degree 5, 37 and 70).
+constexpr int64_t kPackRecs = 32, kPackLen = 128, kPackRecCost = 8, kPackHeads = 8, kPackGraphRecs = 16;
 // Candidates of a pack, at most. Swept at 64 to 2,048 (counts in us, 0: no
 // packs): geometric graph of 2^20 vertices 656 without, 238 at 512, 220 at 1,024;
 // Chung-Lu 2^22 6,133, 5,686, 5,630; R-MAT 2^22 3,538, 3,507, 3,507 (3,533 at
 // 2,048); a batch of 256 graphs 1,860, 1,409, 1,359. Small graphs are cut finer, so
 // that there is a pack for every warp of the GPU: a batch of 32 records takes a warp 1
 // to 2 us, so a record counts as kPackRecCost candidates there (a geometric graph of
-// 2^16 vertices 52 us without packs, 31 with 6,600, 44 with 3,200), and graphs
-// without a batch for every warp have none (a uniform one of 9,645 vertices: 11 us
-// without, 13 with).
+// 2^16 vertices 52 us without packs, 31 with 6,600, 44 with 3,200).
 constexpr int64_t kPackWorkMax = 1024;
 __global__ void k_plan_count(int64_t nv, const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
                              const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp,
@@ -279,11 +311,12 @@ __global__ void k_plan_count(int64_t nv, const int64_t *__restrict__ off, const 
   for (int64_t base = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) & ~int64_t(31); base < nv;
        base += int64_t(gridDim.x) * blockDim.x) {
     const int64_t v = base + lane;
-    int64_t nb = 0, nw = 0, nt = 0, parts, chunks, work = 0, mem = 0, rec = 0;
+    int64_t nb = 0, nw = 0, nt = 0, parts, chunks, work = 0, mem = 0, rec = 0, top = 0;
     if (v < nv) {
       classify(v, off, ioff, iend, P, pp, nb, nw, nt, parts, chunks, work);
       mem = off[v + 1] - off[v];
       rec = ioff[v + 1] - ioff[v];
+      if (rec > 0) top = P[ioff[v] + 1] - P[ioff[v]];  // the longest one
     }
     uint8_t code = 0;
     if (pp.pack_work > 0) {
@@ -295,7 +328,8 @@ __global__ void k_plan_count(int64_t nv, const int64_t *__restrict__ off, const 
         work += __shfl_xor_sync(0xffffffffu, work, o);
         rec += __shfl_xor_sync(0xffffffffu, rec, o);
         busy += __shfl_xor_sync(0xffffffffu, busy, o);
-        if (busy > 1 && mem <= pp.warp_dmax && work <= pp.pack_work && rec <= kPackRecs &&
+        top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+        if (busy > 1 && mem <= pp.warp_dmax && work <= pp.pack_work && rec <= kPackRecs * busy && top <= kPackLen &&
             work + kPackRecCost * rec <= pp.pack_cost)
           code = (lane & (2 * o - 1)) == 0 ? uint8_t(lg) : kPackRest;
       }
@@ -347,7 +381,7 @@ __device__ __forceinline__ Task make_task(int64_t v, int64_t k0, int64_t k1, int
 __global__ void k_plan_fill(int64_t nv, const int64_t *__restrict__ off, const int64_t *__restrict__ ioff,
                             const int64_t *__restrict__ iend, const int64_t *__restrict__ P, const PlanParams pp, const int64_t *__restrict__ nb_pos,
                             const int64_t *__restrict__ nwp_pos, const int64_t *__restrict__ nt_pos,
-                            const uint8_t *__restrict__ pk, Task *__restrict__ bt, Task *__restrict__ wt,
+                            const uint8_t *__restrict__ pk, Task *__restrict__ bt, Task *__restrict__ wt, int64_t n_wt,
                             Task *__restrict__ pt, int32_t *__restrict__ tt) {
   XT_GRID_STRIDE(v, nv) {
     if (pk[v]) {
@@ -387,7 +421,8 @@ __global__ void k_plan_fill(int64_t nv, const int64_t *__restrict__ off, const i
           lg_s = ls;
         }
       }
-      wt[nwp_pos[v] & 0xffffffff] = make_task(v, k0, k1, off[v], off[v + 1], lg_s);
+      const int64_t at = nwp_pos[v] & 0xffffffff;
+      wt[pp.high_first ? n_wt - 1 - at : at] = make_task(v, k0, k1, off[v], off[v + 1], lg_s);
     }
     if (!nb) continue;
     const int64_t base = P[k0];
@@ -1990,16 +2025,16 @@ xt_status make_plan(Graph *g) {
     // CTA task size: large tasks amortise the member-set build and the task
     // barrier, but every CTA should still get about 16 of them
     int64_t total_work = 0;
-    // below 2^17 edges there are at most 2^24.5 candidates and no packs: nothing
-    // here depends on how many
-    if (ne >= (int64_t(1) << 17)) {
+    // by degree, below 2^17 edges there are at most 2^24.5 candidates and no packs:
+    // nothing here depends on how many
+    if (ne >= (int64_t(1) << 17) || g->orient != XT_ORIENT_DEGREE) {
       const void *from = stats + 4;
       if ((s = read_words(c, 1, &from, &total_work)) != XT_OK) break;
     }
     PlanParams pp;
     pp.warp_dmax = kWarpDmax;
-    // graphs of 2^34 or more candidates (R-MAT s24 has 2^35.3) take larger
-    // warp tasks and more record batches per warp
+    // graphs of 2^34 or more candidates (R-MAT s24 has 2^35.3) take more record
+    // batches per warp
     const bool large = total_work >= (int64_t(1) << 34);
     // lane tasks trade latency (a lane's dependent loads set the kernel's
     // tail) for throughput: only graphs with plenty of other work use them
@@ -2007,13 +2042,28 @@ xt_status make_plan(Graph *g) {
     if (g->tier_lane_work >= 0) pp.tiny_work = g->tier_lane_work;
     pp.batches_per_warp = large ? XT_BATCHES_PER_WARP_LARGE : XT_BATCHES_PER_WARP;
     pp.lane_pairs = XT_LANE_PAIRS;
-    pp.warp_work = g->tune_warp_work > 0 ? g->tune_warp_work : (large ? XT_WARP_WORK_LARGE : kWarpWork);
-    if (g->tier_warp_work >= 0) pp.warp_work = g->tier_warp_work;
-    // packs, where every warp has a batch of records to itself; they fill every
-    // warp once before they grow (tiers set by hand: none)
     const int64_t warps = int64_t(pl->grid_global) * kWarps;
+    pl->bitmap_bits = g->tune_bitmap_bits > 0 ? g->tune_bitmap_bits : int64_t(kBlockWords) * 32;
+    pp.col = g->d_col;
+    // the long tasks early: those of high ranks, or, as numbered by the input, of
+    // the low ids that graphs skewed to them have as hubs (65,536 vertices, R-MAT per vertex
+    // in id order 139 us, 175 from the last head)
+    pp.high_first = g->orient == XT_ORIENT_DEGREE;
+    if (g->tune_warp_work > 0 || g->tier_warp_work >= 0) {  // set by hand: candidates alone
+      pp.warp_work = g->tier_warp_work >= 0 ? g->tier_warp_work : g->tune_warp_work;
+      pp.warp_bits = 0;
+      pp.warp_cost = pp.warp_most = INT64_MAX;
+    } else {
+      pp.warp_work = kWarpWork;
+      pp.warp_bits = pl->bitmap_bits;
+      const int64_t share = (total_work + kWarpRecCost * ne) / warps;
+      pp.warp_cost = std::max(kWarpCostMin, std::min(kWarpCost, share));
+      pp.warp_most = std::max(kWarpMostMin, share / 2);
+    }
+    // packs, where every warp has a few heads to itself; they fill every
+    // warp once before they grow (tiers set by hand: none)
     pp.pack_work = pp.pack_cost = 0;
-    if (nv <= kPackMaxNv && ne >= 32 * warps && g->tier_lane_work < 0 && g->tier_warp_work < 0) {
+    if (nv <= kPackMaxNv && nv >= kPackHeads * warps && ne >= kPackGraphRecs * warps && g->tier_lane_work < 0 && g->tier_warp_work < 0) {
       pp.pack_work = kPackWorkMax;
       pp.pack_cost = (total_work + kPackRecCost * ne) / warps;
     }
@@ -2025,7 +2075,6 @@ xt_status make_plan(Graph *g) {
     }
     pl->block_work = pp.block_work;
     pl->warp_work = pp.warp_work;
-    pl->bitmap_bits = g->tune_bitmap_bits > 0 ? g->tune_bitmap_bits : int64_t(kBlockWords) * 32;
     if ((s = dalloc_n(c, &nb, size_t(nv + 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &nw, size_t(nv + 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &nbp, size_t(nv + 1))) != XT_OK) break;
@@ -2069,7 +2118,8 @@ xt_status make_plan(Graph *g) {
     if ((s = dalloc_n(c, &pl->d_pt, size_t(pl->n_ptask > 0 ? pl->n_ptask : 1))) != XT_OK) break;
     if ((s = dalloc_n(c, &pl->d_tt, size_t(pl->n_ttask > 0 ? pl->n_ttask : 1))) != XT_OK) break;
     k_plan_fill<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(
-        nv, g->d_off, g->d_ioff, iend, P, pp, nbp, nwp, ntp, pk, pl->d_bt, pl->d_wt, pl->d_pt, pl->d_tt);
+        nv, g->d_off, g->d_ioff, iend, P, pp, nbp, nwp, ntp, pk, pl->d_bt, pl->d_wt, pl->n_wtask, pl->d_pt,
+        pl->d_tt);
     if ((s = cuda_status(c, cudaGetLastError(), "k_plan_fill")) != XT_OK) break;
     if (pl->n_btask > 1) {  // chunk-major order
       uint32_t *k1 = nullptr, *k2 = nullptr;
