@@ -153,3 +153,31 @@ def test_core_counts_recorded_and_replayed(ctx, first):
         g.capture()
         assert g.count() == g.count_groups()[0] == want
         g.free()
+
+
+def test_core_allocations_that_fail(ctx):
+    """Each allocation of a build and of its counts fails once; the context and
+    the graph stay usable and nothing is left behind."""
+    import xxtric_b200 as xt
+    nv, src, dst = graph(1281)
+    src, dst = src.astype(np.int32), dst.astype(np.int32)
+    want = oracle.count_merge(*oracle.canon_csr(nv, src.astype(np.int64), dst.astype(np.int64)))
+
+    def until_it_passes(call):
+        for k in range(1, 200):
+            ctx.fail_alloc_after(k)
+            try:
+                return call()
+            except xt.XtError as err:
+                assert err.status == xt.XT_ERR_OOM
+            finally:
+                ctx.fail_alloc_after(0)
+        raise AssertionError("still failing")
+
+    held = ctx.mem_stats()[0]
+    g = until_it_passes(lambda: ctx.graph_from_edges(nv, src, dst))
+    assert g.count() == want
+    assert until_it_passes(g.count_edges)[0] == want
+    assert until_it_passes(lambda: g.count(per_vertex=True))[0] == want
+    g.free()
+    assert ctx.mem_stats()[0] == held

@@ -813,25 +813,26 @@ xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d
   const int width = 2 * k.jtop;
   uint8_t *sym = k.d_sym, *xt = k.d_xt;
   int32_t *list = k.d_list;
-  if (!sym) {
-    XT_TRY(dalloc_n(c, &sym, size_t(width) * width * kCoreTile));
+  const int64_t rows = int64_t(k.nb) * kCoreRows;
+  unsigned long long *rows2 = nullptr;
+  xt_status s = XT_OK;
+  if (!sym && (s = dalloc_n(c, &sym, size_t(width) * width * kCoreTile)) == XT_OK) {
     if (keep) k.d_sym = sym;
     k_core_sym<<<counted(c, dim3(unsigned(width * width))), 256, 0, c->stream>>>(width, k.d_tile0, k.d_tiles, sym);
   }
-  if (d_es && !xt) {
-    if (!list) XT_TRY(dalloc_n(c, &list, size_t(k.jtop) * k.nb + k.jtop));
+  if (s == XT_OK && d_es && !xt) {
+    if (!list) s = dalloc_n(c, &list, size_t(k.jtop) * k.nb + k.jtop);
     if (keep) k.d_list = list;
-    XT_TRY(dalloc_n(c, &xt, size_t(k.n_tiles) * kCoreTile));
-    if (keep) k.d_xt = xt;
-    k_core_turn<<<counted(c, dim3(unsigned(k.n_tiles))), 256, 0, c->stream>>>(k.d_tiles, xt);
-    k_core_levels<<<counted(c, dim3(unsigned(k.jtop))), 1024, 0, c->stream>>>(k.nb, k.d_jw, k.d_tile0, list,
-                                                                             list + int64_t(k.jtop) * k.nb);
+    if (s == XT_OK) s = dalloc_n(c, &xt, size_t(k.n_tiles) * kCoreTile);
+    if (s == XT_OK) {
+      if (keep) k.d_xt = xt;
+      k_core_turn<<<counted(c, dim3(unsigned(k.n_tiles))), 256, 0, c->stream>>>(k.d_tiles, xt);
+      k_core_levels<<<counted(c, dim3(unsigned(k.jtop))), 1024, 0, c->stream>>>(k.nb, k.d_jw, k.d_tile0, list,
+                                                                               list + int64_t(k.jtop) * k.nb);
+    }
   }
-  XT_CUDA(c, cudaGetLastError());
-  const int64_t rows = int64_t(k.nb) * kCoreRows;
-  unsigned long long *rows2 = nullptr;
-  XT_TRY(dalloc_n(c, &rows2, size_t(rows)));
-  cudaError_t e = cudaMemsetAsync(rows2, 0, sizeof(*rows2) * rows, c->stream);
+  if (s == XT_OK) s = dalloc_n(c, &rows2, size_t(rows));
+  cudaError_t e = s == XT_OK ? cudaMemsetAsync(rows2, 0, sizeof(*rows2) * rows, c->stream) : cudaSuccess;
   a.sym = sym;
   a.jw = k.d_jw;
   a.jtop = k.jtop;
@@ -848,7 +849,7 @@ xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d
   a.count = list + int64_t(k.jtop) * k.nb;
   a.nb = k.nb;
   const unsigned grid = unsigned(c->sm_count);
-  if (e == cudaSuccess) {
+  if (s == XT_OK && e == cudaSuccess) {
     if (d_es) {
       k_core_count<kCoreEdges><<<counted(c, dim3(grid)), kCoreThreads, kCoreSmem, c->stream>>>(a);
       k_core_count<kCoreInner><<<counted(c, dim3(grid)), kCoreThreads, kCoreSmem, c->stream>>>(a);
@@ -863,6 +864,7 @@ xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d
   if (sym != k.d_sym) dfree(c, sym);
   if (xt != k.d_xt) dfree(c, xt);
   if (list != k.d_list) dfree(c, list);
+  XT_TRY(s);
   XT_CUDA(c, e);
   return XT_OK;
 }
