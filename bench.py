@@ -624,7 +624,7 @@ def roofline_fields(args, info: dict, t_kernel: float) -> dict:
         iss = profiled_value(small, "issue_slots_busy_frac")
         if iss is not None:
             r["issue_frac"] = iss
-            r["issue_source"] = f"profiles/{small} (ncu --set full, R-MAT scale 22: sm__inst_issued / issue slots)"
+            r["issue_source"] = f"profiles/{small} (ncu, R-MAT scale 22: sm__inst_issued / issue slots)"
     return r
 
 

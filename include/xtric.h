@@ -67,11 +67,12 @@ typedef struct {
   int64_t max_out_degree; /* max d+ after orientation */
   int64_t max_in_degree;  /* max d- after orientation */
   int64_t wedge_work;     /* sum over oriented (u,v) of d+(v): items a tail-grouped count streams */
-  int64_t stream_work;    /* sum over u of C(d+(u),2): candidate columns this count streams (the
-                             suffix of N+(u) after each out-neighbour) */
-  int64_t alg_bytes;      /* bytes the count's loads request, repeats included (a suffix streamed by
-                             several heads counts each time; L2 serves many of the repeats):
-                             16(nv+1) offsets + 4|E+| member columns + 8|E+| in-records +
+  int64_t stream_work;    /* sum over u of C(d+(u),2): the count's candidate columns (the suffix of
+                             N+(u) after each out-neighbour); those of a dense core, which large
+                             power-law graphs have, are counted on the tensor cores, not streamed */
+  int64_t alg_bytes;      /* bytes the loads of a count that streams every candidate request, repeats
+                             included (a suffix streamed by several heads counts each time; L2 serves
+                             many of the repeats): 16(nv+1) offsets + 4|E+| member columns + 8|E+| in-records +
                              4 stream_work candidate columns */
   int64_t tail_alg_bytes; /* the tail-grouped figure: 8(nv+1) + 4|E+| + sum (16 + 4 d+(v)) */
   int32_t orient;         /* xt_orient used */
@@ -232,7 +233,7 @@ int64_t xt_graph_groups(const xt_graph *g);
 /* total and per-graph counts (host buffer of xt_graph_groups entries, nullable) */
 xt_status xt_count_groups(xt_graph *g, int64_t *total, int64_t *per_group);
 xt_status xt_count_groups_async(xt_graph *g, int64_t *d_total, int64_t *d_per_group);
-/* Capture the graph's count (its memsets and its one persistent launch) into
+/* Capture the graph's count (its memsets and its persistent launches) into
  * a CUDA graph once; xt_count_groups then replays it. */
 xt_status xt_graph_capture(xt_graph *g);
 /* Schedule thresholds (0 = automatic): items per CTA task, the work limit of
@@ -282,8 +283,8 @@ xt_status xt_graph_set_lane_intersect(xt_graph *g, int kind);
  * index): warp tasks, and lane tasks in groups of 32 heads, are taken from
  * their global cursor `claim` at a time (1..64; 0, the default: 4 for a
  * graph built as a batch, 1 otherwise). One atomic on one address per task
- * limits schedules of many small tasks (the 4,096-graph batch: 38.2 ms a
- * count with 1, 30.4 ms with 4); larger blocks leave a longer tail on
+ * limits schedules of many small tasks (the 4,096-graph batch, before small
+ * heads were packed: 38.2 ms a count with 1, 30.4 ms with 4); larger blocks leave a longer tail on
  * graphs whose warp tasks are fewer (R-MAT scale 22: 4.69 ms with 1, 4.79
  * with 4). The autotuner tries 1, 4 and 16. Counts are identical.
  * Re-captures a captured graph. */
