@@ -1,0 +1,57 @@
+"""Bounded device waits that run out: the call reports it, its copies and
+products in flight end first, and the next call is exact."""
+import contextlib
+
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+NV = 1281  # dense enough for the tensor-core part of the count (its kernels hold the waits)
+
+
+@contextlib.contextmanager
+def wait_limit(tries):
+    import xxtric_b200 as xt
+    xt.debug_wait_limit(tries)
+    try:
+        yield
+    finally:
+        xt.debug_wait_limit(-1)
+
+
+def dense_graph():
+    rng = np.random.default_rng(3)
+    a, b = np.triu_indices(NV, 1)
+    keep = rng.random(len(a)) < 0.8
+    off, tails = oracle.canon_csr(NV, a[keep], b[keep])
+    return off, tails, oracle.count_merge(off, tails, per_vertex=True)
+
+
+@pytest.fixture(scope="module")
+def dense():
+    return dense_graph()
+
+
+@pytest.mark.parametrize("tries", [0, 1, 3])
+def test_core_waits_that_run_out_are_reported(dense, tries):
+    """A limit of 0 gives up at the first wait of each warp, 1 and 3 in the
+    middle of the copies and products, or not at all: then the count is exact."""
+    import xxtric_b200 as xt
+    off, tails, (want, pv) = dense
+    with xt.Context(0) as c:
+        g = c.graph_from_csr(off, tails)
+        for call in (g.count, lambda: g.count(per_vertex=True), g.count_edges):
+            with wait_limit(tries):
+                try:
+                    r = call()
+                    assert tries > 0 and (r[0] if isinstance(r, tuple) else r) == want
+                except xt.XtError as err:
+                    assert err.status == xt.XT_ERR_TIMEOUT
+            assert g.count() == want
+        total, each = g.count(per_vertex=True)
+        assert total == want
+        np.testing.assert_array_equal(each, pv)
+        g.free()

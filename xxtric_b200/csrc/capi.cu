@@ -204,6 +204,11 @@ xt_status xt_debug_fail_alloc(xt_ctx *ctx, int64_t k) {
   return XT_OK;
 }
 
+xt_status xt_debug_wait_limit(int64_t tries) {
+  core_wait_limit(tries);
+  return XT_OK;
+}
+
 int64_t xt_launch_count(const xt_ctx *ctx) { return ctx ? ctx->c.launches : -1; }
 
 xt_status xt_mem_stats(xt_ctx *ctx, int64_t *live, int64_t *peak, int reset_peak) {

@@ -302,6 +302,7 @@ struct CoreArgs {
   int64_t stride;
   unsigned long long *global;
   int *err;
+  uint32_t wait_limit;  // tries of a barrier wait
   // per vertex and per edge
   const uint8_t *sym;      // S: tile (row block, chunk) at row block * 2 jtop + chunk
   const int32_t *jw;
@@ -333,10 +334,10 @@ __device__ __forceinline__ void core_expect(uint64_t *bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(core_smem(bar)), "r"(bytes)
                : "memory");
 }
-// waits for the barrier's phase, at most kCoreWaitLimit tries; gives up early
-// once another warp of the CTA has
-__device__ __forceinline__ bool core_wait(uint64_t *bar, uint32_t parity, volatile int *fail) {
-  for (uint32_t it = 0; it < kCoreWaitLimit; it++) {
+// waits for the barrier's phase, at most `limit` tries; gives up early once
+// another warp of the CTA has
+__device__ __forceinline__ bool core_wait(uint64_t *bar, uint32_t parity, volatile int *fail, uint32_t limit) {
+  for (uint32_t it = 0; it < limit; it++) {
     uint32_t done;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
     // stage k's buffer once it is free, its barrier expecting the step's bytes
     auto stage = [&]() -> uint8_t * {
       const uint32_t sg = k % kCoreStages;
-      if (!core_wait(&s_empty[sg], ((k / kCoreStages) & 1u) ^ 1u, fail)) return nullptr;
+      if (!core_wait(&s_empty[sg], ((k / kCoreStages) & 1u) ^ 1u, fail, a.wait_limit)) return nullptr;
       core_expect(&s_full[sg], kCoreStageBytes);
       return st + sg * kCoreStageBytes;
     };
@@ -526,10 +527,12 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
         }
       }
     }
-    if (lane == 0 && *fail)  // the copies in flight land before the CTA leaves
+    // the copies in flight land before the CTA leaves its shared memory to another:
+    // always, as the products may give up after the last copy has been issued
+    if (lane == 0)
       for (uint32_t q = k > kCoreStages ? k - kCoreStages : 0; q < k; q++) {
         int quiet = 0;
-        core_wait(&s_full[q % kCoreStages], (q / kCoreStages) & 1u, &quiet);
+        core_wait(&s_full[q % kCoreStages], (q / kCoreStages) & 1u, &quiet, kCoreWaitLimit);
       }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -537,13 +540,13 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
       uint32_t k = 0, t = 0;
       for (int64_t i = blockIdx.x; i < n && !*fail; i += gridDim.x) {
         if (!core_item<KIND>(a, s_pfx, i, it)) continue;
-        if (!core_wait(&s_tempty[t & 1], ((t >> 1) & 1u) ^ 1u, fail)) break;
+        if (!core_wait(&s_tempty[t & 1], ((t >> 1) & 1u) ^ 1u, fail, a.wait_limit)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d = tmem + (t & 1) * kCoreStep;
         bool ok = true;
         for (int c = 0; c < it.steps; c++, k++) {
           const uint32_t sg = k % kCoreStages;
-          if (!core_wait(&s_full[sg], (k / kCoreStages) & 1u, fail)) {
+          if (!core_wait(&s_full[sg], (k / kCoreStages) & 1u, fail, a.wait_limit)) {
             ok = false;
             break;
           }
@@ -561,7 +564,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
       }
       core_commit(&s_drain);  // every product issued is done before the accumulators are given back
       int quiet = 0;
-      core_wait(&s_drain, 0, &quiet);
+      core_wait(&s_drain, 0, &quiet, kCoreWaitLimit);
     }
     __syncwarp();
   } else {
@@ -580,7 +583,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
       unsigned int *es = nullptr;  // per edge: the row's entry at the next position
       if ((KIND == kCoreEdges || KIND == kCoreInner) && u >= 0)
         es = a.es + a.poff[u] + (a.off[u + 1] - a.off[u]) - 1 - a.before[mt / 2 * kCoreRows + r];
-      if (!__all_sync(0xffffffffu, core_wait(&s_tfull[t & 1], (t >> 1) & 1u, fail))) break;
+      if (!__all_sync(0xffffffffu, core_wait(&s_tfull[t & 1], (t >> 1) & 1u, fail, a.wait_limit))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       int32_t sum = 0;
 #pragma unroll
@@ -722,6 +725,9 @@ __global__ void __launch_bounds__(256) k_core_halves(const unsigned long long *_
 
 // ---- host side ------------------------------------------------------------------
 
+static thread_local int64_t t_wait_limit = -1;  // xt_debug_wait_limit
+void core_wait_limit(int64_t tries) { t_wait_limit = tries; }
+
 // Widths of the row blocks from the unique rows (row u: cols[rstart[u]] on, as
 // many as off says), and their layout; *d_sums has kCoreSums words once the
 // stream gets there. Leaves g->core empty (and *d_sums null) for graphs that
@@ -796,6 +802,7 @@ xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d
   a.stride = 1;
   a.global = reinterpret_cast<unsigned long long *>(d_global);
   a.err = c->d_err;
+  a.wait_limit = t_wait_limit < 0 ? kCoreWaitLimit : uint32_t(std::min<int64_t>(t_wait_limit, kCoreWaitLimit));
   a.nv = g->nv;
   if (!d_pv && !d_es) {
     if (k.n_items <= shard) return XT_OK;
