@@ -55,3 +55,19 @@ def test_core_waits_that_run_out_are_reported(dense, tries):
         assert total == want
         np.testing.assert_array_equal(each, pv)
         g.free()
+
+
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_count_device_reports_a_wait_that_ran_out(dense, accumulate):
+    import torch
+    import xxtric_b200 as xt
+    off, tails, (want, _) = dense
+    d_off, d_t = torch.from_numpy(off).cuda(), torch.from_numpy(tails).cuda()
+    out = torch.full((1,), 41, dtype=torch.int64, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    with wait_limit(0), pytest.raises(xt.XtError) as err:
+        xt.count_device(NV, d_off, d_t, out, accumulate=accumulate, stream=stream)
+    assert err.value.status == xt.XT_ERR_TIMEOUT
+    assert int(out) == 41, "the counter is left alone"
+    xt.count_device(NV, d_off, d_t, out, accumulate=accumulate, stream=stream)
+    assert int(out) == want + (41 if accumulate else 0)

@@ -446,23 +446,22 @@ xt_status xt_count_device(int64_t nv, const int64_t *d_indices, const int64_t *d
   Ctx *c = &ctx->c;
   Graph g;
   xt_status s = build_from_csr(c, nv, d_indices, d_edge_list, true, XT_ORIENT_DEGREE, &g);
-  int64_t *tmp = nullptr;
   if (s == XT_OK) s = make_plan(&g);
-  if (s == XT_OK) s = dalloc_n(c, &tmp, 1);
-  if (s == XT_OK) s = count_graph(&g, tmp, nullptr);
+  if (s == XT_OK) s = count_graph(&g, &c->d_out->total, nullptr);
+  // a count whose device waits gave up is reported, and leaves *d_count as it was
+  int64_t add = 0;
+  if (s == XT_OK) s = count_status(c, &add);
   if (s == XT_OK && accumulate) {
-    int64_t h = 0, add = 0;
+    int64_t h = 0;
     s = cuda_status(c, cudaMemcpyAsync(&h, d_count, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream), "D2H");
-    if (s == XT_OK)
-      s = cuda_status(c, cudaMemcpyAsync(&add, tmp, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream), "D2H");
     if (s == XT_OK) s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync");
     h += add;
     if (s == XT_OK)
       s = cuda_status(c, cudaMemcpyAsync(d_count, &h, sizeof(int64_t), cudaMemcpyHostToDevice, c->stream), "H2D");
   } else if (s == XT_OK) {
-    s = cuda_status(c, cudaMemcpyAsync(d_count, tmp, sizeof(int64_t), cudaMemcpyDeviceToDevice, c->stream), "D2D");
+    s = cuda_status(c, cudaMemcpyAsync(d_count, &c->d_out->total, sizeof(int64_t), cudaMemcpyDeviceToDevice,
+                                       c->stream), "D2D");
   }
-  dfree(c, tmp);
   free_graph_device(&g);
   cudaFreeAsync(c->d_out, c->stream);
   cudaStreamSynchronize(c->stream);
