@@ -71,3 +71,39 @@ def test_count_device_reports_a_wait_that_ran_out(dense, accumulate):
     assert int(out) == 41, "the counter is left alone"
     xt.count_device(NV, d_off, d_t, out, accumulate=accumulate, stream=stream)
     assert int(out) == want + (41 if accumulate else 0)
+
+
+@pytest.mark.parametrize("form", ["edges", "edges by id", "csr", "canonical csr"])
+def test_a_build_leaves_an_asynchronous_timeout_to_the_next_count(dense, form):
+    """A count_async whose waits ran out is not an error of the next build's
+    input: the build succeeds (and still refuses bad input), the next
+    synchronous count reports the timeout, and the one after is exact."""
+    import torch
+    import xxtric_b200 as xt
+    off, tails, (want, _) = dense
+    with xt.Context(0) as c:
+        g = c.graph_from_csr(off, tails)
+        total = torch.zeros(1, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        with wait_limit(0):
+            g.count_async(total)
+        c.synchronize()
+        if form.startswith("edges"):
+            orient = 0 if form == "edges by id" else 1
+            rows = np.array([0, 0, 1], np.int32), np.array([1, 2, 2], np.int32)
+            with pytest.raises(xt.XtError) as err:
+                c.graph_from_edges(2, *rows, orient)
+            assert err.value.status == xt.XT_ERR_INVALID
+            small = c.graph_from_edges(3, *rows, orient)
+        else:
+            o, t = np.array([0, 2, 4, 6]), np.array([1, 2, 0, 2, 0, 1])
+            with pytest.raises(xt.XtError) as err:
+                c.graph_from_csr(o[[0, 2, 1, 3]], t, canonical=form != "csr")
+            assert err.value.status == xt.XT_ERR_INVALID
+            small = c.graph_from_csr(o, t, canonical=form != "csr")
+        with pytest.raises(xt.XtError) as err:
+            small.count()
+        assert err.value.status == xt.XT_ERR_TIMEOUT
+        assert small.count() == 1 and g.count() == want
+        small.free()
+        g.free()

@@ -660,7 +660,7 @@ __global__ void k_csr_entries(const int64_t *__restrict__ off, const int64_t *__
 __global__ void k_csr_back(const int64_t *__restrict__ off, int64_t nv, const int32_t *__restrict__ rows,
                            const int32_t *__restrict__ t32, int64_t e_first, int64_t ne,
                            const int *__restrict__ err, unsigned long long *__restrict__ chk) {
-  if (*err || chk[0] || chk[1]) return;  // decided already
+  if ((*err & kErrInput) || chk[0] || chk[1]) return;  // decided already
   bool bad = false;
   const double per = 1.0 / double(nv);
   for (int64_t e = e_first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < ne;
@@ -818,10 +818,12 @@ static xt_status exclusive_scan_i64(Ctx *c, In in, int64_t *out, int64_t n) {
   return XT_OK;
 }
 
-// the error word of the context's block, as read from the device
+// the input's bits of the error word, as read from the device; the others, of an
+// asynchronous count whose waits gave up, stay for the next synchronous count
 static xt_status check_err_word(Ctx *c, int h, const char *what) {
-  if (!h) return XT_OK;
-  XT_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
+  if (!(h & kErrInput)) return XT_OK;
+  const int rest = h & ~kErrInput;
+  XT_CUDA(c, cudaMemcpyAsync(c->d_err, &rest, sizeof(int), cudaMemcpyHostToDevice, c->stream));
   const char *why = (h & 1) ? ": vertex id outside [0,nv)" : ": offsets not monotone in [0,ne]";
   return set_error(c, XT_ERR_INVALID, std::string(what) + why);
 }

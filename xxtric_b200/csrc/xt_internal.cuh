@@ -19,6 +19,7 @@ constexpr size_t kColPad = 8;
 // ---- context ---------------------------------------------------------------
 // device block read back by the synchronous counts in one copy: the error word
 // that kernels set when their input or a bounded wait fails, and a total
+constexpr int kErrInput = 3;  // its bits of a build: an id out of range (1), offsets not monotone (2)
 struct CountOut {
   int err;
   int reserved;
