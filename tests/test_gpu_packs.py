@@ -127,3 +127,25 @@ def test_long_warp_tasks_match_the_oracle(ctx, span, orient):
     a, b, s = g.edge_support()
     np.testing.assert_array_equal(s[np.lexsort((b, a))], sup[up][np.lexsort((tails[up], u[up]))])
     g.free()
+
+
+@pytest.mark.parametrize("kind", ["ring", "gaps", "er", "mixed"])
+def test_pack_credits_from_both_tables(ctx, kind):
+    """Per-vertex and per-edge counts of packs whose sets are cuckoo tables (the
+    default), and where some (1) or nearly all (0) fall back to linear probing."""
+    nv, src, dst = graph(kind)
+    off, tails = oracle.canon_csr(nv, src.astype(np.int64), dst.astype(np.int64))
+    want, pv = oracle.count_merge(off, tails, per_vertex=True)
+    sup = oracle.edge_support(off, tails)
+    u = np.repeat(np.arange(nv), np.diff(off))
+    up = u < tails
+    sup = sup[up][np.lexsort((tails[up], u[up]))]
+    g = ctx.graph_from_edges(nv, src.astype(np.int32), dst.astype(np.int32))
+    for iters in (-1, 1, 0):
+        g.debug_cuckoo_iters(iters)
+        total, each = g.count(per_vertex=True)
+        assert total == want
+        np.testing.assert_array_equal(each, pv)
+        a, b, s = g.edge_support()
+        np.testing.assert_array_equal(s[np.lexsort((b, a))], sup)
+    g.free()

@@ -1232,9 +1232,20 @@ __device__ __forceinline__ int stage_task_bulk(int32_t *stage, uint64_t *bar, co
 // ---- packs ----------------------------------------------------------------------
 //
 // A pack's members are keyed with their head: (x << 5 | head) + 1 in a cuckoo
-// table (0 empty), (x << 5 | head) in a linear-probing one (kEmpty empty), so
-// ids must lie below 2^26 (kPackMaxNv).
+// table (0 empty), (x << 5 | head) in a linear-probing one (kEmpty empty; where a
+// cuckoo chain ran too long), so ids must lie below 2^26 (kPackMaxNv). Counts with
+// credits keep 16 bits a slot for its member's hits (at most one a record). While
+// these probed linearly and found a member's counter by its slot's index, some
+// lane of a warp followed a chain at nearly every candidate: per edge, uniform graph of
+// 139,811 vertices and mean out-degree 30 in id order 357 us, 334 now, 343 with its
+// heads one by one; geometric one of 262,145 vertices and mean degree 16 145 and 130;
+// per vertex 329 and 311, 129 and 109.
 constexpr int64_t kPackMaxNv = (int64_t(1) << 26) - 2;
+// Eviction chain limit of a pack's table, of at most 256 keys in 1,024 slots: a pack
+// that falls back holds a short count's last warp (uniform graph of 104,857 vertices,
+// mean out-degree 5 in id order, one such pack: per vertex 35 us without it, 46 with a
+// limit of 64, 41 with 16; with 8 packs that would have fitted fall back too, 38 on average)
+constexpr int kPackCuckooIters = 16;
 
 // the pack's heads, one a lane: first record, end of the live records (both
 // from the pack's first) and first member
@@ -1260,20 +1271,29 @@ __device__ __forceinline__ int pack_find(int32_t start, int32_t x) {
   return h;
 }
 
+// one more hit of the member in a slot
+static_assert(32 * kPackRecs < 65536, "a slot's hits fit 16 bits");
+__device__ __forceinline__ void pack_hit(const Members &m, uint32_t slot) {
+  atomicAdd(reinterpret_cast<unsigned int *>(m.idx) + (slot >> 1), 1u << ((slot & 1u) << 4));
+}
 // the candidate w of a record of head `hl` at padded column pos
 template <int MODE, bool CUCKOO>
 __device__ __forceinline__ int pack_probe(const Members &m, int32_t w, uint32_t hl, unsigned int *__restrict__ es,
                                           int64_t pos) {
   if (CUCKOO) {
     const uint32_t key = uint32_t(w) * 32u + hl + 1u;
-    const uint32_t x = uint32_t(m.words[cuckoo_h1(key, m.shift)]);
-    const uint32_t y = uint32_t(m.words[cuckoo_h2(key, m.shift)]);
-    return int(uint32_t(x == key) | uint32_t(y == key));
+    const uint32_t i = cuckoo_h1(key, m.shift), j = cuckoo_h2(key, m.shift);
+    const uint32_t x = uint32_t(m.words[i]), y = uint32_t(m.words[j]);
+    if (MODE == 0) return int(uint32_t(x == key) | uint32_t(y == key));
+    if (x != key && y != key) return 0;
+    pack_hit(m, x == key ? i : j);
+    if (MODE == 2) atomicAdd(&es[pos], 1u);
+    return 1;
   }
   if (uint32_t(w - m.lo) > uint32_t(m.hi - m.lo)) return 0;  // sentinels too
   const int slot = hash_find(m.words, m.mask, m.shift, int32_t(uint32_t(w) * 32u + hl));
   if (slot < 0) return 0;
-  if (MODE != 0) atomicAdd(&m.mcnt[m.idx[slot]], 1);
+  if (MODE != 0) pack_hit(m, uint32_t(slot));
   if (MODE == 2) atomicAdd(&es[pos], 1u);
   return 1;
 }
@@ -1558,12 +1578,15 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
     int32_t *wstage = s_stage + warp * kStageWarp;
     int32_t *words = bwords + warp * kWarpWords;
     int *hcnt = s_hcnt[warp];
+    const int iters = PV ? min(a.cuckoo_iters, kPackCuckooIters) : a.cuckoo_iters;
     const bool heads = PV || a.group;
     ClaimBlock pclaim(a.n_bt == 0 && a.n_wt == 0, a.claim);
     Task t = claim_task_block(pclaim, &cursor[4], a.pt, a.n_pt, a.stride, a.claim, lane);
     int so = stage_task(wstage, col, rec, t, lane);
     PackHeads ph = pack_heads(a, t, lane);
-    if (t.nrec >= 0 && MODE == 0) zero_words(words, kWarpWords, lane, 32);
+    if (t.nrec >= 0) zero_words(words, kWarpWords, lane, 32);
+    if (PV && t.nrec >= 0)  // the slots' hits, two a word
+      zero_words(reinterpret_cast<int32_t *>(bidx + warp * kWarpWords), kWarpWords / 2, lane, 32);
     while (true) {
       cp_async_wait_all();
       __syncwarp();
@@ -1575,17 +1598,15 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
       m.mcnt = bmcnt + warp * kWarpDmax;
       m.mask = kWarpWords - 1;
       m.shift = 32 - kWarpLg;
-      bool ok = MODE == 0;  // the global count's set is a cuckoo table, in a slice that is all zero
+      bool ok = true;  // the set is a cuckoo table, in a slice that is all zero
       if (heads) hcnt[lane] = 0;
-      if (MODE == 0) {
-        for (int i0 = 0; i0 < t.nmem; i0 += 32) {
-          const int i = i0 + lane, hl = pack_find(ph.mem, i);
-          if (i < t.nmem)
-            ok &= cuckoo_insert(words, m.shift, uint32_t(mem[i]) * 32u + uint32_t(hl) + 1u, a.cuckoo_iters);
-        }
-        ok = __all_sync(0xffffffffu, ok);
+      for (int i0 = 0; i0 < t.nmem; i0 += 32) {
+        const int i = i0 + lane, hl = pack_find(ph.mem, i);
+        if (i < t.nmem)
+          ok &= cuckoo_insert(words, m.shift, uint32_t(mem[i]) * 32u + uint32_t(hl) + 1u, iters);
       }
-      if (!ok) {  // linear probing (with member counters), or a cuckoo chain ran too long
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {  // a cuckoo chain ran too long: linear probing
         int32_t lo = 0x7fffffff, hi = -1;
         for (int i = lane; i < kWarpWords; i += 32) words[i] = kEmpty;
         __syncwarp();
@@ -1594,11 +1615,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
           if (i < t.nmem) {
             lo = min(lo, mem[i]);
             hi = max(hi, mem[i]);
-            const uint32_t slot = hash_insert(words, m.mask, m.shift, int32_t(uint32_t(mem[i]) * 32u + uint32_t(hl)));
-            if (PV) {
-              m.idx[slot] = uint16_t(i);
-              m.mcnt[i] = 0;
-            }
+            hash_insert(words, m.mask, m.shift, int32_t(uint32_t(mem[i]) * 32u + uint32_t(hl)));
           }
         }
         m.lo = __reduce_min_sync(0xffffffffu, lo);
@@ -1607,9 +1624,8 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
       __syncwarp();
       const Task tn = claim_task_block(pclaim, &cursor[4], a.pt, a.n_pt, a.stride, a.claim, lane);
       const PackHeads phn = pack_heads(a, tn, lane);
-      if (PV) acc += stream_pack<MODE, false, true>(a, t, ph, m, hcnt, lane);
-      else if (!ok) acc += stream_pack<0, false, true>(a, t, ph, m, hcnt, lane);
-      else if (a.group) acc += stream_pack<0, true, true>(a, t, ph, m, hcnt, lane);
+      if (!ok) acc += stream_pack<MODE, false, true>(a, t, ph, m, hcnt, lane);
+      else if (heads) acc += stream_pack<MODE, true, true>(a, t, ph, m, hcnt, lane);
       else acc += stream_pack<0, true, false>(a, t, ph, m, hcnt, lane);
       __syncwarp();
       if (MODE == 0 && ok) {
@@ -1630,16 +1646,24 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
           atomicAdd(reinterpret_cast<unsigned long long *>(&pv[v]), (unsigned long long)hcnt[lane]);
         if (a.group) atomicAdd(&a.group_out[a.group[v]], (unsigned long long)hcnt[lane]);
       }
-      if (MODE == 1) {
-        for (int i = lane; i < t.nmem; i += 32)
-          if (m.mcnt[i])
-            atomicAdd(reinterpret_cast<unsigned long long *>(&pv[mem[i]]), (unsigned long long)m.mcnt[i]);
-      }
-      if (MODE == 2) {
+      if (PV) {  // the members' hits to their credits, their slots back to zero
         for (int i0 = 0; i0 < t.nmem; i0 += 32) {
           const int i = i0 + lane, hl = pack_find(ph.mem, i);
-          const int32_t r0 = __shfl_sync(0xffffffffu, ph.mem, hl);
-          if (i < t.nmem && m.mcnt[i]) atomicAdd(&es[a.poff[t.v + hl] + (i - r0)], unsigned(m.mcnt[i]));
+          const int32_t r0 = MODE == 2 ? __shfl_sync(0xffffffffu, ph.mem, hl) : 0;
+          if (i >= t.nmem) continue;
+          const uint32_t key = uint32_t(mem[i]) * 32u + uint32_t(hl) + 1u;
+          uint32_t x = cuckoo_h1(key, m.shift);
+          if (!ok) x = uint32_t(hash_find(words, m.mask, m.shift, int32_t(key - 1u)));
+          else if (uint32_t(words[x]) != key) x = cuckoo_h2(key, m.shift);
+          if (ok) words[x] = 0;
+          const unsigned n = m.idx[x];
+          m.idx[x] = 0;
+          if (MODE == 1 && n) atomicAdd(reinterpret_cast<unsigned long long *>(&pv[mem[i]]), (unsigned long long)n);
+          if (MODE == 2 && n) atomicAdd(&es[a.poff[t.v + hl] + (i - r0)], n);
+        }
+        if (!ok) {
+          __syncwarp();
+          zero_words(words, kWarpWords, lane, 32);
         }
       }
       __syncwarp();
