@@ -2087,6 +2087,16 @@ xt_status make_plan(Graph *g) {
       const int64_t share = (total_work + kWarpRecCost * ne) / warps;
       pp.warp_cost = std::max(kWarpCostMin, std::min(kWarpCost, share));
       pp.warp_most = std::max(kWarpMostMin, share / 2);
+      if (g->orient != XT_ORIENT_DEGREE) {
+        // as numbered by the input the long heads are not the first in the list, and
+        // hubs are among the members, so no bitmap beyond kWarpWork and a smaller share:
+        // R-MAT 2^18 vertices (2^20 rows) 288 -> 259 us a count (276 with 4,096 candidates
+        // for every head), Chung-Lu 2^16 (2^20 rows) per edge 248 -> 233 (236); a share's
+        // half without the bitmaps leaves the latter at 248, a quarter costs 2^15 vertices of
+        // Chung-Lu 5%
+        pp.warp_bits = 0;
+        pp.warp_most = std::max(kWarpMostMin, share / 3);
+      }
     }
     // packs, where every warp has a few heads to itself; they fill every
     // warp once before they grow (tiers set by hand: none)
