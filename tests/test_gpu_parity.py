@@ -631,3 +631,26 @@ def test_cpp_mirror_batch_edges_and_server(tmp_path):
     r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     assert r.stdout.split("\n")[:3] == ["batch 5 4 1", "edges 4 6 12", "served 4 1"], r.stdout
+
+
+@pytest.mark.parametrize("rows_per_sm", [128, 1024])
+@pytest.mark.parametrize("more", [0, 1])
+@pytest.mark.parametrize("dropped", [0, 1])
+def test_supports_at_the_limits_of_rows_by_warp(ctx, rows_per_sm, more, dropped):
+    """Per-edge counts of a ring with 8 neighbours a side, at the numbers of rows and
+    of columns where they are moved out by row instead of by span of columns."""
+    n, k = 148 * rows_per_sm + more, 8
+    i = np.arange(n)
+    src = np.concatenate([i] * k)[dropped:]
+    dst = np.concatenate([(i + j) % n for j in range(1, k + 1)])[dropped:]
+    off, tails = oracle.canon_csr(n, src, dst)
+    want, sup = oracle.count_merge(off, tails), oracle.edge_support(off, tails)
+    u = np.repeat(np.arange(n), np.diff(off))
+    up = u < tails
+    g = ctx.graph_from_edges(n, src.astype(np.int32), dst.astype(np.int32))
+    assert g.info()["n_edges"] == k * n - dropped
+    total, _ = g.count_edges()
+    assert total == want
+    a, b, s = g.edge_support()
+    np.testing.assert_array_equal(s[np.lexsort((b, a))], sup[up][np.lexsort((tails[up], u[up]))])
+    g.free()

@@ -2257,10 +2257,15 @@ __global__ void k_rec_tails(const InRec *__restrict__ rec, int64_t ne, const int
 // a chain of loads (uniform graph of 1,639 vertices 25 us, 35 with 256 always).
 // Graphs of at most two rows a warp, or of rows that fill one on average, none
 // longer than a span, take a warp per row (span 0): no search (uniform graph of 8,739 vertices and out-degree 30 40 us
-// with spans, 38 without; R-MAT in id order, 8,192 vertices, 134 us without, 118 with).
+// with spans, 38 without; R-MAT in id order, 8,192 vertices, 134 us without, 118 with), and so
+// do graphs of up to 1,024 rows an SM with 8 columns on average (a geometric graph of
+// 34,953 vertices and mean out-degree 15 72 us with spans, 67 without, a uniform one of mean
+// out-degree 13 60 and 55; beyond that many rows geometric ones in degree order lose, 250,001
+// of mean out-degree 9 149 and 155).
 constexpr int kUnpadSpan = 256;
 static int unpad_span(const Graph *g, int sms) {
-  if (g->max_out_degree <= kUnpadSpan && (g->nv <= int64_t(sms) * 128 || g->ne >= 16 * g->nv)) return 0;
+  const int fill = g->nv <= int64_t(sms) * 1024 ? 8 : 16;
+  if (g->max_out_degree <= kUnpadSpan && (g->nv <= int64_t(sms) * 128 || g->ne >= fill * g->nv)) return 0;
   int span = kUnpadSpan;
   while (span > 32 && g->ne < int64_t(span) * sms * 64) span /= 2;
   return span;
