@@ -126,3 +126,21 @@ def test_batch_rejects_bad_tables(ctx):
     total, per = g.count_groups()
     assert total == 1 and per.tolist() == [1, 0]
     g.free()
+
+
+def test_batch_names_an_id_outside_its_graph(ctx):
+    """An id past its own graph, inside the union: from host and from device rows."""
+    import torch
+    voff, eoff = np.array([0, 3, 6]), np.array([0, 1, 2])
+    src, dst = np.array([0, 0], np.int32), np.array([3, 1], np.int32)
+    for orient in (0, 1):
+        with pytest.raises(xt.XtError) as e:
+            ctx.graph_from_batch(voff, eoff, src, dst, orient)
+        assert e.value.status == xt.XT_ERR_INVALID and "outside its graph" in ctx.last_error
+        ts, td = torch.from_numpy(src).cuda(), torch.from_numpy(dst).cuda()
+        with pytest.raises(xt.XtError) as e:
+            ctx.graph_from_batch(voff, eoff, ts, td, orient, device=True)
+        assert e.value.status == xt.XT_ERR_INVALID and "outside its graph" in ctx.last_error
+    with pytest.raises(xt.XtError):  # a graph of its own
+        ctx.graph_from_edges(3, src, dst)
+    assert "outside [0,nv)" in ctx.last_error

@@ -604,6 +604,7 @@ __global__ void k_csr_offsets(const int64_t *__restrict__ off, int64_t nv, int64
 // the entries above their row's id less those below it, modulo 2^64; word 2
 // is set when an entry is missing from its other end's row.
 constexpr int kCsrWords = 3;
+constexpr const char *kCsrBadId = "csr: vertex id outside [0,nv)";
 
 // Every CSR entry's row and its tail in 32 bits (ids outside [0, nv): bit 1
 // of *err), with the row checks above. A warp takes spans of kCsrSpan
@@ -820,18 +821,17 @@ static xt_status exclusive_scan_i64(Ctx *c, In in, int64_t *out, int64_t n) {
 
 // the input's bits of the error word, as read from the device; the others, of an
 // asynchronous count whose waits gave up, stay for the next synchronous count
-static xt_status check_err_word(Ctx *c, int h, const char *what) {
+static xt_status check_err_word(Ctx *c, int h, const char *bad_id) {
   if (!(h & kErrInput)) return XT_OK;
   const int rest = h & ~kErrInput;
   XT_CUDA(c, cudaMemcpyAsync(c->d_err, &rest, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  const char *why = (h & 1) ? ": vertex id outside [0,nv)" : ": offsets not monotone in [0,ne]";
-  return set_error(c, XT_ERR_INVALID, std::string(what) + why);
+  return set_error(c, XT_ERR_INVALID, (h & 1) ? bad_id : "csr: offsets not monotone in [0,ne]");
 }
-static xt_status check_err(Ctx *c, const char *what) {
+static xt_status check_err(Ctx *c, const char *bad_id) {
   int64_t h = 0;
   const void *at = c->d_out;
   XT_TRY(read_words(c, 1, &at, &h));
-  return check_err_word(c, int(h & 0xffffffff), what);
+  return check_err_word(c, int(h & 0xffffffff), bad_id);
 }
 
 // Degree orientation: ranks the vertices by (deg, id) into g->d_perm
@@ -839,8 +839,8 @@ static xt_status check_err(Ctx *c, const char *what) {
 // The rank is a stable sort of the ids keyed by degree alone (the ids enter
 // in ascending order, so ties keep id order), on as many key bits as the
 // largest degree needs; deg is consumed. The error word is read with that
-// degree: `what` names the input its checks belong to.
-static xt_status rank_vertices(Ctx *c, int32_t *deg, int64_t nv, Graph *g, int32_t **o2n, const char *what) {
+// degree: `bad_id` says what its first bit means for the input.
+static xt_status rank_vertices(Ctx *c, int32_t *deg, int64_t nv, Graph *g, int32_t **o2n, const char *bad_id) {
   const int B = 256;
   int32_t *ids = nullptr, *dalt = nullptr;
   unsigned int *d_dmax = nullptr;  // two words, to be read as one of 64 bits
@@ -860,7 +860,7 @@ static xt_status rank_vertices(Ctx *c, int32_t *deg, int64_t nv, Graph *g, int32
     int64_t h[2] = {0, 0};
     s = read_words(c, 2, from, h);
     dmax = (unsigned int)h[0];
-    if (s == XT_OK) s = check_err_word(c, int(h[1] & 0xffffffff), what);
+    if (s == XT_OK) s = check_err_word(c, int(h[1] & 0xffffffff), bad_id);
   }
   uint32_t *dk = nullptr;
   int32_t *perm = nullptr;
@@ -1111,7 +1111,7 @@ xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src,
   xt_status s = XT_OK;
   const size_t n1 = size_t(ne > 0 ? ne : 1);
   const int64_t ne4 = (ne + 3) & ~int64_t(3);
-  const char *what = bt.ng > 0 ? "batch" : "edge list";
+  const char *bad_id = bt.ng > 0 ? "batch: a vertex id is outside its graph" : "edge list: vertex id outside [0,nv)";
   do {
     if ((s = dalloc_n(c, &k0, n1 + 2)) != XT_OK) break;
     if ((s = dalloc_n(c, &k1, n1 + 2)) != XT_OK) break;
@@ -1132,11 +1132,11 @@ xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src,
                                                                            0, bt);
         if ((s = cuda_status(c, cudaGetLastError(), "k_edge_keys")) != XT_OK) break;
       }
-      if (orient != XT_ORIENT_DEGREE && (s = check_err(c, what)) != XT_OK) break;  // else with the largest degree
+      if (orient != XT_ORIENT_DEGREE && (s = check_err(c, bad_id)) != XT_OK) break;  // else with the largest degree
     }
     // rank, then relabel every row in place
     if (orient == XT_ORIENT_DEGREE) {
-      if ((s = rank_vertices(c, deg, nv, g, &o2n, what)) != XT_OK) break;
+      if ((s = rank_vertices(c, deg, nv, g, &o2n, bad_id)) != XT_OK) break;
       if (ne > 0)
         k_relabel_split<<<counted(c, grid_for(ne, B, c->sm_count)), B, 0, c->stream>>>(lo, hi, ne, o2n);
       if ((s = cuda_status(c, cudaGetLastError(), "relabel")) != XT_OK) break;
@@ -1178,7 +1178,7 @@ static xt_status build_canonical(Ctx *c, int64_t nv, const int64_t *d_off, int32
     if (orient == XT_ORIENT_DEGREE) {
       if ((s = dalloc_n(c, &deg, size_t(nv))) != XT_OK) break;
       k_degree_from_off<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(d_off, nv, deg);
-      if ((s = rank_vertices(c, deg, nv, g, &o2n, "csr")) != XT_OK) break;
+      if ((s = rank_vertices(c, deg, nv, g, &o2n, kCsrBadId)) != XT_OK) break;
       dfree(c, deg);
       deg = nullptr;
     }
@@ -1251,7 +1251,7 @@ xt_status build_from_csr(Ctx *c, int64_t nv, const int64_t *d_off, const int64_t
       const void *from[kCsrWords + 1] = {chk, chk + 1, chk + 2, c->d_out};
       if ((s = read_words(c, kCsrWords + 1, from, h)) != XT_OK) break;
     }
-    if ((s = check_err_word(c, int(h[kCsrWords] & 0xffffffff), "csr")) != XT_OK) break;
+    if ((s = check_err_word(c, int(h[kCsrWords] & 0xffffffff), kCsrBadId)) != XT_OK) break;
     // rows that are canonical, promised or not, need no edge sort
     const bool sorted = h[0] == 0 && h[1] == 0 && h[2] == 0;
     if (canonical && !sorted) {
