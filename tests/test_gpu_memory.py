@@ -1,0 +1,127 @@
+"""Memory that cannot be had for the dense core: the build goes on without it, with
+the same counts."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import xxtric_b200 as xt
+    with xt.Context(0) as c:
+        yield c
+
+
+def wide_core(n_core=600, n_band=20000, per_row=120):
+    """A dense core below a band of rows that reach into it: some 160 row blocks of
+    three column steps."""
+    rng = np.random.default_rng(17)
+    a, b = np.triu_indices(n_core, 1)
+    keep = rng.random(len(a)) < 0.8
+    band = np.repeat(np.arange(n_core, n_core + n_band), per_row)
+    t = rng.integers(n_core, n_core + n_band, (2, 30000))
+    src = np.concatenate([a[keep], band, t[0]])
+    dst = np.concatenate([b[keep], rng.integers(0, n_core, len(band)), t[1]])
+    n = n_core + n_band
+    p = rng.permutation(n)
+    return n, p[src].astype(np.int32), p[dst].astype(np.int32)
+
+
+class Want:
+    def __init__(self):
+        self.nv, self.src, self.dst = wide_core()
+        off, tails = oracle.canon_csr(self.nv, self.src.astype(np.int64), self.dst.astype(np.int64))
+        self.total, self.pv = oracle.count_merge(off, tails, per_vertex=True)
+        u = np.repeat(np.arange(self.nv), np.diff(off))
+        up = u < tails
+        self.by_position = None
+        self.sup = oracle.edge_support(off, tails)[up][np.lexsort((tails[up], u[up]))]
+
+    def build(self, ctx):
+        return ctx.graph_from_edges(self.nv, self.src, self.dst)
+
+    def check_vertices(self, g):
+        total, each = g.count(per_vertex=True)
+        assert total == self.total
+        np.testing.assert_array_equal(each, self.pv)
+
+    def check_edges(self, g):
+        total, sup = g.count_edges()
+        assert total == self.total
+        if self.by_position is None:  # the supports in the graph's own order, the same for every build
+            off, col = g.csr()
+            p = g.perm().astype(np.int64)
+            a, b = p[np.repeat(np.arange(self.nv), np.diff(off))], p[col]
+            self.by_position = np.empty_like(self.sup)
+            self.by_position[np.lexsort((np.maximum(a, b), np.minimum(a, b)))] = self.sup
+        np.testing.assert_array_equal(sup, self.by_position)
+
+
+@pytest.fixture(scope="module")
+def want():
+    return Want()
+
+
+def count_launches(ctx, g, want):
+    before = ctx.launches
+    assert g.count() == want.total
+    return ctx.launches - before
+
+
+def test_a_build_goes_on_without_its_core(ctx, want):
+    import xxtric_b200 as xt
+    g = want.build(ctx)
+    full = count_launches(ctx, g, want)
+    g.free()
+    held = ctx.mem_stats()[0]
+    dropped, k = 0, 0
+    while True:
+        k += 1
+        assert k < 200
+        ctx.fail_alloc_after(k)
+        before = ctx.mem_stats()[0]
+        try:
+            g = want.build(ctx)
+        except xt.XtError as err:
+            assert err.status == xt.XT_ERR_OOM
+            assert ctx.mem_stats()[0] == before
+            continue
+        finally:
+            ctx.fail_alloc_after(0)
+        if count_launches(ctx, g, want) == full:  # no allocation failed
+            g.free()
+            break
+        dropped += 1
+        want.check_vertices(g)
+        want.check_edges(g)
+        g.free()
+        assert ctx.mem_stats()[0] == held
+    # the tables of its row blocks, their sums, the tiles, the entries before them, the items
+    assert dropped == 5
+
+
+def test_a_core_does_not_raise_the_builds_peak(ctx, want):
+    def peak():
+        ctx.synchronize()
+        before = ctx.mem_stats(reset_peak=True)[0]
+        g = want.build(ctx)
+        p = ctx.mem_stats()[1] - before
+        n = count_launches(ctx, g, want)
+        g.free()
+        return p, n
+
+    with_core, launches = peak()
+    for k in range(1, 200):  # the first allocation whose failure drops the core
+        ctx.fail_alloc_after(k)
+        try:
+            without, n = peak()
+            break
+        except Exception:
+            continue
+        finally:
+            ctx.fail_alloc_after(0)
+    assert n < launches
+    assert with_core <= without + (64 << 10)  # the row blocks' tables

@@ -1019,7 +1019,7 @@ static xt_status rows_to_csr(Ctx *c, const int64_t *rstart, uint32_t *cols_s, in
     // the out-CSR, with the in-records in position order and their sort keys
     // (head << lb | class, in kbuf), sorted by head and then class (stable:
     // records of one (head, class) stay in position order)
-    if ((s = core_decide(c, g, sums)) != XT_OK) break;
+    core_decide(c, g, sums);
     const int lb = g->core.n_items > 0 ? std::min(8, 32 - b) : (b + 7 <= 31 ? 7 : 31 - b);
     uint32_t *kin = reinterpret_cast<uint32_t *>(kbuf), *kalt = kin + m;
     if ((s = dalloc_n(c, &r0, size_t(m) + 2)) != XT_OK) break;
@@ -1035,7 +1035,6 @@ static xt_status rows_to_csr(Ctx *c, const int64_t *rstart, uint32_t *cols_s, in
     const uint32_t dead = lb - (core ? 1 : 0) == 7 ? 127u : core ? 1u << (lb - 1) : 1u << lb;
     if ((s = dalloc_n(c, &g->d_iend, size_t(nv))) != XT_OK) break;
     if ((s = key_bounds(c, ks, m, nv, lb, dead, g->d_ioff, g->d_iend)) != XT_OK) break;
-    if ((s = core_finish(c, g)) != XT_OK) break;
     g->d_irec = rs;
     if (rs == r0) r0 = nullptr;
     else r1 = nullptr;
@@ -1158,6 +1157,7 @@ xt_status build_from_edges(Ctx *c, int64_t nv, int64_t ne, const int32_t *d_src,
   dfree(c, deg);
   dfree(c, o2n);
   dfree(c, rstart);
+  if (s == XT_OK) s = core_finish(c, g);
   if (s != XT_OK) free_graph_device(g);
   return s;
 }
@@ -1210,6 +1210,7 @@ static xt_status build_canonical(Ctx *c, int64_t nv, const int64_t *d_off, int32
   dfree(c, rstart);
   dfree(c, bk);
   dfree(c, kbuf);
+  if (s == XT_OK) s = core_finish(c, g);
   return s;
 }
 

@@ -731,7 +731,7 @@ void core_wait_limit(int64_t tries) { t_wait_limit = tries; }
 // Widths of the row blocks from the unique rows (row u: cols[rstart[u]] on, as
 // many as off says), and their layout; *d_sums has kCoreSums words once the
 // stream gets there. Leaves g->core empty (and *d_sums null) for graphs that
-// cannot gain.
+// cannot gain, and where the tables' memory cannot be had.
 xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *cols, int64_t n, int64_t **d_sums) {
   *d_sums = nullptr;
   Core &k = g->core;
@@ -740,11 +740,14 @@ xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *col
   const int64_t blocks = (g->nv + kCoreRows - 1) / kCoreRows;
   k.nb = int(std::max<int64_t>(kCoreMinBlk, std::min<int64_t>(blocks, kCoreMaxBlk)));
   // one allocation for the row blocks' tables: tile0, then jw, cut, item0
-  XT_TRY(dalloc_n(c, &k.d_tile0, size_t(k.nb + 1) + size_t(3 * k.nb + 1) / 2));
+  if (dalloc_n(c, &k.d_tile0, size_t(k.nb + 1) + size_t(3 * k.nb + 1) / 2) != XT_OK ||
+      dalloc_n(c, d_sums, kCoreSums) != XT_OK) {
+    core_free(g);
+    return XT_OK;
+  }
   k.d_jw = reinterpret_cast<int32_t *>(k.d_tile0 + k.nb + 1);
   k.d_cut = k.d_jw + k.nb;
   k.d_item0 = k.d_cut + k.nb;
-  XT_TRY(dalloc_n(c, d_sums, kCoreSums));
   XT_CUDA(c, cudaMemsetAsync(*d_sums, 0, kCoreSums * sizeof(int64_t), c->stream));
   k_core_pick<<<counted(c, dim3(k.nb)), 1024, 0, c->stream>>>(g->nv, rstart, g->d_off, cols, k.d_jw, k.d_cut,
                                                              reinterpret_cast<unsigned long long *>(*d_sums) + 3);
@@ -753,28 +756,35 @@ xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *col
   return XT_OK;
 }
 
-// sums read back: keeps the core (its memory allocated) or drops it
-xt_status core_decide(Ctx *c, Graph *g, const int64_t *sums) {
+// sums read back: keeps the core or drops it
+void core_decide(Ctx *c, Graph *g, const int64_t *sums) {
   Core &k = g->core;
-  if (k.nb == 0) return XT_OK;
+  if (k.nb == 0) return;
   // dropped also where the operands would outgrow the edges' own memory (a few
   // dense rows that reach far into a sparse core)
   if (sums[3] < kCoreMinFs || sums[1] == 0 || sums[0] * kCoreTile > kCoreMaxBytes * g->ne) {
     core_free(g);
-    return XT_OK;
+    return;
   }
   k.n_tiles = sums[0];
   k.n_items = sums[1];
   k.jtop = int(sums[2]);
-  XT_TRY(dalloc_n(c, &k.d_tiles, size_t(sums[0]) * kCoreTile));
-  XT_TRY(dalloc_n(c, &k.d_before, size_t(sums[0] / 2) * kCoreRows));
-  return dalloc_n(c, &k.d_items, size_t(sums[1]));
 }
 
-// operands and work items from the finished out-CSR
+// Operands and work items from the finished out-CSR. Called when the build's
+// scratch has been given back (more of it than the operands' 16 bytes an edge, so
+// they do not raise the build's peak); where their memory cannot be had the graph
+// goes on without a core, all of its records streamed.
 xt_status core_finish(Ctx *c, Graph *g) {
   Core &k = g->core;
   if (k.n_items == 0) return XT_OK;
+  if (dalloc_n(c, &k.d_tiles, size_t(k.n_tiles) * kCoreTile) != XT_OK ||
+      dalloc_n(c, &k.d_before, size_t(k.n_tiles / 2) * kCoreRows) != XT_OK ||
+      dalloc_n(c, &k.d_items, size_t(k.n_items)) != XT_OK) {
+    core_free(g);
+    return cuda_status(c, cudaMemcpyAsync(g->d_iend, g->d_ioff + 1, sizeof(int64_t) * g->nv,
+                                          cudaMemcpyDeviceToDevice, c->stream), "records without a core");
+  }
   k_core_tiles<<<counted(c, dim3(unsigned(k.n_tiles / 2))), 256, 0, c->stream>>>(g->nv, k.nb, g->d_off, g->d_col,
                                                                                  k.d_tile0, k.d_tiles, k.d_before);
   k_core_items<<<counted(c, dim3(unsigned((k.nb + 255) / 256))), 256, 0, c->stream>>>(k.nb, k.d_jw, k.d_item0,

@@ -226,7 +226,7 @@ xt_status build_batch(Ctx *c, int64_t ng, const int64_t *h_voff, const int64_t *
 constexpr int kCoreSums = 4;
 constexpr int kErrCoreTimeout = 16;  // bit of the context's error word: a bounded wait of the core's kernel gave up
 xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *cols, int64_t m, int64_t **d_sums);
-xt_status core_decide(Ctx *c, Graph *g, const int64_t *sums);
+void core_decide(Ctx *c, Graph *g, const int64_t *sums);
 xt_status core_finish(Ctx *c, Graph *g);
 xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d_es, int shard, int nshards);
 void core_free(Graph *g);
