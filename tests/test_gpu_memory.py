@@ -1,5 +1,5 @@
-"""Memory that cannot be had for the dense core: the build goes on without it, with
-the same counts."""
+"""Memory that cannot be had for the dense core: the build goes on without it,
+per-vertex and per-edge counts without its operands, all exact."""
 import numpy as np
 import pytest
 
@@ -125,3 +125,63 @@ def test_a_core_does_not_raise_the_builds_peak(ctx, want):
             ctx.fail_alloc_after(0)
     assert n < launches
     assert with_core <= without + (64 << 10)  # the row blocks' tables
+
+
+@pytest.mark.parametrize("mode", ["vertices", "edges"])
+def test_counts_without_operands(ctx, want, mode):
+    """The k-th allocation of the first such count fails, on a graph of its own."""
+    import xxtric_b200 as xt
+    call = want.check_vertices if mode == "vertices" else want.check_edges
+    # per vertex: the result, the records' tails, the counts; then S and the rows' sums
+    # per edge: the result, the counts; then S, the lists, the transposes and the rows' sums
+    needed, core = (3, 2) if mode == "vertices" else (2, 4)
+    g = want.build(ctx)
+    call(g)
+    full = ctx.mem_stats()[0]
+    g.free()
+    for k in range(1, needed + core + 2):
+        g = want.build(ctx)
+        ctx.fail_alloc_after(k)
+        try:
+            call(g)
+            assert k > needed
+        except xt.XtError as err:
+            assert k <= needed and err.status == xt.XT_ERR_OOM
+        finally:
+            ctx.fail_alloc_after(0)
+        call(g)  # and with the memory
+        assert ctx.mem_stats()[0] == full
+        g.free()
+
+
+@pytest.mark.parametrize("nshards", [2, 5])
+def test_shards_with_and_without_operands_add_up(ctx, want, nshards):
+    """One shard counts without the operands, the others with them."""
+    import torch
+    part = torch.zeros(1, dtype=torch.int64, device="cuda")
+    g = want.build(ctx)
+    m = g.info()["n_edges"]
+    want.check_edges(g)
+    g.free()
+    for alone in range(nshards):
+        pv, es, totals = np.zeros(want.nv, np.int64), np.zeros(m, np.int64), np.zeros(2, np.int64)
+        for i in range(nshards):
+            g = want.build(ctx)
+            each = torch.zeros(want.nv, dtype=torch.int64, device="cuda")
+            edge = torch.zeros(m, dtype=torch.int64, device="cuda")
+            torch.cuda.synchronize()
+            ctx.fail_alloc_after(3 if i == alone else 0)  # the records' tails, the counts, S
+            g.count_shard_async(i, nshards, part, each)
+            ctx.synchronize()
+            totals[0] += int(part)
+            ctx.fail_alloc_after(3 if i == alone else 0)  # counts, S, the lists
+            g.count_edges_shard_async(i, nshards, part, edge)
+            ctx.synchronize()
+            ctx.fail_alloc_after(0)
+            totals[1] += int(part)
+            pv += each.cpu().numpy()
+            es += edge.cpu().numpy()
+            g.free()
+        assert (totals == want.total).all()
+        np.testing.assert_array_equal(pv, want.pv)
+        np.testing.assert_array_equal(es, want.by_position)

@@ -723,6 +723,131 @@ __global__ void __launch_bounds__(256) k_core_halves(const unsigned long long *_
   if (threadIdx.x == 0 && sum) atomicAdd(total, sum);
 }
 
+// ---- per vertex and per edge without operands ---------------------------------------
+
+// The credits of the core's records where the operands' memory cannot be had: a
+// CTA per head of the core, a warp per record, each candidate looked up among the
+// head's columns. No memory of its own; slower than the products (R-MAT 2^20 per
+// edge 5.7 ms a count against 1.6, 2^21 per vertex 9.4 against 3.1), so only then.
+// Shards take the same shares as the products', whatever path the others are on: a
+// record's by its row block, the third edge's by the item of kCoreInner that holds it.
+constexpr int kSearchThreads = 512;
+constexpr int kSearchSmem = kCoreWidth * int(sizeof(unsigned));  // a counter a position of the core
+template <bool EDGES>
+__global__ void __launch_bounds__(kSearchThreads)
+    k_core_search(const CoreArgs a, const int64_t *__restrict__ ioff, const int64_t *__restrict__ iend,
+                  const InRec *__restrict__ rec, const int32_t *__restrict__ colp) {
+  using Scan = cub::BlockScan<int, kSearchThreads>;
+  using Red = cub::BlockReduce<unsigned long long, kSearchThreads>;
+  extern __shared__ unsigned s_hits[];  // by position, of the head's columns, this shard's
+  __shared__ uint32_t s_in[kCoreWidth / 32];  // the positions that are the head's columns
+  __shared__ union {
+    typename Scan::TempStorage scan;
+    typename Red::TempStorage red;
+  } ts;
+  __shared__ int s_wider[kCoreMaxJ + 1];         // row blocks wider than t steps
+  __shared__ int64_t s_item0[kCoreMaxJ + 1];     // kCoreInner's items before level t
+  __shared__ uint8_t s_seg[kCoreMaxBlk];         // level t: each row block's segment
+  constexpr int kPer = kCoreMaxBlk / kSearchThreads;
+  static_assert(kCoreMaxBlk / kCoreSeg <= 256, "a segment's index fits a byte");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool split = EDGES && a.nshards > 1;
+  if (split) {
+    for (int t = threadIdx.x; t <= kCoreMaxJ; t += kSearchThreads) s_wider[t] = 0;
+    __syncthreads();
+    for (int b = threadIdx.x; b < a.nb; b += kSearchThreads)
+      if (a.jw[b] > 0) atomicAdd(&s_wider[a.jw[b] - 1], 1);  // exactly that wide, first
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int t = kCoreMaxJ - 1; t >= 0; t--) s_wider[t] += s_wider[t + 1];
+      int64_t at = 0;
+      for (int t = 0; t <= kCoreMaxJ; t++) {
+        s_item0[t] = at;
+        at += 2 * (t + 1) * ((s_wider[t] + kCoreSeg - 1) / kCoreSeg);
+      }
+    }
+    __syncthreads();
+  }
+  unsigned long long total = 0;
+  int level = -1;
+  const int64_t heads = min(a.nv, int64_t(a.jtop) * kCoreStep);
+  for (int64_t pos = blockIdx.x; pos < heads; pos += gridDim.x) {
+    const int64_t v = a.nv - 1 - pos, k0 = iend[v], k1 = ioff[v + 1];
+    const int64_t m0 = a.poff[v];
+    const int32_t dv = int32_t(a.off[v + 1] - a.off[v]);
+    const int t = int(pos / kCoreStep);
+    const int segs = split ? (s_wider[t] + kCoreSeg - 1) / kCoreSeg : 1;
+    if (split && t != level) {
+      level = t;
+      int own = 0, at, wide[kPer];
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < kPer; i++) {
+        const int b = threadIdx.x * kPer + i;
+        wide[i] = b < a.nb && a.jw[b] > t;
+        own += wide[i];
+      }
+      Scan(ts.scan).ExclusiveSum(own, at);
+#pragma unroll
+      for (int i = 0; i < kPer; i++) {
+        s_seg[threadIdx.x * kPer + i] = uint8_t(at / kCoreSeg);
+        at += wide[i];
+      }
+      __syncthreads();
+    }
+    for (int i = threadIdx.x; i < kCoreWidth / 32; i += kSearchThreads) s_in[i] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < dv; i += kSearchThreads) {
+      const int x = int(a.nv - 1 - colp[m0 + i]);  // below pos
+      atomicOr(&s_in[x >> 5], 1u << (x & 31));
+      s_hits[x] = 0;
+    }
+    __syncthreads();
+    unsigned long long hv = 0;
+    for (int64_t k = k0 + warp; k < k1; k += kSearchThreads / 32) {
+      const InRec r = rec[k];
+      const int64_t s = rec_s(r);
+      const int32_t len = rec_len(r);
+      if (len == 0 || dv == 0) continue;
+      const int64_t u = row_of(a.poff, a.nv, s - 1, lane);
+      const int b = int((a.nv - 1 - u) / kCoreRows);
+      const bool mine = a.nshards <= 1 || b % a.nshards == a.shard;
+      if (!mine && !EDGES) continue;
+      const int64_t item = split ? s_item0[t] + int64_t((pos / kCoreRows) & 1) * (t + 1) * segs + s_seg[b] : 0;
+      unsigned h = 0;
+      for (int32_t q = lane; q < len; q += 32) {
+        const int x = int(a.nv - 1 - colp[s + q]);  // below pos
+        if (!((s_in[x >> 5] >> (x & 31)) & 1u)) continue;
+        h++;
+        if (EDGES && mine) atomicAdd(&a.es[s + q], 1u);
+        if (!split || (item + x / kCoreStep * segs) % a.nshards == a.shard) atomicAdd(&s_hits[x], 1u);
+      }
+      if (!mine) continue;
+      hv += h;
+      h = __reduce_add_sync(0xffffffffu, h);
+      if (lane == 0 && h) {
+        if (EDGES) atomicAdd(&a.es[s - 1], h);
+        else atomicAdd(&a.pv[u], (unsigned long long)h);
+      }
+    }
+    total += hv;
+    for (int o = 16; o; o >>= 1) hv += __shfl_xor_sync(0xffffffffu, hv, o);
+    if (!EDGES && hv && lane == 0) atomicAdd(&a.pv[v], hv);
+    __syncthreads();
+    for (int i = threadIdx.x; i < dv; i += kSearchThreads) {
+      const int32_t w = colp[m0 + i];
+      const unsigned h = s_hits[a.nv - 1 - w];
+      if (!h) continue;
+      if (EDGES) atomicAdd(&a.es[m0 + i], h);
+      else atomicAdd(&a.pv[w], (unsigned long long)h);
+    }
+    __syncthreads();
+  }
+  __syncthreads();
+  total = Red(ts.red).Sum(total);
+  if (threadIdx.x == 0 && total) atomicAdd(a.global, total);
+}
+
 // ---- host side ------------------------------------------------------------------
 
 static thread_local int64_t t_wait_limit = -1;  // xt_debug_wait_limit
@@ -800,7 +925,8 @@ xt_status core_finish(Ctx *c, Graph *g) {
 // `shard`, or, with d_pv (internal numbering) or d_es (padded column positions),
 // of every nshards-th row block, with each triangle credited to its vertices
 // or edges. The operands of the latter are built by their first count and kept;
-// a count recorded into a CUDA graph before that builds its own each time.
+// a count recorded into a CUDA graph before that builds its own each time, and
+// one that cannot have their memory searches instead (k_core_search).
 xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d_es, int shard, int nshards) {
   Ctx *c = g->ctx;
   Core &k = g->core;
@@ -832,24 +958,24 @@ xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d
   int32_t *list = k.d_list;
   const int64_t rows = int64_t(k.nb) * kCoreRows;
   unsigned long long *rows2 = nullptr;
-  xt_status s = XT_OK;
-  if (!sym && (s = dalloc_n(c, &sym, size_t(width) * width * kCoreTile)) == XT_OK) {
+  bool have = sym || dalloc_n(c, &sym, size_t(width) * width * kCoreTile) == XT_OK;
+  if (have && !k.d_sym) {
     if (keep) k.d_sym = sym;
     k_core_sym<<<counted(c, dim3(unsigned(width * width))), 256, 0, c->stream>>>(width, k.d_tile0, k.d_tiles, sym);
   }
-  if (s == XT_OK && d_es && !xt) {
-    if (!list) s = dalloc_n(c, &list, size_t(k.jtop) * k.nb + k.jtop);
+  if (have && d_es && !xt) {
+    if (!list) have = dalloc_n(c, &list, size_t(k.jtop) * k.nb + k.jtop) == XT_OK;
     if (keep) k.d_list = list;
-    if (s == XT_OK) s = dalloc_n(c, &xt, size_t(k.n_tiles) * kCoreTile);
-    if (s == XT_OK) {
+    have = have && dalloc_n(c, &xt, size_t(k.n_tiles) * kCoreTile) == XT_OK;
+    if (have) {
       if (keep) k.d_xt = xt;
       k_core_turn<<<counted(c, dim3(unsigned(k.n_tiles))), 256, 0, c->stream>>>(k.d_tiles, xt);
       k_core_levels<<<counted(c, dim3(unsigned(k.jtop))), 1024, 0, c->stream>>>(k.nb, k.d_jw, k.d_tile0, list,
                                                                                list + int64_t(k.jtop) * k.nb);
     }
   }
-  if (s == XT_OK) s = dalloc_n(c, &rows2, size_t(rows));
-  cudaError_t e = s == XT_OK ? cudaMemsetAsync(rows2, 0, sizeof(*rows2) * rows, c->stream) : cudaSuccess;
+  have = have && dalloc_n(c, &rows2, size_t(rows)) == XT_OK;
+  cudaError_t e = have ? cudaMemsetAsync(rows2, 0, sizeof(*rows2) * rows, c->stream) : cudaSuccess;
   a.sym = sym;
   a.jw = k.d_jw;
   a.jtop = k.jtop;
@@ -863,10 +989,17 @@ xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d
   a.es = d_es;
   a.xt = xt;
   a.list = list;
-  a.count = list + int64_t(k.jtop) * k.nb;
+  a.count = list ? list + int64_t(k.jtop) * k.nb : nullptr;
   a.nb = k.nb;
-  const unsigned grid = unsigned(c->sm_count);
-  if (s == XT_OK && e == cudaSuccess) {
+  if (!have) {
+    const auto search = d_es ? k_core_search<true> : k_core_search<false>;
+    const int64_t heads = std::min(g->nv, int64_t(k.jtop) * kCoreStep);
+    e = cudaFuncSetAttribute(search, cudaFuncAttributeMaxDynamicSharedMemorySize, kSearchSmem);
+    search<<<counted(c, dim3(unsigned(std::min<int64_t>(heads, c->sm_count * 3)))), kSearchThreads, kSearchSmem,
+             c->stream>>>(a, g->d_ioff, g->d_iend, g->d_irec, g->d_colp);
+    if (e == cudaSuccess) e = cudaGetLastError();
+  } else if (e == cudaSuccess) {
+    const unsigned grid = unsigned(c->sm_count);
     if (d_es) {
       k_core_count<kCoreEdges><<<counted(c, dim3(grid)), kCoreThreads, kCoreSmem, c->stream>>>(a);
       k_core_count<kCoreInner><<<counted(c, dim3(grid)), kCoreThreads, kCoreSmem, c->stream>>>(a);
@@ -881,7 +1014,6 @@ xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d
   if (sym != k.d_sym) dfree(c, sym);
   if (xt != k.d_xt) dfree(c, xt);
   if (list != k.d_list) dfree(c, list);
-  XT_TRY(s);
   XT_CUDA(c, e);
   return XT_OK;
 }
