@@ -77,3 +77,24 @@ def test_rows_without_their_back_entries_take_the_general_path(ctx, drop):
     g = ctx.graph_from_csr(off2, tails[keep], canonical=False)
     assert g.count() == want
     g.free()
+
+
+@pytest.mark.parametrize("before", [1, 70000])
+def test_entries_before_the_first_row_are_checked(before):
+    """A device CSR whose rows start past entry 0: the entries before them are no
+    edges, but an id out of range among them is refused like any other."""
+    import torch
+    import xxtric_b200 as xt
+    off = torch.tensor([0, 2, 4, 6], dtype=torch.int64, device="cuda") + before
+    tails = torch.zeros(before + 6, dtype=torch.int64, device="cuda")
+    tails[before:] = torch.tensor([1, 2, 0, 2, 0, 1])
+    out = torch.zeros(1, dtype=torch.int64, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    xt.count_device(3, off, tails, out, stream=stream)
+    assert int(out) == 1
+    for rows in (off, torch.full_like(off, before)):  # and where no row has an entry
+        for bad in (3, -1):
+            tails[before // 2] = bad
+            with pytest.raises(xt.XtError) as e:
+                xt.count_device(3, rows, tails, out, stream=stream)
+            assert e.value.status == xt.XT_ERR_INVALID

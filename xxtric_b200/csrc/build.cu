@@ -621,6 +621,9 @@ __global__ void k_csr_entries(const int64_t *__restrict__ off, const int64_t *__
   const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
   long long tilt = 0;  // entries above their row's id less those below it
   bool bad = false;
+  // entries before the first row are no edges, but ids all the same
+  for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < e_first; e += int64_t(gridDim.x) * blockDim.x)
+    if (tails[e] < 0 || tails[e] >= nv) atomicOr(err, 1);
   for (int64_t w = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; e_first + w * kCsrSpan < ne; w += nw) {
     const int64_t b0 = e_first + w * kCsrSpan;
     int64_t r = row_of(off, nv, b0, lane);
@@ -1240,8 +1243,8 @@ xt_status build_from_csr(Ctx *c, int64_t nv, const int64_t *d_off, const int64_t
     if ((s = dalloc_n(c, &chk, kCsrWords)) != XT_OK) break;
     if ((s = cuda_status(c, cudaMemsetAsync(chk, 0, kCsrWords * sizeof(*chk), c->stream), "memset")) != XT_OK) break;
     k_csr_offsets<<<counted(c, grid_for(nv, B, c->sm_count)), B, 0, c->stream>>>(d_off, nv, ne_in, c->d_err);
-    if (n > 0) {
-      const int64_t warps = (n + kCsrSpan - 1) / kCsrSpan;
+    if (ne_in > 0) {
+      const int64_t warps = (ne_in + kCsrSpan - 1) / kCsrSpan;
       k_csr_entries<<<counted(c, grid_for(warps * 32, B, c->sm_count)), B, 0, c->stream>>>(
           d_off, d_tails, nv, e_first, ne_in, rows, t32, c->d_err, chk);
       k_csr_back<<<counted(c, grid_for(n, B, c->sm_count)), B, 0, c->stream>>>(d_off, nv, rows, t32, e_first, ne_in,
