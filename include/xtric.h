@@ -78,8 +78,9 @@ typedef struct {
   int32_t orient;         /* xt_orient used */
   int32_t reserved;
   int64_t footprint_bytes; /* bytes of the arrays the count reads, each counted once: offsets and
-                              in-record offsets 16(nv+1), columns 4|E+|, padded columns, in-records
-                              8|E+|: the DRAM traffic of a count that never re-reads */
+                              in-record offsets 16(nv+1), the ends of the streamed records 8 nv,
+                              columns 4|E+|, padded columns, in-records 8|E+|, a dense core's tiles
+                              and items: the DRAM traffic of a count that never re-reads */
   int64_t cluster_tasks;   /* global count: the tasks of its thread-block cluster tier (see
                               xt_graph_set_cluster); 0 when no head needs it */
 } xt_graph_info;

@@ -181,3 +181,23 @@ def test_core_allocations_that_fail(ctx):
     assert until_it_passes(lambda: g.count(per_vertex=True))[0] == want
     g.free()
     assert ctx.mem_stats()[0] == held
+
+
+def test_footprint_counts_the_core(ctx):
+    """footprint_bytes: every array a count reads, the core's tiles (16 KB each) and
+    items (8 bytes) among them."""
+    def parts(g, nv):
+        i, off = g.info(), g.csr()[0]
+        padded = int(((np.diff(off) + 7) // 8 * 8).sum())
+        return i["footprint_bytes"] - (16 * (nv + 1) + 8 * nv + 12 * i["n_edges"] + 4 * padded)
+    g = ctx.graph_from_edges(3, np.array([0, 0, 1], np.int32), np.array([1, 2, 2], np.int32))
+    assert parts(g, 3) == 0
+    g.free()
+    # 1,280 dense vertices: 10 row blocks, pairs of them of width 1 to 5 column steps, each
+    # stored in an even number of chunks
+    nv, src, dst = graph(1280)
+    g = ctx.graph_from_edges(nv, src.astype(np.int32), dst.astype(np.int32))
+    core = parts(g, nv)
+    assert core >= 16384 * 2 * 2 * (1 + 2 + 3 + 4 + 5)
+    assert core <= 16384 * (2 * 2 * (1 + 2 + 3 + 4 + 5) + 2 * 5 * 128)
+    g.free()

@@ -1018,6 +1018,12 @@ xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d
   return XT_OK;
 }
 
+int64_t core_bytes(const Graph *g) {
+  const Core &k = g->core;
+  if (k.n_items == 0) return 0;
+  return k.n_tiles * kCoreTile + k.n_items * int64_t(sizeof(int2)) + int64_t(sizeof(int64_t)) * (k.nb + 1);
+}
+
 void core_free(Graph *g) {
   Core &k = g->core;
   for (void *p : {(void *)k.d_tile0, (void *)k.d_tiles, (void *)k.d_before, (void *)k.d_items, (void *)k.d_sym, (void *)k.d_xt,

@@ -230,6 +230,7 @@ void core_decide(Ctx *c, Graph *g, const int64_t *sums);
 xt_status core_finish(Ctx *c, Graph *g);
 xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d_es, int shard, int nshards);
 void core_free(Graph *g);
+int64_t core_bytes(const Graph *g);  // what a count reads of it
 // test hook: tries of each barrier wait of the core's kernels that the calling thread launches (< 0: the default)
 void core_wait_limit(int64_t tries);
 
