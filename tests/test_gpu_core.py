@@ -201,3 +201,28 @@ def test_footprint_counts_the_core(ctx):
     assert core >= 16384 * 2 * 2 * (1 + 2 + 3 + 4 + 5)
     assert core <= 16384 * (2 * 2 * (1 + 2 + 3 + 4 + 5) + 2 * 5 * 128)
     g.free()
+
+
+def test_supports_of_a_wide_core_sum_to_the_vertices_counts(ctx):
+    """R-MAT 2^20, whose core is thousands of positions wide and its products cut into
+    many segments: the supports sum to three times the total, and those around each
+    vertex to twice its own count (which the oracle's digests check elsewhere)."""
+    import torch
+    scale = 20
+    rows = 16 << scale
+    src = torch.empty(rows, dtype=torch.int32, device="cuda")
+    dst = torch.empty_like(src)
+    torch.cuda.synchronize()
+    ctx.gen_rmat(scale, rows, 5, src, dst)
+    g = ctx.graph_from_device_edges(1 << scale, rows, src, dst)
+    total, each = g.count(per_vertex=True)
+    total_e, sup = g.count_edges()
+    assert total == total_e == g.count()
+    off, col = g.csr()
+    p = g.perm()
+    a, b = p[np.repeat(np.arange(len(off) - 1), np.diff(off))], p[col]
+    n = len(off) - 1
+    around = np.bincount(a, sup, n) + np.bincount(b, sup, n)  # whole numbers far below 2^53
+    assert int(sup.sum()) == 3 * total
+    np.testing.assert_array_equal(around.astype(np.int64), 2 * each)
+    g.free()
