@@ -99,10 +99,10 @@ const char *xt_strerror(xt_status s);
 const char *xt_last_error(const xt_ctx *ctx);
 /* test hook: make the k-th device allocation from now fail (k<=0 disarms) */
 xt_status xt_debug_fail_alloc(xt_ctx *ctx, int64_t k);
-/* test hook: the barrier waits of the dense core's kernels in counts that the
- * calling thread starts from now on give up after `tries` tries (negative: the
- * default), which lets a test reach XT_ERR_TIMEOUT */
-xt_status xt_debug_wait_limit(int64_t tries);
+/* test hook: while on, the dense core's kernels of counts that the calling
+ * thread starts begin as if one of their bounded waits had given up, with
+ * copies in flight, which lets a test reach XT_ERR_TIMEOUT */
+xt_status xt_debug_give_up(int on);
 /* number of this library's own kernels launched on the context so far
  * (library sorts and scans from CUB are not included) */
 int64_t xt_launch_count(const xt_ctx *ctx);

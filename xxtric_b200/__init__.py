@@ -70,7 +70,7 @@ _proto("xt_open", _int, _int, _P(_vp))
 _proto("xt_close", _int, _vp)
 _proto("xt_set_stream", _int, _vp, _vp)
 _proto("xt_debug_fail_alloc", _int, _vp, _i64)
-_proto("xt_debug_wait_limit", _int, _i64)
+_proto("xt_debug_give_up", _int, _int)
 _proto("xt_launch_count", _i64, _vp)
 _proto("xt_synchronize", _int, _vp)
 _proto("xt_graph_get_perm", _int, _vp, _vp)
@@ -129,7 +129,7 @@ _proto("xt_vite_write", _int, ctypes.c_char_p, _int, _i64, _vp, _vp)
 _proto("xt_rgg_generate", _int, _i64, _int, _dbl, _dbl, _u64, _i64, _P(_i64), _vp, _vp)
 
 EXPORTED = ["xt_strerror", "xt_last_error", "xt_open", "xt_close", "xt_set_stream", "xt_debug_fail_alloc",
-            "xt_debug_wait_limit", "xt_launch_count", "xt_synchronize", "xt_graph_get_perm",
+            "xt_debug_give_up", "xt_launch_count", "xt_synchronize", "xt_graph_get_perm",
             "xt_graph_from_csr", "xt_graph_from_edges", "xt_graph_from_device_edges", "xt_graph_get_info",
             "xt_graph_get_csr", "xt_graph_free", "xt_count", "xt_count_async", "xt_count_edges", "xt_count_edges_async",
             "xt_count_shard_async", "xt_count_edges_shard_async", "xt_count_device",
@@ -601,10 +601,9 @@ class DeviceGraph:
             pass
 
 
-def debug_wait_limit(tries: int) -> None:
-    """Test hook: tries of each barrier wait of the dense core's kernels that this
-    thread starts (negative: the default)."""
-    _check(_L.xt_debug_wait_limit(tries), "xt_debug_wait_limit")
+def debug_give_up(on: bool) -> None:
+    """Test hook: the dense core's kernels of this thread's counts give up at once."""
+    _check(_L.xt_debug_give_up(int(on)), "xt_debug_give_up")
 
 
 def count_device(nv: int, d_indices, d_edge_list, d_count, accumulate: bool = False, stream: int = 0) -> None:

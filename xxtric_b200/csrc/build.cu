@@ -717,7 +717,8 @@ __global__ void k_csr_back(const int64_t *__restrict__ off, int64_t nv, const in
 // place (-1: not kept), and counts the kept ones per row; pass 2
 // (k_csr_place) writes them at the scanned starts. Entries of one row are
 // consecutive, so a warp adds one count per run of equal rows.
-// run of equal rows around this lane: its first lane, and its lanes
+
+// the run of equal rows around this lane: its first lane, and the mask of its lanes
 __device__ __forceinline__ unsigned row_run(int32_t row, int lane, int &first) {
   const int32_t p = __shfl_up_sync(0xffffffffu, row, 1);
   const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || p != row);

@@ -204,8 +204,8 @@ xt_status xt_debug_fail_alloc(xt_ctx *ctx, int64_t k) {
   return XT_OK;
 }
 
-xt_status xt_debug_wait_limit(int64_t tries) {
-  core_wait_limit(tries);
+xt_status xt_debug_give_up(int on) {
+  core_give_up(on != 0);
   return XT_OK;
 }
 

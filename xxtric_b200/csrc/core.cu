@@ -60,8 +60,6 @@ constexpr int64_t kStepFs = 2200000;
 constexpr int64_t kCoreMinFs = int64_t(20) * 1000 * 1000 * 1000;
 constexpr int64_t kCoreMaxBytes = 16;  // operand bytes per edge, at most
 
-// the kCoreSums words: tiles, items, widest J, gain in fs
-
 // J = T_b / 256 of row block blockIdx.x: four rows a warp, each lane holding
 // the benefit of two widths. A row has C(c, 2) candidates whose v lies in the
 // top T positions, c its columns there: its entries from the end on, 128 at a
@@ -302,7 +300,7 @@ struct CoreArgs {
   int64_t stride;
   unsigned long long *global;
   int *err;
-  uint32_t wait_limit;  // tries of a barrier wait
+  int give_up;     // as if a wait had given up already (test hook)
   // per vertex and per edge
   const uint8_t *sym;      // S: tile (row block, chunk) at row block * 2 jtop + chunk
   const int32_t *jw;
@@ -334,10 +332,11 @@ __device__ __forceinline__ void core_expect(uint64_t *bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(core_smem(bar)), "r"(bytes)
                : "memory");
 }
-// waits for the barrier's phase, at most `limit` tries; gives up early once
-// another warp of the CTA has
-__device__ __forceinline__ bool core_wait(uint64_t *bar, uint32_t parity, volatile int *fail, uint32_t limit) {
-  for (uint32_t it = 0; it < limit; it++) {
+// waits for the barrier's phase, at most kCoreWaitLimit tries; gives up early
+// once another warp of the CTA has (the limit as a kernel argument cost the products
+// 3%, 70 us of a R-MAT 2^24 count)
+__device__ __forceinline__ bool core_wait(uint64_t *bar, uint32_t parity, volatile int *fail) {
+  for (uint32_t it = 0; it < kCoreWaitLimit; it++) {
     uint32_t done;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
@@ -444,7 +443,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
       core_bar_init(&s_tempty[i], 4);
     }
     core_bar_init(&s_drain, 1);
-    s_fail = 0;
+    s_fail = a.give_up;
     if (KIND == kCoreInner) {  // items before each level
       int32_t at = 0;
       for (int t = 0; t < a.jtop; t++) {
@@ -474,7 +473,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
     // stage k's buffer once it is free, its barrier expecting the step's bytes
     auto stage = [&]() -> uint8_t * {
       const uint32_t sg = k % kCoreStages;
-      if (!core_wait(&s_empty[sg], ((k / kCoreStages) & 1u) ^ 1u, fail, a.wait_limit)) return nullptr;
+      if (!core_wait(&s_empty[sg], ((k / kCoreStages) & 1u) ^ 1u, fail)) return nullptr;
       core_expect(&s_full[sg], kCoreStageBytes);
       return st + sg * kCoreStageBytes;
     };
@@ -532,7 +531,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
     if (lane == 0)
       for (uint32_t q = k > kCoreStages ? k - kCoreStages : 0; q < k; q++) {
         int quiet = 0;
-        core_wait(&s_full[q % kCoreStages], (q / kCoreStages) & 1u, &quiet, kCoreWaitLimit);
+        core_wait(&s_full[q % kCoreStages], (q / kCoreStages) & 1u, &quiet);
       }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -540,13 +539,13 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
       uint32_t k = 0, t = 0;
       for (int64_t i = blockIdx.x; i < n && !*fail; i += gridDim.x) {
         if (!core_item<KIND>(a, s_pfx, i, it)) continue;
-        if (!core_wait(&s_tempty[t & 1], ((t >> 1) & 1u) ^ 1u, fail, a.wait_limit)) break;
+        if (!core_wait(&s_tempty[t & 1], ((t >> 1) & 1u) ^ 1u, fail)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d = tmem + (t & 1) * kCoreStep;
         bool ok = true;
         for (int c = 0; c < it.steps; c++, k++) {
           const uint32_t sg = k % kCoreStages;
-          if (!core_wait(&s_full[sg], (k / kCoreStages) & 1u, fail, a.wait_limit)) {
+          if (!core_wait(&s_full[sg], (k / kCoreStages) & 1u, fail)) {
             ok = false;
             break;
           }
@@ -564,7 +563,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
       }
       core_commit(&s_drain);  // every product issued is done before the accumulators are given back
       int quiet = 0;
-      core_wait(&s_drain, 0, &quiet, kCoreWaitLimit);
+      core_wait(&s_drain, 0, &quiet);
     }
     __syncwarp();
   } else {
@@ -583,7 +582,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) k_core_count(const CoreArgs a
       unsigned int *es = nullptr;  // per edge: the row's entry at the next position
       if ((KIND == kCoreEdges || KIND == kCoreInner) && u >= 0)
         es = a.es + a.poff[u] + (a.off[u + 1] - a.off[u]) - 1 - a.before[mt / 2 * kCoreRows + r];
-      if (!__all_sync(0xffffffffu, core_wait(&s_tfull[t & 1], (t >> 1) & 1u, fail, a.wait_limit))) break;
+      if (!__all_sync(0xffffffffu, core_wait(&s_tfull[t & 1], (t >> 1) & 1u, fail))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       int32_t sum = 0;
 #pragma unroll
@@ -850,8 +849,8 @@ __global__ void __launch_bounds__(kSearchThreads)
 
 // ---- host side ------------------------------------------------------------------
 
-static thread_local int64_t t_wait_limit = -1;  // xt_debug_wait_limit
-void core_wait_limit(int64_t tries) { t_wait_limit = tries; }
+static thread_local bool t_give_up = false;  // xt_debug_give_up
+void core_give_up(bool on) { t_give_up = on; }
 
 // Widths of the row blocks from the unique rows (row u: cols[rstart[u]] on, as
 // many as off says), and their layout; *d_sums has kCoreSums words once the
@@ -860,7 +859,9 @@ void core_wait_limit(int64_t tries) { t_wait_limit = tries; }
 xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *cols, int64_t n, int64_t **d_sums) {
   *d_sums = nullptr;
   Core &k = g->core;
-  // m edges have at most (2m)^1.5 / 6 candidates: below 2^17 edges (of at most n rows), less than the least gain
+  // by degree, n rows without many repeats have some (2n)^1.5 / 6 candidates at most: below
+  // 2^17 rows less than the least gain. By id there is no such bound; small id-ordered graphs
+  // go without a core all the same, as their builds are short next to picking one
   if (g->no_core || n < (int64_t(1) << 17)) return XT_OK;
   const int64_t blocks = (g->nv + kCoreRows - 1) / kCoreRows;
   k.nb = int(std::max<int64_t>(kCoreMinBlk, std::min<int64_t>(blocks, kCoreMaxBlk)));
@@ -938,7 +939,7 @@ xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d
   a.stride = 1;
   a.global = reinterpret_cast<unsigned long long *>(d_global);
   a.err = c->d_err;
-  a.wait_limit = t_wait_limit < 0 ? kCoreWaitLimit : uint32_t(std::min<int64_t>(t_wait_limit, kCoreWaitLimit));
+  a.give_up = t_give_up ? 1 : 0;
   a.nv = g->nv;
   if (!d_pv && !d_es) {
     if (k.n_items <= shard) return XT_OK;

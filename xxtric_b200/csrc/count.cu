@@ -74,7 +74,8 @@ constexpr int kWarps = kThreads / 32;
 #define XT_MIN_BLOCKS 4
 #endif
 // CTAs per SM the register budget is sized for: 4 x 256 threads leave 64
-// registers a thread (no spills). Swept with the task size at R-MAT s24
+// registers a thread (with the packs in the kernel ptxas keeps 16 bytes of a thread's
+// state on the stack; which tier's it has not been settled). Swept with the task size at R-MAT s24
 // (before the cuckoo sets): 3 CTAs/SM with 2^17-candidate tasks 34.2 ms, 4
 // with 2^17 33.8 ms, 4 with 2^16 32.1 ms, 4 with 2^15 35.1 ms, 5 (spilling)
 // 53.9 ms
@@ -407,8 +408,8 @@ __global__ void k_plan_fill(int64_t nv, const int64_t *__restrict__ off, const i
       // steps as its first record needs on S lanes (its pairs: the suffix
       // length plus an average offset into its first pair, over 8); each
       // batch also costs about one step of set-up. Heads of many records are
-      // sampled, at most kPlanSamples batches for each choice (one thread walking all
-      // of a head's 4,000 short records held the R-MAT 2^18 plan for 440 us; with
+      // sampled, about kPlanSamples batches for each choice, each standing for a stride
+      // of them (a short last stride is charged whole; one thread walking all of a head's 4,000 short records held the R-MAT 2^18 plan for 440 us; with
       // 64 samples a batch of 256 graphs spends 137 us here, with 16 110, and the
       // counts are the same to 0.2%).
       int32_t lg_s = 0;
@@ -1784,8 +1785,6 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
   }
 }
 
-// dynamic shared memory: member words; in modes 1 and 2 also hash counters
-// or bitmap word starts, and bitmap member counters
 // ---- the cluster tier (global count) ---------------------------------------
 //
 // A cluster of kCluster CTAs counts one cluster task at a time: the part's
@@ -1893,6 +1892,8 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, XT_
   }
 }
 
+// dynamic shared memory: member words; in modes 1 and 2 also 16 bits a word (member
+// indices, a pack's hits) and member counters
 static size_t count_smem_bytes(bool pv) {
   return pv ? sizeof(int32_t) * (kBlockWords + kBlockDmax) + sizeof(uint16_t) * kBlockWords
             : sizeof(int32_t) * kBlockWords;
@@ -2052,7 +2053,9 @@ xt_status make_plan(Graph *g) {
     // CTA task size: large tasks amortise the member-set build and the task
     // barrier, but every CTA should still get about 16 of them
     int64_t total_work = 0;
-    // by degree, below 2^17 edges there are some 2^25 candidates at most: sizes are
+    // by degree, below 2^17 edges there are some 2^25 candidates (out-degrees stay below
+    // the root of twice the rows that the degrees are counted from; a list that repeats
+    // its rows many times over can exceed it and gets the sizes all the same): sizes are
     // the smallest whatever their number, packs go by records (waiting for it costs a
     // build of 100,000 edges 16 us of 530, and saves its count 1 of 40)
     if (ne >= (int64_t(1) << 17) || g->orient != XT_ORIENT_DEGREE) {

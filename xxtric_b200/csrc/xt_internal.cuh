@@ -223,7 +223,7 @@ xt_status build_batch(Ctx *c, int64_t ng, const int64_t *h_voff, const int64_t *
 // The dense core (core.cu), in the builder's order: widths chosen from the
 // unique rows, kept or dropped once their sums are read back, then operands
 // and items from the finished graph; its part of a count.
-constexpr int kCoreSums = 4;
+constexpr int kCoreSums = 4;  // words read back: tiles, items, widest row block, gain in fs
 constexpr int kErrCoreTimeout = 16;  // bit of the context's error word: a bounded wait of the core's kernel gave up
 xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *cols, int64_t m, int64_t **d_sums);
 void core_decide(Ctx *c, Graph *g, const int64_t *sums);
@@ -231,8 +231,8 @@ xt_status core_finish(Ctx *c, Graph *g);
 xt_status core_count(Graph *g, int64_t *d_global, int64_t *d_pv, unsigned int *d_es, int shard, int nshards);
 void core_free(Graph *g);
 int64_t core_bytes(const Graph *g);  // what a count reads of it
-// test hook: tries of each barrier wait of the core's kernels that the calling thread launches (< 0: the default)
-void core_wait_limit(int64_t tries);
+// test hook: whether the core's kernels that the calling thread launches give up at once
+void core_give_up(bool on);
 
 // Builds (or rebuilds) the per-graph schedule and graph statistics.
 xt_status make_plan(Graph *g);
