@@ -66,6 +66,12 @@ void dfree(Ctx *c, void *p) {
   cudaFreeAsync(p, c->stream);
 }
 
+// what a caller's counter (words[0], as it was) becomes: unchanged where a wait of
+// the count gave up
+__global__ void k_deliver(CountOut *__restrict__ out, int accumulate) {
+  if (!(out->err & kErrWaits)) out->words[0] = out->total + (accumulate ? out->words[0] : 0);
+}
+
 struct WordList {
   const int64_t *p[12];
 };
@@ -448,24 +454,22 @@ xt_status xt_count_device(int64_t nv, const int64_t *d_indices, const int64_t *d
   Graph g;
   xt_status s = build_from_csr(c, nv, d_indices, d_edge_list, true, XT_ORIENT_DEGREE, &g);
   if (s == XT_OK) s = make_plan(&g);
+  // the counter goes through the result block, so that one wait serves the error word too
+  if (s == XT_OK)
+    s = cuda_status(c, cudaMemcpyAsync(c->d_out->words, d_count, sizeof(int64_t), cudaMemcpyDeviceToDevice, c->stream),
+                    "D2D");
   if (s == XT_OK) s = count_graph(&g, &c->d_out->total, nullptr);
-  // a count whose device waits gave up is reported, and leaves *d_count as it was
-  int64_t add = 0;
-  if (s == XT_OK) s = count_status(c, &add);
-  if (s == XT_OK && accumulate) {
-    int64_t h = 0;
-    s = cuda_status(c, cudaMemcpyAsync(&h, d_count, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream), "D2H");
-    if (s == XT_OK) s = cuda_status(c, cudaStreamSynchronize(c->stream), "sync");
-    h += add;
-    if (s == XT_OK)
-      s = cuda_status(c, cudaMemcpyAsync(d_count, &h, sizeof(int64_t), cudaMemcpyHostToDevice, c->stream), "H2D");
-  } else if (s == XT_OK) {
-    s = cuda_status(c, cudaMemcpyAsync(d_count, &c->d_out->total, sizeof(int64_t), cudaMemcpyDeviceToDevice,
-                                       c->stream), "D2D");
+  if (s == XT_OK) {
+    k_deliver<<<counted(c, dim3(1)), 1, 0, c->stream>>>(c->d_out, accumulate);
+    s = cuda_status(c, cudaGetLastError(), "k_deliver");
   }
+  if (s == XT_OK)
+    s = cuda_status(c, cudaMemcpyAsync(d_count, c->d_out->words, sizeof(int64_t), cudaMemcpyDeviceToDevice, c->stream),
+                    "D2D");
   free_graph_device(&g);
+  const xt_status done = count_status(c);  // waits for the stream
+  if (s == XT_OK) s = done;
   cudaFreeAsync(c->d_out, c->stream);
-  cudaStreamSynchronize(c->stream);
   delete ctx;
   return s;
 }

@@ -156,8 +156,6 @@ struct PlanParams {
 #define XT_LANE_LOOP 0
 #endif
 constexpr bool kWarpCuckoo = XT_WARP_CUCKOO != 0;
-// bit of the context's error word set when a bounded staging wait gave up
-constexpr int kErrStageTimeout = 8;
 constexpr int32_t kEmpty = -1;
 
 // A warp or CTA task: the in-records [k0, k0 + nrec) of head v streamed
@@ -2228,7 +2226,7 @@ xt_status count_status(Ctx *c, int64_t *total) {
   XT_CUDA(c, cudaStreamSynchronize(c->stream));
   if (total) *total = o.total;
   const int h = o.err;
-  if (h & (kErrStageTimeout | kErrCoreTimeout)) {
+  if (h & kErrWaits) {
     XT_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
     return set_error(c, XT_ERR_TIMEOUT, "count: a CTA's wait for its staged data timed out");
   }

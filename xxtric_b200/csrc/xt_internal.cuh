@@ -20,6 +20,8 @@ constexpr size_t kColPad = 8;
 // device block read back by the synchronous counts in one copy: the error word
 // that kernels set when their input or a bounded wait fails, and a total
 constexpr int kErrInput = 3;  // its bits of a build: an id out of range (1), offsets not monotone (2)
+constexpr int kErrStageTimeout = 8, kErrCoreTimeout = 16;  // of a count: a staging wait, a wait of the core's gave up
+constexpr int kErrWaits = kErrStageTimeout | kErrCoreTimeout;
 struct CountOut {
   int err;
   int reserved;
@@ -224,7 +226,6 @@ xt_status build_batch(Ctx *c, int64_t ng, const int64_t *h_voff, const int64_t *
 // unique rows, kept or dropped once their sums are read back, then operands
 // and items from the finished graph; its part of a count.
 constexpr int kCoreSums = 4;  // words read back: tiles, items, widest row block, gain in fs
-constexpr int kErrCoreTimeout = 16;  // bit of the context's error word: a bounded wait of the core's kernel gave up
 xt_status core_plan(Ctx *c, Graph *g, const int64_t *rstart, const uint32_t *cols, int64_t m, int64_t **d_sums);
 void core_decide(Ctx *c, Graph *g, const int64_t *sums);
 xt_status core_finish(Ctx *c, Graph *g);
