@@ -588,12 +588,13 @@ def run_e2e(args, ctx, stream, torch, n, ne, src, dst, g, counts, info) -> dict:
 
 
 def roofline_fields(args, info: dict, t_kernel: float) -> dict:
-    """The count kernel's roofline. `achieved` is DRAM bytes per launch over
-    the kernel's CUDA-event time in this run, the DRAM bytes taken from the
-    committed ncu capture of one launch of this workload (`traffic_source`);
-    without a capture it falls back to the bytes the schedule's loads request
-    (`basis` says which). Beside it: the requested (logical) bytes, the
-    compulsory footprint (each array read once), the tail-grouped formula's
+    """The count's roofline, over its kernels together (the streaming one and, where
+    the graph has a dense core, the core's). `achieved` is DRAM bytes per count over
+    the kernels' CUDA-event time in this run, the DRAM bytes taken from the
+    committed ncu capture of one count of this workload (`traffic_source`);
+    without a capture it falls back to the bytes that a count streaming every
+    candidate requests, the core's among them (`basis` says which). Beside it: those
+    (logical) bytes, the compulsory footprint (each array read once), the tail-grouped formula's
     bytes, and the issue-slot utilisation of the small-case capture."""
     peaks = measured_peaks()
     peak = peaks["hbm_gbs"]
@@ -603,16 +604,19 @@ def roofline_fields(args, info: dict, t_kernel: float) -> dict:
     dram = profiled_value(name, "dram_bytes_per_launch_full_size") if name and args.scale == SCALE else None
     logical = info["alg_bytes"] / t_kernel / 1e9
     r = {"bound": "hbm", "peak": peak, "unit": "GB/s", "peak_source": peaks["source"],
-         "kernel": {"global": "k_count<0>", "per-vertex": "k_count<1>",
-                    "per-edge": "k_count<2>"}[getattr(args, "mode", "global")], "kernel_ms": 1e3 * t_kernel}
+         "kernel": {"global": "k_count<0>, with k_core_count<0> where the graph has a dense core",
+                    "per-vertex": "k_count<1>, with k_core_count<1> where the graph has a dense core",
+                    "per-edge": "k_count<2>, with k_core_count<2> and <3> where the graph has a dense core",
+                    }[getattr(args, "mode", "global")], "kernel_ms": 1e3 * t_kernel}
     if dram:
         a = dram / t_kernel / 1e9
         r.update({"achieved": a, "frac": a / peak, "traffic": int(dram),
-                  "basis": "DRAM bytes per launch (ncu capture of one full-size launch) / kernel time in this run",
+                  "basis": "DRAM bytes per count (ncu capture of one full-size count's kernels) / their time in this run",
                   "traffic_source": f"profiles/{name} (dram__bytes_read.sum + dram__bytes_write.sum)"})
     else:
         r.update({"achieved": logical, "frac": logical / peak, "traffic": None,
-                  "basis": "bytes the schedule's loads request (no ncu capture of this workload committed)",
+                  "basis": "bytes a count that streams every candidate requests, those counted in a dense core "
+                           "included (no ncu capture of this workload committed)",
                   "traffic_source": None})
     r.update({"logical_bytes": info["alg_bytes"], "logical_achieved": logical, "logical_frac": logical / peak,
               "footprint_bytes": info["footprint_bytes"],
