@@ -158,3 +158,29 @@ def test_chunglu_config_properties(ctx):
     rng = np.random.default_rng(3)
     sel = np.concatenate([np.argsort(deg)[-32:], rng.choice(n, 2000, replace=False)])
     assert (oracle.local_counts(off, tails, sel) == pv[sel]).all()
+
+
+@pytest.mark.parametrize("rows", [66_000_000, 69_000_000])
+def test_warp_tasks_from_either_end(ctx, rows):
+    """A uniform graph, all warp tasks and packs, below and above the 2^26 edges from
+    which the global count takes the warp tasks in ascending order: whole and in
+    shards it agrees with the per-vertex count, which does not."""
+    import torch
+    n = 3_000_001
+    s = torch.empty(rows, dtype=torch.int32, device="cuda")
+    d = torch.empty_like(s)
+    torch.cuda.synchronize()
+    ctx.gen_er(n, rows, 3, s, d)
+    g = ctx.graph_from_device_edges(n, rows, s, d)
+    assert (g.info()["n_edges"] >= 1 << 26) == (rows > 1 << 26)
+    t, pv = g.count(per_vertex=True)
+    assert pv.sum() == 3 * t and g.count() == t
+    part = torch.zeros(1, dtype=torch.int64, device="cuda")
+    for shards in (2, 5):
+        got = 0
+        for i in range(shards):
+            g.count_shard_async(i, shards, part)
+            ctx.synchronize()
+            got += int(part)
+        assert got == t
+    g.free()

@@ -91,6 +91,13 @@ constexpr int64_t kWarpCost = 32768, kWarpRecCost = 16;
 // candidates (kWarpCostMin 12,288 / 8,192 / 4,096: Chung-Lu 2^14 50 / 53 / 60 us,
 // R-MAT 2^12 49 / 39 / 37)
 constexpr int64_t kWarpCostMin = 8192, kWarpMostMin = 4096;
+// Warp tasks go from the high ranks down, so that the long ones come early and the
+// last are short (R-MAT 2^18 140 -> 130 us, Chung-Lu 2^14 45 -> 40). The global
+// count of this many edges takes them the other way: its warps outrun the memory where
+// the graph is all warp tasks, and from the top down a uniform one of 2^22 vertices
+// takes 5.2 ms with 24 rows a vertex (4.65 ascending) and 7.2 with 32 (6.7); graphs with CTA
+// tasks are the same to 0.1% either way.
+constexpr int64_t kAscendEdges = int64_t(1) << 26;
 #ifndef XT_BLOCK_DMAX
 #define XT_BLOCK_DMAX 2048
 #endif
@@ -177,6 +184,7 @@ struct Plan {
   Task *d_bt = nullptr;
   int64_t n_wtask = 0;         // warp tasks
   Task *d_wt = nullptr;
+  bool high_first = false;     // the warp tasks stand from the last head to the first
   int64_t n_ptask = 0;         // packs
   Task *d_pt = nullptr;
   int64_t n_ttask = 0;         // lane tasks: one head per lane
@@ -1049,6 +1057,7 @@ struct CountArgs {
   int64_t n_ct;
   int lane_merge;  // lane tasks: members found by a two-pointer merge (1) or binary search (0)
   int64_t stride;  // task lists hold every stride-th task of the schedule (a shard of it), else 1
+  int64_t wstride;  // the same of the warp tasks, negative from the list's end to its start
   int beside;      // launched as the core's kernel drains: waits for it at the end
   int claim;       // warp tasks (and groups of 32 lane tasks) taken from their cursor per atomic
   unsigned long long *cursor;     // [0] CTA, [1] warp, [2] lane, [4] pack cursors
@@ -1488,7 +1497,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
     // the whole 1,024-word slice per task.
     int32_t *wstage = s_stage + warp * kStageWarp;
     int32_t *words = bwords + warp * kWarpWords;
-    Task t = claim_task_block(wclaim, &cursor[1], a.wt, a.n_wt, a.stride, a.claim, lane);
+    Task t = claim_task_block(wclaim, &cursor[1], a.wt, a.n_wt, a.wstride, a.claim, lane);
     int so = stage_task(wstage, col, rec, t, lane);
     zero_words(words, kWarpWords, lane, 32);
     while (true) {
@@ -1502,7 +1511,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
       m.mcnt = nullptr;
       const bool ok = warp_set_build(m, mem, t.nmem, kWarpWords, a.bitmap_bits, a.cuckoo_iters, lane);
       __syncwarp();
-      const Task tn = claim_task_block(wclaim, &cursor[1], a.wt, a.n_wt, a.stride, a.claim, lane);  // read after the stream
+      const Task tn = claim_task_block(wclaim, &cursor[1], a.wt, a.n_wt, a.wstride, a.claim, lane);  // read after the stream
       int64_t h;
       if (ok) {
         h = stream_suffixes<MODE, PF>(rec, a.rec_u, a.colp, t.k0, t.k0 + t.nrec, t.lg_s, nullptr, m, pv, es, off, a.poff, lane);
@@ -1530,7 +1539,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
     }
   } else {
     int32_t *wstage = s_stage + warp * kStageWarp;
-    Task t = claim_task_block(wclaim, &cursor[1], a.wt, a.n_wt, a.stride, a.claim, lane);
+    Task t = claim_task_block(wclaim, &cursor[1], a.wt, a.n_wt, a.wstride, a.claim, lane);
     int so = stage_task(wstage, col, rec, t, lane);
     while (true) {
       cp_async_wait_all();
@@ -1546,7 +1555,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
       __syncwarp();
       for (int i = lane; i < t.nmem; i += 32) members_insert_at<PV>(m, mem, i);
       __syncwarp();
-      const Task tn = claim_task_block(wclaim, &cursor[1], a.wt, a.n_wt, a.stride, a.claim, lane);  // read after the stream
+      const Task tn = claim_task_block(wclaim, &cursor[1], a.wt, a.n_wt, a.wstride, a.claim, lane);  // read after the stream
       int64_t h = stream_suffixes<MODE, PF>(rec, a.rec_u, a.colp, t.k0, t.k0 + t.nrec, t.lg_s, nullptr, m, pv, es, off, a.poff,
                                         lane);
       acc += h;
@@ -2112,6 +2121,7 @@ xt_status make_plan(Graph *g) {
       pp.block_work = kBlockWorkMin;
       while (pp.block_work < kBlockWorkMax && pp.block_work * 16 * pl->grid_global < total_work) pp.block_work *= 2;
     }
+    pl->high_first = pp.high_first;
     pl->block_work = pp.block_work;
     pl->warp_work = pp.warp_work;
     if ((s = dalloc_n(c, &nb, size_t(nv + 1))) != XT_OK) break;
@@ -2383,7 +2393,7 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   a.n_tt = shard_len(pl->n_ttask, shard, nshards);
   a.ct = shard_first(pl->d_ct, pl->n_ctask, shard);
   a.n_ct = shard_len(pl->n_ctask, shard, nshards);
-  a.stride = nshards;
+  a.stride = a.wstride = nshards;
   a.beside = 0;
   a.claim = g->claim_block > 0 ? g->claim_block : (g->n_groups > 0 ? 4 : 1);
   a.lane_merge = g->lane_merge;
@@ -2411,6 +2421,10 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
       if (pl->n_ctask > 0) {
         a0.bt = shard_first(pl->d_bt0, pl->n_btask0, shard);
         a0.n_bt = shard_len(pl->n_btask0, shard, nshards);
+      }
+      if (pl->high_first && g->ne >= kAscendEdges && a0.n_wt > 0) {
+        a0.wt += (a0.n_wt - 1) * nshards;
+        a0.wstride = -nshards;
       }
       a0.beside = core ? 1 : 0;
       s = launch_count(c, g->prefetch_suffix > 0 ? k_count<0, true> : k_count<0, false>, pl->grid_global,
