@@ -286,8 +286,8 @@ xt_status xt_graph_set_cluster(xt_graph *g, int on);
 xt_status xt_graph_set_lane_intersect(xt_graph *g, int kind);
 /* No counterpart in the reference (its kernels take vertices by grid
  * index): warp tasks, and lane tasks in groups of 32 heads, are taken from
- * their global cursor `claim` at a time (1..64; 0, the default: 4 for a
- * graph built as a batch, 1 otherwise). One atomic on one address per task
+ * their global cursor `claim` at a time (1..64; 0, the default: 1, and up to
+ * 4 for a graph built as a batch whose tasks leave every warp 8 such blocks). One atomic on one address per task
  * limits schedules of many small tasks (the 4,096-graph batch, before small
  * heads were packed: 38.2 ms a count with 1, 30.4 ms with 4); larger blocks leave a longer tail on
  * graphs whose warp tasks are fewer (R-MAT scale 22: 4.69 ms with 1, 4.79

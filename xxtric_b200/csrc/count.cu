@@ -1154,7 +1154,10 @@ __device__ __forceinline__ Task claim_task(unsigned long long *cursor, const Tas
 // tasks are many and small (the 4,096-graph batch: 38.2 -> 30.4 ms with 4)
 // that atomic is the limit; elsewhere a block lengthens the tail (R-MAT s22
 // 4.69 -> 4.79 ms with 4; s24 and Chung-Lu unchanged), so a plain graph
-// claims one at a time and a batch four (xt_graph_set_claim, the autotuner).
+// claims one at a time and a batch up to four, but no fewer than eight blocks a
+// warp (xt_graph_set_claim, the autotuner). With four always, a batch of 8 graphs took
+// 179 us in id order (153 with one), of 32 graphs 256 (229); from 128 on four is as good or
+// better (256 graphs in id order 1,399 us, 1,486 with one).
 // Where no CTA tasks come first, every warp starts on the block of its own
 // index, without an atomic (first != 0: the blocks given out that way).
 struct ClaimBlock {
@@ -2395,7 +2398,8 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   a.n_ct = shard_len(pl->n_ctask, shard, nshards);
   a.stride = a.wstride = nshards;
   a.beside = 0;
-  a.claim = g->claim_block > 0 ? g->claim_block : (g->n_groups > 0 ? 4 : 1);
+  const int64_t blocks = (a.n_wt + a.n_pt) / (8 * int64_t(pl->grid_global) * kWarps);
+  a.claim = g->claim_block > 0 ? g->claim_block : g->n_groups > 0 ? int(std::max<int64_t>(1, std::min<int64_t>(blocks, 4))) : 1;
   a.lane_merge = g->lane_merge;
   a.cursor = pl->d_cursor;
   a.global = reinterpret_cast<unsigned long long *>(d_global);
