@@ -733,12 +733,21 @@ xt_status xt_count_groups(xt_graph *gr, int64_t *total, int64_t *per_group) {
   Ctx *c = g.ctx;
   cudaSetDevice(c->device);
   XT_TRY(run_count_res(&g));
-  XT_CUDA(c, cudaMemcpyAsync(total, g.d_res, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
-  if (per_group && g.n_groups > 0)
-    XT_CUDA(c, cudaMemcpyAsync(per_group, g.d_res + 1, sizeof(int64_t) * g.n_groups, cudaMemcpyDeviceToHost,
-                               c->stream));
-  XT_CUDA(c, cudaStreamSynchronize(c->stream));
-  return count_status(c);
+  // the total and the graphs' counts in one copy (each into pageable memory holds the host for 7 us)
+  const size_t n = 1 + size_t(per_group && g.n_groups > 0 ? g.n_groups : 0);
+  int64_t *res = new (std::nothrow) int64_t[n];
+  if (!res) return set_error(c, XT_ERR_OOM, "host memory for the counts");
+  xt_status s = cuda_status(c, cudaMemcpyAsync(res, g.d_res, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, c->stream),
+                            "D2H");
+  if (s == XT_OK) s = count_status(c);  // waits for the stream
+  if (s == XT_OK) {
+    *total = res[0];
+    if (n > 1) std::memcpy(per_group, res + 1, sizeof(int64_t) * (n - 1));
+  } else {
+    cudaStreamSynchronize(c->stream);  // no copy outlives the buffer
+  }
+  delete[] res;
+  return s;
 }
 
 int64_t xt_graph_groups(const xt_graph *gr) { return gr ? gr->g.n_groups : -1; }
