@@ -149,3 +149,19 @@ def test_pack_credits_from_both_tables(ctx, kind):
         a, b, s = g.edge_support()
         np.testing.assert_array_equal(s[np.lexsort((b, a))], sup)
     g.free()
+
+
+@pytest.mark.parametrize("orient", [0, 1])
+@pytest.mark.parametrize("ng", [3, 256, 257])
+def test_packs_credit_few_and_many_graphs(ctx, ng, orient):
+    """Batches of 3 to 257 rings (as many triangles as vertices), whose heads are
+    credited to their graphs together or one by one."""
+    n = 60000 // ng + np.arange(ng) % 5
+    voff = np.concatenate([[0], np.cumsum(n)])
+    i = [np.arange(k) for k in n]
+    src = np.concatenate([np.concatenate([a, a]) for a in i]).astype(np.int32)
+    dst = np.concatenate([np.concatenate([(a + 1) % k, (a + 2) % k]) for a, k in zip(i, n)]).astype(np.int32)
+    b = ctx.graph_from_batch(voff, 2 * voff, src, dst, orient)
+    total, per = b.count_groups()
+    assert total == n.sum() and per.tolist() == n.tolist()
+    b.free()
