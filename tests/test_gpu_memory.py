@@ -15,7 +15,7 @@ def ctx():
         yield c
 
 
-def wide_core(n_core=600, n_band=20000, per_row=120):
+def wide_core(n_core=600, n_band=20000, per_row=160):
     """A dense core below a band of rows that reach into it: some 160 row blocks of
     three column steps."""
     rng = np.random.default_rng(17)
@@ -154,7 +154,7 @@ def test_counts_without_operands(ctx, want, mode):
         g.free()
 
 
-@pytest.mark.parametrize("nshards", [2, 5])
+@pytest.mark.parametrize("nshards", [2, 3])
 def test_shards_with_and_without_operands_add_up(ctx, want, nshards):
     """One shard counts without the operands, the others with them."""
     import torch
@@ -170,6 +170,7 @@ def test_shards_with_and_without_operands_add_up(ctx, want, nshards):
             each = torch.zeros(want.nv, dtype=torch.int64, device="cuda")
             edge = torch.zeros(m, dtype=torch.int64, device="cuda")
             torch.cuda.synchronize()
+            g.count_shard_async(i, nshards, part)  # the shards' schedule
             ctx.fail_alloc_after(3 if i == alone else 0)  # the records' tails, the counts, S
             g.count_shard_async(i, nshards, part, each)
             ctx.synchronize()
@@ -185,3 +186,45 @@ def test_shards_with_and_without_operands_add_up(ctx, want, nshards):
         assert (totals == want.total).all()
         np.testing.assert_array_equal(pv, want.pv)
         np.testing.assert_array_equal(es, want.by_position)
+
+
+@pytest.mark.parametrize("nshards", [2, 16])
+def test_shards_of_every_size_add_up(ctx, want, nshards):
+    """Two shards count their part of the core, sixteen stream all their records; the
+    same after the schedule has been made anew."""
+    import torch
+    g = want.build(ctx)
+    want.check_edges(g)
+    part = torch.zeros(1, dtype=torch.int64, device="cuda")
+    each = torch.zeros(want.nv, dtype=torch.int64, device="cuda")
+    edge = torch.zeros(len(want.by_position), dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    for again in range(2):
+        totals, pv, es = np.zeros(3, np.int64), np.zeros(want.nv, np.int64), np.zeros(len(edge), np.int64)
+        before = ctx.launches
+        for i in range(nshards):
+            g.count_shard_async(i, nshards, part)
+            ctx.synchronize()
+            totals[0] += int(part)
+        if again:
+            assert (ctx.launches - before == 3 * nshards) == (nshards == 2), "with the core's kernel, or without"
+        for i in range(nshards):
+            g.count_shard_async(i, nshards, part, each)
+            ctx.synchronize()
+            totals[1] += int(part)
+            pv += each.cpu().numpy()
+            g.count_edges_shard_async(i, nshards, part, edge)
+            ctx.synchronize()
+            totals[2] += int(part)
+            es += edge.cpu().numpy()
+        assert (totals == want.total).all()
+        np.testing.assert_array_equal(pv, want.pv)
+        np.testing.assert_array_equal(es, want.by_position)
+        want.check_vertices(g)
+        if not again:
+            g.set_tuning(0, 2048, 0)
+            g.set_tuning(0, 0, 0)
+            g.count_shard_async(0, nshards, part)  # builds what the next launches do not
+            g.count_shard_async(0, nshards, part, each)
+            ctx.synchronize()
+    g.free()

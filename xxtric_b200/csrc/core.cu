@@ -896,6 +896,7 @@ void core_decide(Ctx *c, Graph *g, const int64_t *sums) {
   k.n_tiles = sums[0];
   k.n_items = sums[1];
   k.jtop = int(sums[2]);
+  k.gain_fs = sums[3];
 }
 
 // Operands and work items from the finished out-CSR. Called when the build's

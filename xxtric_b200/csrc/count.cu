@@ -184,6 +184,7 @@ struct Plan {
   Task *d_bt = nullptr;
   int64_t n_wtask = 0;         // warp tasks
   Task *d_wt = nullptr;
+  int64_t load = 0;            // candidates and kWarpRecCost a record, for each of the GPU's warps
   bool high_first = false;     // the warp tasks stand from the last head to the first
   int64_t n_ptask = 0;         // packs
   Task *d_pt = nullptr;
@@ -1938,10 +1939,8 @@ static xt_status exclusive_scan(Ctx *c, const int64_t *in, int64_t *out, int64_t
   return XT_OK;
 }
 
-void free_plan(Graph *g) {
-  Plan *pl = g->plan;
+static void free_one_plan(Ctx *c, Plan *&pl) {
   if (!pl) return;
-  Ctx *c = g->ctx;
   dfree(c, pl->d_bt);
   dfree(c, pl->d_ct);
   dfree(c, pl->d_bt0);
@@ -1950,7 +1949,12 @@ void free_plan(Graph *g) {
   dfree(c, pl->d_tt);
   dfree(c, pl->d_cursor);
   delete pl;
-  g->plan = nullptr;
+  pl = nullptr;
+}
+void free_plan(Graph *g) {
+  free_one_plan(g->ctx, g->plan);
+  free_one_plan(g->ctx, g->shard_plan);
+  g->shard_plan_n = 0;
 }
 
 static xt_status d2h(Ctx *c, void *h, const void *d, size_t bytes) {
@@ -2093,7 +2097,9 @@ xt_status make_plan(Graph *g) {
     if (g->tier_lane_work >= 0) pp.tiny_work = g->tier_lane_work;
     pp.batches_per_warp = large ? XT_BATCHES_PER_WARP_LARGE : XT_BATCHES_PER_WARP;
     pp.lane_pairs = XT_LANE_PAIRS;
-    const int64_t warps = int64_t(pl->grid_global) * kWarps;
+    // a shard's GPU holds 1 / plan_for of the work, as if the GPU were that many times as large
+    const int64_t warps1 = int64_t(pl->grid_global) * kWarps, warps = warps1 * g->plan_for;
+    pl->load = (total_work + kWarpRecCost * ne) / warps;
     pl->bitmap_bits = g->tune_bitmap_bits > 0 ? g->tune_bitmap_bits : int64_t(kBlockWords) * 32;
     pp.col = g->d_col;
     // the long tasks early: those of high ranks, or, as numbered by the input, of
@@ -2124,7 +2130,7 @@ xt_status make_plan(Graph *g) {
     // packs, where every warp has a few heads to itself; they fill every
     // warp once before they grow (tiers set by hand: none)
     pp.pack_work = pp.pack_cost = 0;
-    if (nv <= kPackMaxNv && nv >= kPackHeads * warps && ne >= kPackGraphRecs * warps && g->tier_lane_work < 0 && g->tier_warp_work < 0) {
+    if (nv <= kPackMaxNv && nv >= kPackHeads * warps1 && ne >= kPackGraphRecs * warps1 && g->tier_lane_work < 0 && g->tier_warp_work < 0) {
       pp.pack_work = kPackWorkMax;
       pp.pack_cost = (total_work + kPackRecCost * ne) / warps;
     }
@@ -2132,7 +2138,10 @@ xt_status make_plan(Graph *g) {
       pp.block_work = g->tune_block_work;
     } else {
       pp.block_work = kBlockWorkMin;
-      while (pp.block_work < kBlockWorkMax && pp.block_work * 16 * pl->grid_global < total_work) pp.block_work *= 2;
+      // (of a shard's about four, while tasks are of some size: an eighth of R-MAT 2^20 per
+      // vertex 264 to 270 us so, 300 with 16)
+      const int64_t tasks = 16 * int64_t(pl->grid_global) * std::max(1, g->plan_for / 4);
+      while (pp.block_work < kBlockWorkMax && pp.block_work * tasks < total_work) pp.block_work *= 2;
     }
     pl->high_first = pp.high_first;
     pl->block_work = pp.block_work;
@@ -2349,13 +2358,53 @@ static xt_status launch_count(Ctx *c, void (*fn)(const CountArgs), int grid, siz
   return cuda_status(c, cudaLaunchKernelEx(&cfg, fn, a), "k_count");
 }
 
+// A shard's part of the core costs its kernels' longest items however many the shards:
+// below this estimated gain a shard, its records are streamed (R-MAT 2^18, gain 40 us:
+// a sixteenth per edge 205 us with the core; 2^20, 208 us: a sixteenth per edge 456 us, 447
+// before there was a core).
+constexpr int64_t kShardFs = int64_t(8) * 1000 * 1000 * 1000;
+
+// The schedule cut for nshards shards, of all records or of the streamed ones. Tasks
+// as long as one GPU's share allows leave a shard waiting for its longest ones.
+static xt_status make_shard_plan(Graph *g, int nshards, bool all) {
+  Plan *main = g->plan;
+  int64_t *iend = g->d_iend;
+  free_one_plan(g->ctx, g->shard_plan);
+  g->shard_plan_n = 0;
+  g->plan = nullptr;
+  if (all) g->d_iend = g->d_ioff + 1;  // every record of a head
+  g->plan_for = nshards;
+  const xt_status s = make_plan(g);
+  g->shard_plan = g->plan;
+  g->shard_plan_n = s == XT_OK ? nshards : 0;
+  g->shard_plan_all = all;
+  g->plan = main;
+  g->d_iend = iend;
+  g->plan_for = 1;
+  return s;
+}
+
 xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_groups, int64_t *d_support, int shard,
                       int nshards) {
   Ctx *c = g->ctx;
   if (nshards < 1 || shard < 0 || shard >= nshards)
     return set_error(c, XT_ERR_INVALID, "shard must lie in [0, nshards) and nshards be at least 1");
   if (!g->plan) XT_TRY(make_plan(g));
+  // (the same for every shard of a count: all of them share the work out alike)
   Plan *pl = g->plan;
+  bool all = nshards > 1 && g->core.n_items > 0 && g->core.gain_fs / nshards < kShardFs;
+  if (nshards > 1 && (all || pl->load / nshards < 2 * kWarpCost)) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) cudaGetLastError();
+    const bool have = g->shard_plan_n == nshards && g->shard_plan_all == all;
+    if (have || cap == cudaStreamCaptureStatusNone) {  // a schedule is not built while recording
+      if (!have) XT_TRY(make_shard_plan(g, nshards, all));
+      pl = g->shard_plan;
+    } else {
+      all = false;
+    }
+  }
+  const bool with_core = g->core.n_items > 0 && !all;
   // pairs of columns are read with 32-byte vector loads
   if (reinterpret_cast<uintptr_t>(g->d_colp) % 32 != 0)
     return set_error(c, XT_ERR_CUDA, "padded column array is not 32-byte aligned");
@@ -2393,7 +2442,7 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   a.colp = g->d_colp;
   a.poff = g->d_poff;
   a.ioff = g->d_ioff;
-  a.iend = g->d_iend;
+  a.iend = all ? g->d_ioff + 1 : g->d_iend;
   a.rec = g->d_irec;
   a.rec_u = g->d_irec_u;
   a.bt = shard_first(pl->d_bt, pl->n_btask, shard);
@@ -2426,8 +2475,8 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   a.err = c->d_err;
   xt_status s = XT_OK;
   // the core's total is one launch, straight ahead of the streaming kernel
-  const bool core = g->core.n_items > shard && !d_pv && !d_support;
-  if (g->core.n_items > 0) s = core_count(g, d_global, pv_int, es, shard, nshards);
+  const bool core = with_core && g->core.n_items > shard && !d_pv && !d_support;
+  if (with_core) s = core_count(g, d_global, pv_int, es, shard, nshards);
   if (g->ne > 0 && s == XT_OK) {
     if (d_support)
       k_count<2, false><<<counted(c, pl->grid_es), kThreads, count_smem_bytes(true), c->stream>>>(a);

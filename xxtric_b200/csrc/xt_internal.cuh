@@ -132,6 +132,7 @@ struct Core {
   uint8_t *d_sym = nullptr, *d_xt = nullptr;
   int32_t *d_list = nullptr;
   int64_t n_tiles = 0, n_items = 0;
+  int64_t gain_fs = 0;        // estimated, of a global count
 };
 
 struct Graph {
@@ -186,6 +187,12 @@ struct Graph {
   int64_t stream_work = 0;  // sum over u of C(d+(u), 2): the suffix columns the count streams
   int64_t colp_len = 0;     // entries of the padded column array
   Plan *plan = nullptr;
+  // a schedule cut for shard_plan_n shards (0: none), of all records where shard_plan_all is
+  // set (a core's among them), else of the streamed ones; built by the first count that needs it
+  Plan *shard_plan = nullptr;
+  int shard_plan_n = 0;
+  bool shard_plan_all = false;
+  int plan_for = 1;  // the shards make_plan cuts for
 };
 
 // Optional: the rows still in host memory. build_from_edges then copies
