@@ -1070,6 +1070,7 @@ struct CountArgs {
   int group_runs;  // packs: heads of one graph credited together
   int64_t bitmap_bits;            // largest member id range kept as a bitmap
   int cuckoo_iters;               // cuckoo eviction chain limit
+  int pack_iters;                 // the same of a pack's table
   int *err;                       // error word: kErrStageTimeout when a staging wait gave up
 };
 
@@ -1257,7 +1258,8 @@ constexpr int64_t kPackMaxNv = (int64_t(1) << 26) - 2;
 // Eviction chain limit of a pack's table, of at most 256 keys in 1,024 slots: a pack
 // that falls back holds a short count's last warp (uniform graph of 104,857 vertices,
 // mean out-degree 5 in id order, one such pack: per vertex 35 us without it, 46 with a
-// limit of 64, 41 with 16; with 8 packs that would have fitted fall back too, 38 on average)
+// limit of 64, 41 with 16; with 8 packs that would have fitted fall back too, 38 on average;
+// a global count of such a graph with out-degree 8 67 and 60)
 constexpr int kPackCuckooIters = 16;
 
 // the pack's heads, one a lane: first record, end of the live records (both
@@ -1591,7 +1593,6 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
     int32_t *wstage = s_stage + warp * kStageWarp;
     int32_t *words = bwords + warp * kWarpWords;
     int *hcnt = s_hcnt[warp];
-    const int iters = PV ? min(a.cuckoo_iters, kPackCuckooIters) : a.cuckoo_iters;
     const bool heads = PV || a.group;
     ClaimBlock pclaim(a.n_bt == 0 && a.n_wt == 0, a.claim);
     Task t = claim_task_block(pclaim, &cursor[4], a.pt, a.n_pt, a.stride, a.claim, lane);
@@ -1616,7 +1617,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? kMinBlocks : 3) k_count(
       for (int i0 = 0; i0 < t.nmem; i0 += 32) {
         const int i = i0 + lane, hl = pack_find(ph.mem, i);
         if (i < t.nmem)
-          ok &= cuckoo_insert(words, m.shift, uint32_t(mem[i]) * 32u + uint32_t(hl) + 1u, iters);
+          ok &= cuckoo_insert(words, m.shift, uint32_t(mem[i]) * 32u + uint32_t(hl) + 1u, a.pack_iters);
       }
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) {  // a cuckoo chain ran too long: linear probing
@@ -2472,6 +2473,7 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   a.group_out = reinterpret_cast<unsigned long long *>(d_groups);
   a.bitmap_bits = pl->bitmap_bits;
   a.cuckoo_iters = g->cuckoo_iters >= 0 ? g->cuckoo_iters : kCuckooIters;
+  a.pack_iters = std::min(a.cuckoo_iters, kPackCuckooIters);
   a.err = c->d_err;
   xt_status s = XT_OK;
   // the core's total is one launch, straight ahead of the streaming kernel
