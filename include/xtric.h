@@ -176,6 +176,8 @@ xt_status xt_count_edges_async(xt_graph *g, int64_t *d_global, int64_t *d_suppor
  * (xxtric_b200.shards does it over NCCL). Asynchronous on the context
  * stream, device outputs overwritten with the shard's part (d_per_vertex:
  * nv int64, nullable; d_support: n_edges int64 in xt_graph_get_csr order).
+ * The first such count of a small graph builds a schedule for that number of
+ * shards (the graph keeps the last eight, and those that a recorded count uses).
  * XT_ERR_INVALID unless 0 <= shard < nshards. */
 xt_status xt_count_shard_async(xt_graph *g, int shard, int nshards, int64_t *d_global, int64_t *d_per_vertex);
 xt_status xt_count_edges_shard_async(xt_graph *g, int shard, int nshards, int64_t *d_global, int64_t *d_support);

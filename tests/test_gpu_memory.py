@@ -228,3 +228,38 @@ def test_shards_of_every_size_add_up(ctx, want, nshards):
             g.count_shard_async(0, nshards, part, each)
             ctx.synchronize()
     g.free()
+
+
+def test_shards_recorded_before_they_ran(want):
+    """Shards whose first count is recorded, and those that run, share the work out
+    alike; a recorded one stays right after counts of many other numbers of shards."""
+    import torch
+    import xxtric_b200 as xt
+    stream = torch.cuda.Stream()
+    with xt.Context(0) as c:
+        c.set_stream(stream.cuda_stream)
+        for nshards in (2, 16):
+            graphs = [want.build(c) for _ in range(2)]
+            part = torch.zeros(2, dtype=torch.int64, device="cuda")
+            torch.cuda.synchronize()
+            rec = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(rec, stream=stream):
+                graphs[0].count_shard_async(0, nshards, part[0:1])
+            got = 0
+            for i in range(1, nshards):  # the others, run on a graph of their own
+                graphs[1].count_shard_async(i, nshards, part[1:2])
+                c.synchronize()
+                got += int(part[1])
+            for others in (range(2, 3), range(2, 14)):
+                for k in others:
+                    graphs[0].count_shard_async(k - 1, k, part[1:2])
+                c.synchronize()
+                part.zero_()
+                torch.cuda.synchronize()
+                rec.replay()
+                torch.cuda.synchronize()
+                assert int(part[0]) + got == want.total
+            del rec
+            torch.cuda.synchronize()
+            for g in graphs:
+                g.free()

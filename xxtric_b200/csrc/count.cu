@@ -185,6 +185,11 @@ struct Plan {
   int64_t n_wtask = 0;         // warp tasks
   Task *d_wt = nullptr;
   int64_t load = 0;            // candidates and kWarpRecCost a record, for each of the GPU's warps
+  // of Graph::shard_plans: the shards it is cut for; whether of all records (a core's among
+  // them) or of the streamed ones; whether a CUDA graph may hold its addresses
+  int shards = 1;
+  bool all = false, recorded = false;
+  Plan *next = nullptr;
   bool high_first = false;     // the warp tasks stand from the last head to the first
   int64_t n_ptask = 0;         // packs
   Task *d_pt = nullptr;
@@ -1954,8 +1959,10 @@ static void free_one_plan(Ctx *c, Plan *&pl) {
 }
 void free_plan(Graph *g) {
   free_one_plan(g->ctx, g->plan);
-  free_one_plan(g->ctx, g->shard_plan);
-  g->shard_plan_n = 0;
+  while (Plan *pl = g->shard_plans) {
+    g->shard_plans = pl->next;
+    free_one_plan(g->ctx, pl);
+  }
 }
 
 static xt_status d2h(Ctx *c, void *h, const void *d, size_t bytes) {
@@ -2366,22 +2373,72 @@ static xt_status launch_count(Ctx *c, void (*fn)(const CountArgs), int grid, siz
 constexpr int64_t kShardFs = int64_t(8) * 1000 * 1000 * 1000;
 
 // The schedule cut for nshards shards, of all records or of the streamed ones. Tasks
-// as long as one GPU's share allows leave a shard waiting for its longest ones.
-static xt_status make_shard_plan(Graph *g, int nshards, bool all) {
-  Plan *main = g->plan;
+// as long as one GPU's share allows leave a shard waiting for its longest ones. While
+// the context's stream is being recorded it is built on a stream of its own (a recorded
+// first count must not share the work out otherwise than another rank's run one).
+constexpr int kShardPlans = 8;  // kept, beside recorded ones
+static xt_status shard_plan(Graph *g, int nshards, bool all, Plan **out) {
+  Ctx *c = g->ctx;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) cudaGetLastError();
+  const bool recording = cap != cudaStreamCaptureStatusNone;
+  int loose = 0;
+  Plan **last = nullptr;  // the link to the oldest that is not recorded
+  for (Plan **at = &g->shard_plans; *at; at = &(*at)->next) {
+    Plan *pl = *at;
+    if (pl->shards == nshards && pl->all == all) {
+      pl->recorded |= recording;
+      *out = pl;
+      return XT_OK;
+    }
+    if (!pl->recorded) {
+      loose++;
+      last = at;
+    }
+  }
+  if (loose >= kShardPlans && !recording) {
+    Plan *old = *last;
+    *last = old->next;
+    free_one_plan(c, old);
+  }
+  const cudaStream_t stream = c->stream;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (recording) {
+    XT_CUDA(c, cudaThreadExchangeStreamCaptureMode(&mode));
+    if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
+      cudaGetLastError();
+      c->stream = stream;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      return set_error(c, XT_ERR_CUDA, "a stream for the shards' schedule");
+    }
+  }
+  Plan *main = g->plan, *kept = g->shard_plans;
   int64_t *iend = g->d_iend;
-  free_one_plan(g->ctx, g->shard_plan);
-  g->shard_plan_n = 0;
-  g->plan = nullptr;
+  g->plan = g->shard_plans = nullptr;  // make_plan frees the graph's schedules before it makes one
   if (all) g->d_iend = g->d_ioff + 1;  // every record of a head
   g->plan_for = nshards;
-  const xt_status s = make_plan(g);
-  g->shard_plan = g->plan;
-  g->shard_plan_n = s == XT_OK ? nshards : 0;
-  g->shard_plan_all = all;
+  xt_status s = make_plan(g);
+  if (s == XT_OK) s = cuda_status(c, cudaStreamSynchronize(c->stream), "shards' schedule");
+  Plan *pl = g->plan;
   g->plan = main;
+  g->shard_plans = kept;
   g->d_iend = iend;
   g->plan_for = 1;
+  if (s == XT_OK) {
+    pl->shards = nshards;
+    pl->all = all;
+    pl->recorded = recording;
+    pl->next = kept;
+    g->shard_plans = pl;
+    *out = pl;
+  } else {
+    free_one_plan(c, pl);
+  }
+  if (recording) {
+    cudaStreamDestroy(c->stream);
+    c->stream = stream;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
   return s;
 }
 
@@ -2393,18 +2450,8 @@ xt_status count_graph(Graph *g, int64_t *d_global, int64_t *d_pv, int64_t *d_gro
   if (!g->plan) XT_TRY(make_plan(g));
   // (the same for every shard of a count: all of them share the work out alike)
   Plan *pl = g->plan;
-  bool all = nshards > 1 && g->core.n_items > 0 && g->core.gain_fs / nshards < kShardFs;
-  if (nshards > 1 && (all || pl->load / nshards < 2 * kWarpCost)) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) cudaGetLastError();
-    const bool have = g->shard_plan_n == nshards && g->shard_plan_all == all;
-    if (have || cap == cudaStreamCaptureStatusNone) {  // a schedule is not built while recording
-      if (!have) XT_TRY(make_shard_plan(g, nshards, all));
-      pl = g->shard_plan;
-    } else {
-      all = false;
-    }
-  }
+  const bool all = nshards > 1 && g->core.n_items > 0 && g->core.gain_fs / nshards < kShardFs;
+  if (nshards > 1 && (all || pl->load / nshards < 2 * kWarpCost)) XT_TRY(shard_plan(g, nshards, all, &pl));
   const bool with_core = g->core.n_items > 0 && !all;
   // pairs of columns are read with 32-byte vector loads
   if (reinterpret_cast<uintptr_t>(g->d_colp) % 32 != 0)

@@ -187,12 +187,9 @@ struct Graph {
   int64_t stream_work = 0;  // sum over u of C(d+(u), 2): the suffix columns the count streams
   int64_t colp_len = 0;     // entries of the padded column array
   Plan *plan = nullptr;
-  // a schedule cut for shard_plan_n shards (0: none), of all records where shard_plan_all is
-  // set (a core's among them), else of the streamed ones; built by the first count that needs it
-  Plan *shard_plan = nullptr;
-  int shard_plan_n = 0;
-  bool shard_plan_all = false;
-  int plan_for = 1;  // the shards make_plan cuts for
+  Plan *shard_plans = nullptr;  // schedules cut for numbers of shards, each built by the first count that
+                                //   needs it, the last one first
+  int plan_for = 1;             // the shards make_plan cuts for
 };
 
 // Optional: the rows still in host memory. build_from_edges then copies
