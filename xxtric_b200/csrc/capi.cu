@@ -66,11 +66,8 @@ void dfree(Ctx *c, void *p) {
   cudaFreeAsync(p, c->stream);
 }
 
-// what a caller's counter (words[0], as it was) becomes: unchanged where a wait of
-// the count gave up
-__global__ void k_deliver(CountOut *__restrict__ out, int accumulate) {
-  if (!(out->err & kErrWaits)) out->words[0] = out->total + (accumulate ? out->words[0] : 0);
-}
+// *to = total + what it was (words[0])
+__global__ void k_add_total(const CountOut *__restrict__ out, int64_t *__restrict__ to) { *to = out->total + out->words[0]; }
 
 struct WordList {
   const int64_t *p[12];
@@ -454,21 +451,25 @@ xt_status xt_count_device(int64_t nv, const int64_t *d_indices, const int64_t *d
   Graph g;
   xt_status s = build_from_csr(c, nv, d_indices, d_edge_list, true, XT_ORIENT_DEGREE, &g);
   if (s == XT_OK) s = make_plan(&g);
-  // the counter goes through the result block, so that one wait serves the error word too
+  // the counter as it was, for a sum and in case a wait of the count gives up
+  int64_t *was = c->d_out->words, *sum = c->d_out->words + 1, *total = &c->d_out->total;
   if (s == XT_OK)
-    s = cuda_status(c, cudaMemcpyAsync(c->d_out->words, d_count, sizeof(int64_t), cudaMemcpyDeviceToDevice, c->stream),
-                    "D2D");
-  if (s == XT_OK) s = count_graph(&g, &c->d_out->total, nullptr);
-  if (s == XT_OK) {
-    k_deliver<<<counted(c, dim3(1)), 1, 0, c->stream>>>(c->d_out, accumulate);
-    s = cuda_status(c, cudaGetLastError(), "k_deliver");
+    s = cuda_status(c, cudaMemcpyAsync(was, d_count, sizeof(int64_t), cudaMemcpyDeviceToDevice, c->stream), "D2D");
+  if (s == XT_OK) s = count_graph(&g, total, nullptr);
+  if (s == XT_OK && accumulate) {
+    k_add_total<<<counted(c, dim3(1)), 1, 0, c->stream>>>(c->d_out, sum);
+    s = cuda_status(c, cudaGetLastError(), "k_add_total");
   }
   if (s == XT_OK)
-    s = cuda_status(c, cudaMemcpyAsync(d_count, c->d_out->words, sizeof(int64_t), cudaMemcpyDeviceToDevice, c->stream),
-                    "D2D");
+    s = cuda_status(c, cudaMemcpyAsync(d_count, accumulate ? sum : total, sizeof(int64_t), cudaMemcpyDeviceToDevice,
+                                       c->stream), "D2D");
   free_graph_device(&g);
   const xt_status done = count_status(c);  // waits for the stream
-  if (s == XT_OK) s = done;
+  if (s == XT_OK && done != XT_OK) {
+    s = done;
+    cudaMemcpyAsync(d_count, was, sizeof(int64_t), cudaMemcpyDeviceToDevice, c->stream);
+    cudaStreamSynchronize(c->stream);
+  }
   cudaFreeAsync(c->d_out, c->stream);
   delete ctx;
   return s;
